@@ -576,7 +576,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // once per element).
       const bool acc = MODE == 1;
       if (EPI == TC_EPI_PIXEL) {
-        const int cpc = (P.bn + cz - 1) / cz, c_lo = zr * cpc + (t >> 7), c_hi = min(min(P.bn, zr * cpc + cpc), P.N - n0);
+        const TcSlice slice(P.bn, cz, zr, P.N - n0);
+        const int c_lo = slice.lo + (t >> 7), c_hi = slice.hi;
         const int row = t & 127;
         const int m = m_tile * 128 + row;
         int pix; const int img = P.by_pix.divmod(m, pix);
@@ -602,16 +603,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       } else {
         // rows of the slice go round the eight warps, a lane takes every 32nd column: a warp's stores cover 128 contiguous bytes
-        const int rpc = (128 + cz - 1) / cz, r_lo = zr * rpc, r_hi = min(min(128, r_lo + rpc), (int)min(128ll, (long long)P.M - (long long)m_tile * 128));
-        const int w = t >> 5, cchunks = P.bn >> 5, cshift = cchunks == 4 ? 2 : cchunks == 2 ? 1 : 0;
-        const int n_rows = r_hi - r_lo - w > 0 ? (r_hi - r_lo - w + 7) / 8 : 0, items = n_rows << cshift;
-        for (int ib = 0; ib < items; ib += 8) {
+        const TcSliceRows rows(TcSlice(128, cz, zr, (int)min(128ll, (long long)P.M - (long long)m_tile * 128)), P.bn, t >> 5);
+        for (int ib = 0; ib < rows.items; ib += 8) {
           float v[8], old[8]; float* o[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const int i = ib + u; v[u] = 0.0f; old[u] = 0.0f; o[u] = nullptr;
-            const int row = r_lo + w + 8 * (i >> cshift), c = ((i & (cchunks - 1)) << 5) + lane, n = n0 + c;
-            if (i < items && n < P.N) {
+            const int row = rows.row(i), c = (rows.run(i) << 5) + lane, n = n0 + c;
+            if (i < rows.items && n < P.N) {
 #pragma unroll
               for (int z = 0; z < 8; ++z) if (z < cz) v[u] += remote[z][row * (P.bn + 1) + c];
               const long long col = out_column<EPI>(P, n);

@@ -65,6 +65,32 @@ struct TcOperand {
 struct TcWalk { int n0, n1; int inc[3][5]; };
 bool tc_walk_of(const TcOperand& o, TcWalk& w);
 
+// A cluster of `cz` splits adds its partial tiles up: CTA `rank` owns rows (row-major epilogues) or columns (pixel-major) lo .. hi - 1 of
+// the tile, `extent` of them in the tile and `limit` inside the result.  Used by the kernel and by the CPU check of the plans.
+#ifdef __CUDACC__
+#define LTB_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define LTB_HOST_DEVICE inline
+#endif
+struct TcSlice {
+  int lo, hi;
+  LTB_HOST_DEVICE TcSlice(int extent, int cz, int rank, int limit) {
+    const int per = (extent + cz - 1) / cz;
+    lo = rank * per; hi = lo + per < extent ? lo + per : extent;
+    if (limit < hi) hi = limit;
+  }
+};
+// The rows of a slice as eight warps share them: warp w takes the rows lo + w, lo + w + 8, .., each as bn / 32 runs of 32 columns.
+struct TcSliceRows {
+  int first, items, shift;
+  LTB_HOST_DEVICE TcSliceRows(const TcSlice& s, int bn, int w) : first(s.lo + w), shift(0) {
+    while ((64 << shift) <= bn) ++shift;                       // runs of a row: 1 << shift
+    items = s.hi > first ? ((s.hi - first + 7) / 8) << shift : 0;
+  }
+  LTB_HOST_DEVICE int row(int i) const { return first + 8 * (i >> shift); }
+  LTB_HOST_DEVICE int run(int i) const { return i & ((1 << shift) - 1); }
+};
+
 enum TcEpilogue {
   TC_EPI_PIXEL = 0,   // D row = pixel, D column = channel: out[img][chan][pix]   (conv forward / data-grad)
   TC_EPI_ROWMAJOR = 1,// D row = row, D column contiguous:   out[row*ld + col]      (gemm, weight-grad)

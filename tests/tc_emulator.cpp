@@ -134,6 +134,29 @@ static bool run_plan(const TcPlan& p, size_t out_count) {
   return true;
 }
 
+// The deterministic mode's sum over a cluster of splits: whatever the tile's width, the cluster's size and the part of the tile inside
+// the result, its CTAs together write every output of the tile once.
+static bool slices_cover() {
+  for (int bn : {64, 128, 256}) for (int cz : {2, 4, 8}) for (int limit = 1; limit <= 256; ++limit) {
+    std::vector<int> rows((size_t)128 * bn, 0), cols(bn, 0);
+    for (int rank = 0; rank < cz; ++rank) {
+      if (limit <= 128) for (int w = 0; w < 8; ++w) {
+        const TcSliceRows s(TcSlice(128, cz, rank, limit), bn, w);
+        for (int i = 0; i < s.items; ++i) {
+          if (s.row(i) >= limit || s.run(i) >= bn / 32) { printf("slice of %d columns, %d CTAs: row %d, run %d\n", bn, cz, s.row(i), s.run(i)); return false; }
+          for (int lane = 0; lane < 32; ++lane) ++rows[(size_t)s.row(i) * bn + s.run(i) * 32 + lane];
+        }
+      }
+      const TcSlice c(bn, cz, rank, limit);
+      for (int half = 0; half < 2; ++half) for (int j = c.lo + half; j < c.hi; j += 2) ++cols[j];
+    }
+    for (int r = 0; r < 128 && limit <= 128; ++r) for (int c = 0; c < bn; ++c)
+      if (rows[(size_t)r * bn + c] != (r < limit)) { printf("tile of %d columns, %d CTAs, %d rows: (%d, %d) written %d times\n", bn, cz, limit, r, c, rows[(size_t)r * bn + c]); return false; }
+    for (int c = 0; c < bn; ++c) if (cols[c] != (c < limit)) { printf("tile of %d columns, %d CTAs, %d inside: column %d written %d times\n", bn, cz, limit, c, cols[c]); return false; }
+  }
+  return true;
+}
+
 static std::vector<float> rnd(size_t n, unsigned seed) { std::vector<float> v(n); srand(seed); for (auto& x : v) x = (float)(rand() % 17 - 8) / 4.0f; return v; }
 static bool close(const std::vector<float>& a, const std::vector<float>& b, const char* what) {
   for (size_t i = 0; i < a.size(); ++i) if (std::fabs(a[i] - b[i]) > 1e-3f * (1.0f + std::fabs(a[i]))) { printf("%s: mismatch at %zu: %f vs %f\n", what, i, a[i], b[i]); return false; }
@@ -235,7 +258,7 @@ static int gemm_case(int M, int N, int K, bool ak, bool bk, bool acc) {
 }
 
 int main() {
-  int bad = 0, taken = 0;
+  int bad = slices_cover() ? 0 : 1, taken = 0;
   const int convs[][4] = {{2, 64, 64, 256}, {3, 64, 256, 256}, {4, 128, 96, 64}, {5, 256, 128, 64}, {11, 256, 128, 16}, {35, 512, 64, 4}, {1, 32, 48, 1024},
                           {8, 576, 64, 256}, {2, 40, 64, 32}, {3, 64, 64, 36}, {2, 2048, 512, 4}, {9, 1024, 256, 16}, {70, 512, 32, 1},
                           // filter rows that need padding (3x3 over 3, 16 and 48 channels; 1x1 over 16 and 48) and few output channels

@@ -445,10 +445,16 @@ def test_gemm_of_ragged_rows_tf32(ora, gpu, ta, tb, M, N, K):
         assert_close(ref[k], got[k], FP32_RTOL, k)
 
 
-@pytest.mark.parametrize("M,N,K,ta,tb", [(4740, 1000, 516, 0, 1), (512, 508, 20000, 1, 0)])
-def test_gemm_in_wide_tiles_tf32(ora, gpu, M, N, K, ta, tb):
-    """256-wide tiles: enough of them, and few that are split over a long K."""
-    test_gemm_of_ragged_rows_tf32(ora, gpu, ta=ta, tb=tb, M=M, N=N, K=K)
+@pytest.mark.parametrize("det", [0, 1])
+@pytest.mark.parametrize("M,N,K,ta,tb", [(4740, 1000, 516, 0, 1), (512, 508, 20000, 1, 0), (4096, 1196, 996, 0, 1)])
+def test_gemm_in_wide_tiles_tf32(ora, gpu, M, N, K, ta, tb, det):
+    """256-wide tiles: enough of them, a product of 13 splits that is stored, and a gradient of 3 splits that is added; by atomics and, in
+    deterministic mode, by clusters (13 splits: two clusters of eight and a sum of their slabs)."""
+    gpu.lib.set_deterministic(det)
+    try:
+        test_gemm_of_ragged_rows_tf32(ora, gpu, ta=ta, tb=tb, M=M, N=N, K=K)
+    finally:
+        gpu.lib.set_deterministic(0)
 
 
 def test_tensor_core_engine_reports_no_timeouts(gpu):
