@@ -147,3 +147,45 @@ def test_deferred_zero_fill_is_invisible_on_the_oracle(oracle_lib):
         m.use_deferred_zero(True)
         m.close(); oracle_lib.reset(mark)
     assert res[0][0] == res[1][0] and np.array_equal(res[0][1], res[1][1])
+
+
+@pytest.mark.parametrize("batch", [1, 252, 253, 505])
+def test_submitted_batches_arrive_whole(oracle_lib, batch):
+    """submit() copies a batch into its staging pair in pieces of 512 KB, 64 bytes at a time: batches of one row (2,080 bytes),
+    of 128 bytes less than a piece, of a piece and 1,952 bytes and of two and 1,824 train as the blocking steps do, bit for bit, whatever the address of the array."""
+    mark = oracle_lib.mark()
+    rng = np.random.default_rng(batch)
+    n = 20 * 26 * batch
+    batches = [(rng.standard_normal(n + 1).astype(np.float32)[k % 2:n + k % 2], rng.integers(0, 26, 20 * batch).astype(np.int32)) for k in range(3)]
+    res = []
+    for feed in (False, True):
+        m = _model(oracle_lib, "rnn_26_50", batch)
+        if feed:
+            losses = []
+            for x, y in batches:
+                losses.append(m.collect(m.submit(x, y, 0.01)))
+        else:
+            losses = [m.step(x, y, 0.01) for x, y in batches]
+        res.append((losses, m.slab_params()))
+        m.close(); oracle_lib.reset(mark)
+    assert res[0][0] == res[1][0] and np.array_equal(res[0][1], res[1][1])
+
+
+def test_programs_start_no_threads(oracle_lib):
+    """Opening, stepping and closing a program costs no thread: neither the first step of a large batch nor the close of the last program
+    may pay for helpers, and a process at its limit of threads must be able to train."""
+    mark = oracle_lib.mark()
+    rng = np.random.default_rng(1)
+    x, y = rng.standard_normal(20 * 80 * 256).astype(np.float32), rng.integers(0, 80, 20 * 256).astype(np.int32)
+
+    def threads():
+        return len(os.listdir("/proc/self/task"))
+    m = _model(oracle_lib, "rnn", 2)
+    m.step(x[:20 * 80 * 2], y[:40], 0.01)                # the oracle's own OpenMP threads are there from now on
+    m.close(); oracle_lib.reset(mark)
+    before = threads()
+    m = _model(oracle_lib, "rnn", 256)
+    m.collect(m.submit(x, y, 0.01)); m.step(x, y, 0.01)
+    assert threads() == before
+    m.close(); oracle_lib.reset(mark)
+    assert threads() == before
