@@ -136,7 +136,7 @@ int64_t LTB_FN(kernel_launches)(void);                  /* kernels launched by t
 void*  LTB_FN(malloc)(size_t bytes);
 void*  LTB_FN(malloc_uninit)(size_t bytes);
 int    LTB_FN(free)(void* p, size_t bytes);             /* LIFO pop: p must be the newest block */
-void*  LTB_FN(mark)(void);
+void*  LTB_FN(mark)(void);                              /* the arena's position for ltb_reset; NULL when work in flight could not be joined */
 int    LTB_FN(reset)(void* mark);
 size_t LTB_FN(arena_used)(void);
 

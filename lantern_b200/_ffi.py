@@ -113,7 +113,7 @@ class BoundLibrary:
             raise AttributeError(name)
         f, ret = fns[name], self.decls[name][0]
         checked = ret is ctypes.c_int and name not in self._NO_CHECK
-        allocates = ret is ctypes.c_void_p and name in ("malloc", "malloc_uninit")
+        allocates = ret is ctypes.c_void_p and name in ("malloc", "malloc_uninit", "mark")
 
         # Kept on the instance: this method then runs once per entry point, not once per call (a small layer is a dozen calls of
         # a few microseconds each).  Tensors among the arguments are the exception, found when ctypes declines one.
@@ -125,7 +125,7 @@ class BoundLibrary:
             if checked and r < 0:
                 raise LanternError(r, self.error_message())
             if allocates and not r:
-                raise LanternError(-3, self.error_message())
+                raise LanternError(self._fns["last_error"](None, 0) or -3, self.error_message())
             return r
         call.__name__ = name
         self.__dict__[name] = call

@@ -242,10 +242,10 @@ struct SideRange { const char* p; size_t bytes; bool written; };
 static std::vector<SideRange> side_ranges;
 int side_join() {
   if (!g.side_open) return LTB_OK;
-  g.side_open = false; side_ranges.clear();
-  g.used = g.side_base;
   LTB_CUDA(cudaEventRecord(g.join_ev, g.side));
   LTB_CUDA(cudaStreamWaitEvent(g.stream, g.join_ev, 0));
+  g.side_open = false; side_ranges.clear();              // only now: without the wait the staging blocks stay held and the next call tries again
+  g.used = g.side_base;
   return LTB_OK;
 }
 void side_add(const void* p, size_t bytes, bool written) { side_ranges.push_back(SideRange{(const char*)p, bytes, written}); }
@@ -282,7 +282,7 @@ int ltb_free(void* p, size_t bytes) {
   cl_cache_drop_from(p); filter_cache_drop_from(p); grad_unset_drop_from(p);
   return LTB_OK;
 }
-void* ltb_mark(void) { if (g.inited) side_join(); return g.heap + g.used; }
+void* ltb_mark(void) { if (g.inited && side_join()) return nullptr; return g.heap + g.used; }
 int ltb_reset(void* mark) {
   LTB_INITED();
   char* m = (char*)mark;

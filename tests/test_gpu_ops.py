@@ -3,6 +3,7 @@ FP32 paths: 1e-4 relative; TF32 tensor-core paths: 2e-3 relative; indices bit-ex
 import numpy as np
 import pytest
 
+from lantern_b200 import LanternError
 from lantern_b200.backend import TensorR
 from tests.golden.reference_known_answers import CASES
 from tests.parity import FP32_RTOL, TF32_RTOL, assert_close, check
@@ -649,6 +650,48 @@ def test_empty_ragged_and_misaligned_vectors(ora, gpu, n):
         out["x"], out["d"], out["guard_x"], out["guard_d"] = full.toCPU()[1:], dfull.toCPU()[1:], full.toCPU()[:1], dfull.toCPU()[:1]
         return out
     check(f, ora, gpu)
+
+
+def test_a_failed_wait_for_the_weight_gradient_is_reported_and_made_up_for(ora, gpu):
+    """With fusion on a weight gradient may still run on the library's second stream when ltb_conv2d_bwd returns.  Here the stream's owner
+    records it in the meantime, so that the wait for the second stream is refused by the host API (no device error): ltb_mark says so
+    instead of returning a mark, and the next call outside the recording waits and finds the gradient complete."""
+    import ctypes
+
+    import torch  # noqa: F401  (loads the CUDA runtime)
+    rt = ctypes.CDLL("libcudart.so.12")
+    lib = gpu.lib
+    N, C, H, K = 64, 64, 16, 64
+    x0, dy0 = (R(i).standard_normal((N, C, H, H)).astype(np.float32) for i in (1, 2))
+    w0 = (R(3).standard_normal((K, C, 1, 1)) / 8).astype(np.float32)
+
+    def f(b):
+        b.lib.set_math(0)
+        x, w, dy = TensorR(b.fromNumpy(x0)), TensorR(b.fromNumpy(w0)), b.fromNumpy(dy0)
+        x.d, w.d = b.zeros(N, C, H, H), b.zeros(K, C, 1, 1)
+        if b is gpu:
+            b.lib.set_fusion(1)
+            stream = ctypes.c_void_p(b.lib.get_stream())
+            b.lib.sync()
+        b.lib.conv2d_bwd(x.x.ptr, x.d.ptr, w.x.ptr, w.d.ptr, 0, dy.ptr, N, C, H, H, K, 1, 1, 1, 1, 0, 0)
+        if b is gpu:
+            graph = ctypes.c_void_p()
+            assert rt.cudaStreamBeginCapture(stream, 1) == 0                  # thread-local mode
+            try:
+                with pytest.raises(LanternError):
+                    b.lib.mark()
+            finally:
+                assert rt.cudaStreamEndCapture(stream, ctypes.byref(graph)) != 0    # the refused wait ended the recording
+            assert not graph.value
+            assert b.lib.mark()
+        return {"dw": w.d.toCPU(), "dx": x.d.toCPU()}
+    ref = f(ora)
+    try:
+        got = f(gpu)
+    finally:
+        lib.set_fusion(0)
+    for k in ref:
+        assert_close(ref[k], got[k], FP32_RTOL, k)
 
 
 def test_sgd_step_over_a_list_of_tensors(ora, gpu):
