@@ -167,6 +167,7 @@ int ltb_set_deterministic(int on) { LTB_INITED(); LTB_REQUIRE(!g.capturing, "ltb
 int ltb_params_changed(void) { LTB_INITED(); filter_cache_note_write(nullptr, 0); return LTB_OK; }
 int ltb_set_math(int mode) {
   LTB_REQUIRE(mode == LTB_MATH_FP32 || mode == LTB_MATH_TF32, "ltb_set_math: unknown mode %d", mode);
+  if (g.inited && g.pending.kind) { int rc = flush_pending(); if (rc) return rc; }      // a held convolution runs in the mode it was called in
   g.math = mode; return LTB_OK;
 }
 int ltb_device_status(void) {

@@ -627,6 +627,21 @@ def test_lookahead_fusion_flushes_on_any_other_call(ora, gpu):
         assert_close(ref[k], got[k], 2e-4, k)
 
 
+@pytest.mark.parametrize("called,then", [(1, 0), (0, 1)])
+def test_a_held_convolution_runs_in_the_math_mode_it_was_called_in(gpu, called, then):
+    x0, w0, b0 = (R(i).standard_normal(s).astype(np.float32) for i, s in enumerate(((4, 64, 16, 16), (64, 64, 1, 1), (64,))))
+
+    def f(fusion, after):
+        gpu.lib.set_fusion(fusion); gpu.lib.set_math(called); gpu.lib.set_deterministic(1)
+        try:
+            y, _, _ = gpu.conv2D_batch(gpu.fromNumpy(x0), gpu.fromNumpy(w0), gpu.fromNumpy(b0), (1, 1), (0, 0, 0, 0))
+            gpu.lib.set_math(after)
+            return y.toCPU()
+        finally:
+            gpu.lib.set_fusion(0); gpu.lib.set_deterministic(0); gpu.lib.set_math(1)
+    assert np.array_equal(f(1, then), f(0, called))
+
+
 @pytest.mark.parametrize("n", [0, 1, 3, 5, 1027, 65537])
 def test_empty_ragged_and_misaligned_vectors(ora, gpu, n):
     """Element counts that are zero, smaller than a float4 or not a multiple of four, on buffers that start one float past
