@@ -1,8 +1,6 @@
 // Planner of the TF32 tensor-core engine: see tc_plan.h.  Pure host code.
 #include "tc_plan.h"
 
-#include <cstdio>
-#include <cstdlib>
 #include <cstring>
 
 namespace ltb {
@@ -310,20 +308,6 @@ bool operand_im2col_mn(TcOperand& o, const float* act, int n_img, int eh, int ew
 // Tile width.  The MMA-issuing thread spends a few hundred cycles per k-iteration whatever the width, so narrow tiles
 // leave the tensor core idle; 128 columns with three stages lets two CTAs share an SM (one's epilogue and issue gaps
 // overlap the other's main loop).  Parallelism for small outputs comes from split-K, not from narrower tiles.
-// Split policy knobs, read once from LTB_SPLIT="fill,min_iters,prefer64,long_iters" (a sweep aid; the defaults are the measured optimum):
-// fill = CTAs per SM that split-K aims for (x 100), min_iters = fewest k-iterations a split may have, prefer64 = 64-wide tiles
-// whenever 128-wide ones would not cover the SMs, long_iters = k-iterations that a split must keep for two CTAs per SM.
-struct SplitKnobs { int fill100 = 70, min_iters = 4, prefer64 = 0, long_iters = 24; };
-const SplitKnobs& split_knobs() {
-  static SplitKnobs k = [] {
-    SplitKnobs v;
-    if (const char* e = std::getenv("LTB_SPLIT")) std::sscanf(e, "%d,%d,%d,%d", &v.fill100, &v.min_iters, &v.prefer64, &v.long_iters);
-    if (v.fill100 < 10) v.fill100 = 10;
-    if (v.min_iters < 1) v.min_iters = 1;
-    return v;
-  }();
-  return k;
-}
 // 256 columns where such tiles alone, or in splits of 32 k-iterations, cover the SMs and pad no more than 128-wide ones: shared memory
 // is what the main loop of a 128 x 128 tile waits for (32 KB written and 32 KB read per k-iteration of 268 tensor cycles), twice the
 // width moves a quarter less of it per product (8192 x 1000 x 2048 and its gradients: 287 -> 242 us).
@@ -331,7 +315,6 @@ int pick_bn(int n_extent, int m_tiles, int sm_count, int k_iters = 0) {
   if (n_extent <= 64) return 64;
   const int64_t wide = (int64_t)m_tiles * cdiv(n_extent, 256);
   if (k_iters >= 16 && cdiv(n_extent, 256) * 256 <= cdiv(n_extent, 128) * 128 && (wide * 10 >= 8 * (int64_t)sm_count || wide * (k_iters / 32) >= sm_count)) return 256;
-  if (split_knobs().prefer64 && (int64_t)m_tiles * cdiv(n_extent, 128) * 10 < (int64_t)8 * sm_count) return 64;
   return 128;
 }
 
@@ -341,14 +324,16 @@ void finish(TcPlan& p, int M, int N, int k_iters, int sm_count, bool may_split) 
   p.splits = 1;
   if (may_split) {
     const int tiles = p.m_tiles * p.n_tiles;
-    // Split-K pays with atomic traffic (splits x the output) and a zero-fill, so it is used sparingly.  Swept on the cases of perf/cases.py:
+    // Split-K pays with atomic traffic (splits x the output) and a zero-fill, so it is used sparingly.  Swept on three workloads, ResNet-50 at
+    // batch 128 and at batch 8 and a 64 -> 64 3x3 layer on 32 images of 56 x 56:
     // 0.7 CTAs per SM (ResNet-50 at batch 128 3.41 ms; at 1.0 3.46, at 0.5 3.44, at 2 3.50), four k-iterations per split at least
     // (batch 8: 1.65 ms; eight 1.72, sixteen 1.96), no split once the tiles alone cover 80 % of the SMs; and two CTAs per SM, whose
     // main loops overlap, where each still has 24 iterations (56 x 56 layer 223 us; without 264).
-    int s = cdiv(sm_count * split_knobs().fill100 / 100, tiles);
+    constexpr int kFill100 = 70, kMinIters = 4, kLongIters = 24;
+    int s = cdiv(sm_count * kFill100 / 100, tiles);
     const int two = cdiv(2 * sm_count, tiles);
-    if (p.bn <= 128 && k_iters / two >= split_knobs().long_iters) s = two;
-    int mx = k_iters / split_knobs().min_iters; if (mx < 1) mx = 1;
+    if (p.bn <= 128 && k_iters / two >= kLongIters) s = two;
+    int mx = k_iters / kMinIters; if (mx < 1) mx = 1;
     if (s > mx) s = mx;
     if ((int64_t)tiles * 10 >= (int64_t)8 * sm_count) s = 1;
     p.splits = s < 1 ? 1 : s;
