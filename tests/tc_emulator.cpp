@@ -1,11 +1,13 @@
 // CPU check of the tensor-core engine's bookkeeping (test infrastructure).
 //
-// Emulates, for every plan the planner produces, (1) what a tiled TMA load writes to shared memory (box order, out-of-
-// bounds zero fill, 32/64/128-byte swizzle as an XOR of address bits [4,7) with bits [7,10)), (2) which element the
-// tensor core reads for (row, k) of an MMA step from the canonical UMMA layout described by the step's descriptor
-// (start offset, LBO, SBO, swizzle, major-ness), and (3) the epilogue's output indexing.  The result of the emulated
-// engine is compared with a direct evaluation of the convolution / GEMM.  This pins coordinates, strides, descriptors
-// and tile/split arithmetic without a GPU; it does not prove that the hardware follows the emulated conventions.
+// Emulates, for every kind of plan the planner produces, (1) what the TMA loads of a stage write to shared memory (one box, several
+// boxes clipped at the row's end, the im2col mode's walk over output pixels; box order, out-of-bounds zero fill, 32/64/128-byte
+// swizzle as an XOR of address bits [4,7) with bits [7,10)), (2) which element the tensor core reads for (row, k) of an MMA step
+// from the canonical UMMA layout described by the step's descriptor (start offset, LBO, SBO, swizzle, major-ness), and (3) the
+// epilogue's output indexing.  The result of the emulated engine is compared with a direct evaluation of the convolution / GEMM.
+// The splits are added up in any order here; how a cluster deals a tile out to its CTAs in deterministic mode is checked by itself.
+// This pins coordinates, strides, descriptors and tile/split arithmetic without a GPU; it does not prove that the hardware follows
+// the emulated conventions.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -27,25 +29,79 @@ static int span(int mode) { return (mode == TC_SW_128 || mode == TC_SW_128_32B) 
 static void coords_of(const TcOperand& o, int tile, int kiter, int64_t* c) {
   for (int d = 0; d < 5; ++d) c[d] = (int64_t)o.c_off[d] + (int64_t)((tile / o.t_div[d]) % o.t_mod[d]) * o.t_mul[d] + (int64_t)((kiter / o.k_div[d]) % o.k_mod[d]) * o.k_mul[d];
 }
+// The im2col mode: `pixels` consecutive output pixels of the walk from `first` on, 32 channels from `chan` on at tap (s, r), written to
+// shared memory from `at` on, a row of 128 bytes per pixel.
+static void im2col_box(const TcOperand& o, int64_t first, int64_t chan, int64_t s, int64_t r, uint32_t at, std::vector<float>& smem) {
+  const TcTensorMap& m = o.map; const TcIm2col& g = o.im;
+  for (int64_t q = 0; q < g.pixels; ++q) {
+    const int64_t per = (int64_t)g.grid_w * g.grid_h, img = (first + q) / per, j = (first + q) % per / g.grid_w, i = (first + q) % g.grid_w;
+    const int64_t w = g.low_w + i * g.step_w + s, h = g.low_h + j * g.step_h + r;
+    for (int64_t c = 0; c < 32; ++c) {
+      const bool inb = chan + c < (int64_t)m.dims[0] && w >= 0 && w < (int64_t)m.dims[1] && h >= 0 && h < (int64_t)m.dims[2] && img < (int64_t)m.dims[3];
+      const float v = inb ? *(const float*)((const char*)m.base + (chan + c) * 4 + w * m.strides[1] + h * m.strides[2] + img * m.strides[3]) : 0.0f;
+      smem[swz(at + (uint32_t)(q * 128 + c * 4), m.swizzle) / 4] = v;
+    }
+  }
+}
+static bool im2col_load(const TcOperand& o, int tile, int kiter, std::vector<float>& smem) {
+  const TcIm2col& g = o.im;
+  for (int d = 1; d < 4; ++d) if (o.map.strides[d] % 16) { printf("stride %d not a multiple of 16 bytes\n", d); return false; }
+  // the box corners of the map: the walk's first and last base pixel relative to the image's first and last pixel
+  if (g.upper_w != g.low_w + (g.grid_w - 1) * g.step_w - ((int)o.map.dims[1] - 1) || g.upper_h != g.low_h + (g.grid_h - 1) * g.step_h - ((int)o.map.dims[2] - 1)) { printf("im2col corners\n"); return false; }
+  smem.assign(o.stage_bytes / 4, 1e30f);                       // a box that is not loaded leaves what was there before
+  if (o.load == TC_LOAD_IM2COL) {
+    int64_t c[5]; coords_of(o, 0, kiter, c);
+    if (g.pixels * 128 != (int)o.stage_bytes || c[0] % 4) { printf("im2col stage\n"); return false; }
+    im2col_box(o, (int64_t)tile * g.pixels, c[0], c[1], c[2], 0, smem);
+    return true;
+  }
+  if (o.nbox * 4096 != (int)o.stage_bytes) { printf("im2col boxes\n"); return false; }
+  for (int b = 0; b < o.nbox; ++b) {
+    const int q = tile * o.nbox + b, blk = q / g.taps, tap = q - blk * g.taps;
+    if (blk < g.ch_blocks) im2col_box(o, (int64_t)kiter * g.pixels, (int64_t)blk * 32, tap % g.tap_s, tap / g.tap_s, (uint32_t)b * 4096, smem);
+  }
+  return true;
+}
+// The producer advances the walk's pixel by additions: from any starting iteration it must be where the division says.
+static bool pixel_walk_matches(const TcOperand& o, int k_iters) {
+  const TcIm2col& g = o.im;
+  for (int k0 = 0; k0 < k_iters; k0 += (k_iters > 5 ? k_iters / 5 : 1)) {
+    const int per = g.grid_w * g.grid_h;
+    int pn = k0 * 32 / per, pj = k0 * 32 % per / g.grid_w, pi = k0 * 32 % g.grid_w;
+    for (int it = k0; it < k_iters; ++it) {
+      if (pn != it * 32 / per || pj != it * 32 % per / g.grid_w || pi != it * 32 % g.grid_w) { printf("pixel walk at iteration %d from %d\n", it, k0); return false; }
+      pi += g.adv_i; pj += g.adv_j; pn += g.adv_n;
+      if (pi >= g.grid_w) { pi -= g.grid_w; ++pj; }
+      if (pj >= g.grid_h) { pj -= g.grid_h; ++pn; }
+    }
+  }
+  return true;
+}
 static bool tma_load(const TcOperand& o, int tile, int kiter, std::vector<float>& smem) {
   const TcTensorMap& m = o.map;
+  if (o.load == TC_LOAD_IM2COL || o.load == TC_LOAD_IM2COL_MN) return im2col_load(o, tile, kiter, smem);
   int64_t c[5]; coords_of(o, tile, kiter, c);
   if ((c[0] * 4) % 16) { printf("unaligned innermost TMA coordinate %lld\n", (long long)c[0]); return false; }
   for (int d = 1; d < m.rank; ++d) if (m.strides[d] % 16) { printf("stride %d not a multiple of 16 bytes\n", d); return false; }
   if ((m.box[0] * 4) % 16 || (int)m.box[0] * 4 > span(m.swizzle) && m.swizzle != TC_SW_NONE) { printf("bad inner box\n"); return false; }
   int64_t total = 1; for (int d = 0; d < m.rank; ++d) { if (m.box[d] > 256) { printf("box > 256\n"); return false; } total *= m.box[d]; }
-  if (total * 4 != o.stage_bytes) { printf("stage_bytes %u != box bytes %lld\n", o.stage_bytes, (long long)total * 4); return false; }
-  smem.assign(o.stage_bytes / 4, 0.0f);
-  for (int64_t lin = 0; lin < total; ++lin) {
-    int64_t r = lin, goff = 0; bool inb = true;
-    for (int d = 0; d < m.rank; ++d) {
-      int64_t i = r % m.box[d]; r /= m.box[d];
-      int64_t g = c[d] + i;
-      if (g < 0 || g >= (int64_t)m.dims[d]) inb = false;
-      goff += g * (d == 0 ? 4 : (int64_t)m.strides[d]);
+  const int boxes = o.load == TC_LOAD_BOXES ? o.nbox : 1;
+  if (boxes > 1 && total * 4 != 4096) { printf("box of several not 4096 bytes\n"); return false; }
+  if (total * 4 * boxes != o.stage_bytes) { printf("stage_bytes %u != box bytes %lld\n", o.stage_bytes, (long long)total * 4); return false; }
+  smem.assign(o.stage_bytes / 4, 1e30f);
+  for (int b = 0; b < boxes; ++b, c[0] += 32) {
+    if (o.load == TC_LOAD_BOXES && c[0] >= (int64_t)m.dims[0]) break;       // wholly beyond the row: not loaded
+    for (int64_t lin = 0; lin < total; ++lin) {
+      int64_t r = lin, goff = 0; bool inb = true;
+      for (int d = 0; d < m.rank; ++d) {
+        int64_t i = r % m.box[d]; r /= m.box[d];
+        int64_t g = c[d] + i;
+        if (g < 0 || g >= (int64_t)m.dims[d]) inb = false;
+        goff += g * (d == 0 ? 4 : (int64_t)m.strides[d]);
+      }
+      float v = inb ? *(const float*)((const char*)m.base + goff) : 0.0f;
+      smem[swz((uint32_t)(b * 4096 + lin * 4), m.swizzle) / 4] = v;
     }
-    float v = inb ? *(const float*)((const char*)m.base + goff) : 0.0f;
-    smem[swz((uint32_t)lin * 4, m.swizzle) / 4] = v;
   }
   return true;
 }
@@ -106,6 +162,7 @@ static bool walk_matches(const TcOperand& o, int tile, int k_iters) {
 static bool run_plan(const TcPlan& p, size_t out_count) {
   if (p.a.nk != p.b.nk) { printf("nk mismatch\n"); return false; }
   if (!walk_matches(p.a, p.m_tiles - 1, p.k_iters) || !walk_matches(p.b, p.n_tiles - 1, p.k_iters)) return false;
+  for (const TcOperand* o : {&p.a, &p.b}) if (o->load == TC_LOAD_IM2COL_MN && !pixel_walk_matches(*o, p.k_iters)) return false;
   // overwrite semantics under split-K: the partial results of the splits are summed and then stored; emulated by zeroing first
   if (p.splits > 1 && !p.accumulate) for (size_t i = 0; i < out_count; ++i) p.out[i] = 0.0f;
   std::vector<float> sa, sb;
@@ -124,8 +181,16 @@ static bool run_plan(const TcPlan& p, size_t out_count) {
     for (int r = 0; r < 128; ++r) for (int c = 0; c < p.bn; ++c) {
       int64_t m = (int64_t)mt * 128 + r, n = (int64_t)nt * p.bn + c;
       if (m >= p.M || n >= p.N) continue;
-      int64_t idx = p.epilogue == TC_EPI_PIXEL ? (m / p.pix_per_img) * p.img_stride + n * p.chan_stride + (m % p.pix_per_img)
-                                                : m * p.ld + (p.col_mul ? (n % p.col_mod) * p.col_mul + n / p.col_mod : n);
+      int64_t idx;
+      if (p.epilogue == TC_EPI_PIXEL) {
+        const int64_t per = p.pix_pad ? p.pix_pad : p.pix_per_img;
+        if (m % per >= p.pix_per_img) continue;                       // a row of the image's last tile beyond the image
+        idx = m / per * p.img_stride + n * p.chan_stride + m % per;
+      } else if (p.epilogue == TC_EPI_TAPS) {
+        const int64_t q = n / 32, blk = q / p.col_mul, ch = blk * 32 + n % 32;
+        if (ch >= p.col_mod) continue;                                // a channel that only fills up the last block
+        idx = m * p.ld + ch * p.col_mul + q % p.col_mul;
+      } else idx = m * p.ld + (p.col_mul ? (n % p.col_mod) * p.col_mul + n / p.col_mod : n);
       if ((size_t)idx >= out_count) { printf("epilogue index out of range\n"); return false; }
       float v = p.alpha * (float)D[(size_t)r * p.bn + c] + ((p.bias && z == 0) ? p.bias[n] : 0.0f);
       if (p.accumulate || atomic) p.out[idx] += v; else p.out[idx] = v;
@@ -204,24 +269,53 @@ static int conv_case(int n_img, int ck, int co, int pix) {
       tc_plan_gather(p, dy.data(), n_img, co, pix); ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "dgrad (gather)")) return -1; }
   }
   if (tc_plan_conv_wgrad(p, x.data(), dy.data(), dw.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "wgrad")) return -1; }
-  printf("conv n=%d ck=%d co=%d pix=%d: %d of 3 plans taken, all match\n", n_img, ck, co, pix, taken);
+  printf("conv n=%d ck=%d co=%d pix=%d: %d of 3 plans (5 with the gathered ones) taken, all match\n", n_img, ck, co, pix, taken);
   return taken;
 }
 
-// R x S convolution with stride 1 through the tap-loop plans, against a direct evaluation.
-static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph, int pw) {
-  const int oH = H + 2 * ph - R + 1, oW = W + 2 * pw - S + 1, taps = R * S;
+// Images of a size that fills no tiles, straight from x[n][k][p].
+static int ragged_case(int n_img, int ck, int co, int pix) {
+  auto x = rnd((size_t)n_img * ck * pix, 1), w = rnd((size_t)co * ck, 2), dy = rnd((size_t)n_img * co * pix, 3), bias = rnd(co, 4);
+  std::vector<float> y(dy.size(), 7.0f), yr(y.size()), dx(x.size(), 0.5f), dxr(dx), dw(w.size(), -1.0f), dwr(dw);
+  for (int n = 0; n < n_img; ++n) for (int q = 0; q < pix; ++q) {
+    for (int c = 0; c < co; ++c) {
+      double s = bias[c]; for (int k = 0; k < ck; ++k) s += (double)w[(size_t)c * ck + k] * x[((size_t)n * ck + k) * pix + q];
+      yr[((size_t)n * co + c) * pix + q] = (float)s;
+    }
+    for (int k = 0; k < ck; ++k) {
+      double s = 0; for (int c = 0; c < co; ++c) s += (double)w[(size_t)c * ck + k] * dy[((size_t)n * co + c) * pix + q];
+      dxr[((size_t)n * ck + k) * pix + q] += (float)s;
+    }
+  }
+  for (int c = 0; c < co; ++c) for (int k = 0; k < ck; ++k) {
+    double s = 0; for (int n = 0; n < n_img; ++n) for (int q = 0; q < pix; ++q) s += (double)dy[((size_t)n * co + c) * pix + q] * x[((size_t)n * ck + k) * pix + q];
+    dwr[(size_t)c * ck + k] += (float)s;
+  }
+  const int ld = (ck + 3) / 4 * 4; std::vector<float> wp((size_t)co * ld, 0.0f);
+  for (int c = 0; c < co; ++c) for (int k = 0; k < ck; ++k) wp[(size_t)c * ld + k] = w[(size_t)c * ck + k];
+  int taken = 0; TcPlan p;
+  if (tc_plan_conv_ragged_fwd(p, x.data(), wp.data(), ld, bias.data(), y.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "ragged fwd")) return -1; }
+  if (tc_plan_conv_ragged_dgrad(p, dy.data(), wp.data(), ld, dx.data(), n_img, ck, co, pix, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "ragged dgrad")) return -1; }
+  if (tc_plan_conv_ragged_wgrad(p, x.data(), dy.data(), dw.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "ragged wgrad")) return -1; }
+  printf("ragged conv n=%d ck=%d co=%d pix=%d: %d of 3 plans taken, all match\n", n_img, ck, co, pix, taken);
+  return taken;
+}
+
+// R x S convolution against a direct evaluation: through the tap-loop plans (stride 1), and through the im2col-mode plans from
+// channels-last copies whose channels are padded to a multiple of 4.
+static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph, int pw, int sh = 1, int sw = 1) {
+  const int oH = (H + 2 * ph - R) / sh + 1, oW = (W + 2 * pw - S) / sw + 1, taps = R * S;
   TcConvGeom g{n_img, C, H, W, K, R, S, ph, pw, oH, oW};
   auto x = rnd((size_t)n_img * C * H * W, 11), w = rnd((size_t)K * C * taps, 12), dy = rnd((size_t)n_img * K * oH * oW, 13), bias = rnd(K, 14);
   std::vector<float> y((size_t)n_img * K * oH * oW, 7.0f), yr(y.size()), dx(x.size(), 0.5f), dxr(dx), dw(w.size(), -1.0f), dwr(dw);
   auto X = [&](int n, int c, int h, int ww) -> double { return (h < 0 || h >= H || ww < 0 || ww >= W) ? 0.0 : x[(((size_t)n * C + c) * H + h) * W + ww]; };
   for (int n = 0; n < n_img; ++n) for (int k = 0; k < K; ++k) for (int oh = 0; oh < oH; ++oh) for (int ow = 0; ow < oW; ++ow) {
     double s = bias[k];
-    for (int c = 0; c < C; ++c) for (int r = 0; r < R; ++r) for (int q = 0; q < S; ++q) s += X(n, c, oh - ph + r, ow - pw + q) * w[(((size_t)k * C + c) * R + r) * S + q];
+    for (int c = 0; c < C; ++c) for (int r = 0; r < R; ++r) for (int q = 0; q < S; ++q) s += X(n, c, oh * sh - ph + r, ow * sw - pw + q) * w[(((size_t)k * C + c) * R + r) * S + q];
     yr[(((size_t)n * K + k) * oH + oh) * oW + ow] = (float)s;
     const double d = dy[(((size_t)n * K + k) * oH + oh) * oW + ow];
     for (int c = 0; c < C; ++c) for (int r = 0; r < R; ++r) for (int q = 0; q < S; ++q) {
-      const int h = oh - ph + r, ww = ow - pw + q;
+      const int h = oh * sh - ph + r, ww = ow * sw - pw + q;
       if (h < 0 || h >= H || ww < 0 || ww >= W) continue;
       dxr[(((size_t)n * C + c) * H + h) * W + ww] += (float)(d * w[(((size_t)k * C + c) * R + r) * S + q]);
       dwr[(((size_t)k * C + c) * R + r) * S + q] += (float)(d * x[(((size_t)n * C + c) * H + h) * W + ww]);
@@ -236,14 +330,34 @@ static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph
     wd[((size_t)t * C + c) * K + k] = w[((size_t)k * C + c) * taps + t];
   }
   int taken = 0; TcPlan p;
-  if (tc_plan_conv_taps_fwd(p, xr.data(), wt.data(), bias.data(), y.data(), g, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "taps fwd")) return -1; }
-  if (tc_plan_conv_taps_dgrad(p, dyr.data(), wd.data(), dx.data(), g, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "taps dgrad")) return -1; }
-  if (tc_plan_conv_taps_wgrad(p, dyr.data(), xr.data(), dw.data(), g, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "taps wgrad")) return -1; }
-  printf("taps conv n=%d C=%d K=%d %dx%d k%dx%d pad %d,%d: %d of 3 plans taken, all match\n", n_img, C, K, H, W, R, S, ph, pw, taken);
+  if (sh == 1 && sw == 1) {
+    if (tc_plan_conv_taps_fwd(p, xr.data(), wt.data(), bias.data(), y.data(), g, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "taps fwd")) return -1; }
+    if (tc_plan_conv_taps_dgrad(p, dyr.data(), wd.data(), dx.data(), g, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "taps dgrad")) return -1; }
+    if (tc_plan_conv_taps_wgrad(p, dyr.data(), xr.data(), dw.data(), g, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "taps wgrad")) return -1; }
+  }
+  // im2col mode; the data gradient of a strided convolution is a stride-1 one of dy with zeros between its pixels
+  const int ldc = (C + 3) / 4 * 4, ldk = (K + 3) / 4 * 4, uH = H + 2 * ph - R + 1, uW = W + 2 * pw - S + 1;
+  std::vector<float> xp((size_t)n_img * H * W * ldc, 0.0f), dyp((size_t)n_img * oH * oW * ldk, 0.0f), up((size_t)n_img * uH * uW * ldk, 0.0f), wtp((size_t)taps * K * ldc, 0.0f), wdp((size_t)taps * C * ldk, 0.0f);
+  for (size_t i = 0; i < (size_t)n_img * H * W; ++i) for (int c = 0; c < C; ++c) xp[i * ldc + c] = xr[i * C + c];
+  for (int n = 0; n < n_img; ++n) for (int a = 0; a < oH; ++a) for (int b = 0; b < oW; ++b) for (int k = 0; k < K; ++k) {
+    const float v = dyr[(((size_t)n * oH + a) * oW + b) * K + k];
+    dyp[(((size_t)n * oH + a) * oW + b) * ldk + k] = v; up[(((size_t)n * uH + a * sh) * uW + b * sw) * ldk + k] = v;
+  }
+  for (int t = 0; t < taps; ++t) for (int k = 0; k < K; ++k) for (int c = 0; c < C; ++c) {
+    wtp[((size_t)t * K + k) * ldc + c] = wt[((size_t)t * K + k) * C + c]; wdp[((size_t)t * C + c) * ldk + k] = wd[((size_t)t * C + c) * K + k];
+  }
+  std::fill(y.begin(), y.end(), 7.0f); std::fill(dx.begin(), dx.end(), 0.5f); std::fill(dw.begin(), dw.end(), -1.0f);
+  TcConvAny a{n_img, C, H, W, K, R, S, sh, sw, ph, pw, oH, oW, ldc, ldk}, u{n_img, C, H, W, K, R, S, 1, 1, ph, pw, uH, uW, ldc, ldk};
+  int any = 0;
+  if (tc_plan_conv_any_fwd(p, xp.data(), wtp.data(), bias.data(), y.data(), a, 148)) { ++any; if (!run_plan(p, y.size()) || !close(yr, y, "im2col fwd")) return -1; }
+  if (tc_plan_conv_any_dgrad(p, up.data(), wdp.data(), dx.data(), u, true, 148)) { ++any; if (!run_plan(p, dx.size()) || !close(dxr, dx, "im2col dgrad")) return -1; }
+  if (tc_plan_conv_any_wgrad(p, dyp.data(), xp.data(), dw.data(), a, 148)) { ++any; if (!run_plan(p, dw.size()) || !close(dwr, dw, "im2col wgrad")) return -1; }
+  if (any != 3) { printf("only %d of 3 im2col plans taken\n", any); return -1; }
+  printf("taps conv n=%d C=%d K=%d %dx%d k%dx%d pad %d,%d stride %d,%d: %d of 3 window plans and 3 im2col plans taken, all match\n", n_img, C, K, H, W, R, S, ph, pw, sh, sw, taken);
   return taken;
 }
 
-static int gemm_case(int M, int N, int K, bool ak, bool bk, bool acc) {
+static int gemm_case(int M, int N, int K, bool ak, bool bk, bool acc, int sms = 148) {
   auto a = rnd((size_t)M * K, 5), b = rnd((size_t)N * K, 6);
   std::vector<float> c((size_t)M * N, 2.0f), cr(c);
   for (int m = 0; m < M; ++m) for (int n = 0; n < N; ++n) {
@@ -251,8 +365,18 @@ static int gemm_case(int M, int N, int K, bool ak, bool bk, bool acc) {
     cr[(size_t)m * N + n] = (acc ? cr[(size_t)m * N + n] : 0.0f) + 0.5f * (float)s;
   }
   TcPlan p;
-  if (!tc_plan_gemm(p, a.data(), ak, b.data(), bk, c.data(), M, N, K, 0.5f, acc, 148)) { printf("gemm %dx%dx%d ak=%d bk=%d: not eligible\n", M, N, K, ak, bk); return 0; }
-  if (!run_plan(p, c.size()) || !close(cr, c, "gemm")) return -1;
+  const int wa = ak ? K : M, ha = ak ? M : K, wb = bk ? K : N, hb = bk ? N : K;
+  if (wa % 4 == 0 && wb % 4 == 0) {
+    if (!tc_plan_gemm(p, a.data(), ak, b.data(), bk, c.data(), M, N, K, 0.5f, acc, sms)) { printf("gemm %dx%dx%d ak=%d bk=%d: not eligible\n", M, N, K, ak, bk); return 0; }
+    if (!run_plan(p, c.size()) || !close(cr, c, "gemm")) return -1;
+  } else {                     // rows of no whole 16-byte unit: copies padded with zeros, as the library makes them
+    const int lda = (wa + 3) / 4 * 4, ldb = (wb + 3) / 4 * 4;
+    std::vector<float> ap((size_t)ha * lda, 0.0f), bp((size_t)hb * ldb, 0.0f);
+    for (int i = 0; i < ha; ++i) for (int j = 0; j < wa; ++j) ap[(size_t)i * lda + j] = a[(size_t)i * wa + j];
+    for (int i = 0; i < hb; ++i) for (int j = 0; j < wb; ++j) bp[(size_t)i * ldb + j] = b[(size_t)i * wb + j];
+    if (!tc_plan_gemm_ld(p, ap.data(), ak, lda, bp.data(), bk, ldb, c.data(), M, N, K, 0.5f, acc, sms)) { printf("gemm %dx%dx%d ak=%d bk=%d: padded copies not eligible\n", M, N, K, ak, bk); return -1; }
+    if (!run_plan(p, c.size()) || !close(cr, c, "padded gemm")) return -1;
+  }
   printf("gemm %dx%dx%d ak=%d bk=%d acc=%d: bn=%d splits=%d match\n", M, N, K, ak, bk, acc, p.bn, p.splits);
   return 1;
 }
@@ -275,7 +399,19 @@ int main() {
   for (int ak = 0; ak < 2; ++ak) for (int bk = 0; bk < 2; ++bk) for (int acc = 0; acc < 2; ++acc) {
     int r = gemm_case(160, 96, 72, ak, bk, acc); if (r < 0) ++bad; else taken += r;
     r = gemm_case(128, 256, 2048, ak, bk, acc); if (r < 0) ++bad; else taken += r;
+    r = gemm_case(68, 36, 100, ak, bk, acc); if (r < 0) ++bad; else taken += r;                 // row lengths that are no multiple of 32
+    r = gemm_case(131, 17, 67, ak, bk, acc); if (r < 0) ++bad; else taken += r;                 // nor of 4
+  }
+  // 256-wide tiles, as small products have them on a machine of a few SMs: enough of them, and one in two splits
+  { int r = gemm_case(250, 508, 520, true, true, true, 4); if (r < 0) ++bad; else taken += r; }
+  { int r = gemm_case(128, 244, 3100, false, false, false, 3); if (r < 0) ++bad; else taken += r; }
+  const int ragged[][4] = {{2, 64, 72, 100}, {3, 36, 24, 196}, {1, 33, 132, 68}, {2, 40, 64, 132}};
+  for (auto& c : ragged) { int r = ragged_case(c[0], c[1], c[2], c[3]); if (r < 0) ++bad; else taken += r; }
+  const int any[][11] = {{2, 12, 20, 7, 9, 3, 3, 1, 1, 1, 1}, {3, 40, 72, 11, 7, 3, 3, 1, 1, 2, 2}, {2, 33, 8, 9, 9, 5, 5, 2, 2, 1, 1}, {2, 64, 48, 14, 14, 1, 1, 0, 0, 2, 2},
+                         {1, 96, 64, 27, 27, 5, 5, 2, 2, 1, 1}, {5, 8, 136, 5, 13, 3, 2, 0, 1, 2, 1}};
+  for (auto& c : any) {
+    int r = taps_case(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9], c[10]); if (r < 0) ++bad; else taken += r;
   }
   printf("%d plans emulated, %d failures\n", taken, bad);
-  return bad ? 1 : (taken >= 40 ? 0 : 2);
+  return bad ? 1 : (taken >= 140 ? 0 : 2);
 }
