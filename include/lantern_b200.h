@@ -56,6 +56,12 @@ enum { LTB_ADD = 0, LTB_SUB = 1, LTB_MUL = 2, LTB_DIV = 3 };
 enum { LTB_RELU = 0, LTB_TANH = 1, LTB_SIGMOID = 2, LTB_EXP = 3, LTB_LOG = 4, LTB_SQRT = 5, LTB_SQUARE = 6 };
 /* Math mode, the counterpart of `cudnnMathType` (TensorDslCudnn.scala:133-136). */
 enum { LTB_MATH_FP32 = 0, LTB_MATH_TF32 = 1 };
+/* LTB_MATH_TF32 lets convolutions (each of forward, data gradient and weight gradient by itself) and matrix products run on the tensor
+ * cores wherever there is a plan for the shape, images and rows of any length among them: both factors are cut to 10 mantissa bits, the
+ * products are summed in FP32.  Which shapes have a plan is no part of the contract.  Always in FP32, in either mode: convolutions with fewer than 8 output channels or fewer than 8 filter elements per output
+ * channel (16 in the weight gradient), products with M or N below 16 or K below 32, the matrix-vector and dot products, the fused
+ * recurrent entry points (affine_act*, rnn_seq_*, tree_node*) and everything that is no contraction.  A caller that needs FP32 in a
+ * contraction sets LTB_MATH_FP32 for it; the mode may be changed between any two calls. */
 
 /* ---------------------------------------------------------------- lifetime / context
  * Replaces backend.setup()/cleanup(): TensorDslCublas.scala:113-124, TensorDslCudnn.scala:143-151
@@ -72,7 +78,7 @@ int    LTB_FN(set_math)(int mode);                      /* LTB_MATH_TF32 (defaul
  * add are issued one call late so that an in-place ReLU of their result joins the same kernel, and an in-place ReLU gradient is held
  * so that the batch-norm backward, convolution backward with a bias or add gradient that reads it applies it on the fly. Results are those of the separate calls; only the moment
  * of the launch moves: a held operation is issued by the next call of this library whatever it is (sync, copies,
- * get_stream and graph_end included; malloc, malloc_uninit and grad_unset only keep books on a block no held operation can
+ * get_stream and graph_end included; malloc, malloc_uninit, mark and grad_unset only keep books on a block no held operation can
  * name yet and issue nothing). A host that enqueues its own work on the stream must call get_stream or sync first.  In the same
  * spirit conv2d_bwd may return while its weight gradient still runs on a second stream: the gradient calls of the chain
  * (conv2d_bwd, bn_bwd, unary_grad, concat_grad, the gradient of an add) wait for it only when their buffers meet, every other call does first.

@@ -1,10 +1,12 @@
 // TF32 tensor-core engine for sm_100a: one warp-specialised kernel for every dense contraction of the training step
 // (convolution forward / data-grad / weight-grad and gemm), driven by the plans of tc_plan.cpp.
 //
-//   warp 0      : TMA producer.  One lane issues cp.async.bulk.tensor loads of the A and B boxes of each k-iteration into a
-//                 4-stage shared-memory ring; completion is signalled on the stage's "full" mbarrier by byte count.
+//   warp 0      : TMA producer: cp.async.bulk.tensor loads of the A and B boxes of each k-iteration into a shared-memory ring of
+//                 four stages (three for 128-wide tiles, so that two CTAs share an SM); completion is signalled on the stage's
+//                 "full" mbarrier by byte count.  With one box per operand the elected lane issues both, with several
+//                 boxes or the im2col mode every lane its own (BoxLane::issue).
 //   warp 1      : owns the tensor memory (tcgen05.alloc / dealloc) and issues tcgen05.mma.kind::tf32 (M = 128, N = tile
-//                 width, K = 8) from one lane, four per stage, accumulating in TMEM; tcgen05.commit releases the stage
+//                 width, K = 8) from the elected lane, four per stage, accumulating in TMEM; tcgen05.commit releases the stage
 //                 ("empty" mbarrier) and finally signals the epilogue.
 //   warps 2..9  : epilogue.  Each warp reads its 32-lane quarter of the accumulator with tcgen05.ld (32 columns at a time)
 //                 and writes the result: pixel-major for convolutions (a warp store covers 32 consecutive pixels of one
@@ -14,8 +16,10 @@
 // contiguous one and the activation operand is fed M/N-major (tcgen05 allows it for tf32) straight from the tensor with a
 // 4-D tiled tensor map.  R x S convolutions with stride 1 run in tap-loop form from a channels-last copy (one transposing
 // pass, see channels_last_kernel): a TMA box is then a window of whole image rows whose coordinates the tap shifts, and
-// zero fill outside the image is the padding.  Smaller images, strided forward convolutions and weight-grads of R x S
-// filters are staged as row matrices or unfolded matrices by the helper kernels at the end of this file.
+// zero fill outside the image is the padding.  Images that fill no tiles, and strides, go through the TMA unit's im2col mode on the
+// same copies (conv_fwd_any and its neighbours), 1x1 convolutions on such images through several clipped boxes per tile.  1x1
+// convolutions on maps of 4 and 16 pixels are gathered by the epilogue warps.  Filters over a few channels, and strided ones where
+// the unfolded matrix is no larger than two copies, are unfolded by the helper kernels below (wants_im2col).
 // Every mbarrier wait is bounded: after about a second it records a code in the library's device status word and the CTA
 // runs to its normal teardown (TMEM is released on every path).  The single issuing lanes of warps 0 and 1 are rejoined by
 // their warps (__syncwarp) before the block-wide barrier, which needs converged warps.
@@ -1315,7 +1319,8 @@ static int conv_dgrad_taps(const float* dy, const float* w, float* dx, const Con
 // of 32.  In im2col mode the TMA unit walks the output pixels itself, image after image, at any stride, so a tile is any 128
 // consecutive output pixels and nothing is unfolded or folded back: per call one channels-last copy of the activation (shared with
 // the other passes when the operand cache is on) and the contraction.  Before, such a convolution was unfolded into a matrix R x S
-// times the size of its input element by element (56 x 56, 64 -> 64, 3x3, batch 32: forward 476 us, with this path 67 us; the layer's whole training pass 920 -> 310 us).
+// times the size of its input element by element (56 x 56, 64 -> 64, 3x3, batch 32: forward 476 us, with this path 67 us; the layer's
+// whole training pass 920 -> 310 us, 215 with what followed).
 // A filter of fewer than 32 elements per output channel fills less than one k-iteration and stays with the other paths, and so do
 // forward and data-gradient of such images when their rows would need padding (below): those have always been computed in FP32.
 static bool any_geometry(const ConvDims& d, TcConvAny& a) {

@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(kSeqThreads) rnn_seq_bwd_kernel(const float* _
 // and hold its H weights in registers, so a step is H / 16 vector loads of h, H / 4 FMAs, two shuffles and a barrier.
 // Matrices come in by cp.async, all copies in flight at once; Who is never transposed (a product of rows with rows, its pitch
 // padded by 4 floats against bank conflicts); with one CTA the gradients are added in place, without the slab and its sum.
-// 20 steps, vocabulary 80, hidden 100, batch 1: the step 116 -> 90 us (forward 38 -> 24, backward with its sum 41 -> 27); batch 256: 158 -> 150.
+// 20 steps, vocabulary 80, hidden 100, batch 1: the step 116 -> 90 us (forward 38 -> 24, backward with its sum 41 -> 27); batch 256: 158 -> 150 (124 with the
+// batch uploaded while it is copied).
 constexpr int kRegHidden = 128;
 __device__ __forceinline__ void copy_async16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");

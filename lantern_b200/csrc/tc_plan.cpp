@@ -395,7 +395,7 @@ bool tc_plan_conv_dgrad(TcPlan& p, const float* dy, bool a_rows, const float* w,
   const int M = n_img * pix;
   if (!(a_rows ? operand_k_rows(p.a, dy, M, co, kTileM, &ka) : operand_mn_pixels(p.a, dy, n_img, co, pix, &ka))) return false;
   p.bn = pick_bn(ck, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_mn_cols(p.b, w, co, ldw, p.bn, &kb) || ka != kb) return false;      // w is stored with ldw (a multiple of 32) columns
+  if (!operand_mn_cols(p.b, w, co, ldw, p.bn, &kb) || ka != kb) return false;      // columns ck .. ldw of w are zero padding
   finish(p, M, ck, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = dx; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = accumulate ? 1 : 0;
   p.pix_per_img = pix; p.img_stride = (int64_t)ck * pix; p.chan_stride = pix;

@@ -120,7 +120,7 @@ struct TcPlan {
 
 // "Flat" convolution view: activations X[n][k][p] with p contiguous (k = channels, or channels*kh*kw after unfolding),
 // weights W[co][k] row-major with ldw >= k floats per row (zeros beyond k: the caller pads a copy when the engine needs a
-// wider row -- forward: ldw a multiple of 4, dgrad: a multiple of 32), outputs Y[n][co][p].  P is the number of pixels per image.
+// wider row, ldw a multiple of 4), outputs Y[n][co][p].  P is the number of pixels per image.
 //   forward : Y[n][co][p]  = sum_k  W[co][k] X[n][k][p] (+ bias[co])         D = pixels x co
 //   dgrad   : dX[n][k][p] (+)= sum_co W[co][k] dY[n][co][p]                   D = pixels x k
 //   wgrad   : dW[co][k]  += sum_{n,p} dY[n][co][p] X[n][k][p]                 D = co x k

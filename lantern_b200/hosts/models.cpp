@@ -34,8 +34,8 @@ namespace {
 
 // A batch's copy into pinned memory.  The processor never reads the copy back, so it is written with streaming stores, which leave out the
 // read of the destination that an ordinary store begins with: 1.6 MB in 69 us, 93 with memcpy.  One thread is enough: the recurrent program
-// at batch 256, whose batch that is, takes 124 us a step with this, 158 with memcpy and slower kernels, and 125 with three helper threads,
-// which cost a program 0.3 ms at its first step and 0.1 ms at its close.
+// at batch 256, whose batch that is, takes 124 us a step with this, 150 with memcpy, and 125 with three helper threads, which
+// cost a program 0.3 ms at its first step and 0.1 ms at its close.
 void copy_to_staging(void* dst, const void* src, size_t bytes) {
 #ifdef __SSE2__
   if (((uintptr_t)dst & 15) == 0) {

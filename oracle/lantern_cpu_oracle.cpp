@@ -62,7 +62,8 @@ struct Ctx {
 // TF32 emulation.  In LTB_MATH_TF32 mode the oracle reproduces what the product's tensor-core path computes for the
 // shapes that path accepts: both operands of the contraction reduced to TF32 (10-bit mantissa, low 13 bits dropped, as the
 // tensor core reads FP32 words), products and sums in FP32.  Shapes the engine declines are computed in plain FP32 on both
-// sides.  This turns the 2e-3 "TF32 tolerance" into a check at FP32 rounding level.  Default is plain FP32: the reference's
+// sides.  Not known here are the plans for images and rows of any length (im2col mode, clipped boxes, padded copies): their tests
+// use factors that have ten mantissa bits to begin with, whose TF32 products are exact.  This turns the 2e-3 "TF32 tolerance" into a check at FP32 rounding level.  Default is plain FP32: the reference's
 // CPU backend.
 inline float tf32_trunc(float v) { uint32_t u; memcpy(&u, &v, 4); u &= 0xFFFFE000u; memcpy(&v, &u, 4); return v; }
 std::vector<float> truncated(const float* p, size_t n) { std::vector<float> v(n); for (size_t i = 0; i < n; ++i) v[i] = tf32_trunc(p[i]); return v; }
@@ -81,9 +82,9 @@ bool tc_conv_taken(int kind, int n_img, int ck, int co, int pix, bool full_image
     return tc_gemm_taken(false, false, co, ck, n_img);                    // dw[K][CHW] += dy^T[K][N] x[N][CHW]
   }
   ltb::TcPlan p; const bool rows = ltb::tc_conv_needs_rows(pix);
-  // the product pads filter rows to 4 floats (forward) or 32 (data-grad) in a staging copy when they are not
+  // the product pads filter rows to 4 floats in a staging copy when they are not
   if (kind == 0) return ltb::tc_plan_conv_fwd(p, tc_dummy, rows, tc_dummy, (ck + 3) / 4 * 4, nullptr, tc_dummy, n_img, ck, co, pix, 148);
-  if (kind == 1) return ltb::tc_plan_conv_dgrad(p, tc_dummy, rows, tc_dummy, (ck + 31) / 32 * 32, tc_dummy, n_img, ck, co, pix, true, 148);
+  if (kind == 1) return ltb::tc_plan_conv_dgrad(p, tc_dummy, rows, tc_dummy, (ck + 3) / 4 * 4, tc_dummy, n_img, ck, co, pix, true, 148);
   return ltb::tc_plan_conv_wgrad(p, tc_dummy, tc_dummy, tc_dummy, n_img, ck, co, pix, 148);
 }
 

@@ -1,7 +1,7 @@
 """Helpers shared by the GPU parity tests: run the same calls on the CPU oracle and on the CUDA library."""
 import numpy as np
 
-FP32_RTOL = 1e-4      # FP32 CUDA-core paths: 1e-4 relative (north star)
+FP32_RTOL = 1e-4      # FP32 CUDA-core paths: 1e-4 relative (the bound every FP32 path is held to)
 TF32_RTOL = 2e-3      # TF32 tensor-core paths: 2e-3 relative
 
 

@@ -254,18 +254,18 @@ static int conv_case(int n_img, int ck, int co, int pix) {
       for (int c = 0; c < co; ++c) dyt[((size_t)n * pix + q) * co + c] = dy[((size_t)n * co + c) * pix + q];
     }
   }
-  // filter rows padded with zeros the way the library stages them: to 4 floats for forward, to 32 for data-grad
+  // filter rows padded with zeros to 4 floats, the way the library stages them
   auto padded = [&](int ld) { std::vector<float> o((size_t)co * ld, 0.0f); for (int c = 0; c < co; ++c) for (int k = 0; k < ck; ++k) o[(size_t)c * ld + k] = w[(size_t)c * ck + k]; return o; };
-  const int ld4 = (ck + 3) / 4 * 4, ld32 = (ck + 31) / 32 * 32;
-  const std::vector<float> w4 = padded(ld4), w32 = padded(ld32);
+  const int ld4 = (ck + 3) / 4 * 4;
+  const std::vector<float> w4 = padded(ld4);
   if (tc_plan_conv_fwd(p, rows ? xt.data() : x.data(), rows, w4.data(), ld4, bias.data(), y.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "fwd")) return -1; }
-  if (tc_plan_conv_dgrad(p, rows ? dyt.data() : dy.data(), rows, w32.data(), ld32, dx.data(), n_img, ck, co, pix, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "dgrad")) return -1; }
+  if (tc_plan_conv_dgrad(p, rows ? dyt.data() : dy.data(), rows, w4.data(), ld4, dx.data(), n_img, ck, co, pix, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "dgrad")) return -1; }
   // the same two contractions with the kernel gathering the activation itself (small images: 4 or 16 pixels)
   if (rows && tc_gather_possible(x.data(), ck, pix) && tc_gather_possible(dy.data(), co, pix)) {
     std::fill(y.begin(), y.end(), 7.0f); std::fill(dx.begin(), dx.end(), 0.5f);
     if (tc_plan_conv_fwd(p, x.data(), true, w4.data(), ld4, bias.data(), y.data(), n_img, ck, co, pix, 148)) {
       tc_plan_gather(p, x.data(), n_img, ck, pix); ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "fwd (gather)")) return -1; }
-    if (tc_plan_conv_dgrad(p, dy.data(), true, w32.data(), ld32, dx.data(), n_img, ck, co, pix, true, 148)) {
+    if (tc_plan_conv_dgrad(p, dy.data(), true, w4.data(), ld4, dx.data(), n_img, ck, co, pix, true, 148)) {
       tc_plan_gather(p, dy.data(), n_img, co, pix); ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "dgrad (gather)")) return -1; }
   }
   if (tc_plan_conv_wgrad(p, x.data(), dy.data(), dw.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "wgrad")) return -1; }

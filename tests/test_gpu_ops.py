@@ -458,6 +458,38 @@ def test_gemm_in_wide_tiles_tf32(ora, gpu, M, N, K, ta, tb, det):
         gpu.lib.set_deterministic(0)
 
 
+def _on_the_tensor_cores(lib, call):
+    import ctypes
+    lib.profile(1)
+    call()
+    lib.profile(0)
+    buf = ctypes.create_string_buffer(1 << 14)
+    lib.profile_report(ctypes.addressof(buf), len(buf))
+    return "tc_gemm_kernel" in buf.value.decode()
+
+
+@pytest.mark.parametrize("cfg,taken", [((8, 3, 32, 64, 3, 1), (1, 1, 1)), ((4, 64, 7, 64, 3, 1), (1, 1, 1)), ((4, 64, 14, 32, 1, 0), (1, 1, 1)),
+                                       ((2, 64, 27, 96, 3, 1), (1, 1, 1)), ((8, 1, 28, 10, 5, 0), (0, 0, 1)), ((4, 32, 8, 7, 3, 1), (0, 0, 0)), ((4, 7, 8, 32, 1, 0), (0, 0, 0))])
+def test_which_convolutions_run_in_tf32(gpu, cfg, taken):
+    """The shapes that the header names as always FP32, and the pass by pass choice next to them."""
+    N, C, H, K, Rk, p = cfg
+    O = H + 2 * p - Rk + 1
+    x, w, dy = gpu.zeros(N, C, H, H), gpu.zeros(K, C, Rk, Rk), gpu.zeros(N, K, O, O)
+    dx, dw, y = gpu.zeros(N, C, H, H), gpu.zeros(K, C, Rk, Rk), gpu.zeros(N, K, O, O)
+    dims = (N, C, H, H, K, Rk, Rk, 1, 1, p, p)
+    lib = gpu.lib
+    got = (_on_the_tensor_cores(lib, lambda: lib.conv2d_fwd(x.ptr, w.ptr, 0, y.ptr, *dims)),
+           _on_the_tensor_cores(lib, lambda: lib.conv2d_bwd(x.ptr, dx.ptr, w.ptr, 0, 0, dy.ptr, *dims)),
+           _on_the_tensor_cores(lib, lambda: lib.conv2d_bwd(x.ptr, 0, w.ptr, dw.ptr, 0, dy.ptr, *dims)))
+    assert got == tuple(map(bool, taken))
+
+
+@pytest.mark.parametrize("M,N,K,taken", [(64, 32, 32, 1), (128, 10, 2048, 0), (15, 4096, 4096, 0), (4096, 4096, 31, 0), (1000, 1001, 127, 1), (500, 500, 127, 0)])
+def test_which_products_run_in_tf32(gpu, M, N, K, taken):
+    a, b, c = gpu.zeros(M, K), gpu.zeros(N, K), gpu.zeros(M, N)
+    assert _on_the_tensor_cores(gpu.lib, lambda: gpu.lib.gemm(a.ptr, 0, b.ptr, 1, 1.0, c.ptr, M, N, K)) == bool(taken)
+
+
 def test_tensor_core_engine_reports_no_timeouts(gpu):
     assert gpu.lib.device_status() == 0
 
