@@ -149,10 +149,10 @@ def test_deferred_zero_fill_is_invisible_on_the_oracle(oracle_lib):
     assert res[0][0] == res[1][0] and np.array_equal(res[0][1], res[1][1])
 
 
-@pytest.mark.parametrize("batch", [1, 252, 253, 505])
+@pytest.mark.parametrize("batch", [1, 101, 252, 253, 505])
 def test_submitted_batches_arrive_whole(oracle_lib, batch):
-    """submit() copies a batch into its staging pair in pieces of 512 KB, 64 bytes at a time: batches of one row (2,080 bytes),
-    of 128 bytes less than a piece, of a piece and 1,952 bytes and of two and 1,824 train as the blocking steps do, bit for bit, whatever the address of the array."""
+    """submit() copies a batch into its staging pair in pieces of 512 KB, those of 32 KB and more 64 bytes at a time: batches of one
+    row (2,080 bytes), of 32 bytes more than a multiple of 64, of 128 bytes less than a piece, of a piece and 1,952 bytes and of two and 1,824 train as the blocking steps do, bit for bit, whatever the address of the array."""
     mark = oracle_lib.mark()
     rng = np.random.default_rng(batch)
     n = 20 * 26 * batch
