@@ -94,10 +94,12 @@ int    LTB_FN(set_fusion)(int on);
 /* Filter cache, off by default (no counterpart in the reference, where cuDNN reads OIHW filters as they are). The tensor-core
  * engine reads the filter of an R x S convolution as one matrix per tap; forward and data-grad each need their own form, and
  * without the cache both are rebuilt at every call. With it on they are kept, keyed by the filter's address and shape, and
- * rebuilt once after the parameters changed. The library notes a change by itself in every entry point through which a
- * generated program writes parameters: the optimizer steps (sgd_step*, adagrad_update, momentum_update, allreduce_*), h2d,
- * d2d, fill*, randinit, clip, geam, the in-place elementwise forms, and a replayed step. A host that writes a filter by
- * any other route (as the output of another operator, or with its own kernel) must call params_changed afterwards. */
+ * rebuilt once after the parameters changed. Every entry point of the library notes what it writes (a replayed step counts as having
+ * written everything). A host that writes a filter with its own kernel must call params_changed afterwards.
+ * A convolution's forward call also keeps its copy of x in the engine's layout for the weight gradient of the same convolution.  It is
+ * dropped when the library writes x, by params_changed and by reset; between a forward call and the backward call that belongs to it a
+ * host's own kernel must not write x without params_changed.  Nothing is kept from one forward call for the next, nor of dy from one
+ * backward call for the next. */
 /* Deterministic mode, off by default (the counterpart of choosing cuDNN's deterministic algorithms, which the reference does
  * not do: it takes whatever cudnnFind*Algorithm ranks first, TensorDslCudnn.scala:515-624). A contraction whose output has few
  * tiles is split over its reduction dimension. By default the splits add their partial results into the output atomically,

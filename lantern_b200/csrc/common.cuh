@@ -112,7 +112,8 @@ void cl_cache_clear();               // gemm_tc.cu: kept channels-last copies (t
 void cl_cache_drop_from(const void* p);
 // A block from the far end of the arena that stays until ltb_reset; nullptr when the two ends would meet (context.cu).
 void* step_alloc(size_t bytes);
-// A call is about to write [p, p + bytes): cached filter forms whose source overlaps it are stale (p == nullptr: all of them).
+// A call is about to write [p, p + bytes): kept copies and cached filter forms whose source overlaps it are stale (p == nullptr: all of
+// them).  Every entry point reports every buffer it writes (LTB_WRITES).
 void filter_cache_note_write(const void* p, size_t bytes);
 // Gradient buffers declared unset (ltb_grad_unset): logically zero, physically not yet written.
 //   grad_take_unset(p, bytes)  true when [p, p + bytes) is exactly one declared block: the caller WRITES its result instead
@@ -142,6 +143,8 @@ void profile_after();
 
 #define LTB_REQUIRE(cond, ...) do { if (!(cond)) return ::ltb::fail(LTB_E_ARG, __VA_ARGS__); } while (0)
 // A gradient buffer that was declared unset and is about to be used in any way but as a whole, writable destination: zeros first.
+// The entry point writes `count` floats at ptr (null: not asked for): kept copies and cached forms of what was there are stale.
+#define LTB_WRITES(ptr, count) do { if (ptr) ::ltb::filter_cache_note_write((ptr), (size_t)(count) * 4); } while (0)
 #define LTB_SETTLE(ptr) do { int rc_s_ = ::ltb::grad_settle((ptr), 0); if (rc_s_) return rc_s_; } while (0)
 #define LTB_CUDA(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) return ::ltb::fail(LTB_E_CUDA, "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); } while (0)
 #define LTB_INITED_CHAIN() do { if (!::ltb::g.inited) return ::ltb::fail(LTB_E_STATE, "%s: library not initialised (call ltb_init)", __func__); } while (0)

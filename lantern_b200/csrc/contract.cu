@@ -45,25 +45,30 @@ extern "C" {
 // matrixMatrixDot and the (2,2) case of dot_grad: TensorDslCPU.scala:158-169, 208-225.
 int ltb_mm_dot(const float* a, const float* b, float* out, int m, int k, int n) {
   LTB_INITED(); LTB_REQUIRE(a && b && out && m > 0 && k > 0 && n > 0, "ltb_mm_dot: bad argument");
+  LTB_WRITES(out, (size_t)m * n);
   return gemm_any(a, false, b, false, out, m, n, k, 1.0f, false);
 }
 int ltb_add_dot_trans1(float* db, const float* a, const float* dc, int m, int k, int n) {   // dB[k,n] += A^T[k,m] dC[m,n]
   LTB_INITED(); LTB_SETTLE(db); LTB_SETTLE(dc); LTB_REQUIRE(db && a && dc && m > 0 && k > 0 && n > 0, "ltb_add_dot_trans1: bad argument");
+  LTB_WRITES(db, (size_t)k * n);
   return gemm_any(a, true, dc, false, db, k, n, m, 1.0f, true);
 }
 int ltb_add_dot_trans2(float* da, const float* dc, const float* b, int m, int k, int n) {   // dA[m,k] += dC[m,n] B^T[n,k]
   LTB_INITED(); LTB_SETTLE(da); LTB_SETTLE(dc); LTB_REQUIRE(da && dc && b && m > 0 && k > 0 && n > 0, "ltb_add_dot_trans2: bad argument");
+  LTB_WRITES(da, (size_t)m * k);
   return gemm_any(dc, false, b, true, da, m, k, n, 1.0f, true);
 }
 
 // gemm: TensorDslCPU.scala:379-426.
 int ltb_gemm(const float* a, int ta, const float* b, int tb, float alpha, float* c, int M, int N, int K) {
   LTB_INITED(); LTB_REQUIRE(a && b && c && M > 0 && N > 0 && K > 0, "ltb_gemm: bad argument");
+  LTB_WRITES(c, (size_t)M * N);
   return gemm_any(a, ta != 0, b, tb != 0, c, M, N, K, alpha, false);
 }
 // gemm_grad: the eight cblas_sgemm calls of TensorDslCPU.scala:428-472, all with beta = 1.
 int ltb_gemm_grad(const float* a, float* da, int ta, const float* b, float* db, int tb, float alpha, const float* dc, int M, int N, int K) {
   LTB_INITED(); LTB_SETTLE(da); LTB_SETTLE(db); LTB_SETTLE(dc); LTB_REQUIRE(a && b && dc && M > 0 && N > 0 && K > 0, "ltb_gemm_grad: bad argument");
+  LTB_WRITES(da, (size_t)M * K); LTB_WRITES(db, (size_t)K * N);
   int rc = LTB_OK;
   if (!ta && !tb) {
     if (da) rc = gemm_any(dc, false, b, true, da, M, K, N, alpha, true);             // dA[M,K] += dC B^T
@@ -86,6 +91,7 @@ int ltb_conv2d_fwd(const float* x, const float* w, const float* bias, float* y, 
                    int sh, int sw, int ph, int pw) {
   LTB_INITED(); ConvDims d;
   LTB_REQUIRE(x && w && y && conv_dims(d, N, C, H, W, K, R, S, sh, sw, ph, pw), "ltb_conv2d_fwd: bad argument");
+  LTB_WRITES(y, (size_t)N * K * d.oH * d.oW);
   if (covers_image(d) && d.R * d.S > 1) {
     if (bias) { int rc = ltb_fill_with_bias(y, bias, N, K, 1); if (rc) return rc; }
     return gemm_any(x, false, w, true, y, N, K, C * R * S, 1.0f, bias != nullptr);
@@ -104,6 +110,7 @@ int ltb_conv2d_bwd(const float* x, float* dx, const float* w, float* dw, float* 
   if (g.side_open && g.used - g.side_base > g.heap_bytes / 8) { rc = side_join(); if (rc) return rc; }      // held staging blocks must not crowd the arena
   LTB_SIDE_CHECK(dx, nx, true); LTB_SIDE_CHECK(dw, nw, true); LTB_SIDE_CHECK(dbias, K, true); LTB_SIDE_CHECK(dy, ny, true);
   LTB_SIDE_CHECK(x, nx, false); LTB_SIDE_CHECK(w, nw, false);
+  LTB_WRITES(dx, nx); LTB_WRITES(dw, nw); LTB_WRITES(dbias, K);
   if (dbias && g.pending.kind == PEND_RELU_GRAD && g.pending.d == dy && g.pending.n == (int64_t)N * K * d.oH * d.oW && dbias != dy) {
     // the held ReLU gradient of dy: masked in the pass that sums the bias gradient, ahead of the two contractions
     const float* y = g.pending.relu_y;

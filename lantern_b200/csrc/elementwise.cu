@@ -533,6 +533,11 @@ using namespace ltb;
 
 extern "C" {
 
+static size_t shape_count(const int* shape, int rank) {
+  size_t n = 1;
+  for (int i = 0; i < rank && i < 8 && shape; ++i) n *= (size_t)(shape[i] > 0 ? shape[i] : 1);
+  return n;
+}
 // fill / fillInPlace: TensorDslCPU.scala:30-35, 65-67.
 int ltb_fill(float* x, float v, int64_t n) {
   LTB_INITED(); filter_cache_note_write(x, (size_t)(n > 0 ? n : 0) * 4); LTB_REQUIRE(x && n >= 0, "ltb_fill: bad argument");
@@ -557,6 +562,7 @@ int ltb_ew_binary(int op, const float* a, const int* as, const float* b, const i
   LTB_INITED_NOFLUSH(); LTB_REQUIRE(a && b && out && op >= LTB_ADD && op <= LTB_DIV, "ltb_ew_binary: bad argument");
   Bcast p; int64_t n; bool ab, bb;
   LTB_REQUIRE(make_bcast(as, bs, rank, p, n, ab, bb), "ltb_ew_binary: shapes do not broadcast");
+  LTB_WRITES(out, n);
   if (g.pending.kind == PEND_BN_FWD && g.fusion_single_use && !ab && !bb && op == LTB_ADD && g.pending.n == n && a != b &&
       (a == g.pending.y || b == g.pending.y)) {                 // the held batch norm's result plus a shortcut: held once more, for the ReLU
     const float* other = a == g.pending.y ? b : a;
@@ -581,6 +587,7 @@ int ltb_ew_binary_grad(int op, const float* a, float* da, const int* as, const f
   LTB_REQUIRE(make_bcast(as, bs, rank, p, n, ab, bb), "ltb_ew_binary_grad: shapes do not broadcast");
   // n bounds the size of either operand
   LTB_SIDE_CHECK(da, n, true); LTB_SIDE_CHECK(db, n, true); LTB_SIDE_CHECK(dout, n, true); LTB_SIDE_CHECK(a, n, false); LTB_SIDE_CHECK(b, n, false);
+  LTB_WRITES(da, shape_count(as, rank)); LTB_WRITES(db, shape_count(bs, rank));
   if (g.pending.kind == PEND_RELU_GRAD && !ab && !bb && op == LTB_ADD && g.pending.d == dout && g.pending.n == n && n > 0) {
     // the held ReLU gradient of dout and this add's gradient in one pass (dout is rewritten with the masked values)
     const float* y = g.pending.relu_y; float* d = g.pending.d;
@@ -620,7 +627,7 @@ int ltb_ew_inplace_scalar(int op, float* x, float s, int64_t n) { return ltb_ew_
 
 // inplaceElementWiseOpWithBroadCastOrReduce: TensorDslCPU.scala:265-279.
 int ltb_ew_inplace(int op, float* x, const int* xs, const float* y, const int* ys, int rank) {
-  LTB_INITED(); LTB_SETTLE(x); LTB_SETTLE(y); { size_t cnt_ = 1; for (int i_ = 0; i_ < rank && i_ < 8 && xs; ++i_) cnt_ *= (size_t)(xs[i_] > 0 ? xs[i_] : 1); filter_cache_note_write(x, cnt_ * 4); } LTB_REQUIRE(x && y && op >= LTB_ADD && op <= LTB_DIV, "ltb_ew_inplace: bad argument");
+  LTB_INITED(); LTB_SETTLE(x); LTB_SETTLE(y); LTB_WRITES(x, shape_count(xs, rank)); LTB_REQUIRE(x && y && op >= LTB_ADD && op <= LTB_DIV, "ltb_ew_inplace: bad argument");
   Bcast p; int64_t n; bool xb, yb;
   LTB_REQUIRE(make_bcast(xs, ys, rank, p, n, xb, yb), "ltb_ew_inplace: shapes do not broadcast");
   if (!xb && !yb) return launch_map<2>(x, y, nullptr, x, n, [op] __device__(float u, float v, float) { return bin_op(op, u, v); });
@@ -658,11 +665,13 @@ int ltb_geam(const float* x, int tx, float alpha, const float* y, int ty, float 
 // trans / trans_grad: TensorDslCPU.scala:349-374.
 int ltb_trans(const float* x, float* out, int rows, int cols) {
   LTB_INITED(); LTB_REQUIRE(x && out && rows > 0 && cols > 0, "ltb_trans: bad argument");
+  LTB_WRITES(out, (size_t)rows * cols);
   LTB_LAUNCH(transpose_kernel<false>, dim3((cols + 31) / 32, (rows + 31) / 32), dim3(32, 8), 0, x, out, rows, cols);
   return LTB_OK;
 }
 int ltb_trans_grad(float* dx, const float* dy, int rows, int cols) {
   LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && dy && rows > 0 && cols > 0, "ltb_trans_grad: bad argument");
+  LTB_WRITES(dx, (size_t)rows * cols);
   // dy is [cols, rows]; dx[rows, cols] += dy^T
   LTB_LAUNCH(transpose_kernel<true>, dim3((rows + 31) / 32, (cols + 31) / 32), dim3(32, 8), 0, dy, dx, cols, rows);
   return LTB_OK;
@@ -671,6 +680,7 @@ int ltb_trans_grad(float* dx, const float* dy, int rows, int cols) {
 // relu/tanh/sigmoid/exp/log/sqrt/square: TensorDslCPU.scala:710-781.
 int ltb_unary(int op, const float* x, float* out, int64_t n) {
   LTB_INITED_NOFLUSH(); LTB_REQUIRE(x && out && n >= 0 && op >= LTB_RELU && op <= LTB_SQUARE, "ltb_unary: bad argument");
+  LTB_WRITES(out, n);
   if (g.pending.kind && op == LTB_RELU && x == out && g.pending.n == n) {      // in-place ReLU of the result that was just held back
     const Pending h = g.pending;
     if (h.kind == PEND_BN_FWD && h.y == out) { g.pending.kind = PEND_NONE; return bn_fwd_issue(h, true); }
@@ -690,7 +700,7 @@ int ltb_unary_grad(int op, const float* x, float* dx, const float* y, const floa
   LTB_SIDE_CHECK(dx, n, true); LTB_SIDE_CHECK(x, n, false); LTB_SIDE_CHECK(y, n, false); LTB_SIDE_CHECK(dy, n, false);
   if (g.pending.kind) { int rc_ = flush_pending(); if (rc_) return rc_; }
   LTB_REQUIRE(dx && dy && n >= 0 && op >= LTB_RELU && op <= LTB_SQUARE, "ltb_unary_grad: bad argument");
-  LTB_SETTLE(dx); LTB_SETTLE(dy);
+  LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_WRITES(dx, n);
   if (op == LTB_RELU && in_place) {
     LTB_REQUIRE(y, "ltb_unary_grad: relu in place needs the result");
     if (g.fusion && n > 0) { Pending h; h.kind = PEND_RELU_GRAD; h.n = n; h.relu_y = y; h.d = dx; g.pending = h; return LTB_OK; }   // BN backward or an add's gradient may absorb it
@@ -709,11 +719,13 @@ int ltb_unary_grad(int op, const float* x, float* dx, const float* y, const floa
 // with time(NULL) (TensorDslCudnn.scala:1301) and cannot be reproduced.
 int ltb_dropout_masked(const float* x, float* y, const float* mask, int64_t n) {
   LTB_INITED(); LTB_REQUIRE(x && y && mask && n >= 0, "ltb_dropout_masked: bad argument");
+  LTB_WRITES(y, n);
   return launch_map<2>(x, mask, nullptr, y, n, [] __device__(float v, float m, float) { return v * m; });
 }
 int ltb_dropout(const float* x, float* y, float* mask, float p, int64_t n) {
   LTB_INITED(); LTB_REQUIRE(x && y && mask && n >= 0 && p >= 0.0f && p < 1.0f, "ltb_dropout: rate must be in [0,1)");
   LTB_REQUIRE(!g.capturing, "ltb_dropout: host RNG while recording a step");
+  LTB_WRITES(mask, n);
   if (n) {
     // drawn into pinned memory that the copy reads later: the stream is not drained (a step of the MNIST program waited here for its
     // whole forward pass, 0.225 -> 0.21 ms).  (float)rand() / RAND_MAX > p compares against p * 2^31: RAND_MAX as a float is 2^31, an exact scale.
@@ -728,6 +740,7 @@ int ltb_dropout(const float* x, float* y, float* mask, float p, int64_t n) {
 }
 int ltb_dropout_grad(float* dx, const float* mask, const float* dy, int64_t n) {
   LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && mask && dy && n >= 0, "ltb_dropout_grad: bad argument");
+  LTB_WRITES(dx, n);
   return launch_map<3>(dx, mask, dy, dx, n, [] __device__(float g0, float m, float d) { return g0 + m * d; });
 }
 
@@ -737,6 +750,7 @@ int ltb_concat(float* out, const float* const* inputs, const int* dims, int n_in
   LTB_INITED(); LTB_REQUIRE(out && inputs && dims && n_inputs > 0 && outer > 0 && inner > 0, "ltb_concat: bad argument");
   int64_t total = 0;
   for (int k = 0; k < n_inputs; ++k) { LTB_REQUIRE(inputs[k] && dims[k] > 0, "ltb_concat: bad input %d", k); total += dims[k]; }
+  LTB_WRITES(out, total * inner * outer);
   int64_t off = 0;
   if (n_inputs <= kPieces && total * inner * outer < (1ll << 31)) {
     float* p[kPieces]; int64_t len[kPieces];
@@ -762,6 +776,7 @@ int ltb_concat_grad(float* const* dinputs, const float* dout, const int* dims, i
   LTB_SETTLE(dout); LTB_REQUIRE(dinputs && dout && dims && n_inputs > 0 && outer > 0 && inner > 0, "ltb_concat_grad: bad argument");
   int64_t total = 0;
   for (int k = 0; k < n_inputs; ++k) { LTB_REQUIRE(dims[k] > 0, "ltb_concat_grad: bad input %d", k); total += dims[k]; }
+  for (int k = 0; k < n_inputs; ++k) LTB_WRITES(dinputs[k], (size_t)dims[k] * inner * outer);
   int64_t off = 0;
   bool distinct = true;                                       // one buffer named twice is added into piece after piece
   for (int k = 0; k < n_inputs; ++k) for (int j = 0; j < k; ++j) distinct = distinct && (!dinputs[k] || dinputs[k] != dinputs[j]);

@@ -1048,13 +1048,35 @@ namespace ltb {
 // copy in a staging block and gives it back.  With it, a copy made by a forward convolution, or of dy at the start of a
 // convolution's backward call, is kept in a block taken from the far end of the arena (those blocks live until ltb_reset)
 // and found again by address and shape: the weight-gradient of that convolution reads the forward copy of x, and data-grad
-// and weight-grad share one copy of dy.  A copy is dropped when one of the entry points that report their writes
-// (filter_cache_note_write) touches its source, when ltb_free releases the source, and at ltb_reset.
-struct ClCopy { const float* src; int n_img, chan, pix; float* cl; int geom; };   // geom 0: channels-last copy; else the key of an unfolded matrix (unfold_key)
+// and weight-grad share one copy of dy.  Only backward looks a copy up, dy's within its own call: a forward call makes its copy in any
+// case, and so does a backward call for dy, because the caller may have written the buffer by its own means.  A copy is dropped when
+// any entry point writes its source (LTB_WRITES), when ltb_free releases the source, where a recording begins or ends, and at ltb_reset.
+struct ClCopy { const float* src; size_t src_floats; int n_img, chan, pix; float* cl; int geom; };   // geom 0: channels-last copy; else the key of an unfolded matrix (unfold_key)
 static std::vector<ClCopy> cl_cache;
 void cl_cache_clear() { cl_cache.clear(); }
 void cl_cache_drop_from(const void* p) {                   // ltb_free: everything at or above p is gone
   for (size_t i = 0; i < cl_cache.size();) { if (in_arena_from(cl_cache[i].src, p)) { cl_cache[i] = cl_cache.back(); cl_cache.pop_back(); } else ++i; }
+}
+static void cl_cache_drop(const void* p, size_t bytes) {       // every copy whose source overlaps [p, p + bytes); p null: all
+  for (size_t i = 0; i < cl_cache.size();) {
+    const char* sl = (const char*)cl_cache[i].src; const char* sh = sl + cl_cache[i].src_floats * 4;
+    if (!p || ((const char*)p < sh && sl < (const char*)p + bytes)) { cl_cache[i] = cl_cache.back(); cl_cache.pop_back(); } else ++i;
+  }
+}
+// A block for a new copy of src that is to be kept (null: no room): the block of the copy it replaces where that has the same shape, so
+// that calls on the same buffers without an ltb_reset between do not use the arena up.  Every reader of the old copy runs before on
+// the same stream or has been waited for; not so in a branch region, whose two streams may read one source.
+static float* kept_block(const float* src, size_t src_floats, int n_img, int chan, int pix, int geom, size_t floats) {
+  for (size_t i = 0; i < cl_cache.size(); ++i) {
+    ClCopy& e = cl_cache[i];
+    if (e.src != src || e.geom != geom) continue;
+    if (e.n_img == n_img && e.chan == chan && e.pix == pix && !g.branch_marked) return e.cl;
+    e = cl_cache.back(); cl_cache.pop_back();
+    break;
+  }
+  float* p = (float*)step_alloc(floats * 4);
+  if (p) cl_cache.push_back(ClCopy{src, src_floats, n_img, chan, pix, p, geom});
+  return p;
 }
 static float* cl_lookup(const float* src, int n_img, int chan, int pix) {
   for (auto& e : cl_cache) if (e.src == src && e.n_img == n_img && e.chan == chan && e.pix == pix && e.geom == 0) return e.cl;
@@ -1119,12 +1141,11 @@ static int unfolded(const float* x, const ConvDims& d, const float** col, float*
   const size_t n = (size_t)d.N * ck * pix;
   *temp = nullptr; *floats = 0; *col = nullptr;
   if (g.filter_cache && !(g.tune & 4)) {
-    float* kept = unfold_lookup(x, d);
-    if (!kept && (kept = (float*)step_alloc(n * 4)) != nullptr) {
-      int rc = launch_unfold(x, kept, d); if (rc) return rc;
-      cl_cache.push_back(ClCopy{x, d.N, ck, pix, kept, unfold_key(d)});
+    if (float* kept = kept_block(x, (size_t)d.N * d.C * d.H * d.W, d.N, ck, pix, unfold_key(d), n)) {
+      *col = kept;
+      int rc = launch_unfold(x, kept, d); if (rc) cl_cache_drop(x, 1);
+      return rc;
     }
-    if (kept) { *col = kept; return LTB_OK; }
   }
   float* buf = temp_alloc(n);
   if (!buf) return LTB_OK;
@@ -1158,12 +1179,10 @@ static int channels_last(const float* src, int n_img, int chan, int pix, float**
   const size_t n = (size_t)n_img * up4(chan) * pix;
   *floats = 0; *out = nullptr;
   if (keep && g.filter_cache && !(g.tune & 4)) {
-    if (float* kept = (float*)step_alloc(n * 4)) {
-      int rc = channels_last_into(src, n_img, chan, pix, kept); if (rc) return rc;
-      for (size_t i = 0; i < cl_cache.size(); ++i) if (cl_cache[i].src == src && cl_cache[i].geom == 0) { cl_cache[i] = cl_cache.back(); cl_cache.pop_back(); break; }
-      cl_cache.push_back(ClCopy{src, n_img, chan, pix, kept, 0});
+    if (float* kept = kept_block(src, (size_t)n_img * chan * pix, n_img, chan, pix, 0, n)) {
       *out = kept;
-      return LTB_OK;
+      int rc = channels_last_into(src, n_img, chan, pix, kept); if (rc) cl_cache_drop(src, 1);
+      return rc;
     }
   }
   *out = temp_alloc(n); *floats = n;
@@ -1173,8 +1192,8 @@ static int channels_last(const float* src, int n_img, int chan, int pix, float**
 // ---- filter cache (ltb_set_filter_cache) ------------------------------------------------------------------------------------
 // The per-tap forms of a filter are needed twice per step (forward and data-grad) and change once per step (the optimizer).
 // With the cache on they live in private device memory, keyed by the filter's address and shape, and are refreshed -- all
-// stale filters together, in ONE launch -- at the first use after a write that overlaps a filter (filter_cache_note_write, called by the optimizer, transfer,
-// fill and in-place entry points with their destination; a replayed step and ltb_params_changed mark every filter).  A filter first seen while a step is being recorded takes
+// stale filters together, in ONE launch -- at the first use after a write that overlaps a filter (LTB_WRITES in every entry point that
+// writes; a replayed step and ltb_params_changed mark every filter).  A filter first seen while a step is being recorded takes
 // the uncached path (no allocation inside a capture).
 struct FilterForms { const float* w; int K, C, taps; float *fwd, *dgrad; bool stale, gone; };
 static std::vector<FilterForms> filter_cache;
@@ -1187,10 +1206,7 @@ void filter_cache_clear() {
 // recorded step may name them) until a filter of that address and shape comes again or the cache is cleared.
 void filter_cache_drop_from(const void* p) { for (auto& e : filter_cache) if (in_arena_from(e.w, p)) { e.gone = true; e.stale = true; } }
 void filter_cache_note_write(const void* p, size_t bytes) {
-  for (size_t i = 0; i < cl_cache.size();) {
-    const char* sl = (const char*)cl_cache[i].src; const char* sh = sl + (size_t)cl_cache[i].n_img * cl_cache[i].chan * cl_cache[i].pix * 4;
-    if (!p || ((const char*)p < sh && sl < (const char*)p + bytes)) { cl_cache[i] = cl_cache.back(); cl_cache.pop_back(); } else ++i;
-  }
+  cl_cache_drop(p, bytes);
   if (filter_cache.empty()) return;
   const char* lo = (const char*)p; const char* hi = lo + bytes;
   for (auto& e : filter_cache) {
@@ -1333,8 +1349,8 @@ static int conv_fwd_any(const float* x, const float* w, const float* bias, float
   TcConvAny a; TcPlan p;
   if (tc_conv_needs_rows(d.oH * d.oW) && d.C * d.R * d.S % 4) return 0;
   if (!any_geometry(d, a) || !tc_plan_conv_any_fwd(p, (const float*)g.heap, (const float*)g.heap, bias, y, a, g.sm_count)) return 0;     // eligibility with any aligned pointers
-  float *xr = cl_lookup(x, d.N, d.C, d.H * d.W), *wt = nullptr; size_t nx = 0, nw = 0;
-  int rc = xr ? LTB_OK : channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true); if (rc) return rc;
+  float *xr = nullptr, *wt = nullptr; size_t nx = 0, nw = 0;
+  int rc = channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true); if (rc) return rc;
   if (!xr) return 0;
   rc = tap_matrices(w, d, 0, &wt, &nw);
   bool ok = !rc && wt && tc_plan_conv_any_fwd(p, xr, wt, bias, y, a, g.sm_count);
@@ -1421,10 +1437,11 @@ static bool wants_im2col(const ConvDims& d) {
 // Start of a convolution's backward call, before its two halves part onto two streams: one channels-last copy of dy for both.
 int conv_bwd_prestage(const float* dy, const ConvDims& d, bool both_halves) {
   TcConvGeom gm; TcConvAny a;
-  if (!g.filter_cache || !both_halves) return LTB_OK;
   const bool window = taps_geometry(d, gm) && d.C % 64 == 0 && d.K % 32 == 0;
-  if (!window && !(wants_im2col(d) && d.sh == 1 && d.sw == 1 && any_geometry(d, a))) return LTB_OK;
-  if (cl_lookup(dy, d.N, d.K, d.oH * d.oW)) return LTB_OK;
+  if (!g.filter_cache || !both_halves || (!window && !(wants_im2col(d) && d.sh == 1 && d.sw == 1 && any_geometry(d, a)))) {
+    cl_cache_drop(dy, (size_t)d.N * d.K * d.oH * d.oW * 4);              // a copy from an earlier call is not this gradient's
+    return LTB_OK;
+  }
   float* dyr; size_t ny;
   int rc = channels_last(dy, d.N, d.K, d.oH * d.oW, &dyr, &ny, /*keep=*/true);
   if (!rc && dyr && ny) temp_free(dyr, ny);                 // no room to keep it: each half makes its own, as before

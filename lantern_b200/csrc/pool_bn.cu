@@ -677,6 +677,7 @@ int ltb_maxpool_fwd(const float* x, float* y, int32_t* idx, int N, int C, int H,
   LTB_REQUIRE((int64_t)N * C * H * W < ((int64_t)1 << 31), "ltb_maxpool_fwd: tensor too large for int32 indices");
   int oH = (H + 2 * pad - kh) / sh + 1, oW = (W + 2 * pad - kw) / sw + 1;
   int64_t n_out = (int64_t)N * C * oH * oW;
+  LTB_WRITES(y, n_out);
   if (kh == 2 && kw == 2 && sh == 2 && sw == 2 && pad == 0 && (W & 3) == 0 && (H & 1) == 0 && aligned16(x) && aligned16(y) && aligned16(idx)) {
     int64_t pairs = n_out / 2;
     LTB_LAUNCH(maxpool2x2_fwd_kernel, grid_for(pairs, 256), 256, 0, x, y, idx, pairs, H, W, oH, oW / 2);
@@ -687,6 +688,7 @@ int ltb_maxpool_fwd(const float* x, float* y, int32_t* idx, int N, int C, int H,
 }
 int ltb_maxpool_bwd(float* dx, const float* dy, const int32_t* idx, int64_t n_out) {
   LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && dy && idx && n_out >= 0, "ltb_maxpool_bwd: bad argument");
+  LTB_WRITES(dx, n_out * 4);            // its extent is not an argument: 2 x 2 windows, of larger ones the part that is sure
   if (n_out) LTB_LAUNCH(maxpool_bwd_kernel, grid_for(n_out, 256), 256, 0, dx, dy, idx, n_out);
   return LTB_OK;
 }
@@ -695,6 +697,7 @@ int ltb_avgpool_fwd(const float* x, float* y, int N, int C, int H, int W, int kh
   LTB_REQUIRE(x && y && N > 0 && C > 0 && kh >= 1 && kw >= 1 && sh >= 1 && sw >= 1 && H >= kh && W >= kw, "ltb_avgpool_fwd: bad argument");
   int oH = (H - kh) / sh + 1, oW = (W - kw) / sw + 1;
   int64_t n_out = (int64_t)N * C * oH * oW;
+  LTB_WRITES(y, n_out);
   LTB_LAUNCH(avgpool_fwd_kernel, grid_for(n_out, 256), 256, 0, x, y, n_out, H, W, oH, oW, kh, kw, sh, sw);
   return LTB_OK;
 }
@@ -703,6 +706,7 @@ int ltb_avgpool_bwd(float* dx, const float* dy, int N, int C, int H, int W, int 
   LTB_REQUIRE(dx && dy && N > 0 && C > 0 && kh >= 1 && kw >= 1 && sh >= 1 && sw >= 1 && H >= kh && W >= kw, "ltb_avgpool_bwd: bad argument");
   int oH = (H - kh) / sh + 1, oW = (W - kw) / sw + 1;
   int64_t n_in = (int64_t)N * C * H * W;
+  LTB_WRITES(dx, n_in);
   LTB_LAUNCH(avgpool_bwd_kernel, grid_for(n_in, 256), 256, 0, dx, dy, n_in, H, W, oH, oW, kh, kw, sh, sw);
   return LTB_OK;
 }
@@ -714,6 +718,7 @@ int ltb_bn_train_fwd(const float* x, float* y, const float* gamma, const float* 
   int S = bn_splits(N, C);
   LTB_REQUIRE((size_t)C * S * 2 * 4 <= g.cur_scratch_bytes(), "ltb_bn_train_fwd: too many channels");
   int64_t n = (int64_t)N * C * HW;
+  LTB_WRITES(y, n); LTB_WRITES(save_mean, C); LTB_WRITES(save_istd, C); LTB_WRITES(run_mean, C); LTB_WRITES(run_var, C);
   bool vec = (HW & 3) == 0 && aligned16(x) && aligned16(y);
   if (vec && (int64_t)N * (HW >> 2) < ((int64_t)1 << 30)) {      // one cluster launch: statistics and result in the same kernel
     Pending p;
@@ -739,6 +744,7 @@ int ltb_bn_bwd(const float* x, float* dx, const float* dy, const float* gamma, f
   LTB_REQUIRE((size_t)C * (S * 2 + 3) * 4 <= g.cur_scratch_bytes(), "ltb_bn_bwd: too many channels");
   float* coef = g.cur_scratch() + (size_t)C * S * 2;
   int64_t n = (int64_t)N * C * HW;
+  LTB_WRITES(dx, n); LTB_WRITES(dgamma, C); LTB_WRITES(dbeta, C);
   bool vec = (HW & 3) == 0 && aligned16(x) && aligned16(dy) && aligned16(dx);
   const bool cluster_path = vec && (int64_t)N * (HW >> 2) < ((int64_t)1 << 30);
   // a held in-place ReLU gradient on exactly this dy is applied by the kernel itself
@@ -789,6 +795,7 @@ int ltb_bn_bwd(const float* x, float* dx, const float* dy, const float* gamma, f
 int ltb_bn_inference(const float* x, float* y, const float* gamma, const float* beta, const float* rm, const float* rv,
                      int N, int C, int HW, float eps) {
   LTB_INITED(); LTB_REQUIRE(x && y && gamma && beta && rm && rv && N > 0 && C > 0 && HW > 0, "ltb_bn_inference: bad argument");
+  LTB_WRITES(y, (size_t)N * C * HW);
   Pending h; h.kind = PEND_BN_INF; h.n = (int64_t)N * C * HW; h.x = x; h.y = y; h.gamma = gamma; h.beta = beta;
   h.run_mean = const_cast<float*>(rm); h.run_var = const_cast<float*>(rv); h.N = N; h.C = C; h.HW = HW; h.eps = eps;
   if (g.fusion) { g.pending = h; return LTB_OK; }            // an in-place ReLU of y may join it

@@ -539,6 +539,7 @@ extern "C" {
 int ltb_rnn_seq_fwd(const float* x, const int32_t* y, const float* h0, const float* Wxh, const float* Whh, const float* bh, const float* Who,
                     const float* bo, float* h, float* logp, float* loss, int T, int B, int V, int H) {
   LTB_INITED(); LTB_REQUIRE(x && y && Wxh && Whh && bh && Who && bo && h && logp && loss && T > 0 && B > 0 && V > 0 && H > 0, "ltb_rnn_seq_fwd: bad argument");
+  LTB_WRITES(h, (size_t)T * B * H); LTB_WRITES(logp, (size_t)T * B * V); LTB_WRITES(loss, 1);
   int rows; size_t sf, sb;
   if (!seq_plan(T, B, V, H, &rows, &sf, &sb))
     return fail(LTB_E_LIMIT, "ltb_rnn_seq_fwd: the weights (vocabulary %d, hidden %d) and %d steps of one batch row do not fit one SM's shared memory", V, H, T);
@@ -560,6 +561,7 @@ int ltb_rnn_seq_fwd(const float* x, const int32_t* y, const float* h0, const flo
 int ltb_rnn_seq_bwd(const float* x, const int32_t* y, const float* h0, const float* Whh, const float* Who, const float* h, const float* logp,
                     const float* dloss, float* dWxh, float* dWhh, float* dbh, float* dWho, float* dbo, int T, int B, int V, int H) {
   LTB_INITED(); LTB_SETTLE(dloss); LTB_SETTLE(dWxh); LTB_SETTLE(dWhh); LTB_SETTLE(dbh); LTB_SETTLE(dWho); LTB_SETTLE(dbo); LTB_REQUIRE(x && y && Whh && Who && h && logp && dloss && dWxh && dWhh && dbh && dWho && dbo && T > 0 && B > 0 && V > 0 && H > 0, "ltb_rnn_seq_bwd: bad argument");
+  LTB_WRITES(dWxh, (size_t)V * H); LTB_WRITES(dWhh, (size_t)H * H); LTB_WRITES(dbh, H); LTB_WRITES(dWho, (size_t)H * V); LTB_WRITES(dbo, V);
   int rows; size_t sf, sb;
   if (!seq_plan(T, B, V, H, &rows, &sf, &sb) || seq_opted_device != g.device) return fail(LTB_E_STATE, "ltb_rnn_seq_bwd: no forward call came before");
   const int ctas = (int)ceil_div(B, rows), n_sums = 2 * V * H + H * H + H + V;
@@ -786,6 +788,7 @@ static int tree_node_check(const ltb_tree_node* n, const char* who) {
 int ltb_tree_node_fwd(const ltb_tree_node* n) {
   LTB_INITED();
   if (int rc = tree_node_check(n, "ltb_tree_node_fwd")) return rc;
+  filter_cache_note_write(nullptr, 0);                  // what it writes is a score of vectors: everything is taken as stale
   const int G = n->inner ? 5 : 3;
   LTB_LAUNCH(tree_node_fwd_kernel, (unsigned)ceil_div(G * n->hidden, kNodeWarps), kNodeThreads, 0, *n);
   return LTB_OK;
@@ -794,6 +797,7 @@ int ltb_tree_node_fwd(const ltb_tree_node* n) {
 int ltb_tree_node_bwd(const ltb_tree_node* n) {
   LTB_INITED();
   if (int rc = tree_node_check(n, "ltb_tree_node_bwd")) return rc;
+  filter_cache_note_write(nullptr, 0);
   const int G = n->inner ? 5 : 3;
   LTB_REQUIRE(n->dc && n->dh && n->dloss && n->dWhy && n->dby, "ltb_tree_node_bwd: missing gradient operand");
   for (int g = 0; g < G; ++g) {
@@ -812,6 +816,7 @@ int ltb_tree_node_bwd(const ltb_tree_node* n) {
 // call are [first, first + count).
 int ltb_tree_nodes_fwd(const ltb_tree_node* nodes_host, const ltb_tree_node* nodes_dev, int first, int count) {
   LTB_INITED(); LTB_REQUIRE(nodes_host && nodes_dev && first >= 0 && count > 0, "ltb_tree_nodes_fwd: bad argument");
+  filter_cache_note_write(nullptr, 0);
   for (int at = first; at < first + count; at += kNodesPerLaunch) {
     const int n = first + count - at < kNodesPerLaunch ? first + count - at : kNodesPerLaunch;
     int ctas = 1;
@@ -826,6 +831,7 @@ int ltb_tree_nodes_fwd(const ltb_tree_node* nodes_host, const ltb_tree_node* nod
 }
 int ltb_tree_nodes_bwd(const ltb_tree_node* nodes_host, const ltb_tree_node* nodes_dev, int first, int count) {
   LTB_INITED(); LTB_REQUIRE(nodes_host && nodes_dev && first >= 0 && count > 0, "ltb_tree_nodes_bwd: bad argument");
+  filter_cache_note_write(nullptr, 0);
   for (int at = first; at < first + count; at += kNodesPerLaunch) {
     const int n = first + count - at < kNodesPerLaunch ? first + count - at : kNodesPerLaunch;
     int ctas = 1;

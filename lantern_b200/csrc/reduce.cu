@@ -169,27 +169,27 @@ using namespace ltb;
 extern "C" {
 
 // sum / mean and their grads: TensorDslCPU.scala:1115-1124.
-int ltb_sum(const float* x, float* out, int64_t n) { LTB_INITED(); LTB_REQUIRE(x && out && n >= 0, "ltb_sum: bad argument"); return full_sum(x, out, n, 1.0f); }
-int ltb_mean(const float* x, float* out, int64_t n) { LTB_INITED(); LTB_REQUIRE(x && out && n > 0, "ltb_mean: bad argument"); return full_sum(x, out, n, 1.0f / (float)n); }
+int ltb_sum(const float* x, float* out, int64_t n) { LTB_INITED(); LTB_REQUIRE(x && out && n >= 0, "ltb_sum: bad argument"); LTB_WRITES(out, 1); return full_sum(x, out, n, 1.0f); }
+int ltb_mean(const float* x, float* out, int64_t n) { LTB_INITED(); LTB_REQUIRE(x && out && n > 0, "ltb_mean: bad argument"); LTB_WRITES(out, 1); return full_sum(x, out, n, 1.0f / (float)n); }
 int ltb_sum_grad(float* dx, const float* dout, int64_t n) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && n >= 0, "ltb_sum_grad: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && n >= 0, "ltb_sum_grad: bad argument"); LTB_WRITES(dx, n);
   if (n) LTB_LAUNCH(add_scalar_from_kernel, grid_for(n, 256), 256, 0, dx, dout, 1.0f, n);
   return LTB_OK;
 }
 int ltb_mean_grad(float* dx, const float* dout, int64_t n) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && n > 0, "ltb_mean_grad: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && n > 0, "ltb_mean_grad: bad argument"); LTB_WRITES(dx, n);
   LTB_LAUNCH(add_scalar_from_kernel, grid_for(n, 256), 256, 0, dx, dout, 1.0f / (float)n, n);
   return LTB_OK;
 }
 // sum(dim) / sum_grad(dim): TensorDslCPU.scala:1125-1164.
 int ltb_sum_dim(const float* x, float* out, int outer, int d, int inner) {
-  LTB_INITED(); LTB_REQUIRE(x && out && outer > 0 && d > 0 && inner > 0, "ltb_sum_dim: bad argument");
+  LTB_INITED(); LTB_REQUIRE(x && out && outer > 0 && d > 0 && inner > 0, "ltb_sum_dim: bad argument"); LTB_WRITES(out, (size_t)outer * inner);
   if (inner == 1) LTB_LAUNCH(sum_lastdim_kernel, (unsigned)ceil_div((int64_t)outer * 32, 256), 256, 0, x, out, outer, d);
   else LTB_LAUNCH(sum_dim_kernel, grid_for((int64_t)outer * inner, 256), 256, 0, x, out, outer, d, inner);
   return LTB_OK;
 }
 int ltb_sum_dim_grad(float* dx, const float* dout, int outer, int d, int inner) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && outer > 0 && d > 0 && inner > 0, "ltb_sum_dim_grad: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && outer > 0 && d > 0 && inner > 0, "ltb_sum_dim_grad: bad argument"); LTB_WRITES(dx, (size_t)outer * d * inner);
   LTB_LAUNCH(sum_dim_grad_kernel, grid_for((int64_t)outer * d * inner, 256), 256, 0, dx, dout, outer, d, inner);
   return LTB_OK;
 }
@@ -216,7 +216,7 @@ namespace ltb { void static_sum_forget() { for (auto& p : static_sum_ptr) p = nu
 extern "C" {
 
 int ltb_sum_static_scratch(const float* x, float* out, int64_t n) {
-  LTB_INITED(); LTB_REQUIRE(x && out && n >= 0, "ltb_sum_static_scratch: bad argument");
+  LTB_INITED(); LTB_REQUIRE(x && out && n >= 0, "ltb_sum_static_scratch: bad argument"); LTB_WRITES(out, 1);
   if (n > kStaticSumMaxN)
     return fail(LTB_E_LIMIT, "ltb_sum_static_scratch: %lld elements exceed the limit of %lld", (long long)n, (long long)kStaticSumMaxN);
   LTB_REQUIRE(g.device >= 0 && g.device < kStaticSumMaxDevices, "ltb_sum_static_scratch: device index out of range");
@@ -244,38 +244,38 @@ int ltb_sum_static_scratch(const float* x, float* out, int64_t n) {
 
 // softmax / logSoftmax and grads: TensorDslCPU.scala:783-846.
 int ltb_softmax(const float* x, float* y, int rows, int cols) {
-  LTB_INITED(); LTB_REQUIRE(x && y && rows > 0 && cols > 0, "ltb_softmax: bad argument");
+  LTB_INITED(); LTB_REQUIRE(x && y && rows > 0 && cols > 0, "ltb_softmax: bad argument"); LTB_WRITES(y, (size_t)rows * cols);
   LTB_LAUNCH(softmax_kernel<0>, (unsigned)ceil_div((int64_t)rows * 32, 256), 256, 0, x, y, rows, cols); return LTB_OK;
 }
 int ltb_log_softmax(const float* x, float* y, int rows, int cols) {
-  LTB_INITED(); LTB_REQUIRE(x && y && rows > 0 && cols > 0, "ltb_log_softmax: bad argument");
+  LTB_INITED(); LTB_REQUIRE(x && y && rows > 0 && cols > 0, "ltb_log_softmax: bad argument"); LTB_WRITES(y, (size_t)rows * cols);
   LTB_LAUNCH(softmax_kernel<1>, (unsigned)ceil_div((int64_t)rows * 32, 256), 256, 0, x, y, rows, cols); return LTB_OK;
 }
 int ltb_softmax_grad(float* dx, const float* y, const float* dy, int rows, int cols) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_softmax_grad: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_softmax_grad: bad argument"); LTB_WRITES(dx, (size_t)rows * cols);
   LTB_LAUNCH(softmax_grad_kernel<0>, (unsigned)ceil_div((int64_t)rows * 32, 256), 256, 0, dx, y, dy, rows, cols); return LTB_OK;
 }
 int ltb_log_softmax_grad(float* dx, const float* y, const float* dy, int rows, int cols) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_log_softmax_grad: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_log_softmax_grad: bad argument"); LTB_WRITES(dx, (size_t)rows * cols);
   LTB_LAUNCH(softmax_grad_kernel<1>, (unsigned)ceil_div((int64_t)rows * 32, 256), 256, 0, dx, y, dy, rows, cols); return LTB_OK;
 }
 // nllLoss / nllLoss_grad: TensorDslCPU.scala:1090-1110.
 int ltb_nll(const float* x, const int32_t* t, float* out, int rows, int cols) {
-  LTB_INITED(); LTB_REQUIRE(x && t && out && rows > 0 && cols > 0, "ltb_nll: bad argument");
+  LTB_INITED(); LTB_REQUIRE(x && t && out && rows > 0 && cols > 0, "ltb_nll: bad argument"); LTB_WRITES(out, rows);
   LTB_LAUNCH(nll_kernel, (rows + 127) / 128, 128, 0, x, t, out, rows, cols); return LTB_OK;
 }
 int ltb_nll_grad(float* dx, const float* dout, const int32_t* t, int rows, int cols) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && t && rows > 0 && cols > 0, "ltb_nll_grad: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && t && rows > 0 && cols > 0, "ltb_nll_grad: bad argument"); LTB_WRITES(dx, (size_t)rows * cols);
   LTB_LAUNCH(nll_grad_kernel, (rows + 127) / 128, 128, 0, dx, dout, t, rows, cols); return LTB_OK;
 }
 
 // vectorVectorDot / matrixVectorDot and the (1,1), (2,1) cases of dot_grad: TensorDslCPU.scala:135-206.
 int ltb_vv_dot(const float* x, const float* y, float* out, int n) {
-  LTB_INITED(); LTB_REQUIRE(x && y && out && n > 0, "ltb_vv_dot: bad argument");
+  LTB_INITED(); LTB_REQUIRE(x && y && out && n > 0, "ltb_vv_dot: bad argument"); LTB_WRITES(out, 1);
   LTB_LAUNCH(dot_kernel, 1, 1024, 0, x, y, out, n); return LTB_OK;
 }
 int ltb_vv_dot_grad(float* dx, float* dy, const float* x, const float* y, const float* dout, int n) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_SETTLE(dout); LTB_REQUIRE(x && y && dout && n > 0, "ltb_vv_dot_grad: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_SETTLE(dout); LTB_REQUIRE(x && y && dout && n > 0, "ltb_vv_dot_grad: bad argument"); LTB_WRITES(dx, n); LTB_WRITES(dy, n);
   if (dx) LTB_LAUNCH(axpy_from_scalar_kernel, grid_for(n, 256), 256, 0, dx, y, dout, n);
   if (dy) LTB_LAUNCH(axpy_from_scalar_kernel, grid_for(n, 256), 256, 0, dy, x, dout, n);
   return LTB_OK;
@@ -353,7 +353,7 @@ extern "C" {
 int ltb_lstm_cell(const float* i, const float* u, const float* fl, const float* cl, const float* fr, const float* cr,
                   const float* o, float* c, float* tc, float* h, int n) {
   LTB_INITED();
-  LTB_REQUIRE(i && u && o && c && tc && h && n > 0, "ltb_lstm_cell: bad argument");
+  LTB_REQUIRE(i && u && o && c && tc && h && n > 0, "ltb_lstm_cell: bad argument"); LTB_WRITES(c, n); LTB_WRITES(tc, n); LTB_WRITES(h, n);
   LTB_REQUIRE((fl && cl && fr && cr) || (!fl && !cl && !fr && !cr), "ltb_lstm_cell: the four child operands go together");
   LTB_LAUNCH(lstm_cell_kernel, (unsigned)ceil_div(n, 128), 128, 0, i, u, fl, cl, fr, cr, o, c, tc, h, n);
   return LTB_OK;
@@ -362,7 +362,7 @@ int ltb_lstm_cell_grad(const float* i, float* di, const float* u, float* du, con
                        const float* fr, float* dfr, const float* cr, float* dcr, const float* o, float* d_o,
                        const float* tc, const float* dc, const float* dh, int n) {
   LTB_INITED(); LTB_SETTLE(di); LTB_SETTLE(du); LTB_SETTLE(dfl); LTB_SETTLE(dcl); LTB_SETTLE(dfr); LTB_SETTLE(dcr); LTB_SETTLE(d_o); LTB_SETTLE(dc); LTB_SETTLE(dh);
-  LTB_REQUIRE(i && di && u && du && o && d_o && tc && dc && dh && n > 0, "ltb_lstm_cell_grad: bad argument");
+  LTB_REQUIRE(i && di && u && du && o && d_o && tc && dc && dh && n > 0, "ltb_lstm_cell_grad: bad argument"); LTB_WRITES(di, n); LTB_WRITES(du, n); LTB_WRITES(dfl, n); LTB_WRITES(dcl, n); LTB_WRITES(dfr, n); LTB_WRITES(dcr, n); LTB_WRITES(d_o, n);
   LTB_REQUIRE((fl && dfl && cl && dcl && fr && dfr && cr && dcr) || (!fl && !dfl && !cl && !dcl && !fr && !dfr && !cr && !dcr),
               "ltb_lstm_cell_grad: the child operands and their gradients go together");
   LTB_LAUNCH(lstm_cell_grad_kernel, (unsigned)ceil_div(n, 128), 128, 0, i, di, u, du, fl, dfl, cl, dcl, fr, dfr, cr, dcr, o, d_o, tc, dc, dh, n);
@@ -435,6 +435,7 @@ int ltb_affine_act_rows(const float* x0, const float* W0, int cols0, const float
   LTB_INITED();
   LTB_REQUIRE(x0 && W0 && bias && out && cols0 > 0 && batch > 0 && batch <= 65535 && width > 0 && (x1 == nullptr) == (W1 == nullptr) && (!W1 || cols1 > 0),
               "ltb_affine_act_rows: bad argument");
+  LTB_WRITES(out, (size_t)batch * width);
   LTB_REQUIRE(act == -1 || act == LTB_TANH || act == LTB_SIGMOID, "ltb_affine_act_rows: activation must be tanh, sigmoid or -1");
   LTB_LAUNCH(affine_act_rows_kernel, dim3((unsigned)ceil_div(width, 128), batch), 128, 0, x0, W0, cols0, x1, W1, W1 ? cols1 : 0, bias, act, out, batch, width);
   return LTB_OK;
@@ -444,6 +445,7 @@ int ltb_affine_act_rows_grad(const float* x0, float* dx0, const float* W0, float
                              int batch, int width) {
   LTB_INITED(); LTB_SETTLE(dx0); LTB_SETTLE(dW0); LTB_SETTLE(dx1); LTB_SETTLE(dW1); LTB_SETTLE(dbias); LTB_SETTLE(dout);
   LTB_REQUIRE(x0 && W0 && dW0 && dbias && out && dout && cols0 > 0 && batch > 0 && width > 0, "ltb_affine_act_rows_grad: bad argument");
+  LTB_WRITES(dx0, (size_t)batch * cols0); LTB_WRITES(dW0, (size_t)cols0 * width); LTB_WRITES(dx1, (size_t)batch * cols1); LTB_WRITES(dW1, (size_t)cols1 * width); LTB_WRITES(dbias, width);
   LTB_REQUIRE((x1 == nullptr) == (W1 == nullptr) && (W1 == nullptr) == (dW1 == nullptr) && (!W1 || cols1 > 0) && (W1 || !dx1),
               "ltb_affine_act_rows_grad: x1, W1 and dW1 go together");
   LTB_REQUIRE(act == -1 || act == LTB_TANH || act == LTB_SIGMOID, "ltb_affine_act_rows_grad: activation must be tanh, sigmoid or -1");
@@ -459,7 +461,7 @@ int ltb_affine_act_rows_grad(const float* x0, float* dx0, const float* W0, float
 int ltb_affine_act(const float* W0, const float* a, int cols0, const float* W1, const float* b, int cols1, const float* bias,
                    int act, float* out, int rows) {
   LTB_INITED();
-  LTB_REQUIRE(W0 && a && bias && out && rows > 0 && cols0 > 0 && (W1 == nullptr) == (b == nullptr) && (!W1 || cols1 > 0), "ltb_affine_act: bad argument");
+  LTB_REQUIRE(W0 && a && bias && out && rows > 0 && cols0 > 0 && (W1 == nullptr) == (b == nullptr) && (!W1 || cols1 > 0), "ltb_affine_act: bad argument"); LTB_WRITES(out, rows);
   LTB_REQUIRE(act == -1 || act == LTB_TANH || act == LTB_SIGMOID, "ltb_affine_act: activation must be tanh, sigmoid or -1");
   LTB_LAUNCH(affine_act_kernel, (unsigned)ceil_div(rows, 4), 128, 0, W0, a, cols0, W1, b, cols1, bias, act, out, rows);
   return LTB_OK;
@@ -467,22 +469,22 @@ int ltb_affine_act(const float* W0, const float* a, int cols0, const float* W1, 
 int ltb_affine_act_grad(const float* W0, float* dW0, const float* a, float* da, int cols0, const float* W1, float* dW1,
                         const float* b, float* db, int cols1, float* dbias, int act, const float* out, const float* dout, int rows) {
   LTB_INITED(); LTB_SETTLE(dW0); LTB_SETTLE(da); LTB_SETTLE(dW1); LTB_SETTLE(db); LTB_SETTLE(dbias); LTB_SETTLE(dout);
-  LTB_REQUIRE(W0 && dW0 && a && dbias && out && dout && rows > 0 && cols0 > 0, "ltb_affine_act_grad: bad argument");
+  LTB_REQUIRE(W0 && dW0 && a && dbias && out && dout && rows > 0 && cols0 > 0, "ltb_affine_act_grad: bad argument"); LTB_WRITES(dW0, (size_t)rows * cols0); LTB_WRITES(da, cols0); LTB_WRITES(dW1, (size_t)rows * cols1); LTB_WRITES(db, cols1); LTB_WRITES(dbias, rows);
   LTB_REQUIRE((W1 == nullptr) == (b == nullptr) && (W1 == nullptr) == (dW1 == nullptr) && (!W1 || cols1 > 0), "ltb_affine_act_grad: W1, dW1 and b go together");
   LTB_REQUIRE(act == -1 || act == LTB_TANH || act == LTB_SIGMOID, "ltb_affine_act_grad: activation must be tanh, sigmoid or -1");
   LTB_LAUNCH(affine_act_grad_kernel, (unsigned)ceil_div(rows, 4), 128, 0, W0, dW0, a, da, cols0, W1, dW1, b, db, cols1, dbias, act, out, dout, rows);
   return LTB_OK;
 }
 int ltb_mv_dot(const float* a, const float* x, float* out, int m, int k) {
-  LTB_INITED(); LTB_REQUIRE(a && x && out && m > 0 && k > 0, "ltb_mv_dot: bad argument");
+  LTB_INITED(); LTB_REQUIRE(a && x && out && m > 0 && k > 0, "ltb_mv_dot: bad argument"); LTB_WRITES(out, m);
   LTB_LAUNCH(gemv_rows_kernel<false>, (unsigned)ceil_div((int64_t)m * 32, 256), 256, 0, a, x, out, m, k); return LTB_OK;
 }
 int ltb_add_cartesian(float* da, const float* y, const float* dout, int m, int k) {
-  LTB_INITED(); LTB_SETTLE(da); LTB_SETTLE(dout); LTB_REQUIRE(da && y && dout && m > 0 && k > 0, "ltb_add_cartesian: bad argument");
+  LTB_INITED(); LTB_SETTLE(da); LTB_SETTLE(dout); LTB_REQUIRE(da && y && dout && m > 0 && k > 0, "ltb_add_cartesian: bad argument"); LTB_WRITES(da, (size_t)m * k);
   LTB_LAUNCH(outer_acc_kernel, grid_for((int64_t)m * k, 256), 256, 0, da, y, dout, m, k); return LTB_OK;
 }
 int ltb_add_composition(float* dx, const float* a, const float* dout, int m, int k) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && a && dout && m > 0 && k > 0, "ltb_add_composition: bad argument");
+  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && a && dout && m > 0 && k > 0, "ltb_add_composition: bad argument"); LTB_WRITES(dx, k);
   LTB_LAUNCH(gemv_cols_kernel, (k + 127) / 128, 128, 0, a, dout, dx, m, k); return LTB_OK;
 }
 

@@ -490,6 +490,67 @@ def test_which_products_run_in_tf32(gpu, M, N, K, taken):
     assert _on_the_tensor_cores(gpu.lib, lambda: gpu.lib.gemm(a.ptr, 0, b.ptr, 1, 1.0, c.ptr, M, N, K)) == bool(taken)
 
 
+def _exact(seed, shape, scale=1.0):
+    """Normal numbers of ten mantissa bits: their TF32 products are exact."""
+    a = (R(seed).standard_normal(shape) * scale).astype(np.float32)
+    return (np.ascontiguousarray(a).view(np.uint32) & np.uint32(0xFFFFE000)).view(np.float32)
+
+
+KEPT_COPY_CONVS = [(2, 64, 27, 96, 3, 1, 1), (4, 64, 16, 64, 3, 1, 1), (4, 3, 32, 64, 3, 1, 1), (4, 64, 16, 64, 3, 2, 1), (3, 64, 4, 64, 3, 1, 1), (2, 64, 7, 64, 1, 1, 0)]
+
+
+@pytest.mark.parametrize("cfg", KEPT_COPY_CONVS, ids=[str(c) for c in KEPT_COPY_CONVS])
+def test_kept_copies_follow_their_buffers(ora, gpu, cfg):
+    """With the operand cache on, copies of activations and output gradients in the engine's layout are kept.  A buffer that is written
+    again without a reset between -- by any operator, and by the caller's own means before a forward call or as the gradient of a
+    backward call -- is read again: forward, both gradients, twice each on buffers that are used over and over."""
+    N, C, H, K, Rk, s, p = cfg
+    O = (H + 2 * p - Rk) // s + 1
+    xs = [np.abs(_exact(i, (N, C, H, H))) for i in range(4)]
+    dys = [np.abs(_exact(10 + i, (N, K, O, O))) for i in range(3)]
+    w0 = _exact(20, (K, C, Rk, Rk), 1.0 / np.sqrt(C * Rk * Rk))
+    dims = (N, C, H, H, K, Rk, Rk, s, s, p, p)
+
+    def own_means(b, dst, a):                                           # what a caller's own kernel would do
+        if b is ora:
+            b.lib.h2d(dst.ptr, a.ctypes.data, a.nbytes)
+        else:
+            import ctypes
+
+            import torch  # noqa: F401
+            b.lib.sync()
+            assert ctypes.CDLL("libcudart.so.12").cudaMemcpy(ctypes.c_void_p(dst.ptr), ctypes.c_void_p(a.ctypes.data), ctypes.c_size_t(a.nbytes), 1) == 0
+
+    def f(b):
+        lib, out = b.lib, {}
+        x, dy, y, w = b.fromNumpy(xs[0]), b.fromNumpy(dys[0]), b.zeros(N, K, O, O), b.fromNumpy(w0)
+        srcs, dsrcs = [b.fromNumpy(a) for a in xs], [b.fromNumpy(a) for a in dys]
+        dx, dw = b.zeros(N, C, H, H), b.zeros(K, C, Rk, Rk)
+
+        def fwd(k):
+            lib.conv2d_fwd(x.ptr, w.ptr, 0, y.ptr, *dims); out["y%d" % k] = y.toCPU()
+
+        def bwd(k):
+            lib.fill(dx.ptr, 0.0, N * C * H * H); lib.fill(dw.ptr, 0.0, K * C * Rk * Rk)
+            lib.conv2d_bwd(x.ptr, dx.ptr, w.ptr, dw.ptr, 0, dy.ptr, *dims)
+            out["dx%d" % k], out["dw%d" % k] = dx.toCPU(), dw.toCPU()
+        fwd(0); bwd(0)
+        lib.unary(0, srcs[1].ptr, x.ptr, xs[1].size); fwd(1)            # by an operator, then forward
+        lib.unary(0, dsrcs[1].ptr, dy.ptr, dys[1].size); bwd(1)         # a new gradient in the same buffer
+        lib.unary(0, srcs[2].ptr, x.ptr, xs[2].size); bwd(2)            # by an operator, then backward (recomputed activations)
+        own_means(b, x, xs[3]); fwd(3)
+        own_means(b, dy, dys[2]); bwd(3)
+        return out
+    ref = f(ora)
+    gpu.lib.set_filter_cache(1)
+    try:
+        got = f(gpu)
+    finally:
+        gpu.lib.set_filter_cache(0)
+    for k in ref:
+        assert_close(ref[k], got[k], FP32_RTOL, k)
+
+
 def test_tensor_core_engine_reports_no_timeouts(gpu):
     assert gpu.lib.device_status() == 0
 
