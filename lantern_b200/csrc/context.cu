@@ -416,6 +416,7 @@ int ltb_graph_begin(void) {
   LTB_REQUIRE(!g.branch_marked && !g.in_branch, "ltb_graph_begin: a branch region is open (ltb_branch_join missing)");
   LTB_CUDA(cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal));
   g.capturing = true; g.capture_launch_base = g.launches;
+  filter_cache_note_write(nullptr, 0);             // the recorded step makes every copy and filter form it reads: a replay finds other contents
   return LTB_OK;
 }
 void* ltb_graph_end(void) {
@@ -423,6 +424,7 @@ void* ltb_graph_end(void) {
   if (g.pending.kind) flush_pending();             // a held operation belongs to the recorded step
   if (side_join()) { fail(LTB_E_CUDA, "ltb_graph_end: joining the side stream failed"); }
   g.capturing = false;
+  filter_cache_note_write(nullptr, 0);             // and what it makes is there only once it has been replayed
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamEndCapture(g.stream, &graph);
   if (e != cudaSuccess || !graph) { fail(LTB_E_CUDA, "ltb_graph_end: capture failed: %s", cudaGetErrorString(e)); return nullptr; }

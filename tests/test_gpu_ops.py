@@ -551,6 +551,46 @@ def test_kept_copies_follow_their_buffers(ora, gpu, cfg):
         assert_close(ref[k], got[k], FP32_RTOL, k)
 
 
+@pytest.mark.parametrize("cfg", KEPT_COPY_CONVS[:3], ids=[str(c) for c in KEPT_COPY_CONVS[:3]])
+def test_a_recording_shares_no_kept_copies_with_the_calls_around_it(ora, gpu, cfg):
+    """A recorded forward call makes the copies it reads, although an eager call before the recording left some; and an eager backward call
+    before the first replay does not read copies that only the replay will make.  The filter's forms likewise."""
+    N, C, H, K, Rk, s, p = cfg
+    O = (H + 2 * p - Rk) // s + 1
+    xs, ws = [np.abs(_exact(i, (N, C, H, H))) for i in range(2)], [_exact(20 + i, (K, C, Rk, Rk), 1.0 / np.sqrt(C * Rk * Rk)) for i in range(2)]
+    dy0 = _exact(10, (N, K, O, O))
+    dims = (N, C, H, H, K, Rk, Rk, s, s, p, p)
+
+    def f(b):
+        lib, out = b.lib, {}
+        x, dy, y, w = b.fromNumpy(xs[0]), b.fromNumpy(dy0), b.zeros(N, K, O, O), b.fromNumpy(ws[0])
+        dx, dw = b.zeros(N, C, H, H), b.zeros(K, C, Rk, Rk)
+        lib.conv2d_fwd(x.ptr, w.ptr, 0, y.ptr, *dims)
+        graph = None
+        if b is gpu:
+            lib.graph_begin(); lib.conv2d_fwd(x.ptr, w.ptr, 0, y.ptr, *dims); graph = lib.graph_end()
+        lib.conv2d_bwd(x.ptr, dx.ptr, w.ptr, dw.ptr, 0, dy.ptr, *dims)
+        out["dx"], out["dw"] = dx.toCPU(), dw.toCPU()
+        lib.h2d(x.ptr, xs[1].ctypes.data, xs[1].nbytes); lib.h2d(w.ptr, ws[1].ctypes.data, ws[1].nbytes)
+        lib.fill(y.ptr, 0.0, N * K * O * O)
+        if b is gpu:
+            lib.graph_launch(graph)
+        else:
+            lib.conv2d_fwd(x.ptr, w.ptr, 0, y.ptr, *dims)
+        out["y"] = y.toCPU()
+        if graph:
+            lib.graph_destroy(graph)
+        return out
+    ref = f(ora)
+    gpu.lib.set_filter_cache(1)
+    try:
+        got = f(gpu)
+    finally:
+        gpu.lib.set_filter_cache(0)
+    for k in ref:
+        assert_close(ref[k], got[k], FP32_RTOL, k)
+
+
 def test_tensor_core_engine_reports_no_timeouts(gpu):
     assert gpu.lib.device_status() == 0
 
