@@ -6,17 +6,20 @@
 // (TensorDslCudnn.scala:515-831).  Semantics follow TensorDslCPU.scala:379-472 (gemm) and 484-692 (conv).
 //
 // One kernel template: C[m,n] (op)= sum_k A(m,k) * B(k,n), both operands given by tables, so that the convolution variants never
-// materialise the reference's `finput` (im2col) buffer: element (r, k) is p[row(r).off + kk(k).off], or zero where
-// row(r).h + kk(k).h leaves [0, H) or the same for w.  A table entry costs the divisions once per row or once per k, not per element
-// (computed per element they made the data-gradient of SqueezeNet's layers 5 TFLOP/s kernels).
+// materialise the reference's `finput` (im2col) buffer: element (r, k) is p[row(r).off + kk(k).off], or zero where the bits of kk(k) are
+// not all among those of row(r) (a tap outside the image).  A table entry costs the divisions once per row or once per k, not per element
+// (computed per element they made the data-gradient of SqueezeNet's layers 5 TFLOP/s kernels); the bit test and 32-bit offsets, and 16-byte loads
+// where four neighbours lie together, took the contractions of SqueezeNet's step at batch 64 from 1586 to 1448 us, entries made before the
+// kernel waits for its predecessors to 1420.
 //   tiles      : BM x BN outputs, 16 of k per step, 256 threads with (BM/16) x (BN/16) outputs each; the next step's operands travel to
 //                registers while this one is computed, shared memory is double-buffered, one barrier per step.  (Element-wise
 //                cp.async with three steps under way was slower: 41 against 48 TFLOP/s.)
 //   arithmetic : packed pairs (fma.rn.f32x2): half the issue slots of scalar FMAs, which leaves room for the shared-memory loads.
 //   output     : m is the index that is contiguous in memory (the caller swaps the operands for row-major results), so a thread's
 //                four consecutive m leave as one 16-byte store or vector reduction.
-// Bound: the FP32 pipes (128 FMA per SM and cycle, 74 TFLOP/s at 1.97 GHz); 50 TFLOP/s on
-// 4096 x 4096 x 2048 (the scalar 64 x 64 kernel before: 30); all contractions of SqueezeNet's step at batch 64 6.1 -> 1.5 ms.
+// Bound: the FP32 pipes (128 FMA per SM and cycle, 74 TFLOP/s at 1.97 GHz) and, for an 8 x 8 tile of a thread as much, the 32 floats per cycle that
+// shared memory delivers (four FMAs per float loaded); 55 TFLOP/s on 4096 x 4096 x 2048 with k contiguous, 51 without.  The 3x3 layers
+// that conv3x3_direct_kernel below takes make six FMAs per float.
 #include <cooperative_groups.h>
 
 #include "gemm.cuh"
@@ -26,8 +29,22 @@ namespace cg = cooperative_groups;
 namespace ltb {
 
 constexpr int BKK = 16;
-struct Ent { long long off; int h, w; };
+// Narrow entries: element (r, k) is p[row.off + kk.off] where every bit of kk.bits is set in row.bits.  A convolution's row has a bit for
+// each kh and each kw that stays inside the image (R + S <= 30 of them), its k the two of its tap; bit 31 says that the entry exists.
+// Wide entries are for operands of 2^31 elements or more and for larger filters.
+struct Ent { int off; unsigned bits; };
+struct WideEnt { long long off; int h, w; };
+constexpr unsigned kExists = 1u << 31, kNowhere = 1u << 30;  // no row has kNowhere
 constexpr int kOutside = -(1 << 28);                        // an h that no partner brings back into range
+__device__ __forceinline__ void outside_row(Ent& e) { e.off = 0; e.bits = 0; }
+__device__ __forceinline__ void outside_row(WideEnt& e) { e.off = 0; e.h = kOutside; e.w = 0; }
+__device__ __forceinline__ void outside_k(Ent& e) { e.off = 0; e.bits = kNowhere; }
+__device__ __forceinline__ void outside_k(WideEnt& e) { e.off = 0; e.h = kOutside; e.w = 0; }
+__device__ __forceinline__ bool meets(const Ent& r, const Ent& k) { return (r.bits & k.bits) == k.bits; }
+__device__ __forceinline__ bool meets(const WideEnt& r, const WideEnt& k) { return r.h + k.h == 0; }       // entries without a place in an image
+template <class E> __device__ __forceinline__ E plain_entry(long long off);
+template <> __device__ __forceinline__ Ent plain_entry<Ent>(long long off) { return Ent{(int)off, kExists}; }
+template <> __device__ __forceinline__ WideEnt plain_entry<WideEnt>(long long off) { return WideEnt{off, 0, 0}; }
 
 __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
   unsigned long long d;
@@ -46,27 +63,67 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
 }
 
 constexpr int kTables = 4;
-// One operand's share of a step: T rows x BKK, fetched to registers, then stored.  KFAST: k is contiguous in memory (a thread keeps
-// its k), else the row is (it keeps its row).
-template <int T, bool KFAST, class OP>
+// How an operand's elements are fetched.  FEED_ROW: single elements, neighbouring threads on neighbouring rows (a thread keeps its row);
+// FEED_K: neighbouring threads on neighbouring k (a thread keeps its k).  _4: four neighbours at a time with one 16-byte load, where
+// groups of four along the contiguous index are aligned and lie inside together.
+enum { FEED_ROW = 0, FEED_K = 1, FEED_ROW4 = 2, FEED_K4 = 3 };
+// One operand's share of a step: T rows x BKK, fetched to registers, then stored k by k.
+template <int T, int FEED, class OP>
 struct Feed {
-  static constexpr int E = T * BKK / 256, P = T + 4;
-  float v[E];
-  __device__ __forceinline__ void fetch(const OP& op, const Ent& mine, const Ent* rows, const Ent* ks, int tid) {
-    if (KFAST) {
-      const Ent k = ks[tid & 15];
+  using E = typename OP::Entry;
+  static constexpr int P = T + 4;
+  static constexpr int N = FEED >= FEED_ROW4 ? (T * BKK / 4 + 255) / 256 : T * BKK / 256;
+  static constexpr bool whole = T * BKK / 4 >= 256;             // 16-byte items: fewer than threads for 32-row tiles
+  float v[FEED >= FEED_ROW4 ? 4 * N : N];
+  __device__ __forceinline__ void fetch(const OP& op, const E& mine, const E* rows, const E* ks, int tid) {
+    if constexpr (FEED == FEED_K) {
+      const E k = ks[tid & 15];
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = op.get(rows[(tid >> 4) + 16 * e], k);
+      for (int e = 0; e < N; ++e) v[e] = op.get(rows[(tid >> 4) + 16 * e], k);
+    } else if constexpr (FEED == FEED_ROW) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) v[e] = op.get(mine, ks[tid / T + (256 / T) * e]);
+    } else if constexpr (FEED == FEED_ROW4) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        const int k = tid / (T / 4) + (1024 / T) * e;
+        const float4 t = whole || k < BKK ? op.get4(mine, ks[whole ? k : k & 15]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[4 * e] = t.x; v[4 * e + 1] = t.y; v[4 * e + 2] = t.z; v[4 * e + 3] = t.w;
+      }
     } else {
+      const E k = ks[(tid & 3) * 4];
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = op.get(mine, ks[tid / T + (256 / T) * e]);
+      for (int e = 0; e < N; ++e) {
+        const int r = (tid >> 2) + 64 * e;
+        const float4 t = whole || r < T ? op.get4(rows[whole ? r : r & (T - 1)], k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[4 * e] = t.x; v[4 * e + 1] = t.y; v[4 * e + 2] = t.z; v[4 * e + 3] = t.w;
+      }
     }
   }
+  // the row that a thread keeps (its first of four)
+  static __device__ __forceinline__ int my_row(int tid) { return FEED == FEED_ROW4 ? tid % (T / 4) * 4 : tid % T; }
+  static constexpr bool table = FEED == FEED_K || FEED == FEED_K4;
   __device__ __forceinline__ void store(float* s, int tid) const {
+    if constexpr (FEED == FEED_ROW4) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int r = KFAST ? (tid >> 4) + 16 * e : tid % T, k = KFAST ? (tid & 15) : tid / T + (256 / T) * e;
-      s[k * P + r] = v[e];
+      for (int e = 0; e < N; ++e) {
+        const int k = tid / (T / 4) + (1024 / T) * e;
+        if (whole || k < BKK) *reinterpret_cast<float4*>(s + k * P + tid % (T / 4) * 4) = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+      }
+    } else if constexpr (FEED == FEED_K4) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        const int r = (tid >> 2) + 64 * e;
+        if (whole || r < T)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s[((tid & 3) * 4 + i) * P + r] = v[4 * e + i];
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        const int r = FEED == FEED_K ? (tid >> 4) + 16 * e : tid % T, k = FEED == FEED_K ? (tid & 15) : tid / T + (256 / T) * e;
+        s[k * P + r] = v[e];
+      }
     }
   }
 };
@@ -75,30 +132,33 @@ template <int BM, int BN> constexpr int igemm_smem() {
   constexpr int operands = 2 * BKK * (BM + BN + 8) * 4, partial = BM * BN * 4;       // a split's partial tile takes the operands' place
   return operands > partial ? operands : partial;
 }
-template <int BM, int BN, bool AK, bool BK, class OA, class OB, class ST>
+template <int BM, int BN, int AF, int BF, class OA, class OB, class ST>
 __global__ void __launch_bounds__(256, 2) igemm_kernel(int M, int N, int K, int k_per_split, const OA oa, const OB ob, const ST st) {
-  pdl_enter();
+  pdl_launch();
   constexpr int PA = BM + 4, PB = BN + 4, TM = BM / 16, TN = BN / 16;
   extern __shared__ __align__(16) float pool[];
-  __shared__ Ent ka[kTables][BKK], kb[kTables][BKK];
-  __shared__ Ent ra[AK ? BM : 1], rb[BK ? BN : 1];
+  using EA = typename OA::Entry; using EB = typename OB::Entry;
+  using FA = Feed<BM, AF, OA>; using FB = Feed<BN, BF, OB>;
+  __shared__ EA ka[kTables][BKK]; __shared__ EB kb[kTables][BKK];
+  __shared__ EA ra[FA::table ? BM : 1]; __shared__ EB rb[FB::table ? BN : 1];
   const int tid = threadIdx.x;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int k_begin = blockIdx.z * k_per_split, k_end = min(K, k_begin + k_per_split);
   const int steps = k_end > k_begin ? (k_end - k_begin + BKK - 1) / BKK : 0;          // the last splits may have nothing: they contribute zeros
-  const Ent outside{0, kOutside, 0};
-  auto a_row = [&](int r) { return m0 + r < M ? oa.row(m0 + r) : outside; };
-  auto b_row = [&](int r) { return n0 + r < N ? ob.row(n0 + r) : outside; };
+  auto a_row = [&](int r) { EA e; if (m0 + r < M) e = oa.row(m0 + r); else outside_row(e); return e; };
+  auto b_row = [&](int r) { EB e; if (n0 + r < N) e = ob.row(n0 + r); else outside_row(e); return e; };
   auto table = [&](int step, int i, bool second) {
     const int k = k_begin + step * BKK + i;
-    if (second) kb[step & (kTables - 1)][i] = k < k_end ? ob.kk(k) : outside; else ka[step & (kTables - 1)][i] = k < k_end ? oa.kk(k) : outside;
+    if (second) { EB e; if (k < k_end) e = ob.kk(k); else outside_k(e); kb[step & (kTables - 1)][i] = e; }
+    else { EA e; if (k < k_end) e = oa.kk(k); else outside_k(e); ka[step & (kTables - 1)][i] = e; }
   };
-  Ent mine_a = outside, mine_b = outside;
-  if (AK) { for (int r = tid; r < BM; r += 256) ra[r] = a_row(r); } else mine_a = a_row(tid % BM);
-  if (BK) { for (int r = tid; r < BN; r += 256) rb[r] = b_row(r); } else mine_b = b_row(tid % BN);
+  EA mine_a; EB mine_b;
+  if (FA::table) { for (int r = tid; r < BM; r += 256) ra[r] = a_row(r); } else mine_a = a_row(FA::my_row(tid));
+  if (FB::table) { for (int r = tid; r < BN; r += 256) rb[r] = b_row(r); } else mine_b = b_row(FB::my_row(tid));
   if (tid < 4 * BKK) table(tid % (2 * BKK) / BKK, tid % BKK, tid >= 2 * BKK);            // steps 0 and 1
   __syncthreads();
-  Feed<BM, AK, OA> fa; Feed<BN, BK, OB> fb;
+  pdl_wait();                                               // the entries touch no memory: they are made while the kernels before run
+  FA fa; FB fb;
   auto fetch = [&](int step) {
     fa.fetch(oa, mine_a, ra, ka[step & (kTables - 1)], tid);
     fb.fetch(ob, mine_b, rb, kb[step & (kTables - 1)], tid);
@@ -177,67 +237,135 @@ __global__ void __launch_bounds__(256, 2) igemm_kernel(int M, int N, int K, int 
 }
 
 // ---- operands ------------------------------------------------------------------------------------------------------------------
-struct MatOp {                                              // a strided matrix
+__device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+template <class E>
+struct MatOpOf {                                            // a strided matrix
+  using Entry = E;
   const float* p; long long sr, sk;
-  __device__ __forceinline__ Ent row(int r) const { return Ent{r * sr, 0, 0}; }
-  __device__ __forceinline__ Ent kk(int k) const { return Ent{k * sk, 0, 0}; }
-  __device__ __forceinline__ float get(const Ent& r, const Ent& k) const { return r.h + k.h == 0 ? p[r.off + k.off] : 0.0f; }
+  __device__ __forceinline__ E row(int r) const { return plain_entry<E>(r * sr); }
+  __device__ __forceinline__ E kk(int k) const { return plain_entry<E>(k * sk); }
+  __device__ __forceinline__ float get(const E& r, const E& k) const { return meets(r, k) ? __ldg(p + (r.off + k.off)) : 0.0f; }
+  __device__ __forceinline__ float4 get4(const E& r, const E& k) const { return meets(r, k) ? load4(p + (r.off + k.off)) : make_float4(0.f, 0.f, 0.f, 0.f); }
 };
+using MatOp = MatOpOf<Ent>; using WideMatOp = MatOpOf<WideEnt>;
 // Output pixel (n, ho, wo) and tap (ci, kh, kw) of a convolution input.  PIXROW: the pixel is the row index (forward), else k (weight-gradient).
+// The entry of whichever is the row carries a bit for each kh and kw (of the pixel: those inside the image; of the tap: its own), the
+// other's is matched against it; in the weight gradient the roles of the two bit sets are exchanged: see meets().
 template <bool PIXROW>
 struct ConvInput {
+  using Entry = Ent;
   const float* x; ConvDims d; FastDiv oW, oH, S, R;
   ConvInput(const float* x_, const ConvDims& d_) : x(x_), d(d_), oW(d_.oW), oH(d_.oH), S(d_.S), R(d_.R) {}
-  __device__ __forceinline__ Ent pixel(int m) const {
+  // inside: the kh and kw that lie inside for this pixel
+  __device__ __forceinline__ int pixel(int m, unsigned& inside) const {
     int wo, ho; const int n = oH.divmod(oW.divmod(m, wo), ho), h = ho * d.sh - d.ph, w = wo * d.sw - d.pw;
-    return Ent{(long long)n * d.C * d.H * d.W + (long long)h * d.W + w, h, w};
+    inside = 0;
+    for (int i = 0; i < d.R; ++i) if ((unsigned)(h + i) < (unsigned)d.H) inside |= 1u << i;
+    for (int i = 0; i < d.S; ++i) if ((unsigned)(w + i) < (unsigned)d.W) inside |= 1u << (d.R + i);
+    return (n * d.C * d.H + h) * d.W + w;
   }
-  __device__ __forceinline__ Ent tap(int k) const {
+  __device__ __forceinline__ int tap(int k, unsigned& own) const {
     int kw, kh; const int ci = R.divmod(S.divmod(k, kw), kh);
-    return Ent{((long long)ci * d.H + kh) * d.W + kw, kh, kw};
+    own = (1u << kh) | (1u << (d.R + kw));
+    return (ci * d.H + kh) * d.W + kw;
   }
-  __device__ __forceinline__ Ent row(int r) const { return PIXROW ? pixel(r) : tap(r); }
-  __device__ __forceinline__ Ent kk(int k) const { return PIXROW ? tap(k) : pixel(k); }
-  __device__ __forceinline__ float get(const Ent& r, const Ent& k) const {
+  // own bits of the tap must be among the pixel's inside bits: with the tap as the row, the complements change sides
+  __device__ __forceinline__ unsigned all() const { return (1u << (d.R + d.S)) - 1u; }
+  __device__ __forceinline__ Ent row(int r) const {
+    unsigned b; int off;
+    if (PIXROW) off = pixel(r, b); else { off = tap(r, b); b = all() & ~b; }
+    return Ent{off, b | kExists};
+  }
+  __device__ __forceinline__ Ent kk(int k) const {
+    unsigned b; int off;
+    if (PIXROW) off = tap(k, b); else { off = pixel(k, b); b = all() & ~b; }
+    return Ent{off, b | kExists};
+  }
+  __device__ __forceinline__ float get(const Ent& r, const Ent& k) const { return meets(r, k) ? __ldg(x + (r.off + k.off)) : 0.0f; }
+  __device__ __forceinline__ float4 get4(const Ent& r, const Ent& k) const { return meets(r, k) ? load4(x + (r.off + k.off)) : make_float4(0.f, 0.f, 0.f, 0.f); }
+};
+template <bool PIXROW>
+struct WideConvInput {
+  using Entry = WideEnt;
+  const float* x; ConvDims d; FastDiv oW, oH, S, R;
+  WideConvInput(const float* x_, const ConvDims& d_) : x(x_), d(d_), oW(d_.oW), oH(d_.oH), S(d_.S), R(d_.R) {}
+  __device__ __forceinline__ WideEnt pixel(int m) const {
+    int wo, ho; const int n = oH.divmod(oW.divmod(m, wo), ho), h = ho * d.sh - d.ph, w = wo * d.sw - d.pw;
+    return WideEnt{(long long)n * d.C * d.H * d.W + (long long)h * d.W + w, h, w};
+  }
+  __device__ __forceinline__ WideEnt tap(int k) const {
+    int kw, kh; const int ci = R.divmod(S.divmod(k, kw), kh);
+    return WideEnt{((long long)ci * d.H + kh) * d.W + kw, kh, kw};
+  }
+  __device__ __forceinline__ WideEnt row(int r) const { return PIXROW ? pixel(r) : tap(r); }
+  __device__ __forceinline__ WideEnt kk(int k) const { return PIXROW ? tap(k) : pixel(k); }
+  __device__ __forceinline__ float get(const WideEnt& r, const WideEnt& k) const {
     return (unsigned)(r.h + k.h) < (unsigned)d.H && (unsigned)(r.w + k.w) < (unsigned)d.W ? x[r.off + k.off] : 0.0f;
   }
+  __device__ __forceinline__ float4 get4(const WideEnt&, const WideEnt&) const { return make_float4(0.f, 0.f, 0.f, 0.f); }
 };
-// Input pixel (n, h, w) against (co, kh, kw) of dy: the element at ((h + ph - kh) / sh, (w + pw - kw) / sw) where that exists.
-template <bool STRIDED>
+// Input pixel (n, h, w) against (co, kh, kw) of dy: the element at ((h + ph - kh) / sh, (w + pw - kw) / sw) where that exists.  Where it does,
+// h + ph and kh leave the same remainder, so the quotient is the difference of the two quotients and the offset still a sum.
 struct ConvDy {
-  const float* dy; ConvDims d; FastDiv W, H, S, R;
-  ConvDy(const float* dy_, const ConvDims& d_) : dy(dy_), d(d_), W(d_.W), H(d_.H), S(d_.S), R(d_.R) {}
+  using Entry = Ent;
+  const float* dy; ConvDims d; FastDiv W, H, S, R, sh, sw;
+  ConvDy(const float* dy_, const ConvDims& d_) : dy(dy_), d(d_), W(d_.W), H(d_.H), S(d_.S), R(d_.R), sh(d_.sh), sw(d_.sw) {}
   __device__ __forceinline__ Ent row(int m) const {
-    int w, h; const int n = H.divmod(W.divmod(m, w), h); w += d.pw; h += d.ph;
-    return Ent{(long long)n * d.K * d.oH * d.oW + (STRIDED ? 0 : (long long)h * d.oW + w), h, w};
+    int w, h, rh, rw; const int n = H.divmod(W.divmod(m, w), h);
+    const int qh = sh.divmod(h + d.ph, rh), qw = sw.divmod(w + d.pw, rw);
+    unsigned b = kExists;
+    for (int i = rh, q = qh; i < d.R; i += d.sh, --q) if ((unsigned)q < (unsigned)d.oH) b |= 1u << i;
+    for (int i = rw, q = qw; i < d.S; i += d.sw, --q) if ((unsigned)q < (unsigned)d.oW) b |= 1u << (d.R + i);
+    return Ent{(n * d.K * d.oH + qh) * d.oW + qw, b};
   }
   __device__ __forceinline__ Ent kk(int k) const {
     int kw, kh; const int co = R.divmod(S.divmod(k, kw), kh);
-    return Ent{(long long)co * d.oH * d.oW - (STRIDED ? 0 : (long long)kh * d.oW + kw), -kh, -kw};
+    return Ent{(co * d.oH - sh.div(kh)) * d.oW - sw.div(kw), kExists | (1u << kh) | (1u << (d.R + kw))};
   }
-  __device__ __forceinline__ float get(const Ent& r, const Ent& k) const {
-    int h = r.h + k.h, w = r.w + k.w;
-    if (!STRIDED) return (unsigned)h < (unsigned)d.oH && (unsigned)w < (unsigned)d.oW ? dy[r.off + k.off] : 0.0f;
+  __device__ __forceinline__ float get(const Ent& r, const Ent& k) const { return meets(r, k) ? __ldg(dy + (r.off + k.off)) : 0.0f; }
+  __device__ __forceinline__ float4 get4(const Ent& r, const Ent& k) const { return meets(r, k) ? load4(dy + (r.off + k.off)) : make_float4(0.f, 0.f, 0.f, 0.f); }
+};
+struct WideConvDy {
+  using Entry = WideEnt;
+  const float* dy; ConvDims d; FastDiv W, H, S, R;
+  WideConvDy(const float* dy_, const ConvDims& d_) : dy(dy_), d(d_), W(d_.W), H(d_.H), S(d_.S), R(d_.R) {}
+  __device__ __forceinline__ WideEnt row(int m) const {
+    int w, h; const int n = H.divmod(W.divmod(m, w), h);
+    return WideEnt{(long long)n * d.K * d.oH * d.oW, h + d.ph, w + d.pw};
+  }
+  __device__ __forceinline__ WideEnt kk(int k) const {
+    int kw, kh; const int co = R.divmod(S.divmod(k, kw), kh);
+    return WideEnt{(long long)co * d.oH * d.oW, -kh, -kw};
+  }
+  __device__ __forceinline__ float get(const WideEnt& r, const WideEnt& k) const {
+    const int h = r.h + k.h, w = r.w + k.w;
     if (h < 0 || w < 0) return 0.0f;
     const int ho = h / d.sh, wo = w / d.sw;
     return ho * d.sh == h && wo * d.sw == w && ho < d.oH && wo < d.oW ? dy[r.off + k.off + (long long)ho * d.oW + wo] : 0.0f;
   }
+  __device__ __forceinline__ float4 get4(const WideEnt&, const WideEnt&) const { return make_float4(0.f, 0.f, 0.f, 0.f); }
 };
 // Filter w[co][ci][tap] with row ci and k = (co, tap).
+template <class E>
 struct FilterByInput {
+  using Entry = E;
   const float* w; int C, rs; FastDiv by;
   FilterByInput(const float* w_, int C_, int rs_) : w(w_), C(C_), rs(rs_), by(rs_) {}
-  __device__ __forceinline__ Ent row(int ci) const { return Ent{(long long)ci * rs, 0, 0}; }
-  __device__ __forceinline__ Ent kk(int k) const { const int co = by.div(k); return Ent{(long long)co * C * rs + (k - co * rs), 0, 0}; }
-  __device__ __forceinline__ float get(const Ent& r, const Ent& k) const { return r.h + k.h == 0 ? w[r.off + k.off] : 0.0f; }
+  __device__ __forceinline__ E row(int ci) const { return plain_entry<E>((long long)ci * rs); }
+  __device__ __forceinline__ E kk(int k) const { const int co = by.div(k); return plain_entry<E>((long long)co * C * rs + (k - co * rs)); }
+  __device__ __forceinline__ float get(const E& r, const E& k) const { return meets(r, k) ? __ldg(w + (r.off + k.off)) : 0.0f; }
+  __device__ __forceinline__ float4 get4(const E& r, const E& k) const { return meets(r, k) ? load4(w + (r.off + k.off)) : make_float4(0.f, 0.f, 0.f, 0.f); }
 };
 // dy[n][co][pixel] with row co and k = (n, pixel).
+template <class E>
 struct DyByPixel {
+  using Entry = E;
   const float* dy; int K, hw; FastDiv by;
   DyByPixel(const float* dy_, int K_, int hw_) : dy(dy_), K(K_), hw(hw_), by(hw_) {}
-  __device__ __forceinline__ Ent row(int co) const { return Ent{(long long)co * hw, 0, 0}; }
-  __device__ __forceinline__ Ent kk(int k) const { const int n = by.div(k); return Ent{(long long)n * K * hw + (k - n * hw), 0, 0}; }
-  __device__ __forceinline__ float get(const Ent& r, const Ent& k) const { return r.h + k.h == 0 ? dy[r.off + k.off] : 0.0f; }
+  __device__ __forceinline__ E row(int co) const { return plain_entry<E>((long long)co * hw); }
+  __device__ __forceinline__ E kk(int k) const { const int n = by.div(k); return plain_entry<E>((long long)n * K * hw + (k - n * hw)); }
+  __device__ __forceinline__ float get(const E& r, const E& k) const { return meets(r, k) ? __ldg(dy + (r.off + k.off)) : 0.0f; }
+  __device__ __forceinline__ float4 get4(const E& r, const E& k) const { return meets(r, k) ? load4(dy + (r.off + k.off)) : make_float4(0.f, 0.f, 0.f, 0.f); }
 };
 
 // ---- results: four consecutive m of column n, of which `left` exist -------------------------------------------------------------
@@ -301,7 +429,7 @@ static Tiling choose_tiling(int M, int N, int K, bool may_add_atomically) {
   t.groups = (int)ceil_div(K, (int64_t)t.kps * t.cz);                     // only clusters that have work
   return t;
 }
-template <bool AK, bool BK, class OA, class OB, class ST>
+template <int AF, int BF, class OA, class OB, class ST>
 static int launch_igemm(const char* label, const Tiling& t, int M, int N, int K, const OA& oa, const OB& ob, const ST& st) {
   const dim3 grid((unsigned)ceil_div(M, t.bm), (unsigned)ceil_div(N, t.bn), (unsigned)(t.cz * t.groups));
   auto go = [&](auto igemm, int smem, bool& ready) -> int {
@@ -312,7 +440,7 @@ static int launch_igemm(const char* label, const Tiling& t, int M, int N, int K,
     return LTB_OK;
   };
   static bool ready[5];
-#define LTB_TILE(BM, BN, I) go(igemm_kernel<BM, BN, AK, BK, OA, OB, ST>, igemm_smem<BM, BN>(), ready[I])
+#define LTB_TILE(BM, BN, I) go(igemm_kernel<BM, BN, AF, BF, OA, OB, ST>, igemm_smem<BM, BN>(), ready[I])
   if (t.bm == 128) return t.bn == 128 ? LTB_TILE(128, 128, 0) : t.bn == 64 ? LTB_TILE(128, 64, 1) : LTB_TILE(128, 32, 2);
   return t.bn == 64 ? LTB_TILE(64, 64, 3) : LTB_TILE(64, 32, 4);
 #undef LTB_TILE
@@ -462,16 +590,31 @@ static int strided_gemm(const float* a, int64_t sam, int64_t sak, const float* b
   { bool taken = false; int rc = skinny_gemm(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate, &taken); if (rc || taken) return rc; }
   // m of the kernel is the contiguous index of C
   const bool swap = scn == 1 && scm != 1;
-  const MatOp oa = swap ? MatOp{b, sbn, sbk} : MatOp{a, sam, sak}, ob = swap ? MatOp{a, sam, sak} : MatOp{b, sbn, sbk};
   const int m = swap ? N : M, n = swap ? M : N;
   const long long sm = swap ? scn : scm, sn = swap ? scm : scn;
+  const float* pa = swap ? b : a; const float* pb = swap ? a : b;
+  const int64_t ar = swap ? sbn : sam, ak = swap ? sbk : sak, br = swap ? sam : sbn, bk = swap ? sak : sbk;
   const Tiling t = choose_tiling(m, n, K, !g.deterministic && accumulate);
   const MatPut st{c, sm, sn, alpha, t.groups > 1 ? 2 : accumulate ? 1 : 0, sm == 1 && sn % 4 == 0 && aligned16(c)};
-  const bool ak = oa.sk == 1 && oa.sr != 1, bk = ob.sk == 1 && ob.sr != 1;
-  if (ak && bk) return launch_igemm<true, true>("igemm[gemm]", t, m, n, K, oa, ob, st);
-  if (ak) return launch_igemm<true, false>("igemm[gemm]", t, m, n, K, oa, ob, st);
-  if (bk) return launch_igemm<false, true>("igemm[gemm]", t, m, n, K, oa, ob, st);
-  return launch_igemm<false, false>("igemm[gemm]", t, m, n, K, oa, ob, st);
+  const int64_t most = ((int64_t)1 << 31) - 1;
+  if (m * ar + K * ak > most || n * br + K * bk > most) {
+    const WideMatOp oa{pa, ar, ak}, ob{pb, br, bk};
+    if (ak == 1 && ar != 1) return bk == 1 && br != 1 ? launch_igemm<FEED_K, FEED_K>("igemm[gemm]", t, m, n, K, oa, ob, st) : launch_igemm<FEED_K, FEED_ROW>("igemm[gemm]", t, m, n, K, oa, ob, st);
+    return bk == 1 && br != 1 ? launch_igemm<FEED_ROW, FEED_K>("igemm[gemm]", t, m, n, K, oa, ob, st) : launch_igemm<FEED_ROW, FEED_ROW>("igemm[gemm]", t, m, n, K, oa, ob, st);
+  }
+  const MatOp oa{pa, ar, ak}, ob{pb, br, bk};
+  // four at a time along the contiguous index, which must then end on a multiple of four (k also where a split begins, a multiple of 16)
+  auto feed = [&](const float* p, int64_t sr, int64_t sk, int rows) {
+    if (sk == 1 && sr != 1) return sr % 4 == 0 && K % 4 == 0 && aligned16(p) ? FEED_K4 : FEED_K;
+    return sr == 1 && sk % 4 == 0 && rows % 4 == 0 && aligned16(p) ? FEED_ROW4 : FEED_ROW;
+  };
+  int fa = feed(pa, ar, ak, m), fb = feed(pb, br, bk, n);
+  if (fa < FEED_ROW4 || fb < FEED_ROW4) { fa &= FEED_K; fb &= FEED_K; }          // both or neither: half as many kernels
+#define LTB_FEEDS(A, B) if (fa == A && fb == B) return launch_igemm<A, B>("igemm[gemm]", t, m, n, K, oa, ob, st)
+  LTB_FEEDS(FEED_K4, FEED_K4); LTB_FEEDS(FEED_K4, FEED_ROW4); LTB_FEEDS(FEED_ROW4, FEED_K4); LTB_FEEDS(FEED_ROW4, FEED_ROW4);
+  LTB_FEEDS(FEED_K, FEED_K); LTB_FEEDS(FEED_K, FEED_ROW); LTB_FEEDS(FEED_ROW, FEED_K); LTB_FEEDS(FEED_ROW, FEED_ROW);
+#undef LTB_FEEDS
+  return fail(LTB_E_STATE, "igemm: no such feed");
 }
 
 // dbias[co] += sum over n, ho, wo of dy (TensorDslCPU.scala:607-617); MASK: dy is the gradient of a ReLU that ran in place and is
@@ -525,29 +668,251 @@ __global__ void __launch_bounds__(256) conv_bias_grad_kernel(float* dy, const fl
   }
 }
 
+// ---- 3x3, stride 1, padding 1 on maps of 4, 8, 16 or 32 columns: direct -----------------------------------------------------------
+// Forward (FLIP false): out[n][o][p] = sum over (i, r, s) of w[o][i][r][s] in[n][i][p + (r-1, s-1)].  Data gradient (FLIP true): in = dy, out = dx and
+// w[i][o][2-r][2-s], added to what out holds.  A warp owns 32 runs of PX neighbouring pixels (a lane each) times 8 output channels; the CTA's NW warps
+// share the input tile and have 8 channels each.  For one input channel and filter row a lane loads PX + 2 pixels and three times eight
+// weights (the same for the whole warp) and makes 24 PX products of them, so that the FP32 pipes and not the loads are the limit; the
+// matrix form above loads every element of the unfolded operand on its own.  Packed pairs run along the output channel.
+//   shared memory : rows of in with four zeros in front (the left edge of a row and the right edge of the one before), W + 4 floats an odd
+//                   multiple of four so that lanes on neighbouring rows meet no bank twice; weights [channel][tap][output channel].  Double-buffered,
+//                   the next 8 channels arrive by cp.async.
+//   splits        : input channels are dealt to a cluster of up to 8 CTAs, whose tiles are summed in rank order, as in igemm_kernel.
+struct DirectGeo { int N, Ci, Co, H, W; int rows, imgs, rs, ci_per; const float* bias; int relu; FastDiv by_q, by_line, by_ch, by_seg, by_rows, by_group; };
+// Asynchronous copies into shared memory; zeros (and nothing read) where ok is false.
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+constexpr int kDirectCh = 8;                                // input channels per step
+template <int PX, int NW> int direct_smem(int tile) {      // tile: floats of one input channel
+  const int steps = 2 * kDirectCh * (tile + 9 * (NW * 8 + 4)), partial = 32 * PX * NW * 8;
+  return (steps > partial ? steps : partial) * 4;
+}
+template <int PX, int NW, bool FLIP>
+__global__ void __launch_bounds__(NW * 32) conv3x3_direct_kernel(const float* __restrict__ in, const float* __restrict__ w, float* out, const DirectGeo G) {
+  pdl_launch();
+  constexpr int T = NW * 32, KT = NW * 8, KP = KT + 4;       // pitch of the weights: the copies below meet a bank four times at most
+  extern __shared__ __align__(16) float pool[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int hw = G.H * G.W, img_tile = (G.rows + 2) * G.rs, tile = G.imgs * img_tile + 4;    // four more: the right edge of the last row
+  // the group's first image and row, and the lane's own place in it; lanes of neighbouring rows first (see above)
+  int h0, row, r_all;
+  const int n0 = G.by_group.divmod(blockIdx.x, h0) * G.imgs, seg = G.by_seg.divmod(lane, r_all), img = G.by_rows.divmod(r_all, row);
+  h0 *= G.rows;
+  const int o0 = blockIdx.y * KT, c_begin = blockIdx.z * G.ci_per, c_end = min(G.Ci, c_begin + G.ci_per);
+  const int steps = c_end > c_begin ? (c_end - c_begin + kDirectCh - 1) / kDirectCh : 0;
+  float* const buf[2] = {pool, pool + kDirectCh * (tile + 9 * KP)};
+
+  // input rows as 16-byte items: (channel, image, row, quarter), W / 4 quarters; the zeros around them are written once
+  const int q = G.W / 4, per_ch = G.imgs * (G.rows + 2) * q, items = kDirectCh * per_ch;
+  constexpr int kItems = ((PX == 8 ? 640 : 384) + T - 1) / T;      // items of a thread: 4 to 32 columns make 576 or 640 with runs of eight, 320 or 384 with four
+  constexpr int kWeights = kDirectCh * 9 * KT / T;          // 18
+  int src[kItems], dst[kItems];                             // within a channel block; src -1: outside the image, dst -1: no item
+#pragma unroll
+  for (int e = 0; e < kItems; ++e) {
+    const int i = tid + e * T;
+    src[e] = -1; dst[e] = -1;
+    if (i < items) {
+      int j, c4, y;
+      const int c = G.by_ch.divmod(i, j), line = G.by_q.divmod(j, c4), im = G.by_line.divmod(line, y), h = h0 + y - 1;
+      c4 *= 4;
+      dst[e] = c * tile + im * img_tile + y * G.rs + 4 + c4;
+      if ((unsigned)h < (unsigned)G.H && n0 + im < G.N) src[e] = ((im * G.Ci + c) * G.H + h) * G.W + c4;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    for (int i = tid; i < kDirectCh * tile / 4; i += T) reinterpret_cast<float4*>(buf[u])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();                                          // the zeros are down
+  pdl_wait();
+  auto fetch = [&](int step) {
+    float* b = buf[step & 1];
+    const int c0 = c_begin + step * kDirectCh, live = c_end - c0;
+    const float* base = in + ((long long)n0 * G.Ci + c0) * hw;
+#pragma unroll
+    for (int e = 0; e < kItems; ++e)
+      if (dst[e] >= 0) { const bool ok = src[e] >= 0 && tid + e * T < live * per_ch; copy16(b + dst[e], base + (ok ? src[e] : 0), ok); }
+    // weights in the order of memory: (channel, tap) of one output channel after the other, FLIP: (output channel, tap) of one channel after the other
+    float* wb = b + kDirectCh * tile;
+#pragma unroll
+    for (int e = 0; e < kWeights; ++e) {
+      const int i = tid + e * T, a = i / (FLIP ? KT * 9 : kDirectCh * 9), j = i - a * (FLIP ? KT * 9 : kDirectCh * 9), u = j / 9, t = j - u * 9;
+      const int c = FLIP ? a : u, o = FLIP ? u : a;
+      const bool ok = c < live && o0 + o < G.Co;
+      const float* from = FLIP ? w + ((long long)(c0 + c) * G.Co + o0) * 9 + j : w + ((long long)(o0 + o) * G.Ci + c0) * 9 + j;
+      copy4(wb + (c * 9 + (FLIP ? 8 - t : t)) * KP + o, ok ? from : w, ok);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned long long acc[PX][4];
+#pragma unroll
+  for (int p = 0; p < PX; ++p)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[p][j] = 0ull;
+  if (steps > 0) fetch(0);
+  const int at = img * img_tile + row * G.rs + seg * PX + 3;      // the pixel left of the lane's first, one row up
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                        // step s is down for everybody, and everybody is done with step s - 1
+    if (s + 1 < steps) fetch(s + 1);
+    const float* xb = buf[s & 1] + at; const float* wb = buf[s & 1] + kDirectCh * tile + warp * 8;
+#pragma unroll 1
+    for (int c = 0; c < kDirectCh; ++c) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        float x[PX + 2];
+        const float* xr = xb + c * tile + r * G.rs;
+        x[0] = xr[0]; x[PX + 1] = xr[PX + 1];
+#pragma unroll
+        for (int p = 0; p < PX; p += 4) *reinterpret_cast<float4*>(x + 1 + p) = *reinterpret_cast<const float4*>(xr + 1 + p);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+          const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(wb + (c * 9 + r * 3 + t) * KP), wc = *reinterpret_cast<const ulonglong2*>(wb + (c * 9 + r * 3 + t) * KP + 4);
+#pragma unroll
+          for (int p = 0; p < PX; ++p) {
+            const unsigned long long xx = pack2(x[p + t], x[p + t]);
+            acc[p][0] = fma2(wa.x, xx, acc[p][0]); acc[p][1] = fma2(wa.y, xx, acc[p][1]);
+            acc[p][2] = fma2(wc.x, xx, acc[p][2]); acc[p][3] = fma2(wc.y, xx, acc[p][3]);
+          }
+        }
+      }
+    }
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cz = (int)cluster.num_blocks();
+  // eight channels of PX neighbouring pixels leave as 16-byte stores
+  auto emit = [&](int o, int lane_img, int lane_row, int lane_seg, float4 v, int part) {
+    if (n0 + lane_img >= G.N || o >= G.Co) return;
+    float4* dst4 = reinterpret_cast<float4*>(out + ((long long)(n0 + lane_img) * G.Co + o) * hw + (h0 + lane_row) * G.W + lane_seg * PX) + part;
+    if (FLIP) { const float4 old = *dst4; v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w; }
+    else {
+      const float b = G.bias ? G.bias[o] : 0.0f;
+      v.x += b; v.y += b; v.z += b; v.w += b;
+      if (G.relu) { v.x = v.x < 0.0f ? 0.0f : v.x; v.y = v.y < 0.0f ? 0.0f : v.y; v.z = v.z < 0.0f ? 0.0f : v.z; v.w = v.w < 0.0f ? 0.0f : v.w; }
+    }
+    *dst4 = v;
+  };
+  if (cz > 1) __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int p = 0; p < PX; p += 4) {
+      const float2 a = unpack2(acc[p][j]), b = unpack2(acc[p + 1][j]), c = unpack2(acc[p + 2][j]), d = unpack2(acc[p + 3][j]);
+      const float4 lo = make_float4(a.x, b.x, c.x, d.x), hi = make_float4(a.y, b.y, c.y, d.y);
+      const int o = warp * 8 + 2 * j;
+      if (cz > 1) {                                         // [output channel][part][lane]: the sum below runs along the lanes
+        float4* t = reinterpret_cast<float4*>(pool) + (o * (PX / 4) + p / 4) * 32 + lane;
+        t[0] = lo; t[(PX / 4) * 32] = hi;
+      } else { emit(o0 + o, img, row, seg, lo, p / 4); emit(o0 + o + 1, img, row, seg, hi, p / 4); }
+    }
+  if (cz > 1) {
+    cluster.sync();
+    const int rank = (int)cluster.block_rank(), all = KT * (PX / 4) * 32, per = all / cz / 32 * 32 + (all / cz % 32 ? 32 : 0);
+    for (int i = rank * per + tid; i < min(all, (rank + 1) * per); i += T) {
+      float4 p[8];
+#pragma unroll
+      for (int z = 0; z < 8; ++z) if (z < cz) p[z] = reinterpret_cast<const float4*>(cluster.map_shared_rank(pool, z))[i];
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int z = 0; z < 8; ++z) if (z < cz) { v.x += p[z].x; v.y += p[z].y; v.z += p[z].z; v.w += p[z].w; }
+      const int part = (i >> 5) % (PX / 4), o = (i >> 5) / (PX / 4);
+      emit(o0 + o, img, row, seg, v, part);                 // T is a multiple of 32: item i belongs to this thread's lane
+    }
+    cluster.sync();
+  }
+}
+template <int PX, int NW, bool FLIP>
+static int launch_direct(const float* in, const float* w, float* out, DirectGeo& G, int warps, const char* label) {
+  const int segs = G.W / PX, lines = 32 / segs;             // rows of a group
+  G.rows = lines < G.H ? lines : G.H; G.imgs = lines / G.rows;
+  G.rs = G.W + 4; if (G.rs % 8 == 0) G.rs += 4;
+  G.by_q = FastDiv(G.W / 4); G.by_line = FastDiv(G.rows + 2); G.by_ch = FastDiv(G.imgs * (G.rows + 2) * (G.W / 4));
+  G.by_seg = FastDiv(32 / segs); G.by_rows = FastDiv(G.rows); G.by_group = FastDiv(G.H / G.rows);
+  const int groups = (int)ceil_div(G.N, G.imgs) * (G.H / G.rows);
+  const int tiles = groups * (int)ceil_div(G.Co, NW * 8);
+  // CTAs share the input channels until every SM has `warps` warps; small problems of more than 32 channels also until a chain is 144 products
+  // long (the matrix form's in such cases: 64 -> 256 on 8 x 8 at batch 64 is 1.9e-7 off in both, 2.6e-7 with chains of 288)
+  int cz = 1;
+  while (cz < 8 && G.Ci >= kDirectCh * (cz + 1) && (tiles * cz * NW < warps * g.sm_count || (G.Ci > 32 && G.Ci > 16 * cz && tiles * NW < 12 * g.sm_count))) ++cz;
+  G.ci_per = (int)ceil_div(ceil_div(G.Ci, cz), kDirectCh) * kDirectCh;
+  cz = (int)ceil_div(G.Ci, G.ci_per);
+  const int smem = direct_smem<PX, NW>(G.imgs * (G.rows + 2) * G.rs + 4);
+  static int most = 0;
+  if (smem > most) { LTB_CUDA(cudaFuncSetAttribute((conv3x3_direct_kernel<PX, NW, FLIP>), cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); most = smem; }
+  g.label = label;
+  LTB_LAUNCH_CLUSTER_Z((conv3x3_direct_kernel<PX, NW, FLIP>), dim3((unsigned)groups, (unsigned)ceil_div(G.Co, NW * 8), (unsigned)cz), NW * 32, cz, smem, in, w, out, G);
+  g.label = nullptr;
+  return LTB_OK;
+}
+// Few channels into many: runs of eight pixels and 32 output channels per CTA, split until an SM has six warps (a split's sum costs what it
+// saves beyond that).  Many into few: the sums are long and the outputs few, so runs of four and 16 output channels, split until an SM has
+// sixteen warps.  Swept on SqueezeNet's layers at batch 64 (us, 16 -> 64 and 32 -> 128 on 16 x 16, 48 -> 192 and 64 -> 256 on 8 x 8): the first rule
+// 14, 31, 29, 34 forward and 25, 45, 36, 55 in the data gradient, the second 17, 39, 29, 43 and 14, 38, 30, 38.
+template <bool FLIP>
+static int conv_direct(const float* in, const float* w, float* out, DirectGeo& G, const char* label) {
+  if (G.Ci <= G.Co && G.W >= 8 && G.H >= 8) return launch_direct<8, 4, FLIP>(in, w, out, G, 6, label);
+  return launch_direct<4, 2, FLIP>(in, w, out, G, G.Ci <= G.Co ? 6 : 16, label);
+}
+// 3x3, stride 1, padding 1 on maps of 4 to 32 rows and columns (powers of two: whole groups of 32 runs), 16-byte aligned tensors, at least a step of
+// channels on both sides.
+static bool direct_takes(const ConvDims& d, const float* a, const float* b) {
+  if (d.R != 3 || d.S != 3 || d.sh != 1 || d.sw != 1 || d.ph != 1 || d.pw != 1 || !aligned16(a) || !aligned16(b)) return false;
+  if (d.W != 4 && d.W != 8 && d.W != 16 && d.W != 32) return false;
+  if (d.C < 8 || d.K < 8) return false;
+  return d.H <= 32 && (d.H & (d.H - 1)) == 0 && d.H >= 4 && (int64_t)d.C * d.H * d.W * 32 < (1ll << 31) && (int64_t)d.K * d.H * d.W * 32 < (1ll << 31);
+}
+
 // ---- convolution as implicit GEMM -----------------------------------------------------------------------------
+// Whether narrow entries hold this convolution, and whether its pixels are plain runs (1x1, stride 1, no padding, whole groups of four).
+static bool narrow(const ConvDims& d) {
+  const int64_t most = ((int64_t)1 << 31) - 1 - (int64_t)(d.R + d.ph) * (d.W + d.oW) - d.S - d.pw;      // an entry's own offset may lie a filter or the padding outside
+  return d.R + d.S <= 30 && (int64_t)d.N * d.C * d.H * d.W <= most && (int64_t)d.N * d.K * d.oH * d.oW <= most && (int64_t)d.K * d.C * d.R * d.S <= most;
+}
+static bool plain_pixels(const ConvDims& d) { return d.R == 1 && d.S == 1 && d.sh == 1 && d.sw == 1 && d.ph == 0 && d.pw == 0 && d.H * d.W % 4 == 0; }
 int conv_fwd_fp32(const float* x, const float* w, const float* bias, float* y, const ConvDims& d, bool relu) {
   const int hw = d.oH * d.oW, M = d.N * hw, Kd = d.C * d.R * d.S;
+  if (direct_takes(d, x, y)) {
+    DirectGeo G{d.N, d.C, d.K, d.H, d.W, 0, 0, 0, 0, bias, relu ? 1 : 0};
+    return conv_direct<false>(x, w, y, G, "direct[conv_fwd]");
+  }
   const Tiling t = choose_tiling(M, d.K, Kd, false);
   const PixelPut st(y, bias, d.K, hw, 0, relu);
-  return launch_igemm<false, true>("igemm[conv_fwd]", t, M, d.K, Kd, ConvInput<true>(x, d), MatOp{w, Kd, 1}, st);
+  if (!narrow(d)) return launch_igemm<FEED_ROW, FEED_K>("igemm[conv_fwd]", t, M, d.K, Kd, WideConvInput<true>(x, d), WideMatOp{w, Kd, 1}, st);
+  const ConvInput<true> in(x, d); const MatOp fw{w, Kd, 1};
+  const bool w4 = Kd % 4 == 0 && aligned16(w);
+  if (w4 && plain_pixels(d) && aligned16(x)) return launch_igemm<FEED_ROW4, FEED_K4>("igemm[conv_fwd]", t, M, d.K, Kd, in, fw, st);
+  if (w4) return launch_igemm<FEED_ROW, FEED_K4>("igemm[conv_fwd]", t, M, d.K, Kd, in, fw, st);
+  return launch_igemm<FEED_ROW, FEED_K>("igemm[conv_fwd]", t, M, d.K, Kd, in, fw, st);
 }
 int conv_dgrad_fp32(const float* dy, const float* w, float* dx, const ConvDims& d) {
   const int hw = d.H * d.W, M = d.N * hw, rs = d.R * d.S, Kd = d.K * rs;
+  if (direct_takes(d, dy, dx)) {
+    DirectGeo G{d.N, d.K, d.C, d.H, d.W, 0, 0, 0, 0, nullptr, 0};
+    return conv_direct<true>(dy, w, dx, G, "direct[conv_dgrad]");
+  }
   const Tiling t = choose_tiling(M, d.C, Kd, false);
   const PixelPut st(dx, nullptr, d.C, hw, 1, false);
-  const FilterByInput fw(w, d.C, rs);
-  if (d.sh == 1 && d.sw == 1) {
-    if (rs > 1) return launch_igemm<false, true>("igemm[conv_dgrad]", t, M, d.C, Kd, ConvDy<false>(dy, d), fw, st);
-    return launch_igemm<false, false>("igemm[conv_dgrad]", t, M, d.C, Kd, ConvDy<false>(dy, d), fw, st);
-  }
-  return launch_igemm<false, true>("igemm[conv_dgrad]", t, M, d.C, Kd, ConvDy<true>(dy, d), fw, st);
+  if (!narrow(d)) return launch_igemm<FEED_ROW, FEED_K>("igemm[conv_dgrad]", t, M, d.C, Kd, WideConvDy(dy, d), FilterByInput<WideEnt>(w, d.C, rs), st);
+  const FilterByInput<Ent> fw(w, d.C, rs);
+  const ConvDy in(dy, d);
+  if (rs > 1) return launch_igemm<FEED_ROW, FEED_K>("igemm[conv_dgrad]", t, M, d.C, Kd, in, fw, st);
+  const bool w4 = d.C % 4 == 0 && aligned16(w);
+  if (w4 && plain_pixels(d) && aligned16(dy)) return launch_igemm<FEED_ROW4, FEED_ROW4>("igemm[conv_dgrad]", t, M, d.C, Kd, in, fw, st);
+  return launch_igemm<FEED_ROW, FEED_ROW>("igemm[conv_dgrad]", t, M, d.C, Kd, in, fw, st);
 }
 int conv_wgrad_fp32(const float* x, const float* dy, float* dw, const ConvDims& d) {
   const int M = d.C * d.R * d.S, hw = d.oH * d.oW, Kd = d.N * hw;       // dw[co][(ci, kh, kw)]: the filter element is the contiguous index
   const Tiling t = choose_tiling(M, d.K, Kd, !g.deterministic);
   const MatPut st{dw, 1, M, 1.0f, t.groups > 1 ? 2 : 1, M % 4 == 0 && aligned16(dw)};
-  return launch_igemm<true, true>("igemm[conv_wgrad]", t, M, d.K, Kd, ConvInput<false>(x, d), DyByPixel(dy, d.K, hw), st);
+  if (!narrow(d)) return launch_igemm<FEED_K, FEED_K>("igemm[conv_wgrad]", t, M, d.K, Kd, WideConvInput<false>(x, d), DyByPixel<WideEnt>(dy, d.K, hw), st);
+  const ConvInput<false> in(x, d); const DyByPixel<Ent> g4(dy, d.K, hw);
+  const bool d4 = hw % 4 == 0 && aligned16(dy);
+  if (d4 && plain_pixels(d) && aligned16(x)) return launch_igemm<FEED_K4, FEED_K4>("igemm[conv_wgrad]", t, M, d.K, Kd, in, g4, st);
+  if (d4) return launch_igemm<FEED_K, FEED_K4>("igemm[conv_wgrad]", t, M, d.K, Kd, in, g4, st);
+  return launch_igemm<FEED_K, FEED_K>("igemm[conv_wgrad]", t, M, d.K, Kd, in, g4, st);
 }
 int conv_bias_grad(float* dy, const float* relu_y, float* dbias, const ConvDims& d) {
   const int hw = d.oH * d.oW;

@@ -140,6 +140,30 @@ def test_conv_fwd_bwd_fp32(ora, gpu, cfg):
     check(f, ora, gpu)
 
 
+# (N, C, H, W, K, R, S, stride, pad): the direct 3x3 form at the edges of its groups of images, rows, channels and splits; operands fed four at a
+# time and one by one; strides; filters whose rows and columns do not fit a table entry's bits.
+FP32_FORMS = [(1, 8, 4, 4, 8, 3, 3, 1, 1), (9, 13, 4, 4, 70, 3, 3, 1, 1), (3, 40, 8, 8, 33, 3, 3, 1, 1), (5, 17, 16, 16, 9, 3, 3, 1, 1), (2, 9, 32, 32, 34, 3, 3, 1, 1),
+              (2, 64, 8, 16, 16, 3, 3, 1, 1), (3, 16, 32, 4, 48, 3, 3, 1, 1), (2, 24, 4, 32, 40, 3, 3, 1, 1), (2, 70, 16, 8, 100, 3, 3, 1, 1),
+              (3, 20, 6, 6, 36, 1, 1, 1, 0), (3, 18, 5, 5, 34, 1, 1, 1, 0), (4, 10, 12, 9, 12, 3, 5, 3, 2), (2, 6, 11, 13, 8, 4, 3, 2, 3), (1, 2, 16, 17, 5, 15, 15, 1, 2), (2, 3, 20, 18, 5, 17, 16, 2, 4)]
+
+
+@pytest.mark.parametrize("cfg", FP32_FORMS, ids=[str(c) for c in FP32_FORMS])
+def test_conv_forms_fp32(ora, gpu, cfg):
+    n, c, h, w, k, r, s, st, p = cfg
+    x, f, bias = R(1).standard_normal((n, c, h, w)).astype(np.float32), R(2).standard_normal((k, c, r, s)).astype(np.float32), R(3).standard_normal(k).astype(np.float32)
+
+    def run(b):
+        b.lib.set_math(0)
+        X, F, B = TensorR(b.fromNumpy(x)), TensorR(b.fromNumpy(f)), TensorR(b.fromNumpy(bias))
+        y, _, _ = b.conv2D_batch(X.x, F.x, B.x, (st, st), (p, p))
+        dy = b.fromNumpy(R(4).standard_normal(y.shape).astype(np.float32))
+        for _ in range(2):                               # the second call adds to what the first left
+            b.conv2D_batch_grad(X, None, F, TensorR(y, dy), B, (p, p), (st, st))
+        b.lib.set_math(1)
+        return {"y": y.toCPU(), "dx": X.d.toCPU(), "dw": F.d.toCPU(), "db": B.d.toCPU()}
+    check(run, ora, gpu)
+
+
 @pytest.mark.parametrize("cfg", [(2, 3, 8, 8, 2, 2, 0), (2, 3, 9, 7, 3, 2, 1), (4, 16, 32, 32, 2, 2, 0), (1, 1, 3, 3, 2, 1, 0), (3, 5, 6, 10, 2, 2, 0)])
 def test_maxpool_indices_bit_exact(ora, gpu, cfg):
     N, C, H, W, k, s, pad = cfg
