@@ -66,8 +66,7 @@ struct TcParams {
   int cluster_z;               // splits whose partial results are summed inside the kernel: a thread-block cluster of this many CTAs along z
   long long pix_per_img, img_stride, chan_stride, ld;
   FastDiv by_pix;              // by the tile rows of an image (pix_pad)
-  int col_mod, col_mul;        // row-major epilogue: D column n goes to column (n % col_mod) * col_mul + n / col_mod when col_mul != 0
-                               // TC_EPI_TAPS: col_mod channels in blocks of 32, col_mul taps
+  int col_mod, col_mul;        // TC_EPI_TAPS: col_mod channels in blocks of 32, col_mul taps
   // Gather mode (gather_src != null): the A operand is not loaded by TMA but collected by the epilogue warps, which are idle
   // during the main loop, straight from an activation tensor src[img][chan][pix] with pix = 4 or 16 (images too small for a
   // 128-byte run of pixels), transposing it on the way into the K-major rows the tensor core reads.
@@ -192,6 +191,11 @@ struct BoxLane {
     if (GEN && load == TC_LOAD_BOXES) {
       c[0] += 32 * d; offset += 4096u * d; bytes = 4096u;
       if (c[0] >= o.dim0) active = false;
+    } else if (GEN && load == TC_LOAD_TAPS) {
+      const int q = n_tile * o.nbox + d, blk = q / o.im.taps, tap = q - blk * o.im.taps, r = tap / o.im.tap_s;
+      c[1] += tap - r * o.im.tap_s; c[2] += r; c[4] = blk;
+      offset += 4096u * d; bytes = 4096u;
+      if (blk >= o.im.ch_blocks) active = false;
     } else if (GEN && load == TC_LOAD_IM2COL) start(o.im, (long long)m_tile * 128);
     else if (GEN && load == TC_LOAD_IM2COL_MN) {
       const int q = n_tile * o.nbox + d, blk = q / o.im.taps, tap = q - blk * o.im.taps;
@@ -222,7 +226,7 @@ struct BoxLane {
       }
     } else {
       const CUtensorMap* const map = lane & 8 ? map_b : map_a;
-      if (load <= TC_LOAD_BOXES) { if (active) tma_load(map, bar, stage + offset, rank, c); }
+      if (load != TC_LOAD_IM2COL && load != TC_LOAD_IM2COL_MN) { if (active) tma_load(map, bar, stage + offset, rank, c); }
       else if (active) tma_im2col(map, bar, stage + offset, c[0], o.im.low_w + pi * o.im.step_w, o.im.low_h + pj * o.im.step_h, pn, c[1], c[2]);
     }
     if (GEN && load == TC_LOAD_IM2COL_MN) {
@@ -280,7 +284,7 @@ __device__ __forceinline__ long long out_column(const TcParams& P, int n) {
     const int q = n >> 5, blk = q / P.col_mul, c = blk * 32 + (n & 31);
     return c < P.col_mod ? (long long)c * P.col_mul + (q - blk * P.col_mul) : -1;
   }
-  return P.col_mul ? (long long)(n % P.col_mod) * P.col_mul + n / P.col_mod : n;
+  return n;
 }
 
 // EPI (TcEpilogue) and MODE (0 store, 1 accumulate, 2 atomic accumulate) are compile-time: each launch then carries one
@@ -538,13 +542,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const int e = i * 32 + lane, ch = e & (nch - 1), c = e >> shift, n = n_tile * P.bn + ch * 32 + c;
           const long long col = n < P.N ? out_column<EPI>(P, n) : -1;
           if (col < 0) continue;
-          const float* src = tile + ch * kTapChunk + c;
+          const float* src = tile + ch * kTapChunk + c + half * 16 * kTapPitch;
           float* p = P.out + (m0 + half * 16) * P.ld + col;
-#pragma unroll 8
-          for (int r = half * 16; r < r_end; ++r) {
+          const int rows = r_end - half * 16;
+          float old[16];
+          if (MODE == 1)                          // all loads first: added one after the other these take 25 us where everything else takes 11
+#pragma unroll
+            for (int r = 0; r < 16; ++r) old[r] = r < rows ? p[r * P.ld] : 0.0f;
+#pragma unroll
+          for (int r = 0; r < 16; ++r) {
+            if (r >= rows) break;
             const float v = P.alpha * src[r * kTapPitch];
-            if (MODE == 2) atomicAdd(p, v); else if (MODE == 1) *p += v; else *p = v;
-            p += P.ld;
+            if (MODE == 2) atomicAdd(p + r * P.ld, v); else p[r * P.ld] = MODE == 1 ? old[r] + v : v;
           }
         }
       }
@@ -730,18 +739,18 @@ __global__ void permute_taps_kernel(const float* __restrict__ w, float* __restri
     out[i] = a < inner ? w[((int64_t)k * C + c) * taps + t] : 0.0f;
   }
 }
-// Both per-tap forms, fwd[tap][k][c] and dgrad[tap][c][k], of several filters in one launch (every filter the optimizer has
-// just written: one launch per step instead of one per 3x3 layer).  A CTA takes a tile of 32 output channels x 32 input
-// channels x all taps of one filter through shared memory: the 32 x (32 taps) floats of a tile are contiguous runs of w, and
-// both forms leave as runs of 32 consecutive floats (read element by element, w's stride of `taps` floats between
-// neighbouring channels made this copy of 45 MB take 137 us).  Jobs are laid end to end over the tile index.
-struct FormJob { const float* w; float* fwd; float* dgrad; int K, C, taps; int begin; };    // begin: first tile of this job
+// The per-tap matrices of several filters w[k][c][tap] in one launch (every filter the optimizer has just written: one launch per step
+// instead of one per layer): form[tap][k][c], and form_c[tap][c][k] where the data-gradient wants that too (C no multiple of 32).  A CTA takes a tile
+// of 32 output channels x 32 input channels x all taps of one filter through shared memory, runs of 32 consecutive floats on both sides.
+// 3x3 filters of whole channel blocks move 16 bytes at a time with nine loads of a thread in flight.  Bound by memory (ResNet-50: 45 MB each way);
+// 65 us with one load in flight and both forms.  Jobs are laid end to end over the tile index.
+struct FormJob { const float* w; float *form, *form_c; int K, C, taps; int begin; };    // begin: first tile of this job
 constexpr int kFormJobs = 24;
 struct FormJobs { FormJob j[kFormJobs]; int n; int total; };
-constexpr int kFormTaps = 9;                                   // filters with more taps go element by element inside their tile
+constexpr int kFormTaps = 9, kFormRow = 32 * kFormTaps;        // filters with more taps go element by element inside their tile
 __global__ void __launch_bounds__(256) filter_forms_multi_kernel(const FormJobs J) {
   pdl_enter();
-  __shared__ float tile[32][32 * kFormTaps + 1];
+  __shared__ float tile[32][kFormRow + 1];
   int q = 0;
   while (q + 1 < J.n && (int)blockIdx.x >= J.j[q + 1].begin) ++q;
   const FormJob& f = J.j[q];
@@ -749,12 +758,34 @@ __global__ void __launch_bounds__(256) filter_forms_multi_kernel(const FormJobs 
   const int ctiles = (C + 31) / 32, id = (int)blockIdx.x - f.begin;
   const int k0 = (id / ctiles) * 32, c0 = (id % ctiles) * 32;
   const int kn = min(32, K - k0), cn = min(32, C - c0);
+  if (taps == kFormTaps && !f.form_c) {
+    float4 v[kFormTaps];
+#pragma unroll
+    for (int e = 0; e < kFormTaps; ++e) {                      // 32 rows of 72 items over 256 threads
+      const int i = threadIdx.x + e * 256, kk = i / (kFormRow / 4), r = i - kk * (kFormRow / 4);
+      v[e] = kk < kn ? __ldg(reinterpret_cast<const float4*>(f.w + ((long long)(k0 + kk) * C + c0) * kFormTaps) + r) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int e = 0; e < kFormTaps; ++e) {
+      const int i = threadIdx.x + e * 256, kk = i / (kFormRow / 4), r = (i - kk * (kFormRow / 4)) * 4;
+      tile[kk][r] = v[e].x; tile[kk][r + 1] = v[e].y; tile[kk][r + 2] = v[e].z; tile[kk][r + 3] = v[e].w;
+    }
+    __syncthreads();
+    const int kk = threadIdx.x >> 3, c = (threadIdx.x & 7) * 4;
+    if (kk < kn)
+#pragma unroll
+      for (int e = 0; e < kFormTaps; ++e) {                    // tap e: 32 rows of 8 items
+        const float* t = tile[kk] + c * kFormTaps + e;
+        *reinterpret_cast<float4*>(f.form + ((long long)e * K + k0 + kk) * C + c0 + c) = make_float4(t[0], t[kFormTaps], t[2 * kFormTaps], t[3 * kFormTaps]);
+      }
+    return;
+  }
   if (taps > kFormTaps) {
     for (int i = threadIdx.x; i < kn * cn * taps; i += 256) {
       const int t = i % taps, cc = (i / taps) % cn, kk = i / (taps * cn);
       const float v = f.w[((long long)(k0 + kk) * C + c0 + cc) * taps + t];
-      f.fwd[((long long)t * K + k0 + kk) * C + c0 + cc] = v;
-      f.dgrad[((long long)t * C + c0 + cc) * K + k0 + kk] = v;
+      f.form[((long long)t * K + k0 + kk) * C + c0 + cc] = v;
+      if (f.form_c) f.form_c[((long long)t * C + c0 + cc) * K + k0 + kk] = v;
     }
     return;
   }
@@ -765,14 +796,15 @@ __global__ void __launch_bounds__(256) filter_forms_multi_kernel(const FormJobs 
     for (int r = lane; r < run; r += 32) tile[kk][r] = src[r];
   }
   __syncthreads();
-  // both forms leave as rows of up to 32 consecutive floats, a warp per row: fwd[t][k][c0 ..] and dgrad[t][c][k0 ..]
+  // both forms leave as rows of up to 32 consecutive floats, a warp per row: form[t][k][c0 ..] and form_c[t][c][k0 ..]
   for (int row = warp; row < taps * kn; row += 8) {
     const int t = row / kn, kk = row - t * kn;
-    if (lane < cn) f.fwd[((long long)t * K + k0 + kk) * C + c0 + lane] = tile[kk][lane * taps + t];
+    if (lane < cn) f.form[((long long)t * K + k0 + kk) * C + c0 + lane] = tile[kk][lane * taps + t];
   }
+  if (!f.form_c) return;
   for (int row = warp; row < taps * cn; row += 8) {
     const int t = row / cn, cc = row - t * cn;
-    if (lane < kn) f.dgrad[((long long)t * C + c0 + cc) * K + k0 + lane] = tile[lane][cc * taps + t];
+    if (lane < kn) f.form_c[((long long)t * C + c0 + cc) * K + k0 + lane] = tile[lane][cc * taps + t];
   }
 }
 // Filter matrix w[rows][cols] copied with its rows padded by zeros to ld floats (the engine's tensor maps want a row length
@@ -973,7 +1005,7 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr)
   P.idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)p.a.mn_major << 15) | ((uint32_t)p.b.mn_major << 16) | ((uint32_t)(p.bn >> 3) << 17) | ((128u >> 4) << 24);
   P.out = ws ? ws : p.out; P.bias = ws ? nullptr : p.bias; P.alpha = ws ? 1.0f : p.alpha; P.split_stride = ws ? (long long)out_floats : 0;
   P.pix_per_img = p.pix_per_img ? p.pix_per_img : 1; P.by_pix = FastDiv((int)(p.pix_pad ? p.pix_pad : P.pix_per_img));
-  P.img_stride = p.img_stride; P.chan_stride = p.chan_stride; P.ld = p.ld; P.col_mod = p.col_mod ? p.col_mod : 1; P.col_mul = p.col_mul;
+  P.img_stride = p.img_stride; P.chan_stride = p.chan_stride; P.ld = p.ld; P.col_mod = p.col_mod; P.col_mul = p.col_mul;
   P.gather_src = p.gather_src; P.g_pix = p.g_pix; P.g_chan = p.g_chan; P.g_imgs = p.g_imgs;
   P.relu = relu && *relu && !atomic && !ws ? 1 : 0;
   if (P.relu) *relu = false;
@@ -1195,11 +1227,11 @@ static int channels_last(const float* src, int n_img, int chan, int pix, float**
 // stale filters together, in ONE launch -- at the first use after a write that overlaps a filter (LTB_WRITES in every entry point that
 // writes; a replayed step and ltb_params_changed mark every filter).  A filter first seen while a step is being recorded takes
 // the uncached path (no allocation inside a capture).
-struct FilterForms { const float* w; int K, C, taps; float *fwd, *dgrad; bool stale, gone; };
+struct FilterForms { const float* w; int K, C, taps; float *form, *form_c; bool stale, gone; };
 static std::vector<FilterForms> filter_cache;
 static size_t filter_cache_bytes = 0;
 void filter_cache_clear() {
-  for (auto& e : filter_cache) { cudaFree(e.fwd); cudaFree(e.dgrad); }
+  for (auto& e : filter_cache) { cudaFree(e.form); cudaFree(e.form_c); }
   filter_cache.clear(); filter_cache_bytes = 0;
 }
 // ltb_reset / ltb_free: filters at or above p exist no more and are not refreshed with the next program's.  Their blocks stay (a
@@ -1221,22 +1253,23 @@ static FilterForms* filter_cache_entry(const float* w, const ConvDims& d) {
   const size_t bytes = (size_t)d.K * d.C * taps * 4;
   if (filter_cache_bytes + 2 * bytes > ((size_t)2 << 30)) { cudaStreamSynchronize(g.stream); cudaStreamSynchronize(g.side); cudaStreamSynchronize(g.branch); filter_cache_clear(); }
   FilterForms e{w, d.K, d.C, taps, nullptr, nullptr, true, false};
-  if (cudaMalloc((void**)&e.fwd, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  if (cudaMalloc((void**)&e.dgrad, bytes) != cudaSuccess) { cudaGetLastError(); cudaFree(e.fwd); return nullptr; }
-  filter_cache_bytes += 2 * bytes;
+  if (cudaMalloc((void**)&e.form, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (d.C % 32 && cudaMalloc((void**)&e.form_c, bytes) != cudaSuccess) { cudaGetLastError(); cudaFree(e.form); return nullptr; }
+  filter_cache_bytes += d.C % 32 ? 2 * bytes : bytes;
   filter_cache.push_back(e);
   return &filter_cache.back();
 }
-// The per-tap matrices of w: out[tap][k][c] (by_c == 0, forward) or out[tap][c][k] (data-grad), rows padded to 4 floats.  *floats is the size of the
-// staging block to give back afterwards, 0 when the matrices live in the cache.
-static int tap_matrices(const float* w, const ConvDims& d, int by_c, float** out, size_t* floats) {
+// The per-tap matrices of w: out[tap][k][c], rows padded to 4 floats, for forward and, of a filter whose C is a multiple of 32, data-gradient;
+// or out[tap][c][k] for the data-gradient of any other.  *floats is the size of the staging block to give back afterwards, 0 when the matrices live in the cache.
+static int tap_matrices(const float* w, const ConvDims& d, bool dgrad, float** out, size_t* floats) {
+  const int by_c = dgrad && d.C % 32 != 0;
   const int ld = up4(by_c ? d.K : d.C);
   const size_t n = (size_t)(by_c ? d.C : d.K) * ld * d.R * d.S;
   if (!by_c && d.R * d.S == 1 && ld == d.C && aligned16(w)) { *out = const_cast<float*>(w); *floats = 0; return LTB_OK; }   // one tap: the filter is that matrix
   // Only filters in the arena are kept: a refresh reads every filter it knows, and memory of the caller's own may be gone by then,
   // or be another filter written by other means.
   const bool in_arena = (const char*)w >= g.heap && (const char*)w < g.heap + g.heap_bytes;
-  if (g.filter_cache && in_arena && d.R * d.S > 1 && d.C % 4 == 0 && d.K % 4 == 0) {
+  if (g.filter_cache && in_arena && d.R * d.S > 1 && d.C % 4 == 0 && d.K % 4 == 0 && aligned16(w)) {
     if (FilterForms* e = filter_cache_entry(w, d)) {
       if (e->stale) {
         // every stale filter at once: after an optimizer step all of them are, and their values are final until the next write
@@ -1251,13 +1284,13 @@ static int tap_matrices(const float* w, const ConvDims& d, int by_c, float** out
         for (auto& o : filter_cache) {
           if (!o.stale || o.gone) continue;
           if (jobs.n == kFormJobs) { int rc = flush(); if (rc) return rc; }
-          jobs.j[jobs.n++] = FormJob{o.w, o.fwd, o.dgrad, o.K, o.C, o.taps, jobs.total};
+          jobs.j[jobs.n++] = FormJob{o.w, o.form, o.form_c, o.K, o.C, o.taps, jobs.total};
           jobs.total += (int)(ceil_div(o.K, 32) * ceil_div(o.C, 32));
           o.stale = false;
         }
         int rc = flush(); if (rc) return rc;
       }
-      *out = by_c ? e->dgrad : e->fwd; *floats = 0;
+      *out = by_c ? e->form_c : e->form; *floats = 0;
       return LTB_OK;
     }
   }
@@ -1309,7 +1342,7 @@ static int conv_fwd_taps(const float* x, const float* w, const float* bias, floa
   float *xr = nullptr, *wt = nullptr; size_t nx = 0, nw = 0;
   int rc = channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true); if (rc) return rc;     // the weight-gradient of this convolution reads it again
   if (!xr) return 0;
-  rc = tap_matrices(w, d, 0, &wt, &nw);
+  rc = tap_matrices(w, d, false, &wt, &nw);
   bool ok = !rc && wt && tc_plan_conv_taps_fwd(p, xr, wt, bias, y, gm, g.sm_count);
   if (ok) rc = launch_plan(p, "tc_gemm_kernel[conv_fwd taps]", relu);
   if (wt && nw) temp_free(wt, nw);
@@ -1322,7 +1355,7 @@ static int conv_dgrad_taps(const float* dy, const float* w, float* dx, const Con
   float *dyr = cl_lookup(dy, d.N, d.K, d.oH * d.oW), *wd = nullptr; size_t ny = 0, nw = 0;
   int rc = dyr ? LTB_OK : channels_last(dy, d.N, d.K, d.oH * d.oW, &dyr, &ny); if (rc) return rc;
   if (!dyr) return 0;
-  rc = tap_matrices(w, d, 1, &wd, &nw);
+  rc = tap_matrices(w, d, true, &wd, &nw);
   bool ok = !rc && wd && tc_plan_conv_taps_dgrad(p, dyr, wd, dx, gm, accumulate, g.sm_count);
   if (ok) rc = launch_plan(p, "tc_gemm_kernel[conv_dgrad taps]");
   if (wd && nw) temp_free(wd, nw);
@@ -1352,7 +1385,7 @@ static int conv_fwd_any(const float* x, const float* w, const float* bias, float
   float *xr = nullptr, *wt = nullptr; size_t nx = 0, nw = 0;
   int rc = channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true); if (rc) return rc;
   if (!xr) return 0;
-  rc = tap_matrices(w, d, 0, &wt, &nw);
+  rc = tap_matrices(w, d, false, &wt, &nw);
   bool ok = !rc && wt && tc_plan_conv_any_fwd(p, xr, wt, bias, y, a, g.sm_count);
   if (ok) rc = launch_plan(p, "tc_gemm_kernel[conv_fwd im2col]", relu);
   if (wt && nw) temp_free(wt, nw);
@@ -1381,7 +1414,7 @@ static int conv_dgrad_any(const float* dy, const float* w, float* dx, const Conv
   } else if (!dyr) rc = channels_last(dy, d.N, d.K, d.oH * d.oW, &dyr, &ny);
   if (rc) return rc;
   if (!dyr) return 0;
-  rc = tap_matrices(w, d, 1, &wd, &nw);
+  rc = tap_matrices(w, d, true, &wd, &nw);
   bool ok = !rc && wd && (window ? tc_plan_conv_taps_dgrad(p, dyr, wd, dx, gm, accumulate, g.sm_count) : tc_plan_conv_any_dgrad(p, dyr, wd, dx, a, accumulate, g.sm_count));
   if (ok) rc = launch_plan(p, window ? "tc_gemm_kernel[conv_dgrad taps up]" : "tc_gemm_kernel[conv_dgrad im2col]");
   if (wd && nw) temp_free(wd, nw);

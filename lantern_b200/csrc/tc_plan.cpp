@@ -191,16 +191,35 @@ bool operand_k_taps(TcOperand& o, const float* wp, int taps, int rows, int kdim,
   return true;
 }
 
+// The same matrices wp[tap][kdim][cols] used N-major (cols contiguous, a multiple of 32): box (32 of cols, 32 of kdim, tile_cols / 32 chunks, 1 tap).
+bool operand_mn_taps(TcOperand& o, const float* wp, int taps, int kdim, int cols, int tile_cols, int* k_iters) {
+  clear(o);
+  if (!aligned16(wp) || cols % 32 || kdim < 1) return false;
+  const int chunks = cdiv(kdim, kBK);
+  o.map.base = wp; o.mn_major = 1; o.nk = 4; o.stage_bytes = (uint32_t)tile_cols * 128;
+  o.map.rank = 4; o.map.swizzle = TC_SW_128_32B;
+  o.map.dims[0] = 32; o.map.dims[1] = (uint64_t)kdim; o.map.dims[2] = (uint64_t)cols / 32; o.map.dims[3] = (uint64_t)taps;
+  o.map.strides[1] = (uint64_t)cols * 4; o.map.strides[2] = 128; o.map.strides[3] = (uint64_t)kdim * cols * 4;
+  o.map.box[0] = 32; o.map.box[1] = kBK; o.map.box[2] = (uint32_t)tile_cols / 32; o.map.box[3] = 1;
+  if (chunks > 1) { o.k_div[1] = 1; o.k_mod[1] = chunks; o.k_mul[1] = kBK; }
+  o.k_div[3] = chunks; o.k_mul[3] = 1;
+  o.t_mul[2] = tile_cols / 32;
+  o.lbo = kBK * 128; o.sbo = 512;
+  for (int i = 0; i < 4; ++i) o.kstep_off[i] = (uint32_t)i * 1024;
+  *k_iters = taps * chunks;
+  return true;
+}
+
 // M/N-major activation for weight-grad: the M (or N) index is the channel, the K index the pixel.  One stage = 32
 // pixels (a box of whole rows of the th x tw pixel grid the reduction runs over) x tile_ch channels, stored as
-// tile_ch/32 chunks of [32 pixels][32 channels].  The tile index selects the channel block and, when taps > 1, the tap
-// whose shift (r + off_h, s + off_w) is added to the pixel coordinates: tile = (r*S + s)*ch_blocks + block.
+// tile_ch/32 chunks of [32 pixels][32 channels].  taps 1: the tile index selects the channel block.  taps > 1 (TC_LOAD_TAPS): a chunk is a tap of
+// a channel block, whose shift (r + off_h, s + off_w) is added to the pixel coordinates, the taps of a block in a row: neighbouring chunks are then
+// neighbours in dw[k][c][r][s].
 bool operand_mn_window(TcOperand& o, const float* act, int n_img, int eh, int ew, int ch, int th, int tw, int tile_ch, int R, int S, int off_h, int off_w,
                        int* k_iters) {
   clear(o);
   PixelBox b;
   if (!aligned16(act) || ch % 32 || tile_ch % 32 || !pixel_box(kBK, th, tw, b)) return false;
-  const int blocks = cdiv(ch, tile_ch);
   o.map.base = act; o.mn_major = 1; o.nk = 4; o.stage_bytes = (uint32_t)tile_ch * 128;
   o.map.rank = 5; o.map.swizzle = TC_SW_128_32B;
   o.map.dims[0] = 32; o.map.dims[1] = (uint64_t)ew; o.map.dims[2] = (uint64_t)eh; o.map.dims[3] = (uint64_t)n_img; o.map.dims[4] = (uint64_t)ch / 32;
@@ -209,10 +228,10 @@ bool operand_mn_window(TcOperand& o, const float* act, int n_img, int eh, int ew
   // reduction: pixel blocks of the th x tw grid, image after image
   if (b.per_img > 1) { o.k_div[2] = 1; o.k_mod[2] = b.per_img; o.k_mul[2] = b.bh; }
   o.k_div[3] = b.per_img; o.k_mul[3] = b.bi;
-  // tile: channel block, then tap
-  o.t_div[4] = 1; o.t_mod[4] = blocks; o.t_mul[4] = tile_ch / 32;
-  if (S > 1) { o.t_div[1] = blocks; o.t_mod[1] = S; o.t_mul[1] = 1; }
-  if (R > 1) { o.t_div[2] = blocks * S; o.t_mod[2] = R; o.t_mul[2] = 1; }
+  if (R * S > 1) {
+    o.load = TC_LOAD_TAPS; o.nbox = tile_ch / 32; o.map.box[4] = 1;
+    o.im.taps = R * S; o.im.tap_s = S; o.im.ch_blocks = ch / 32;
+  } else o.t_mul[4] = tile_ch / 32;
   o.c_off[1] = off_w; o.c_off[2] = off_h;
   o.lbo = kBK * 128; o.sbo = 512;
   for (int i = 0; i < 4; ++i) o.kstep_off[i] = (uint32_t)i * 1024;
@@ -434,7 +453,7 @@ bool tc_plan_conv_taps_fwd(TcPlan& p, const float* xr, const float* wt, const fl
   return true;
 }
 
-bool tc_plan_conv_taps_dgrad(TcPlan& p, const float* dyr, const float* wd, float* dx, const TcConvGeom& g, bool accumulate, int sm_count) {
+bool tc_plan_conv_taps_dgrad(TcPlan& p, const float* dyr, const float* wt, float* dx, const TcConvGeom& g, bool accumulate, int sm_count) {
   std::memset(&p, 0, sizeof p);
   if (!taps_geometry_ok(g)) return false;
   int ka = 0, kb = 0;
@@ -442,7 +461,7 @@ bool tc_plan_conv_taps_dgrad(TcPlan& p, const float* dyr, const float* wd, float
   // input pixel (h, w) receives dy(h + ph - r, w + pw - s) * w[k][c][r][s]
   if (!operand_k_window(p.a, dyr, g.n_img, g.oH, g.oW, g.K, g.H, g.W, g.R, g.S, g.ph, g.pw, -1, &ka)) return false;
   p.bn = pick_bn(g.C, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_k_taps(p.b, wd, g.R * g.S, g.C, g.K, p.bn, &kb) || ka != kb) return false;
+  if (!operand_mn_taps(p.b, wt, g.R * g.S, g.K, g.C, p.bn, &kb) || ka != kb) return false;
   finish(p, M, g.C, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = dx; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = accumulate ? 1 : 0;
   p.pix_per_img = (int64_t)g.H * g.W; p.img_stride = (int64_t)g.C * g.H * g.W; p.chan_stride = (int64_t)g.H * g.W;
@@ -451,15 +470,15 @@ bool tc_plan_conv_taps_dgrad(TcPlan& p, const float* dyr, const float* wd, float
 
 bool tc_plan_conv_taps_wgrad(TcPlan& p, const float* dyr, const float* xr, float* dw, const TcConvGeom& g, int sm_count) {
   std::memset(&p, 0, sizeof p);
-  if (!taps_geometry_ok(g) || g.C % 64) return false;
+  if (!taps_geometry_ok(g) || g.C % 64 || g.R * g.S == 1) return false;
   int ka = 0, kb = 0;
   const int taps = g.R * g.S;
   // dw[k][c][r][s] += sum over output pixels dy[n][k][oh][ow] * x[n][c][oh - ph + r][ow - pw + s]
   if (!operand_mn_window(p.a, dyr, g.n_img, g.oH, g.oW, g.K, g.oH, g.oW, kTileM, 1, 1, 0, 0, &ka)) return false;
-  p.bn = g.C % 128 == 0 ? 128 : 64;
+  p.bn = 128;
   if (!operand_mn_window(p.b, xr, g.n_img, g.H, g.W, g.C, g.oH, g.oW, p.bn, g.R, g.S, -g.ph, -g.pw, &kb) || ka != kb) return false;
   finish(p, g.K, taps * g.C, ka, sm_count, true);
-  p.epilogue = TC_EPI_ROWMAJOR; p.out = dw; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = 1; p.ld = (int64_t)taps * g.C;
+  p.epilogue = TC_EPI_TAPS; p.out = dw; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = 1; p.ld = (int64_t)taps * g.C;
   p.col_mod = g.C; p.col_mul = taps;
   return true;
 }
@@ -488,7 +507,7 @@ bool tc_plan_conv_any_fwd(TcPlan& p, const float* xr, const float* wt, const flo
   return true;
 }
 
-bool tc_plan_conv_any_dgrad(TcPlan& p, const float* dyr, const float* wd, float* dx, const TcConvAny& g, bool accumulate, int sm_count) {
+bool tc_plan_conv_any_dgrad(TcPlan& p, const float* dyr, const float* wp, float* dx, const TcConvAny& g, bool accumulate, int sm_count) {
   std::memset(&p, 0, sizeof p);
   if (!any_geometry_ok(g) || g.sh != 1 || g.sw != 1) return false;
   int ka = 0, kb = 0;
@@ -496,8 +515,14 @@ bool tc_plan_conv_any_dgrad(TcPlan& p, const float* dyr, const float* wd, float*
   // dx is the convolution of dy with the filter turned round: tap (r', s') = (R - 1 - r, S - 1 - s), padding R - 1 - ph
   if (!operand_im2col(p.a, dyr, g.n_img, g.oH, g.oW, g.K, g.ldk, g.H, g.W, 1, 1, g.ph - g.R + 1, g.pw - g.S + 1, g.R, g.S, &ka) || !corner_ok(p.a)) return false;
   p.bn = pick_bn(g.C, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_k_taps(p.b, wd, g.R * g.S, g.C, g.ldk, p.bn, &kb) || ka != kb) return false;
-  p.b.c_off[2] = g.R * g.S - 1; p.b.k_mul[2] = -1;                  // the taps in reverse
+  // the taps in reverse
+  if (g.C % 32 == 0) {
+    if (!operand_mn_taps(p.b, wp, g.R * g.S, g.K, g.C, p.bn, &kb) || ka != kb) return false;
+    p.b.c_off[3] = g.R * g.S - 1; p.b.k_mul[3] = -1;
+  } else {
+    if (!operand_k_taps(p.b, wp, g.R * g.S, g.C, g.ldk, p.bn, &kb) || ka != kb) return false;
+    p.b.c_off[2] = g.R * g.S - 1; p.b.k_mul[2] = -1;
+  }
   finish(p, M, g.C, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = dx; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = accumulate ? 1 : 0;
   p.pix_per_img = (int64_t)g.H * g.W; p.img_stride = (int64_t)g.C * g.H * g.W; p.chan_stride = (int64_t)g.H * g.W;

@@ -35,7 +35,9 @@ struct TcTensorMap {          // arguments of cuTensorMapEncodeTiled for one FP3
 //                    of 32: the part of a box beyond the row is zero-filled, a box wholly beyond it is not loaded)
 // TC_LOAD_IM2COL     one im2col-mode load: 128 consecutive pixels of the walk, 32 channels, at the tap given by coordinates 1 and 2
 // TC_LOAD_IM2COL_MN  `nbox` im2col-mode loads of 32 pixels x 32 channels; box j is chunk tile * nbox + j of (tap, channel block)
-enum TcLoad { TC_LOAD_BOX = 0, TC_LOAD_BOXES = 1, TC_LOAD_IM2COL = 2, TC_LOAD_IM2COL_MN = 3 };
+// TC_LOAD_TAPS       `nbox` tiled boxes of 32 pixels x 32 channels of a channels-last image; box j is chunk tile * nbox + j of (tap, channel
+//                    block), its tap (s, r) added to coordinates 1 and 2, its channel block to coordinate 4
+enum TcLoad { TC_LOAD_BOX = 0, TC_LOAD_BOXES = 1, TC_LOAD_IM2COL = 2, TC_LOAD_IM2COL_MN = 3, TC_LOAD_TAPS = 4 };
 
 // The walk of an im2col-mode tensor map over channels-last images: base pixels (low_w + i * step_w, low_h + j * step_h), i < grid_w,
 // j < grid_h, image after image; upper_* is the bounding box's upper corner as cuTensorMapEncodeIm2col wants it.
@@ -55,7 +57,7 @@ struct TcOperand {
   uint32_t kstep_off[8];      // start-address offset of each step within the stage
   // How a stage is filled (TcLoad).  The last three modes are described at their operands in tc_plan.cpp.
   int load;
-  int nbox;                   // boxes per stage, 4096 bytes each (TC_LOAD_BOXES, TC_LOAD_IM2COL_MN); 1 otherwise
+  int nbox;                   // boxes per stage, 4096 bytes each (TC_LOAD_BOXES, TC_LOAD_IM2COL_MN, TC_LOAD_TAPS); 1 otherwise
   TcIm2col im;
 };
 
@@ -110,7 +112,7 @@ struct TcPlan {
   int64_t pix_per_img, img_stride, chan_stride;   // TC_EPI_PIXEL
   int64_t pix_pad;            // TC_EPI_PIXEL: tile rows per image, at least pix_per_img (0: pix_per_img); rows beyond the image are not stored
   int64_t ld;                                     // TC_EPI_ROWMAJOR
-  int col_mod, col_mul;                           // TC_EPI_ROWMAJOR, when col_mul != 0: D column n is stored at column (n % col_mod) * col_mul + n / col_mod
+  int col_mod, col_mul;                           // TC_EPI_TAPS: channels, taps
   // Gather mode (tc_plan_gather): operand a keeps its K-major row descriptors but is not loaded by TMA; the kernel's
   // epilogue warps collect it from gather_src[img][chan][pix] (pix = 4 or 16), warp g filling rows 16 g .. 16 g + 15 of
   // the tile, lane = channel within the 32-channel block, 128-byte swizzle.
@@ -139,19 +141,19 @@ bool tc_plan_conv_wgrad(TcPlan& p, const float* x, const float* dy, float* dw, i
 // xr[n][h][w][c] and dyr[n][oh][ow][k] (made by a transposing copy); a TMA box then is a window of whole image rows
 // with 32 channels, and the tap (r, s) only shifts the box coordinates -- the nine-fold unfolded matrix never exists.
 //   forward : rows = output pixels, K loop = (r, s, channel block); weights permuted to wt[r*S+s][k][c]
-//   dgrad   : rows = input pixels,  K loop = (r, s, k block);       weights permuted to wd[r*S+s][c][k]
-//   wgrad   : D = k x (tap, c), K loop = blocks of 32 pixels, both operands M/N-major; stored to OIHW through col_mod/col_mul
+//   dgrad   : rows = input pixels,  K loop = (r, s, k block);       the same weights wt[r*S+s][k][c], read N-major
+//   wgrad   : D = k x (channel block, tap, c), K loop = blocks of 32 pixels, both operands M/N-major; stored to OIHW by TC_EPI_TAPS
 struct TcConvGeom { int n_img, C, H, W, K, R, S, ph, pw, oH, oW; };
 bool tc_plan_conv_taps_fwd(TcPlan& p, const float* xr, const float* wt, const float* bias, float* y, const TcConvGeom& g, int sm_count);
-bool tc_plan_conv_taps_dgrad(TcPlan& p, const float* dyr, const float* wd, float* dx, const TcConvGeom& g, bool accumulate, int sm_count);
+bool tc_plan_conv_taps_dgrad(TcPlan& p, const float* dyr, const float* wt, float* dx, const TcConvGeom& g, bool accumulate, int sm_count);
 bool tc_plan_conv_taps_wgrad(TcPlan& p, const float* dyr, const float* xr, float* dw, const TcConvGeom& g, int sm_count);
 // The same three contractions for any image size, stride and channel count, from channels-last copies whose channel counts
 // are padded to a multiple of 4 (ldc, ldk): the TMA unit's im2col mode walks the output pixels itself, so that a tile is
 // any 128 consecutive ones (a tiled window needs rows of the image that fill a tile exactly).
-//   fwd   : wt[r*S+s][k][ldc];  dgrad (stride 1): wd[r*S+s][c][ldk];  wgrad: D = k x (tap, channel block, channel)
+//   fwd   : wt[r*S+s][k][ldc];  dgrad (stride 1): the same for C a multiple of 32, else wd[r*S+s][c][ldk];  wgrad: D = k x (tap, channel block, channel)
 struct TcConvAny { int n_img, C, H, W, K, R, S, sh, sw, ph, pw, oH, oW, ldc, ldk; };
 bool tc_plan_conv_any_fwd(TcPlan& p, const float* xr, const float* wt, const float* bias, float* y, const TcConvAny& g, int sm_count);
-bool tc_plan_conv_any_dgrad(TcPlan& p, const float* dyr, const float* wd, float* dx, const TcConvAny& g, bool accumulate, int sm_count);
+bool tc_plan_conv_any_dgrad(TcPlan& p, const float* dyr, const float* wp, float* dx, const TcConvAny& g, bool accumulate, int sm_count);
 bool tc_plan_conv_any_wgrad(TcPlan& p, const float* dyr, const float* xr, float* dw, const TcConvAny& g, int sm_count);
 // The flat convolution view straight from x[n][k][p] for image sizes that do not fill tiles (pix a multiple of 4, at least 64):
 // every image is cut into tiles of 128 pixels, the last one partly beyond the image.

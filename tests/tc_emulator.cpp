@@ -85,12 +85,19 @@ static bool tma_load(const TcOperand& o, int tile, int kiter, std::vector<float>
   for (int d = 1; d < m.rank; ++d) if (m.strides[d] % 16) { printf("stride %d not a multiple of 16 bytes\n", d); return false; }
   if ((m.box[0] * 4) % 16 || (int)m.box[0] * 4 > span(m.swizzle) && m.swizzle != TC_SW_NONE) { printf("bad inner box\n"); return false; }
   int64_t total = 1; for (int d = 0; d < m.rank; ++d) { if (m.box[d] > 256) { printf("box > 256\n"); return false; } total *= m.box[d]; }
-  const int boxes = o.load == TC_LOAD_BOXES ? o.nbox : 1;
+  const bool taps = o.load == TC_LOAD_TAPS;
+  const int boxes = o.load == TC_LOAD_BOXES || taps ? o.nbox : 1;
   if (boxes > 1 && total * 4 != 4096) { printf("box of several not 4096 bytes\n"); return false; }
   if (total * 4 * boxes != o.stage_bytes) { printf("stage_bytes %u != box bytes %lld\n", o.stage_bytes, (long long)total * 4); return false; }
   smem.assign(o.stage_bytes / 4, 1e30f);
-  for (int b = 0; b < boxes; ++b, c[0] += 32) {
+  const int64_t w0 = c[1], h0 = c[2];
+  for (int b = 0; b < boxes; ++b, c[0] += taps ? 0 : 32) {
     if (o.load == TC_LOAD_BOXES && c[0] >= (int64_t)m.dims[0]) break;       // wholly beyond the row: not loaded
+    if (taps) {
+      const int q = tile * o.nbox + b, blk = q / o.im.taps, tap = q - blk * o.im.taps;
+      if (blk >= o.im.ch_blocks) break;
+      c[1] = w0 + tap % o.im.tap_s; c[2] = h0 + tap / o.im.tap_s; c[4] = blk;
+    }
     for (int64_t lin = 0; lin < total; ++lin) {
       int64_t r = lin, goff = 0; bool inb = true;
       for (int d = 0; d < m.rank; ++d) {
@@ -190,7 +197,7 @@ static bool run_plan(const TcPlan& p, size_t out_count) {
         const int64_t q = n / 32, blk = q / p.col_mul, ch = blk * 32 + n % 32;
         if (ch >= p.col_mod) continue;                                // a channel that only fills up the last block
         idx = m * p.ld + ch * p.col_mul + q % p.col_mul;
-      } else idx = m * p.ld + (p.col_mul ? (n % p.col_mod) * p.col_mul + n / p.col_mod : n);
+      } else idx = m * p.ld + n;
       if ((size_t)idx >= out_count) { printf("epilogue index out of range\n"); return false; }
       float v = p.alpha * (float)D[(size_t)r * p.bn + c] + ((p.bias && z == 0) ? p.bias[n] : 0.0f);
       if (p.accumulate || atomic) p.out[idx] += v; else p.out[idx] = v;
@@ -332,7 +339,7 @@ static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph
   int taken = 0; TcPlan p;
   if (sh == 1 && sw == 1) {
     if (tc_plan_conv_taps_fwd(p, xr.data(), wt.data(), bias.data(), y.data(), g, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "taps fwd")) return -1; }
-    if (tc_plan_conv_taps_dgrad(p, dyr.data(), wd.data(), dx.data(), g, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "taps dgrad")) return -1; }
+    if (tc_plan_conv_taps_dgrad(p, dyr.data(), wt.data(), dx.data(), g, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "taps dgrad")) return -1; }
     if (tc_plan_conv_taps_wgrad(p, dyr.data(), xr.data(), dw.data(), g, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "taps wgrad")) return -1; }
   }
   // im2col mode; the data gradient of a strided convolution is a stride-1 one of dy with zeros between its pixels
@@ -350,7 +357,7 @@ static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph
   TcConvAny a{n_img, C, H, W, K, R, S, sh, sw, ph, pw, oH, oW, ldc, ldk}, u{n_img, C, H, W, K, R, S, 1, 1, ph, pw, uH, uW, ldc, ldk};
   int any = 0;
   if (tc_plan_conv_any_fwd(p, xp.data(), wtp.data(), bias.data(), y.data(), a, 148)) { ++any; if (!run_plan(p, y.size()) || !close(yr, y, "im2col fwd")) return -1; }
-  if (tc_plan_conv_any_dgrad(p, up.data(), wdp.data(), dx.data(), u, true, 148)) { ++any; if (!run_plan(p, dx.size()) || !close(dxr, dx, "im2col dgrad")) return -1; }
+  if (tc_plan_conv_any_dgrad(p, up.data(), C % 32 == 0 ? wtp.data() : wdp.data(), dx.data(), u, true, 148)) { ++any; if (!run_plan(p, dx.size()) || !close(dxr, dx, "im2col dgrad")) return -1; }
   if (tc_plan_conv_any_wgrad(p, dyp.data(), xp.data(), dw.data(), a, 148)) { ++any; if (!run_plan(p, dw.size()) || !close(dwr, dw, "im2col wgrad")) return -1; }
   if (any != 3) { printf("only %d of 3 im2col plans taken\n", any); return -1; }
   printf("taps conv n=%d C=%d K=%d %dx%d k%dx%d pad %d,%d stride %d,%d: %d of 3 window plans and 3 im2col plans taken, all match\n", n_img, C, K, H, W, R, S, ph, pw, sh, sw, taken);

@@ -452,6 +452,18 @@ def test_conv_of_any_size_tf32(ora, gpu, cfg, cache, det):
         assert_close(ref[k], got[k], FP32_RTOL, k)
 
 
+# Stride-1 filters on maps that tiles fill: rows and chunks (a tap of 32 channels) that end inside a tile, taps that wrap inside one, with and
+# without splits, and the filter matrices read both ways.
+TAP_CONVS = [(3, 64, 16, 16, 32, 3, 1, 1), (5, 128, 8, 8, 96, 3, 1, 1), (9, 192, 4, 4, 160, 3, 1, 1), (35, 64, 2, 2, 64, 3, 1, 1), (2, 64, 8, 8, 32, 5, 1, 2),
+             (32, 512, 2, 2, 512, 3, 1, 1), (16, 32, 16, 16, 64, 3, 1, 1)]
+
+
+@pytest.mark.parametrize("cache,det", [(0, 0), (1, 0), (1, 1)])
+@pytest.mark.parametrize("cfg", TAP_CONVS, ids=[str(c) for c in TAP_CONVS])
+def test_tap_loop_tiles_tf32(ora, gpu, cfg, cache, det):
+    test_conv_of_any_size_tf32(ora, gpu, cfg, cache, det)
+
+
 @pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
 @pytest.mark.parametrize("M,N,K", [(68, 36, 100), (1000, 132, 72), (129, 260, 1028), (4740, 1000, 36)])
 def test_gemm_of_ragged_rows_tf32(ora, gpu, ta, tb, M, N, K):
