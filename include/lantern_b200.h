@@ -77,7 +77,8 @@ int    LTB_FN(set_math)(int mode);                      /* LTB_MATH_TF32 (defaul
 /* Look-ahead fusion, off by default. When on, batch normalisation (training or inference), a convolution with a bias and same-shape
  * add are issued one call late so that an in-place ReLU of their result joins the same kernel, and an in-place ReLU gradient is held
  * so that the batch-norm backward, convolution backward with a bias or add gradient that reads it applies it on the fly. Results are those of the separate calls; only the moment
- * of the launch moves: a held operation is issued by the next call of this library whatever it is (sync, copies,
+ * of the launch moves: a held operation is issued by the next call of this library whatever it is, or joined by it; a batch norm and
+ * the ReLU that joined it are held for one call more, so that a convolution of the result can have them prepare its output (sync, copies,
  * get_stream and graph_end included; malloc, malloc_uninit, mark and grad_unset only keep books on a block no held operation can
  * name yet and issue nothing). A host that enqueues its own work on the stream must call get_stream or sync first.  In the same
  * spirit conv2d_bwd may return while its weight gradient still runs on a second stream: the gradient calls of the chain

@@ -20,7 +20,7 @@ constexpr size_t kGranule = 256;      // arena granule (TMA wants 16 B bases/str
 // in-place ReLU of its result share the contraction's epilogue, and a held ReLU gradient joins the bias-gradient pass of the
 // convolution backward that reads it.  Any other call
 // first issues the held operation on its own, so results never change; only the moment of the launch does.
-enum { PEND_NONE = 0, PEND_BN_FWD = 1, PEND_ADD = 2, PEND_RELU_GRAD = 3, PEND_RELU_ADD_GRAD = 4, PEND_BN_ADD = 5, PEND_CONV = 6, PEND_BN_INF = 7 };
+enum { PEND_NONE = 0, PEND_BN_FWD = 1, PEND_ADD = 2, PEND_RELU_GRAD = 3, PEND_RELU_ADD_GRAD = 4, PEND_BN_ADD = 5, PEND_CONV = 6, PEND_BN_INF = 7, PEND_BN_RELU = 8 };
 struct ConvDims { int N, C, H, W, K, R, S, sh, sw, ph, pw, oH, oW; };
 struct Pending {
   int kind = PEND_NONE;
@@ -38,6 +38,9 @@ struct Pending {
   float *da = nullptr, *db = nullptr; int fa = 0, fb = 0;
   // PEND_CONV: y = conv(x, w) (+ bias)
   const float *w = nullptr, *bias = nullptr; ConvDims dims = {};
+  // PEND_BN_RELU: a PEND_BN_FWD or PEND_BN_ADD (`inner`) and the in-place ReLU of its result, held one call further: the convolution that
+  // reads the result has its own output cleared and its channels-last copy written by the same kernel (BnExtra)
+  int inner = PEND_NONE;
   // PEND_BN_ADD (fusion level 3): the PEND_BN_FWD fields, then out = y + a with y the held batch norm's result; an in-place ReLU of
   // out makes the three one kernel that never writes y
 };
@@ -79,6 +82,7 @@ struct Context {
   bool fusion_single_use = false;     // level 3: a batch-norm result consumed by add + in-place ReLU has no other reader and is not written
   bool fusion_no_writeback = false;   // level 2: an absorbed in-place ReLU gradient is applied on load only (its buffer is dead afterwards)
   Pending pending;
+  Pending ahead;                      // a PEND_BN_RELU taken over by the convolution call that is running; issued by its first launch that reads or clears something
   bool side_open = false;             // weight gradients are running on the side stream that no stream has waited for yet (side_join)
   size_t side_base = 0;               // arena mark below the staging blocks held for them
   bool hold_workspace = false;        // while two halves are in flight their staging blocks are released together at the end
@@ -101,7 +105,18 @@ int relu_add_grad_issue(const Pending& p);                 // issues the held op
 // issue functions shared by the entry points and the flush (pool_bn.cu / elementwise.cu)
 int conv_fwd_issue(const Pending& p, bool relu);           // contract.cu
 int bn_inference_issue(const Pending& p, bool relu);
-int bn_fwd_issue(const Pending& p, bool relu);
+// What a batch norm's kernel does beside its own work for the convolution that follows: clear `zero` (n4 times 16 bytes) and write a
+// channels-last copy of the result.
+struct ZeroFill { float4* p = nullptr; int64_t n4 = 0; };
+struct BnExtra { ZeroFill zero; float* cl = nullptr; };
+bool bn_fwd_writes_copy(const Pending& p);                 // whether the kernel that p takes can write the copy
+int bn_fwd_issue(const Pending& p, bool relu, const BnExtra& extra = BnExtra());
+// A result that the launches of this call add into and that has to be zero before: `p` (null: nothing to clear) is cleared by whichever
+// kernel of the call runs first and can, `done` says that one did.
+struct Clear { float* p = nullptr; size_t floats = 0; bool done = false; };
+ZeroFill take_clear(Clear* c);                             // what a kernel is given to clear (gemm_tc.cu)
+// Issues g.ahead, if there is one, with the clearing and the copy; cl: where the channels-last copy goes.
+int issue_ahead(Clear* clear = nullptr, float* cl = nullptr);
 int add_issue(const float* a, const float* b, float* out, int64_t n, bool relu);
 int relu_issue(float* x, int64_t n);
 int relu_grad_issue(const float* y, float* d, int64_t n);
@@ -176,6 +191,12 @@ struct FastDiv {
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() { pdl_launch(); pdl_wait(); }
+// The whole grid's share of a ZeroFill.
+__device__ __forceinline__ void zero_fill(const ZeroFill& z) {
+  if (z.n4 == 0) return;
+  const int64_t block = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x, per = blockDim.x * blockDim.y;
+  for (int64_t i = block * per + threadIdx.y * blockDim.x + threadIdx.x; i < z.n4; i += (int64_t)gridDim.x * gridDim.y * gridDim.z * per) z.p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
 #endif
 inline void pdl_attribute(cudaLaunchAttribute& a) { a.id = cudaLaunchAttributeProgrammaticStreamSerialization; a.val.programmaticStreamSerializationAllowed = 1; }
 

@@ -35,7 +35,7 @@ int ltb::conv_fwd_issue(const Pending& p, bool relu) {
   const ConvDims& d = p.dims;
   bool left = relu;                                          // the ReLU still to be done
   int r = g.math == LTB_MATH_TF32 ? conv_fwd_tc(p.x, p.w, p.bias, p.y, d, &left) : 0;
-  if (r == 0) { left = false; return conv_fwd_fp32(p.x, p.w, p.bias, p.y, d, relu); }
+  if (r == 0) { left = false; r = issue_ahead(); return r ? r : conv_fwd_fp32(p.x, p.w, p.bias, p.y, d, relu); }
   if (r < 0) return r;
   return left ? relu_issue(p.y, p.n) : LTB_OK;
 }
@@ -89,8 +89,14 @@ int ltb_gemm_grad(const float* a, float* da, int ta, const float* b, float* db, 
 // conv2D_batch: TensorDslCPU.scala:532-571.
 int ltb_conv2d_fwd(const float* x, const float* w, const float* bias, float* y, int N, int C, int H, int W, int K, int R, int S,
                    int sh, int sw, int ph, int pw) {
-  LTB_INITED(); ConvDims d;
-  LTB_REQUIRE(x && w && y && conv_dims(d, N, C, H, W, K, R, S, sh, sw, ph, pw), "ltb_conv2d_fwd: bad argument");
+  LTB_INITED_NOFLUSH(); ConvDims d;
+  const bool ok = x && w && y && conv_dims(d, N, C, H, W, K, R, S, sh, sw, ph, pw);
+  // The batch norm and ReLU that make x may still be held: this call's first launch that reads x, or clears y, issues them (issue_ahead).
+  const int64_t nx = (int64_t)N * C * H * W, nw = (int64_t)K * C * R * S;
+  if (ok && g.pending.kind == PEND_BN_RELU && (g.pending.inner == PEND_BN_ADD ? g.pending.out : g.pending.y) == x && g.pending.n == nx && g.pending.N == N &&
+      (w + nw <= x || x + nx <= w) && g.math == LTB_MATH_TF32 && !bias && !covers_image(d)) { g.ahead = g.pending; g.pending.kind = PEND_NONE; }
+  else if (g.pending.kind) { int rc = flush_pending(); if (rc) return rc; }
+  LTB_REQUIRE(ok, "ltb_conv2d_fwd: bad argument");
   LTB_WRITES(y, (size_t)N * K * d.oH * d.oW);
   if (covers_image(d) && d.R * d.S > 1) {
     if (bias) { int rc = ltb_fill_with_bias(y, bias, N, K, 1); if (rc) return rc; }
@@ -98,7 +104,8 @@ int ltb_conv2d_fwd(const float* x, const float* w, const float* bias, float* y, 
   }
   Pending h; h.kind = PEND_CONV; h.n = (int64_t)N * K * d.oH * d.oW; h.x = x; h.w = w; h.bias = bias; h.y = y; h.dims = d;
   if (g.fusion && bias) { g.pending = h; return LTB_OK; }   // an in-place ReLU of y may join it; without a bias a batch norm follows, which nothing here joins
-  return conv_fwd_issue(h, false);
+  const int rc = conv_fwd_issue(h, false), left = issue_ahead();        // a convolution that failed early leaves it to be issued here
+  return rc ? rc : left;
 }
 // conv2D_batch_grad: TensorDslCPU.scala:575-692. dx, dw, dbias accumulate; dx is NULL for a leaf input.
 int ltb_conv2d_bwd(const float* x, float* dx, const float* w, float* dw, float* dbias, const float* dy, int N, int C, int H, int W,

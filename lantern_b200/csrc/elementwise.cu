@@ -463,6 +463,7 @@ int flush_pending() {
   g.pending.kind = PEND_NONE;
   switch (p.kind) {
     case PEND_BN_FWD: return bn_fwd_issue(p, false);
+    case PEND_BN_RELU: { Pending q = p; q.kind = p.inner; return bn_fwd_issue(q, true); }
     case PEND_CONV: return conv_fwd_issue(p, false);
     case PEND_BN_INF: return bn_inference_issue(p, false);
     case PEND_ADD: return add_issue(p.a, p.b, p.out, p.n, false);
@@ -683,11 +684,10 @@ int ltb_unary(int op, const float* x, float* out, int64_t n) {
   LTB_WRITES(out, n);
   if (g.pending.kind && op == LTB_RELU && x == out && g.pending.n == n) {      // in-place ReLU of the result that was just held back
     const Pending h = g.pending;
-    if (h.kind == PEND_BN_FWD && h.y == out) { g.pending.kind = PEND_NONE; return bn_fwd_issue(h, true); }
+    if ((h.kind == PEND_BN_FWD && h.y == out) || (h.kind == PEND_BN_ADD && h.out == out)) { g.pending.inner = h.kind; g.pending.kind = PEND_BN_RELU; return LTB_OK; }
     if (h.kind == PEND_BN_INF && h.y == out) { g.pending.kind = PEND_NONE; return bn_inference_issue(h, true); }
     if (h.kind == PEND_CONV && h.y == out) { g.pending.kind = PEND_NONE; return conv_fwd_issue(h, true); }
     if (h.kind == PEND_ADD && h.out == out) { g.pending.kind = PEND_NONE; return add_issue(h.a, h.b, h.out, h.n, true); }
-    if (h.kind == PEND_BN_ADD && h.out == out) { g.pending.kind = PEND_NONE; return bn_fwd_issue(h, true); }
   }
   if (g.pending.kind) { int rc = flush_pending(); if (rc) return rc; }
   return launch_map<1>(x, nullptr, nullptr, out, n, [op] __device__(float v, float, float) { return un_op(op, v); });

@@ -648,8 +648,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // col[n][(c*R+r)*S+s][p] = x[n][c][ho*sh-ph+r][wo*sw-pw+s] (0 outside): the reference's `finput` (TensorDslCPU.scala:484-530).
 // A thread owns one output pixel of one input plane (n, c) and writes all R*S taps of it: the plane and pixel
 // decomposition (the only integer divisions) is paid once per R*S elements, the writes of a warp stay contiguous.
-__global__ void unfold_rows_kernel(const float* __restrict__ x, float* __restrict__ col, ConvDims d, int planes_per_block, int threads_per_plane) {
+__global__ void unfold_rows_kernel(const float* __restrict__ x, float* __restrict__ col, ConvDims d, int planes_per_block, int threads_per_plane, const ZeroFill zero) {
   pdl_enter();
+  zero_fill(zero);
   const int pix = d.oH * d.oW, rs = d.R * d.S;
   const int64_t planes = (int64_t)d.N * d.C;
   const int lane_p = threadIdx.x % threads_per_plane;
@@ -676,8 +677,9 @@ __global__ void unfold_rows_kernel(const float* __restrict__ x, float* __restric
 // Channels-last copy dst[n][p][ld] of src[n][chan][p] for any channel and pixel count; channels chan .. ld - 1 are written as zeros.
 // A CTA moves 32 channels x 64 pixels through shared memory, coalesced on both sides, eight loads in flight per thread (tiles of 32 x 32
 // with four took 19 us instead of 15 on 32 x 64 x 56 x 56).  grid (ceil(pix/64), ceil(ld/32), N), block 256.
-__global__ void __launch_bounds__(256) channels_last_kernel(const float* __restrict__ src, float* __restrict__ dst, int chan, int pix, int ld) {
+__global__ void __launch_bounds__(256) channels_last_kernel(const float* __restrict__ src, float* __restrict__ dst, int chan, int pix, int ld, const ZeroFill zero) {
   pdl_enter();
+  zero_fill(zero);
   __shared__ float tile[32][65];
   const int p0 = blockIdx.x * 64, c0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
@@ -694,8 +696,9 @@ __global__ void __launch_bounds__(256) channels_last_kernel(const float* __restr
 }
 // The same copy of small images (fewer than 32 pixels: 64-pixel rows of the tile above would be mostly idle), 32 channels of one image
 // per CTA; chan a multiple of 32.  grid (1, chan/32, N).
-__global__ void to_rows_tiled_kernel(const float* __restrict__ src, float* __restrict__ dst, int chan, int pix) {
+__global__ void to_rows_tiled_kernel(const float* __restrict__ src, float* __restrict__ dst, int chan, int pix, const ZeroFill zero) {
   pdl_enter();
+  zero_fill(zero);
   __shared__ float tile[32][33];
   const int n = blockIdx.z, c0 = blockIdx.y * 32;
   const float* s = src + ((int64_t)n * chan + c0) * pix;
@@ -708,8 +711,9 @@ __global__ void to_rows_tiled_kernel(const float* __restrict__ src, float* __res
 // (up is uH x uW pixels of ld channels).  The data-gradient of a strided convolution is the stride-1 data-gradient of this tensor,
 // so no fold-back pass is needed.  A CTA writes the sh rows that one row of dy owns, 32 channels, through shared memory; wide rows
 // go 32 pixels at a time.  grid (ceil(uH/sh), ceil(ld/32), N), block 256.
-__global__ void __launch_bounds__(256) channels_last_up_kernel(const float* __restrict__ dy, float* __restrict__ up, int K, int ld, int oH, int oW, int uH, int uW, int sh, int sw) {
+__global__ void __launch_bounds__(256) channels_last_up_kernel(const float* __restrict__ dy, float* __restrict__ up, int K, int ld, int oH, int oW, int uH, int uW, int sh, int sw, const ZeroFill zero) {
   pdl_enter();
+  zero_fill(zero);
   __shared__ float tile[32][33];
   const int a = blockIdx.x, k0 = blockIdx.y * 32, n = blockIdx.z;
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
@@ -968,8 +972,47 @@ typedef void (*EngineFn)(const CUtensorMap, const CUtensorMap, const TcParams);
    tc_gemm_kernel<TC_EPI_TAPS, 0, GEN>, tc_gemm_kernel<TC_EPI_TAPS, 1, GEN>, tc_gemm_kernel<TC_EPI_TAPS, 2, GEN>}
 static const EngineFn kEngine[2][9] = {LTB_ENGINE(false), LTB_ENGINE(true)};    // by load modes, epilogue and store mode
 #undef LTB_ENGINE
+static size_t plan_out_floats(const TcPlan& p) {
+  return p.epilogue == TC_EPI_PIXEL ? (size_t)ceil_div(p.M, p.pix_pad ? p.pix_pad : p.pix_per_img ? p.pix_per_img : 1) * (size_t)p.img_stride : (size_t)p.M * (size_t)p.ld;
+}
+// What a plan's launch wants cleared first: a result that its splits add into.  As a node of its own a clearing costs 2.5 to 3 us of a chain of
+// launches and the early start of the launch behind it, 50 times in a step of ResNet-50 at batch 8; beside a kernel that runs anyway
+// nothing measurable.
+static Clear plan_clear(const TcPlan& p) {
+  Clear c;
+  if (p.splits > 1 && !g.deterministic && !p.accumulate) { c.p = p.out; c.floats = plan_out_floats(p); }
+  return c;
+}
+ZeroFill take_clear(Clear* c) {
+  ZeroFill z;
+  if (!c || !c->p || c->done || c->floats % 4 || !aligned16(c->p)) return z;
+  c->done = true; z.p = reinterpret_cast<float4*>(c->p); z.n4 = (int64_t)(c->floats / 4);
+  return z;
+}
+static bool overlaps(const void* a, size_t an, const void* b, size_t bn) {      // floats
+  return a && b && (const char*)a < (const char*)b + bn * 4 && (const char*)b < (const char*)a + an * 4;
+}
+int issue_ahead(Clear* clear, float* cl) {
+  if (!g.ahead.kind) return LTB_OK;
+  Pending p = g.ahead;
+  g.ahead.kind = PEND_NONE;
+  p.kind = p.inner;
+  BnExtra extra;
+  extra.cl = cl;
+  if (clear && clear->p && clear->floats <= 8 * (size_t)p.n) {       // not what the batch norm itself reads or writes, and in proportion to its grid
+    bool apart = true;
+    for (const float* q : {p.x, p.a, (const float*)p.y, (const float*)p.out}) apart = apart && !overlaps(q, (size_t)p.n, clear->p, clear->floats);
+    for (const float* q : {p.gamma, p.beta, (const float*)p.run_mean, (const float*)p.run_var, (const float*)p.save_mean, (const float*)p.save_istd})
+      apart = apart && !overlaps(q, (size_t)p.C, clear->p, clear->floats);
+    if (apart) extra.zero = take_clear(clear);
+  }
+  return bn_fwd_issue(p, true, extra);
+}
 // *relu: the caller wants max(0, result); false on return when the kernel has done it, still true when splits meet outside it.
-static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr) {
+// clear: plan_clear of this plan, if a kernel before this one was to do it.
+static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr, Clear clear = Clear()) {
+  if (!clear.p) clear = plan_clear(p);
+  { int rc = issue_ahead(&clear); if (rc) return rc; }
   CUtensorMap ma, mb;
   int rc = encode_map(p.a, &ma); if (rc) return rc;
   rc = encode_map(p.b, &mb); if (rc) return rc;
@@ -989,7 +1032,7 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr)
     cz = splits <= 2 ? 2 : splits <= 4 ? 4 : 8;
     nslabs = (int)ceil_div(splits, cz);
   }
-  const size_t out_floats = p.epilogue == TC_EPI_PIXEL ? (size_t)ceil_div(p.M, p.pix_pad ? p.pix_pad : p.pix_per_img ? p.pix_per_img : 1) * (size_t)p.img_stride : (size_t)p.M * (size_t)p.ld;
+  const size_t out_floats = plan_out_floats(p);
   float* ws = nullptr;
   if (nslabs > 1) {
     ws = temp_alloc((size_t)nslabs * out_floats);
@@ -1000,7 +1043,7 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr)
   if (atomic) splits = (int)ceil_div(p.k_iters, P.k_per_split);                    // atomic mode: only splits that have work
   P.cluster_z = cz;
   P.epilogue = p.epilogue; P.accumulate = ws ? 0 : p.accumulate; P.atomic = atomic ? 1 : 0;
-  if (atomic && !p.accumulate) LTB_CUDA(cudaMemsetAsync(p.out, 0, out_floats * 4, g.stream));     // overwrite semantics: start from zero, then add
+  if (atomic && !p.accumulate && !clear.done) LTB_CUDA(cudaMemsetAsync(p.out, 0, out_floats * 4, g.stream));     // overwrite semantics: start from zero, then add
   // tf32 x tf32 -> f32: D format 1 at [4,6), A/B format 2 at [7,10)/[10,13), major bits 15/16, N>>3 at [17,23), M>>4 at [24,29)
   P.idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)p.a.mn_major << 15) | ((uint32_t)p.b.mn_major << 16) | ((uint32_t)(p.bn >> 3) << 17) | ((128u >> 4) << 24);
   P.out = ws ? ws : p.out; P.bias = ws ? nullptr : p.bias; P.alpha = ws ? 1.0f : p.alpha; P.split_stride = ws ? (long long)out_floats : 0;
@@ -1122,12 +1165,14 @@ static float* unfold_lookup(const float* src, const ConvDims& d) {
   for (auto& e : cl_cache) if (e.src == src && e.n_img == d.N && e.chan == ck && e.pix == pix && e.geom == key) return e.cl;
   return nullptr;
 }
-static int launch_unfold(const float* x, float* col, const ConvDims& d) {
+static int launch_unfold(const float* x, float* col, const ConvDims& d, Clear* clear = nullptr) {
+  { int rc = issue_ahead(clear); if (rc) return rc; }
+  const ZeroFill zero = clear && !overlaps(clear->p, clear->floats, x, (size_t)d.N * d.C * d.H * d.W) ? take_clear(clear) : ZeroFill();
   const int pix = d.oH * d.oW;
   int tpp = 4; while (tpp < pix && tpp < 256) tpp <<= 1;       // threads per input plane: a power of two in [4, 256] (4 x 4 and 2 x 2 outputs leave no lane idle)
   const int ppb = 256 / tpp;
   const int64_t planes = (int64_t)d.N * d.C;
-  LTB_LAUNCH(unfold_rows_kernel, grid_for(ceil_div(planes, ppb) * 256, 256, 16), 256, 0, x, col, d, ppb, tpp);
+  LTB_LAUNCH(unfold_rows_kernel, grid_for(ceil_div(planes, ppb) * 256, 256, 16), 256, 0, x, col, d, ppb, tpp, zero);
   return LTB_OK;
 }
 // 1x1 convolution with stride 2 and no padding (ResNet's downsampling branch): every gradient element goes to exactly
@@ -1168,21 +1213,21 @@ static float* temp_alloc(size_t floats) {
 // The unfolded form col[n][(c, r, s)][p] of a convolution input for the forward pass: kept for the weight gradient of the same
 // convolution when the operand cache is on, else a staging block of *floats floats to give back (*floats == 0: kept).  *col stays
 // null when there is no room.
-static int unfolded(const float* x, const ConvDims& d, const float** col, float** temp, size_t* floats) {
+static int unfolded(const float* x, const ConvDims& d, const float** col, float** temp, size_t* floats, Clear* clear) {
   const int ck = d.C * d.R * d.S, pix = d.oH * d.oW;
   const size_t n = (size_t)d.N * ck * pix;
   *temp = nullptr; *floats = 0; *col = nullptr;
   if (g.filter_cache && !(g.tune & 4)) {
     if (float* kept = kept_block(x, (size_t)d.N * d.C * d.H * d.W, d.N, ck, pix, unfold_key(d), n)) {
       *col = kept;
-      int rc = launch_unfold(x, kept, d); if (rc) cl_cache_drop(x, 1);
+      int rc = launch_unfold(x, kept, d, clear); if (rc) cl_cache_drop(x, 1);
       return rc;
     }
   }
   float* buf = temp_alloc(n);
   if (!buf) return LTB_OK;
   *temp = buf; *floats = n; *col = buf;
-  return launch_unfold(x, buf, d);
+  return launch_unfold(x, buf, d, clear);
 }
 
 // ---- tap-loop (implicit) path for R x S convolutions with stride 1 ---------------------------------------------------------
@@ -1192,34 +1237,38 @@ static bool taps_geometry(const ConvDims& d, TcConvGeom& gm) {
   return true;
 }
 static int up4(int v) { return (v + 3) / 4 * 4; }
-static int channels_last_into(const float* src, int n_img, int chan, int pix, float* out) {
+static int channels_last_into(const float* src, int n_img, int chan, int pix, float* out, Clear* clear) {
   const int ld = up4(chan);
+  if (g.ahead.kind && g.ahead.N == n_img && g.ahead.C == chan && g.ahead.HW == pix && bn_fwd_writes_copy(g.ahead)) return issue_ahead(clear, out);      // (g.ahead makes src)
+  { int rc = issue_ahead(clear); if (rc) return rc; }
+  ZeroFill zero = clear && !overlaps(clear->p, clear->floats, src, (size_t)n_img * chan * pix) ? take_clear(clear) : ZeroFill();
   if (chan % 32 == 0 && pix < 32 && n_img <= 65535) {
-    LTB_LAUNCH(to_rows_tiled_kernel, dim3(1, chan / 32, n_img), 32 * pix < 256 ? 128 : 256, 0, src, out, chan, pix);
+    LTB_LAUNCH(to_rows_tiled_kernel, dim3(1, chan / 32, n_img), 32 * pix < 256 ? 128 : 256, 0, src, out, chan, pix, zero);
     return LTB_OK;
   }
   for (int n0 = 0; n0 < n_img; n0 += 65535) {                       // gridDim.z holds at most 65535 images
     const int nn = n_img - n0 < 65535 ? n_img - n0 : 65535;
-    LTB_LAUNCH(channels_last_kernel, dim3((unsigned)ceil_div(pix, 64), (unsigned)ceil_div(ld, 32), (unsigned)nn), 256, 0, src + (size_t)n0 * chan * pix, out + (size_t)n0 * pix * ld, chan, pix, ld);
+    LTB_LAUNCH(channels_last_kernel, dim3((unsigned)ceil_div(pix, 64), (unsigned)ceil_div(ld, 32), (unsigned)nn), 256, 0, src + (size_t)n0 * chan * pix, out + (size_t)n0 * pix * ld, chan, pix, ld, zero);
+    zero = ZeroFill();
   }
   return LTB_OK;
 }
 // Channels-last copy [N][pix][ld] of a tensor [N][chan][pix], ld = chan rounded up to 4 (zeros beyond chan: the tensor maps want
 // rows of a multiple of 16 bytes).  keep: put it where it outlives the call and remember it (when the cache is on and the arena has
 // room); otherwise a staging block of *floats floats to give back (*floats == 0: kept).  *out stays null when there is no room at all.
-static int channels_last(const float* src, int n_img, int chan, int pix, float** out, size_t* floats, bool keep = false) {
+static int channels_last(const float* src, int n_img, int chan, int pix, float** out, size_t* floats, bool keep = false, Clear* clear = nullptr) {
   const size_t n = (size_t)n_img * up4(chan) * pix;
   *floats = 0; *out = nullptr;
   if (keep && g.filter_cache && !(g.tune & 4)) {
     if (float* kept = kept_block(src, (size_t)n_img * chan * pix, n_img, chan, pix, 0, n)) {
       *out = kept;
-      int rc = channels_last_into(src, n_img, chan, pix, kept); if (rc) cl_cache_drop(src, 1);
+      int rc = channels_last_into(src, n_img, chan, pix, kept, clear); if (rc) cl_cache_drop(src, 1);
       return rc;
     }
   }
   *out = temp_alloc(n); *floats = n;
   if (!*out) return LTB_OK;
-  return channels_last_into(src, n_img, chan, pix, *out);
+  return channels_last_into(src, n_img, chan, pix, *out, clear);
 }
 // ---- filter cache (ltb_set_filter_cache) ------------------------------------------------------------------------------------
 // The per-tap forms of a filter are needed twice per step (forward and data-grad) and change once per step (the optimizer).
@@ -1340,11 +1389,12 @@ static int conv_fwd_taps(const float* x, const float* w, const float* bias, floa
   TcConvGeom gm; TcPlan p;
   if (!taps_geometry(d, gm) || !tc_plan_conv_taps_fwd(p, y, y, bias, y, gm, g.sm_count)) return 0;     // eligibility with any aligned pointers
   float *xr = nullptr, *wt = nullptr; size_t nx = 0, nw = 0;
-  int rc = channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true); if (rc) return rc;     // the weight-gradient of this convolution reads it again
+  Clear clear = plan_clear(p);
+  int rc = channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true, &clear); if (rc) return rc;     // the weight-gradient of this convolution reads it again
   if (!xr) return 0;
   rc = tap_matrices(w, d, false, &wt, &nw);
   bool ok = !rc && wt && tc_plan_conv_taps_fwd(p, xr, wt, bias, y, gm, g.sm_count);
-  if (ok) rc = launch_plan(p, "tc_gemm_kernel[conv_fwd taps]", relu);
+  if (ok) rc = launch_plan(p, "tc_gemm_kernel[conv_fwd taps]", relu, clear);
   if (wt && nw) temp_free(wt, nw);
   if (nx) temp_free(xr, nx);
   return rc ? rc : (ok ? 1 : 0);
@@ -1383,11 +1433,12 @@ static int conv_fwd_any(const float* x, const float* w, const float* bias, float
   if (tc_conv_needs_rows(d.oH * d.oW) && d.C * d.R * d.S % 4) return 0;
   if (!any_geometry(d, a) || !tc_plan_conv_any_fwd(p, (const float*)g.heap, (const float*)g.heap, bias, y, a, g.sm_count)) return 0;     // eligibility with any aligned pointers
   float *xr = nullptr, *wt = nullptr; size_t nx = 0, nw = 0;
-  int rc = channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true); if (rc) return rc;
+  Clear clear = plan_clear(p);
+  int rc = channels_last(x, d.N, d.C, d.H * d.W, &xr, &nx, /*keep=*/true, &clear); if (rc) return rc;
   if (!xr) return 0;
   rc = tap_matrices(w, d, false, &wt, &nw);
   bool ok = !rc && wt && tc_plan_conv_any_fwd(p, xr, wt, bias, y, a, g.sm_count);
-  if (ok) rc = launch_plan(p, "tc_gemm_kernel[conv_fwd im2col]", relu);
+  if (ok) rc = launch_plan(p, "tc_gemm_kernel[conv_fwd im2col]", relu, clear);
   if (wt && nw) temp_free(wt, nw);
   if (nx) temp_free(xr, nx);
   return rc ? rc : (ok ? 1 : 0);
@@ -1403,20 +1454,22 @@ static int conv_dgrad_any(const float* dy, const float* w, float* dx, const Conv
   }
   gm.n_img = d.N; gm.C = d.C; gm.H = d.H; gm.W = d.W; gm.K = d.K; gm.R = d.R; gm.S = d.S; gm.ph = d.ph; gm.pw = d.pw; gm.oH = a.oH; gm.oW = a.oW;
   const float* any = (const float*)g.heap;
-  const bool window = tc_plan_conv_taps_dgrad(p, any, any, dx, gm, true, g.sm_count);
-  if (!window && !tc_plan_conv_any_dgrad(p, any, any, dx, a, true, g.sm_count)) return 0;
+  const bool window = tc_plan_conv_taps_dgrad(p, any, any, dx, gm, accumulate, g.sm_count);
+  if (!window && !tc_plan_conv_any_dgrad(p, any, any, dx, a, accumulate, g.sm_count)) return 0;
+  Clear clear = plan_clear(p);
   float *dyr = strided ? nullptr : cl_lookup(dy, d.N, d.K, d.oH * d.oW), *wd = nullptr; size_t ny = 0, nw = 0;
   int rc = LTB_OK;
   if (strided) {
     ny = (size_t)d.N * a.oH * a.oW * a.ldk;
     if (!(dyr = temp_alloc(ny))) return 0;
-    LTB_LAUNCH(channels_last_up_kernel, dim3((unsigned)ceil_div(a.oH, d.sh), (unsigned)ceil_div(a.ldk, 32), (unsigned)d.N), 256, 0, dy, dyr, d.K, a.ldk, d.oH, d.oW, a.oH, a.oW, d.sh, d.sw);
-  } else if (!dyr) rc = channels_last(dy, d.N, d.K, d.oH * d.oW, &dyr, &ny);
+    const ZeroFill zero = overlaps(clear.p, clear.floats, dy, (size_t)d.N * d.K * d.oH * d.oW) ? ZeroFill() : take_clear(&clear);
+    LTB_LAUNCH(channels_last_up_kernel, dim3((unsigned)ceil_div(a.oH, d.sh), (unsigned)ceil_div(a.ldk, 32), (unsigned)d.N), 256, 0, dy, dyr, d.K, a.ldk, d.oH, d.oW, a.oH, a.oW, d.sh, d.sw, zero);
+  } else if (!dyr) rc = channels_last(dy, d.N, d.K, d.oH * d.oW, &dyr, &ny, false, &clear);
   if (rc) return rc;
   if (!dyr) return 0;
   rc = tap_matrices(w, d, true, &wd, &nw);
   bool ok = !rc && wd && (window ? tc_plan_conv_taps_dgrad(p, dyr, wd, dx, gm, accumulate, g.sm_count) : tc_plan_conv_any_dgrad(p, dyr, wd, dx, a, accumulate, g.sm_count));
-  if (ok) rc = launch_plan(p, window ? "tc_gemm_kernel[conv_dgrad taps up]" : "tc_gemm_kernel[conv_dgrad im2col]");
+  if (ok) rc = launch_plan(p, window ? "tc_gemm_kernel[conv_dgrad taps up]" : "tc_gemm_kernel[conv_dgrad im2col]", nullptr, clear);
   if (wd && nw) temp_free(wd, nw);
   if (ny) temp_free(dyr, ny);
   return rc ? rc : (ok ? 1 : 0);
@@ -1496,14 +1549,15 @@ int conv_fwd_tc(const float* x, const float* w, const float* bias, float* y, con
   const bool gathered = rows && !ragged && pix > 1 && !(g.tune & 1) && tc_gather_possible(y, ck, pix);
   if (rows && !ragged && !gathered && pix > 1) return 0;
   const float* op = x; float* temp = nullptr; size_t tn = 0;
-  int rc = is_pointwise(d) ? LTB_OK : unfolded(x, d, &op, &temp, &tn);
+  Clear clear = plan_clear(p);
+  int rc = is_pointwise(d) ? LTB_OK : unfolded(x, d, &op, &temp, &tn, &clear);
   if (rc || !op) return rc;
   float* wtemp; size_t wn; const float* wp;
   rc = padded_filter(w, d.K, ck, ldw, &wp, &wtemp, &wn);
   bool ok = !rc && wp && (ragged ? tc_plan_conv_ragged_fwd(p, op, wp, ldw, bias, y, d.N, ck, d.K, pix, g.sm_count)
                                  : tc_plan_conv_fwd(p, op, rows, wp, ldw, bias, y, d.N, ck, d.K, pix, g.sm_count));
   if (ok && gathered) tc_plan_gather(p, op, d.N, ck, pix);
-  if (ok) rc = launch_plan(p, gathered ? "tc_gemm_kernel[conv_fwd gather]" : "tc_gemm_kernel[conv_fwd]", relu);
+  if (ok) rc = launch_plan(p, gathered ? "tc_gemm_kernel[conv_fwd gather]" : "tc_gemm_kernel[conv_fwd]", relu, clear);
   if (wtemp) temp_free(wtemp, wn);
   if (temp) temp_free(temp, tn);
   return rc ? rc : (ok ? 1 : 0);

@@ -285,7 +285,7 @@ constexpr int kBnVptBwd = 4;       // backward keeps x, dy and dx: half the slic
 template <int VPT>
 __global__ void __launch_bounds__(512, 2) bn_fwd_cluster_kernel(const float* x, float* y, const float* __restrict__ gamma, const float* __restrict__ beta,
                                                              float* run_mean, float* run_var, float* save_mean, float* save_istd,
-                                                             const BnGeo geo, int N, int C, int HW, int per_cta, float eps, float momentum, int relu, const float* __restrict__ add) {
+                                                             const BnGeo geo, int N, int C, int HW, int per_cta, float eps, float momentum, int relu, const float* __restrict__ add, const ZeroFill zero) {
   pdl_enter();
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned K = cluster.num_blocks(), r = cluster.block_rank();
@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(512, 2) bn_fwd_cluster_kernel(const float* x, 
       const int t = begin + j * (int)blockDim.x + (int)threadIdx.x;
       if (t < end) { int i; const int n = geo.hw4.divmod(t, i); keep[j] = reinterpret_cast<const float4*>(x + ((int64_t)n * C + c) * HW)[i]; }
     }
+    zero_fill(zero);                                                // while the loads are on their way
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       const int t = begin + j * (int)blockDim.x + (int)threadIdx.x;
@@ -316,6 +317,7 @@ __global__ void __launch_bounds__(512, 2) bn_fwd_cluster_kernel(const float* x, 
       }
     }
   } else {
+    zero_fill(zero);
 #pragma unroll 4
     for (int t = begin + (int)threadIdx.x; t < end; t += (int)blockDim.x) {
       int i; const int n = geo.hw4.divmod(t, i);
@@ -514,7 +516,7 @@ __device__ __forceinline__ void row_sum2(float& a, float& b, float* red) {
 template <int VPT>
 __global__ void __launch_bounds__(512, 2) bn_fwd_packed_kernel(const float* x, float* y, const float* __restrict__ gamma, const float* __restrict__ beta,
                                                             float* run_mean, float* run_var, float* save_mean, float* save_istd,
-                                                            const BnGeo geo, int N, int C, int HW, float eps, float momentum, int relu, const float* __restrict__ add) {
+                                                            const BnGeo geo, int N, int C, int HW, float eps, float momentum, int relu, const float* __restrict__ add, const BnExtra extra) {
   pdl_enter();
   __shared__ float red[32];
   __shared__ float stat[16][2];
@@ -533,6 +535,7 @@ __global__ void __launch_bounds__(512, 2) bn_fwd_packed_kernel(const float* x, f
     const int t = j * T + (int)threadIdx.x;
     if (live && t < total) { int i; const int n = geo.hw4.divmod(t, i); keep[j] = reinterpret_cast<const float4*>(x + ((int64_t)n * C + c) * HW)[i]; }
   }
+  zero_fill(extra.zero);                                                // while the loads are on their way
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const int t = j * T + (int)threadIdx.x;
@@ -565,6 +568,10 @@ __global__ void __launch_bounds__(512, 2) bn_fwd_packed_kernel(const float* x, f
       if (add) v = add4(v, reinterpret_cast<const float4*>(add + ((int64_t)n * C + c) * HW)[i]);
       if (relu) { v.x = v.x < 0.0f ? 0.0f : v.x; v.y = v.y < 0.0f ? 0.0f : v.y; v.z = v.z < 0.0f ? 0.0f : v.z; v.w = v.w < 0.0f ? 0.0f : v.w; }
       reinterpret_cast<float4*>(y + ((int64_t)n * C + c) * HW)[i] = v;
+      if (extra.cl) {
+        float* q = extra.cl + ((int64_t)n * HW + 4 * i) * C + c;
+        q[0] = v.x; q[C] = v.y; q[2 * C] = v.z; q[3 * C] = v.w;
+      }
     }
   }
 }
@@ -642,25 +649,32 @@ static int bn_splits(int N, int C) {
 
 // Issues a BN forward described by `p` (the cluster path), optionally with the ReLU of its result; a PEND_BN_ADD also adds
 // p.a and writes p.out instead of p.y.
-int bn_fwd_issue(const Pending& p, bool relu) {
+// The channels-last copy leaves a packed kernel as single floats, 4 C bytes apart: 16 us of stores per million of them (512 thousand, 256 x 4 x 4 at
+// batch 128: 12.2 us, 4.4 without the copy), where the copy as a launch of its own takes 3.5 us on the smallest maps and 5 on these.
+static bool bn_fwd_packed(const Pending& p, BnPackedPlan& pk) { return (bn_cluster_plan(p.N, p.C, p.HW).K == 1 || p.C >= 96) && bn_packed_plan(p.N, p.C, p.HW, kBnVpt, pk); }
+bool bn_fwd_writes_copy(const Pending& p) {
+  BnPackedPlan pk;
+  return p.C % 4 == 0 && (int64_t)p.N * p.C * p.HW <= (1 << 17) && bn_fwd_packed(p, pk);
+}
+int bn_fwd_issue(const Pending& p, bool relu, const BnExtra& extra) {
   const BnClusterPlan c = bn_cluster_plan(p.N, p.C, p.HW);
   const int r = relu ? 1 : 0;
   const float* add = p.kind == PEND_BN_ADD ? p.a : nullptr;
   float* y = p.kind == PEND_BN_ADD ? p.out : p.y;
   BnPackedPlan pk;
-  if ((c.K == 1 || p.C >= 96) && bn_packed_plan(p.N, p.C, p.HW, kBnVpt, pk)) {
+  if (bn_fwd_packed(p, pk)) {
     PdlUnlessLarge scope(ceil_div(p.C, pk.G));
     LTB_LAUNCH(bn_fwd_packed_kernel<kBnVpt>, (unsigned)ceil_div(p.C, pk.G), dim3(pk.T, pk.G), 0, p.x, y, p.gamma, p.beta, p.run_mean, p.run_var,
-               p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, p.eps, p.momentum, r, add);
+               p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, p.eps, p.momentum, r, add, extra);
     return LTB_OK;
   }
   PdlUnlessLarge scope((int64_t)p.C * c.K);
   if (c.per_cta <= kBnVpt * c.threads)
     LTB_LAUNCH_CLUSTER(bn_fwd_cluster_kernel<kBnVpt>, dim3((unsigned)p.C * c.K), dim3(c.threads), c.K, p.x, y, p.gamma, p.beta, p.run_mean, p.run_var,
-                       p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, c.per_cta, p.eps, p.momentum, r, add);
+                       p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, c.per_cta, p.eps, p.momentum, r, add, extra.zero);
   else
     LTB_LAUNCH_CLUSTER(bn_fwd_cluster_kernel<0>, dim3((unsigned)p.C * c.K), dim3(c.threads), c.K, p.x, y, p.gamma, p.beta, p.run_mean, p.run_var,
-                       p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, c.per_cta, p.eps, p.momentum, r, add);
+                       p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, c.per_cta, p.eps, p.momentum, r, add, extra.zero);
   return LTB_OK;
 }
 
