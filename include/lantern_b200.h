@@ -280,6 +280,45 @@ int LTB_FN(tree_node_bwd)(const ltb_tree_node* node);
 int LTB_FN(tree_nodes_fwd)(const ltb_tree_node* nodes_host, const ltb_tree_node* nodes_dev, int first, int count);
 int LTB_FN(tree_nodes_bwd)(const ltb_tree_node* nodes_host, const ltb_tree_node* nodes_dev, int first, int count);
 
+/* A whole tree of such nodes in one call each way: every inner node has the same parameters and so has every leaf.  The nodes are
+ * sorted by height, leaves first, the root last.  topo is an int32 array, on the host and (the same) in device memory: the nodes' left children
+ * [nodes], right children [nodes] (indices; -1 for leaves), scores [nodes], the leaves' rows of the table [nodes], and the first node of each level
+ * [levels + 1].  values: LTB_TREE_VALUES(hidden) floats per node, 16-byte aligned -- with p = LTB_TREE_PITCH(hidden): gates at 0, c at 5 p, tanh(c) at 6 p, h at 7 p, log
+ * probabilities at 8 p, accumulated loss at 8 p + 32.  grads: LTB_TREE_GRADS(hidden) floats per node -- dc at 0, dh at p, dloss at 2 p; the caller
+ * sets the root's dloss, the rest is zero before tree_bwd.  Results are those of tree_node_fwd / tree_node_bwd node by node with the
+ * children's second state (classify_cell ? h : c) feeding the cell and their first (classify_cell ? c : h) the gates.  Limits (LTB_E_LIMIT beyond: the calls per level and
+ * per node remain): hidden 160, in_len 320, 119 nodes. */
+#define LTB_TREE_PITCH(hidden) (((hidden) + 63) / 64 * 64)
+#define LTB_TREE_VALUES(hidden) (8 * LTB_TREE_PITCH(hidden) + 64)
+#define LTB_TREE_GRADS(hidden) (2 * LTB_TREE_PITCH(hidden) + 64)
+typedef struct ltb_tree {
+  int nodes;
+  int levels;
+  int hidden;
+  int in_len;                 /* length of a leaf's embedding */
+  int classes;                /* at most 32 */
+  int classify_cell;
+  const float* leaf_W[5];     /* slots 0, 3, 4: [hidden][in_len] */
+  float* leaf_dW[5];
+  const float* leaf_bias[5];
+  float* leaf_dbias[5];
+  const float* W[5][2];       /* [hidden][hidden] each */
+  float* dW[5][2];
+  const float* bias[5];       /* slots 1 and 2 may name the same vector */
+  float* dbias[5];
+  const float* Why;
+  const float* by;
+  float* dWhy;
+  float* dby;
+  const float* table;         /* embeddings, rows of in_len floats */
+  const int32_t* topo_host;
+  const int32_t* topo;
+  float* values;
+  float* grads;
+} ltb_tree;
+int LTB_FN(tree_fwd)(const ltb_tree* tree);
+int LTB_FN(tree_bwd)(const ltb_tree* tree);
+
 /* Branch regions (no counterpart in the reference, whose generated programs issue everything on one stream): two runs of
  * calls that do not depend on each other -- the shortcut convolution of a residual block and its main path, the two
  * expand convolutions of a fire module -- may overlap on the device.

@@ -12,7 +12,11 @@
 // log-softmax, and in the backward pass do_t Who^T and all five gradient sums -- runs as register-tiled matrix products
 // over the CTA's T x rows lines at once.  The CTAs' gradient sums are written to slabs and added into the gradient tensors
 // in CTA order by a second small launch (no atomics: the same bits on every run).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace ltb {
 
@@ -851,6 +855,518 @@ int ltb_tree_nodes_bwd(const ltb_tree_node* nodes_host, const ltb_tree_node* nod
     }
     LTB_LAUNCH(tree_nodes_bwd_kernel, dim3((unsigned)ctas, (unsigned)n), kNodeThreads, 0, nodes_dev + at);
   }
+  return LTB_OK;
+}
+
+}  // extern "C"
+
+// ------------------------------------------------------------------------------------------------------------------
+// A whole tree per call (ltb_tree_fwd / ltb_tree_bwd).
+//
+// Level by level (above) a level costs 10 us whatever it holds: a launch, the description, the weights out of L2, a counter, the combination by
+// the last CTA.  Here the chain of levels runs in ONE thread-block cluster of sixteen CTAs, a warp per hidden unit, and a level is one hardware cluster barrier.
+//   tree_leaves_fwd   all leaves, on the whole machine: a warp holds the three gate rows of a unit and takes every `shares`-th leaf.
+//   tree_chain_fwd    a warp holds the five gate rows of its unit (50 floats per lane) and computes gates, cell and hidden state of one node after the other; the two
+//                     states go into the shared memory of all CTAs, where the next level finds them.  Then a warp per node classifies.
+//   tree_chain_bwd    a warp holds the two columns of its unit (50 floats per lane): what reaches the unit in a node's children is the product of those
+//                     with the node's 5 Hd gate gradients.  Everything of a unit -- its states, its gradients in every node -- stays in the warp's own part
+//                     of shared memory; only the gate gradients are written to all CTAs.
+//   tree_weights_bwd  weight gradients on the whole machine: a warp per row, over all nodes in order (a bias that two gates share takes two atomic additions).
+// A grid-wide barrier on a counter in memory instead of the cluster's takes 6 us per level (25 leaves, nine levels: 70 us forward, 81 backward).
+// Bound: the chain, 0.8 us per level (barrier and exchange) and some 0.5 us per node forward, 0.8 backward; 25 leaves 9 + 33 us forward, 45 + 13 backward
+// (event-timed, with some 4 us of the event pair each; level by level 105 and 110 for the two directions), the step 202 -> 123 us.
+namespace ltb {
+
+constexpr int kTreeUnits = 160;                        // warps of a chain kernel: CTAS thread blocks of kTreeUnits / CTAS warps
+constexpr int kTreeHidden = kTreeUnits, kTreeIn = 320, kTreeNodes = 119, kTreeChunk = 8;      // limits; nodes whose gate gradients are exchanged at once
+constexpr int kTreeH = kTreeHidden / 32, kTreeI = kTreeIn / 32, kTreeR = 5 * kTreeHidden / 32;            // floats per lane: half a gate row, a leaf's row, a column
+
+struct TreeView {
+  const ltb_tree& t; int n, p;
+  const int32_t *left, *right, *score, *word, *first;
+  __device__ TreeView(const ltb_tree& t_) : t(t_), n(t_.nodes), p(LTB_TREE_PITCH(t_.hidden)), left(t_.topo), right(left + n), score(right + n), word(score + n), first(word + n) {}
+  __device__ float* V(int i) const { return t.values + (size_t)i * (8 * p + 64); }
+  __device__ float* G(int i) const { return t.grads + (size_t)i * (2 * p + 64); }
+  // a parent's gates read the first state of its children, its cell the second; the classifier reads the first
+  __device__ int first_state() const { return (t.classify_cell ? 5 : 7) * p; }
+  __device__ int second_state() const { return (t.classify_cell ? 7 : 5) * p; }
+};
+
+// Sums of five values over the warp in eight exchanges: a lane ends up with the total of gate five_of(lane) alone.
+__device__ __forceinline__ int five_of(int lane) { return lane & 4 ? 4 : (lane & 8 ? 2 : 0) + (lane & 16 ? 1 : 0); }
+__device__ __forceinline__ float warp_add_five(const float* a, int lane) {
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+  float v0 = (b4 ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, b4 ? a[0] : a[1], 16);
+  const float v1 = (b4 ? a[3] : a[2]) + __shfl_xor_sync(0xffffffffu, b4 ? a[2] : a[3], 16);
+  float v2 = a[4] + __shfl_xor_sync(0xffffffffu, a[4], 16);
+  v0 = (b3 ? v1 : v0) + __shfl_xor_sync(0xffffffffu, b3 ? v0 : v1, 8);
+  v2 += __shfl_xor_sync(0xffffffffu, v2, 8);
+  v0 = (b2 ? v2 : v0) + __shfl_xor_sync(0xffffffffu, b2 ? v0 : v2, 4);
+  v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
+  return v0 + __shfl_xor_sync(0xffffffffu, v0, 1);
+}
+
+__global__ void __launch_bounds__(kNodeThreads) tree_leaves_fwd_kernel(const ltb_tree tree, int shares) {
+  pdl_wait();
+  pdl_launch();                   // in this order: the chain kernel reads the weights before it waits for this one
+  const TreeView T(tree);
+  const int lane = threadIdx.x & 31, Hd = tree.hidden, L = tree.in_len;
+  const int at = (int)blockIdx.x * kNodeWarps + ((int)threadIdx.x >> 5), u = at % Hd, share = at / Hd;
+  if (share >= shares) return;
+  float w[3][kTreeI], bias[3];
+#pragma unroll
+  for (int g = 0; g < 3; ++g) {
+    const int slot = node_slot(false, g);
+    bias[g] = tree.leaf_bias[slot][u];
+#pragma unroll
+    for (int m = 0; m < kTreeI; ++m) { const int k = lane + 32 * m; w[g][m] = k < L ? tree.leaf_W[slot][(size_t)u * L + k] : 0.0f; }
+  }
+  const int leaves = T.first[1];
+  for (int i = share; i < leaves; i += 2 * shares) {           // two leaves' loads in flight; the weights beyond L are zero, so the index may be clamped
+    const int i1 = min(i + shares, leaves - 1);
+    const float* x0 = tree.table + (size_t)__ldg(T.word + i) * L; const float* x1 = tree.table + (size_t)__ldg(T.word + i1) * L;
+    float a[6] = {};
+    float v0[kTreeI], v1[kTreeI];
+#pragma unroll
+    for (int m = 0; m < kTreeI; ++m) { const int k = min(lane + 32 * m, L - 1); v0[m] = __ldg(x0 + k); v1[m] = __ldg(x1 + k); }
+#pragma unroll
+    for (int m = 0; m < kTreeI; ++m)
+#pragma unroll
+      for (int g = 0; g < 3; ++g) { a[g] += w[g][m] * v0[m]; a[3 + g] += w[g][m] * v1[m]; }
+#pragma unroll
+    for (int g = 0; g < 6; ++g) a[g] = warp_add(a[g]) + bias[g % 3];
+    if (lane < 2 && (lane == 0 || i + shares < leaves)) {
+      const float ig = act_apply(0, lane ? a[3] : a[0]), og = act_apply(3, lane ? a[4] : a[1]), uv = act_apply(4, lane ? a[5] : a[2]), c = ig * uv, tc = tanhf(c);
+      float* v = T.V(lane ? i + shares : i);
+      v[u] = ig; v[3 * Hd + u] = og; v[4 * Hd + u] = uv;
+      v[5 * T.p + u] = c; v[6 * T.p + u] = tc; v[7 * T.p + u] = og * tc;
+    }
+  }
+}
+
+// This CTA's units of `rows` vectors of Hs floats into the same place of the other CTAs, eight bytes at a time (a float at a time from each unit's warp
+// the network between the SMs takes 1.5 us per node).
+template <int CTAS>
+__device__ __forceinline__ void tree_spread(const cg::cluster_group& cluster, float* v, int rows, int Hs, int rank) {
+  constexpr int kWarps = kTreeUnits / CTAS, kParts = kWarps / 2;
+  for (int i = threadIdx.x; i < rows * CTAS * kParts; i += 32 * kWarps) {
+    const int rest = i / kParts, row = rest / CTAS, to = rest - row * CTAS, at = rank * kWarps + (i - rest * kParts) * 2;
+    if (to == rank || at >= Hs) continue;
+    float* p = v + (size_t)row * Hs + at;
+    *reinterpret_cast<float2*>(cluster.map_shared_rank(p, to)) = *reinterpret_cast<const float2*>(p);
+  }
+}
+// Shared memory: state [node][2][Hs] (first, second; Hs = hidden rounded up to 32, zeros beyond hidden), kept [unit of the CTA][inner node][8] (gates, c, tanh c,
+// h: they go to memory at the end, because a cluster barrier waits for every store to memory before it), why [classes][hidden], loss [node], left,
+// right [node], first [levels + 1].
+template <int CTAS>
+__global__ void __launch_bounds__(32 * kTreeUnits / CTAS, 1) tree_chain_fwd_kernel(const ltb_tree tree) {
+  constexpr int kWarps = kTreeUnits / CTAS, kThreads = 32 * kWarps;
+  extern __shared__ float sm[];
+  const TreeView T(tree);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster.block_rank();
+  const int Hd = tree.hidden, Hs = (Hd + 31) / 32 * 32, n = T.n, u = rank * kWarps + warp;
+  const int inner = n / 2;                                   // of n nodes, in a tree of which every inner node has two children
+  const int K = tree.classes;
+  float* state = sm; float* kept = state + (size_t)n * 2 * Hs; float* why = kept + (size_t)kWarps * inner * 8; float* loss = why + K * Hd;
+  int* left = reinterpret_cast<int*>(loss + n); int* right = left + n; int* first = right + n;
+  pdl_launch();
+  float w0[5][kTreeH], w1[5][kTreeH], bias = 0.0f;
+#pragma unroll
+  for (int g = 0; g < 5; ++g)
+#pragma unroll
+    for (int m = 0; m < kTreeH; ++m) {
+      const int k = lane + 32 * m; const bool ok = u < Hd && k < Hd && tree.levels > 1;
+      w0[g][m] = ok ? tree.W[g][0][(size_t)u * Hd + k] : 0.0f; w1[g][m] = ok ? tree.W[g][1][(size_t)u * Hd + k] : 0.0f;
+    }
+  const int my_gate = five_of(lane);
+  if (u < Hd && tree.levels > 1) bias = tree.bias[my_gate][u];
+  pdl_wait();
+  for (int i = tid; i < n; i += kThreads) { left[i] = T.left[i]; right[i] = T.right[i]; }
+  for (int i = tid; i <= tree.levels; i += kThreads) first[i] = T.first[i];
+  const int leaves = T.first[1], quads = leaves * 2 * (Hs / 4);
+  for (int i = tid; i < K * Hd; i += kThreads) why[i] = tree.Why[i];
+  for (int i = quads + tid; i < n * 2 * (Hs / 4); i += kThreads) reinterpret_cast<float4*>(state)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i0 = tid; i0 < quads; i0 += 4 * kThreads) {   // the leaves' states, four loads of a thread in flight
+    float4 v[4]; int k[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + e * kThreads, row = i / (Hs / 4), q = row >> 1;
+      k[e] = (i - row * (Hs / 4)) * 4;
+      v[e] = i < quads && k[e] < Hd ? __ldg(reinterpret_cast<const float4*>(T.V(q) + (row & 1 ? T.second_state() : T.first_state()) + k[e])) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + e * kThreads;
+      if (k[e] + 1 >= Hd) v[e].y = 0.0f;
+      if (k[e] + 2 >= Hd) v[e].z = 0.0f;
+      if (k[e] + 3 >= Hd) v[e].w = 0.0f;
+      if (i < quads) reinterpret_cast<float4*>(state)[i] = v[e];
+    }
+  }
+  cluster.sync();                                            // before the first write from another CTA
+  for (int level = 1; level < tree.levels; ++level) {
+    const int begin = first[level], end = first[level + 1];
+    float* const mine = kept + ((size_t)warp * inner + begin - leaves) * 8;      // this unit's values of the level's nodes
+    if (u < Hd) {
+      // the products, two nodes at a time (one after the other their latencies add up: 1800 cycles a node with the gates below)
+      for (int q = begin; q < end; q += 2) {
+        const int q1 = min(q + 1, end - 1);
+        const float* x[4] = {state + (size_t)left[q] * 2 * Hs, state + (size_t)right[q] * 2 * Hs, state + (size_t)left[q1] * 2 * Hs, state + (size_t)right[q1] * 2 * Hs};
+        float a[2][5] = {};
+#pragma unroll
+        for (int m = 0; m < kTreeH; ++m) {
+          if (32 * m >= Hs) break;
+          float v[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = x[e][lane + 32 * m];
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int g = 0; g < 5; ++g) a[e][g] += w0[g][m] * v[2 * e] + w1[g][m] * v[2 * e + 1];
+        }
+        const float p0 = warp_add_five(a[0], lane) + bias, p1 = warp_add_five(a[1], lane) + bias;
+        if ((lane & 3) == 0 && (lane < 5 || !(lane & 4))) { mine[(q - begin) * 8 + my_gate] = p0; mine[(q1 - begin) * 8 + my_gate] = p1; }
+      }
+      __syncwarp();
+      // the gates and the cell, a lane per node
+      for (int i = lane; i < end - begin; i += 32) {
+        float* v = mine + i * 8;
+        const float ig = act_apply(0, v[0]), fl = act_apply(1, v[1]), fr = act_apply(2, v[2]), og = act_apply(3, v[3]), uv = act_apply(4, v[4]);
+        const int q = begin + i;
+        const float c = (ig * uv + fl * state[(size_t)(2 * left[q] + 1) * Hs + u]) + fr * state[(size_t)(2 * right[q] + 1) * Hs + u], tc = tanhf(c), h = og * tc;
+        *reinterpret_cast<float4*>(v) = make_float4(ig, fl, fr, og); *reinterpret_cast<float4*>(v + 4) = make_float4(uv, c, tc, h);
+        state[(size_t)2 * q * Hs + u] = tree.classify_cell ? c : h; state[(size_t)(2 * q + 1) * Hs + u] = tree.classify_cell ? h : c;
+      }
+    }
+    __syncthreads();
+    tree_spread<CTAS>(cluster, state + (size_t)begin * 2 * Hs, 2 * (end - begin), Hs, rank);
+    cluster.sync();                                          // the level's states are in every CTA
+  }
+  for (int i = tid; i < inner * 8 * kWarps; i += kThreads) {          // neighbouring threads on neighbouring units
+    const int ne = i / kWarps, a = i - ne * kWarps, q = ne >> 3, e = ne & 7, unit = rank * kWarps + a;
+    if (unit < Hd) T.V(leaves + q)[(e < 5 ? e * Hd : e * T.p) + unit] = kept[((size_t)a * inner + q) * 8 + e];
+  }
+  // log probabilities and each node's own part of the loss: a warp per node, the parts gathered by CTA 0
+  float* const loss0 = cluster.map_shared_rank(loss, 0);
+  for (int i = rank * kWarps + warp; i < n; i += CTAS * kWarps) {
+    const float* x = state + (size_t)i * 2 * Hs;
+    float o = -3.4028235e38f;
+    for (int k = 0; k < K; ++k) {
+      float a = 0.0f;
+      for (int j = lane; j < Hd; j += 32) a += why[k * Hd + j] * x[j];
+      a = warp_add(a);
+      if (lane == k) o = a + tree.by[k];
+    }
+    const float m = warp_max(o), lse = m + logf(warp_add(lane < K ? expf(o - m) : 0.0f));
+    if (lane < K) T.V(i)[8 * T.p + lane] = o - lse;
+    if (lane == T.score[i]) loss0[i] = -(o - lse);
+  }
+  cluster.sync();
+  if (rank != 0 || warp != 0) return;
+  for (int level = 0; level < tree.levels; ++level) {
+    for (int i = first[level] + lane; i < first[level + 1]; i += 32) {
+      const float v = level == 0 ? loss[i] : (loss[i] + loss[left[i]]) + loss[right[i]];
+      loss[i] = v; T.V(i)[8 * T.p + 32] = v;
+    }
+    __syncwarp();
+  }
+}
+
+// work: per node 5 Hd gate gradients and 32 of the classifier, for tree_weights_bwd.
+// Shared memory: dpre [2][kTreeChunk][5][Hs] (Hs as above), per unit of the CTA and node eight values (five gates, tanh c, the children's second states) and
+// two gradients (first, second state) and the five gate gradients (to memory at the end, as above), why [classes][unit], dpred [node][classes], dloss [node], left, right [node], first [levels + 1].
+template <int CTAS>
+__global__ void __launch_bounds__(32 * kTreeUnits / CTAS, 1) tree_chain_bwd_kernel(const ltb_tree tree, float* work) {
+  constexpr int kWarps = kTreeUnits / CTAS, kThreads = 32 * kWarps;
+  extern __shared__ float sm[];
+  const TreeView T(tree);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster.block_rank();
+  const int Hd = tree.hidden, Hs = (Hd + 31) / 32 * 32, K = tree.classes, n = T.n, R = 5 * Hs, u0 = rank * kWarps, u = u0 + warp, wstride = 5 * Hd + 32;
+  float* dpre = sm; float* vals = dpre + 2 * kTreeChunk * R; float* grad = vals + (size_t)kWarps * n * 8; float* kept = grad + (size_t)kWarps * n * 2; float* why = kept + (size_t)kWarps * n * 5;
+  float* dpred = why + K * kWarps; float* dloss = dpred + n * K;
+  int* left = reinterpret_cast<int*>(dloss + n); int* right = left + n; int* first = right + n;
+  pdl_enter();
+  float w0[kTreeR], w1[kTreeR];
+#pragma unroll
+  for (int m = 0; m < kTreeR; ++m) {
+    const int g = 32 * m / Hs, j = lane + 32 * m - g * Hs; const bool ok = u < Hd && g < 5 && j < Hd && tree.levels > 1;
+    w0[m] = ok ? tree.W[g][0][(size_t)j * Hd + u] : 0.0f; w1[m] = ok ? tree.W[g][1][(size_t)j * Hd + u] : 0.0f;
+  }
+  const int leaves = T.first[1], second = T.second_state();
+  for (int i = tid; i < n; i += kThreads) { left[i] = T.left[i]; right[i] = T.right[i]; dloss[i] = T.G(i)[2 * T.p]; }
+  for (int i = tid; i <= tree.levels; i += kThreads) first[i] = T.first[i];
+  for (int i = tid; i < 2 * kTreeChunk * R; i += kThreads) dpre[i] = 0.0f;
+  for (int i = tid; i < K * kWarps; i += kThreads) { const int k = i / kWarps, a = u0 + i - k * kWarps; why[i] = a < Hd ? tree.Why[(size_t)k * Hd + a] : 0.0f; }
+  for (int i0 = tid; i0 < n * 10 * kWarps; i0 += 8 * kThreads) {      // neighbouring threads on neighbouring units, eight loads of a thread in flight
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int i = i0 + j * kThreads, nu = i / kWarps, a = i - nu * kWarps, q = nu / 10, e = nu - q * 10;
+      v[j] = 0.0f;
+      if (q < n && u0 + a < Hd) {
+        const float* at = nullptr;
+        if (e < 5) at = e == 0 || e > 2 || q >= leaves ? T.V(q) + e * Hd : nullptr;
+        else if (e == 5) at = T.V(q) + 6 * T.p;
+        else if (e < 8) at = q >= leaves ? T.V(e == 6 ? __ldg(T.left + q) : __ldg(T.right + q)) + second : nullptr;
+        else at = T.G(q) + ((e == 8) == (tree.classify_cell != 0) ? 0 : T.p);           // first: dc where the cell is classified, else dh
+        if (at) v[j] = at[u0 + a];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int i = i0 + j * kThreads, nu = i / kWarps, a = i - nu * kWarps, q = nu / 10, e = nu - q * 10;
+      if (q < n) { if (e < 8) vals[((size_t)a * n + q) * 8 + e] = v[j]; else grad[((size_t)a * n + q) * 2 + e - 8] = v[j]; }
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {                                           // the loss gradient goes down the tree unchanged
+    for (int level = tree.levels - 1; level > 0; --level) {
+      for (int q = first[level] + lane; q < first[level + 1]; q += 32) { dloss[left[q]] += dloss[q]; dloss[right[q]] += dloss[q]; }
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < n * K; i += kThreads) {          // nllLoss_grad, logSoftmax_grad
+    const int q = i / K, k = i - q * K;
+    const float d = dloss[q] * (expf(T.V(q)[8 * T.p + k]) - (k == T.score[q] ? 1.0f : 0.0f));
+    dpred[i] = d;
+  }
+  if (rank == 0) for (int i = tid; i < n; i += kThreads) T.G(i)[2 * T.p] = dloss[i];
+  cluster.sync();                                            // shared memory of every CTA is set up
+  float* const my_vals = vals + (size_t)warp * n * 8; float* const my_grad = grad + (size_t)warp * n * 2;
+  // gate gradients of node q at this warp's unit; the children's second states get theirs
+  auto gates_of = [&](int q, bool inner, float* d) {
+    const float* v = my_vals + (size_t)q * 8;
+    float dfirst = my_grad[q * 2];
+    const float dsecond = my_grad[q * 2 + 1];
+    float dcls = 0.0f;
+    for (int k = 0; k < K; ++k) dcls += why[k * kWarps + warp] * dpred[q * K + k];
+    dfirst += dcls;
+    const float dc = tree.classify_cell ? dfirst : dsecond, dh = tree.classify_cell ? dsecond : dfirst;
+    const float ig = v[0], fl = v[1], fr = v[2], og = v[3], uv = v[4], tc = v[5];
+    const float dct = dc + dh * og * (1.0f - tc * tc);
+    d[0] = (dct * uv) * ig * (1.0f - ig); d[3] = (dh * tc) * og * (1.0f - og); d[4] = (dct * ig) * (1.0f - uv * uv);
+    d[1] = (dct * v[6]) * fl * (1.0f - fl); d[2] = (dct * v[7]) * fr * (1.0f - fr);       // zero in a leaf
+    if (inner) { my_grad[left[q] * 2 + 1] += dct * fl; my_grad[right[q] * 2 + 1] += dct * fr; }
+    float* o = kept + ((size_t)warp * n + q) * 5;
+#pragma unroll
+    for (int e = 0; e < 5; ++e) o[e] = d[e];
+  };
+  int turn = 0;
+  for (int level = tree.levels - 1; level > 0; --level)
+    for (int q0 = first[level]; q0 < first[level + 1]; q0 += kTreeChunk, turn ^= 1) {
+      const int nq = min(kTreeChunk, first[level + 1] - q0);
+      float* const buf = dpre + (size_t)turn * kTreeChunk * R;
+      if (u < Hd && lane < nq) {
+        float d[5];
+        gates_of(q0 + lane, true, d);
+#pragma unroll
+        for (int e = 0; e < 5; ++e) buf[(size_t)lane * R + e * Hs + u] = d[e];
+      }
+      __syncthreads();
+      tree_spread<CTAS>(cluster, buf, 5 * nq, Hs, rank);
+      // everybody has the chunk's gate gradients; the buffer of the chunk before is free again once all have met the next time
+      cluster.sync();
+      if (u < Hd)
+        for (int b = 0; b < nq; b += 2) {                    // two nodes at a time
+          const int b1 = min(b + 1, nq - 1);
+          float a[4] = {};
+#pragma unroll
+          for (int m = 0; m < kTreeR; ++m) {
+            if (32 * m >= R) break;
+            const float x0 = buf[(size_t)b * R + lane + 32 * m], x1 = buf[(size_t)b1 * R + lane + 32 * m];
+            a[0] += w0[m] * x0; a[1] += w1[m] * x0; a[2] += w0[m] * x1; a[3] += w1[m] * x1;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] = warp_add(a[e]);
+          if (lane < (b1 > b ? 4 : 2)) {
+            const int q = q0 + (lane < 2 ? b : b1);
+            my_grad[(lane & 1 ? right[q] : left[q]) * 2] += lane == 0 ? a[0] : lane == 1 ? a[1] : lane == 2 ? a[2] : a[3];
+          }
+        }
+      __syncwarp();
+    }
+  if (u < Hd) for (int q = lane; q < leaves; q += 32) { float d[5]; gates_of(q, false, d); }
+  __syncthreads();
+  for (int i = tid; i < n * 2 * kWarps; i += kThreads) {             // what the nodes' gradients have become
+    const int nu = i / kWarps, a = i - nu * kWarps, q = nu >> 1, e = nu & 1;
+    if (u0 + a < Hd) T.G(q)[((e == 0) == (tree.classify_cell != 0) ? 0 : T.p) + u0 + a] = grad[((size_t)a * n + q) * 2 + e];
+  }
+  for (int i = tid; i < n * 5 * kWarps; i += kThreads) {
+    const int ne = i / kWarps, a = i - ne * kWarps, q = ne / 5, e = ne - q * 5;
+    if (u0 + a < Hd) work[(size_t)q * wstride + e * Hd + u0 + a] = kept[((size_t)a * n + q) * 5 + e];
+  }
+  if (rank == 0)
+    for (int i = tid; i < n * K; i += kThreads) { const int q = i / K, k = i - q * K; work[(size_t)q * wstride + 5 * Hd + k] = dpred[i]; }
+  cluster.sync();                                            // nobody leaves while its shared memory may still be written
+}
+
+// acc[m] += dp(q) x(q)[m] over the nodes lo <= q < hi, NB nodes' loads in flight; x writes M floats.  Returns the sum of dp.
+template <int M, int NB, class DP, class X>
+__device__ __forceinline__ float tree_outer(float* acc, int lo, int hi, const DP& dp, const X& x) {
+  float total = 0.0f;
+  for (int q = lo; q < hi; q += NB) {
+    float v[NB][M], d[NB];
+#pragma unroll
+    for (int e = 0; e < NB; ++e) { const int i = min(q + e, hi - 1); d[e] = q + e < hi ? dp(i) : 0.0f; x(i, v[e]); }
+#pragma unroll
+    for (int e = 0; e < NB; ++e) {
+      total += d[e];
+#pragma unroll
+      for (int m = 0; m < M; ++m) acc[m] += d[e] * v[e][m];
+    }
+  }
+  return total;
+}
+// M floats of a vector of `len`, lane + 32 m; the index is clamped, not tested: what comes of the rest is not stored.
+template <int M>
+__device__ __forceinline__ void tree_lane(float* v, const float* p, int lane, int len) {
+#pragma unroll
+  for (int m = 0; m < M; ++m) v[m] = __ldg(p + min(lane + 32 * m, len - 1));
+}
+__global__ void __launch_bounds__(kNodeThreads) tree_weights_bwd_kernel(const ltb_tree tree, const float* __restrict__ work) {
+  pdl_enter();
+  __shared__ int left[kTreeNodes], right[kTreeNodes], word[kTreeNodes];
+  const TreeView T(tree);
+  const int lane = threadIdx.x & 31, Hd = tree.hidden, L = tree.in_len, K = tree.classes, wstride = 5 * Hd + 32;
+  if ((int)threadIdx.x < T.n) { left[threadIdx.x] = T.left[threadIdx.x]; right[threadIdx.x] = T.right[threadIdx.x]; word[threadIdx.x] = T.word[threadIdx.x]; }
+  __syncthreads();
+  const int leaves = T.first[1], inner_rows = 5 * Hd, leaf_rows = 3 * Hd, s = T.first_state();
+  int item = (int)blockIdx.x * kNodeWarps + ((int)threadIdx.x >> 5);
+  float acc[kTreeI], total = 0.0f;
+#pragma unroll
+  for (int m = 0; m < kTreeI; ++m) acc[m] = 0.0f;
+  if (item < inner_rows) {
+    if (leaves == T.n) return;                               // a single leaf: the inner gates may not even exist
+    const int g = item / Hd, u = item - g * Hd;
+    float* d0 = tree.dW[g][0] + (size_t)u * Hd; float* d1 = tree.dW[g][1] + (size_t)u * Hd;
+    float old[kTreeI];
+#pragma unroll
+    for (int m = 0; m < kTreeH; ++m) { const int k = lane + 32 * m; old[m] = k < Hd ? d0[k] : 0.0f; old[kTreeH + m] = k < Hd ? d1[k] : 0.0f; }
+    total = tree_outer<kTreeI, 5>(acc, leaves, T.n, [&](int q) { return __ldg(work + (size_t)q * wstride + item); },
+                                  [&](int q, float* v) { tree_lane<kTreeH>(v, T.V(left[q]) + s, lane, Hd); tree_lane<kTreeH>(v + kTreeH, T.V(right[q]) + s, lane, Hd); });
+#pragma unroll
+    for (int m = 0; m < kTreeH; ++m) { const int k = lane + 32 * m; if (k < Hd) { d0[k] = old[m] + acc[m]; d1[k] = old[kTreeH + m] + acc[kTreeH + m]; } }
+    if (lane == 0) atomicAdd(tree.dbias[g] + u, total);
+    return;
+  }
+  item -= inner_rows;
+  if (item < leaf_rows) {
+    const int g = node_slot(false, item / Hd), u = item % Hd;
+    float* d0 = tree.leaf_dW[g] + (size_t)u * L;
+    float old[kTreeI];
+#pragma unroll
+    for (int m = 0; m < kTreeI; ++m) { const int k = lane + 32 * m; old[m] = k < L ? d0[k] : 0.0f; }
+    total = tree_outer<kTreeI, 5>(acc, 0, leaves, [&](int q) { return __ldg(work + (size_t)q * wstride + g * Hd + u); }, [&](int q, float* v) { tree_lane<kTreeI>(v, tree.table + (size_t)word[q] * L, lane, L); });
+#pragma unroll
+    for (int m = 0; m < kTreeI; ++m) { const int k = lane + 32 * m; if (k < L) d0[k] = old[m] + acc[m]; }
+    if (lane == 0) atomicAdd(tree.leaf_dbias[g] + u, total);
+    return;
+  }
+  item -= leaf_rows;
+  if (item >= K) return;
+  total = tree_outer<kTreeH, 10>(acc, 0, T.n, [&](int q) { return __ldg(work + (size_t)q * wstride + 5 * Hd + item); }, [&](int q, float* v) { tree_lane<kTreeH>(v, T.V(q) + s, lane, Hd); });
+#pragma unroll
+  for (int m = 0; m < kTreeH; ++m) { const int u = lane + 32 * m; if (u < Hd) tree.dWhy[(size_t)item * Hd + u] += acc[m]; }
+  if (lane == 0) tree.dby[item] += total;
+}
+
+static size_t tree_smem_fwd(const ltb_tree& t, int ctas) {
+  return ((size_t)t.nodes * (2 * ((t.hidden + 31) / 32 * 32) + 3) + (size_t)(kTreeUnits / ctas) * (t.nodes / 2) * 8 + (size_t)t.classes * t.hidden + t.levels + 1) * 4;
+}
+static size_t tree_smem_bwd(const ltb_tree& t, int ctas) {
+  return ((size_t)2 * kTreeChunk * 5 * ((t.hidden + 31) / 32 * 32) + (size_t)(kTreeUnits / ctas) * ((size_t)t.nodes * 15 + t.classes) + (size_t)t.nodes * (t.classes + 3) + t.levels + 1) * 4;
+}
+static int tree_check(const ltb_tree* t, bool grads, const char* who) {
+  LTB_REQUIRE(t && t->nodes > 0 && t->levels > 0 && t->hidden > 0 && t->in_len > 0 && t->classes > 0 && t->classes <= 32, "%s: bad argument", who);
+  if (t->hidden > kTreeHidden || t->in_len > kTreeIn || t->nodes > kTreeNodes) return fail(LTB_E_LIMIT, "%s: hidden at most %d, in_len %d, %d nodes", who, kTreeHidden, kTreeIn, kTreeNodes);
+  LTB_REQUIRE(aligned16(t->values), "%s: values must be 16-byte aligned", who);
+  LTB_REQUIRE(t->Why && t->by && t->table && t->topo && t->topo_host && t->values && (!grads || (t->grads && t->dWhy && t->dby)), "%s: missing operand", who);
+  for (int s = 0; s < 5; ++s) {
+    LTB_REQUIRE(s == 1 || s == 2 || (t->leaf_W[s] && t->leaf_bias[s] && (!grads || (t->leaf_dW[s] && t->leaf_dbias[s]))), "%s: missing gate of the leaves", who);
+    LTB_REQUIRE(t->levels == 1 || (t->W[s][0] && t->W[s][1] && t->bias[s] && (!grads || (t->dW[s][0] && t->dW[s][1] && t->dbias[s]))), "%s: missing gate", who);
+  }
+  // the topology the kernels will follow: levels in order, every child in a level below and of one parent
+  const int n = t->nodes; const int32_t *left = t->topo_host, *right = left + n, *score = right + n, *word = score + n, *first = word + n;
+  LTB_REQUIRE(t->levels <= n && first[0] == 0 && first[t->levels] == n, "%s: levels do not cover the nodes", who);
+  bool taken[kTreeNodes] = {};
+  for (int l = 0; l < t->levels; ++l) {
+    LTB_REQUIRE(first[l] < first[l + 1] && first[l + 1] <= n, "%s: bad level", who);
+    for (int i = first[l]; i < first[l + 1]; ++i) {
+      LTB_REQUIRE(score[i] >= 0 && score[i] < t->classes, "%s: score out of range", who);
+      if (l == 0) LTB_REQUIRE(left[i] < 0 && word[i] >= 0, "%s: bad leaf", who);
+      else {
+        LTB_REQUIRE(left[i] >= 0 && right[i] >= 0 && left[i] < first[l] && right[i] < first[l], "%s: a child is not below its parent", who);
+        LTB_REQUIRE(left[i] != right[i] && !taken[left[i]] && !taken[right[i]], "%s: a node with two parents", who);
+        taken[left[i]] = taken[right[i]] = true;
+      }
+    }
+  }
+  return LTB_OK;
+}
+// CTAs of the chain kernels' cluster: sixteen, twice the warps per SM of eight, where the device takes a cluster of that size (25 leaves, before the
+// products went two nodes at a time: 43 us forward, 48 with eight), else eight, which every device does.  0: the kernels could not be set up.
+template <int CTAS>
+static bool tree_set_up() {
+  const int smem = 220 * 1024;
+  bool ok = cudaFuncSetAttribute(tree_chain_fwd_kernel<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+            cudaFuncSetAttribute(tree_chain_bwd_kernel<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+  if (ok && CTAS > 8) {
+    ok = cudaFuncSetAttribute(tree_chain_fwd_kernel<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+         cudaFuncSetAttribute(tree_chain_bwd_kernel<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CTAS); cfg.blockDim = dim3(32 * kTreeUnits / CTAS); cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int f = 0, b = 0;
+    ok = ok && cudaOccupancyMaxActiveClusters(&f, tree_chain_fwd_kernel<CTAS>, &cfg) == cudaSuccess && f > 0 &&
+         cudaOccupancyMaxActiveClusters(&b, tree_chain_bwd_kernel<CTAS>, &cfg) == cudaSuccess && b > 0;
+  }
+  cudaGetLastError();
+  return ok;
+}
+static int tree_ctas() {
+  static int device = -1, ctas = 0;
+  if (device != g.device) { ctas = tree_set_up<16>() ? 16 : tree_set_up<8>() ? 8 : 0; device = g.device; }
+  return ctas;
+}
+
+}  // namespace ltb
+
+extern "C" {
+
+int ltb_tree_fwd(const ltb_tree* t) {
+  LTB_INITED();
+  if (int rc = tree_check(t, false, "ltb_tree_fwd")) return rc;
+  const int ctas = tree_ctas();
+  if (!ctas) return fail(LTB_E_CUDA, "the tree kernels could not be set up");
+  LTB_WRITES(t->values, (size_t)t->nodes * LTB_TREE_VALUES(t->hidden));
+  const int leaves = t->topo_host[4 * t->nodes + 1];
+  int shares = g.sm_count * kNodeWarps / t->hidden;           // a warp per unit and share of the leaves, a CTA per SM
+  shares = shares < 1 ? 1 : shares > leaves ? leaves : shares;
+  LTB_LAUNCH(tree_leaves_fwd_kernel, (unsigned)ceil_div((int64_t)shares * t->hidden, kNodeWarps), kNodeThreads, 0, *t, shares);
+  const unsigned threads = 32 * kTreeUnits / ctas;
+  if (ctas == 16) LTB_LAUNCH_CLUSTER_XZ(tree_chain_fwd_kernel<16>, dim3(16), dim3(threads), 16, 1, tree_smem_fwd(*t, 16), *t);
+  else LTB_LAUNCH_CLUSTER_XZ(tree_chain_fwd_kernel<8>, dim3(8), dim3(threads), 8, 1, tree_smem_fwd(*t, 8), *t);
+  return LTB_OK;
+}
+int ltb_tree_bwd(const ltb_tree* t) {
+  LTB_INITED();
+  if (int rc = tree_check(t, true, "ltb_tree_bwd")) return rc;
+  const int ctas = tree_ctas();
+  if (!ctas) return fail(LTB_E_CUDA, "the tree kernels could not be set up");
+  filter_cache_note_write(nullptr, 0);                  // what it writes is a score of vectors: everything is taken as stale
+  const size_t need = (size_t)t->nodes * (5 * t->hidden + 32) * 4;
+  if (need > g.cur_scratch_bytes()) return fail(LTB_E_LIMIT, "ltb_tree_bwd: too many nodes for the library's workspace");
+  float* work = g.cur_scratch();
+  const unsigned threads = 32 * kTreeUnits / ctas;
+  if (ctas == 16) LTB_LAUNCH_CLUSTER_XZ(tree_chain_bwd_kernel<16>, dim3(16), dim3(threads), 16, 1, tree_smem_bwd(*t, 16), *t, work);
+  else LTB_LAUNCH_CLUSTER_XZ(tree_chain_bwd_kernel<8>, dim3(8), dim3(threads), 8, 1, tree_smem_bwd(*t, 8), *t, work);
+  LTB_LAUNCH(tree_weights_bwd_kernel, (unsigned)ceil_div(8 * t->hidden + t->classes, kNodeWarps), kNodeThreads, 0, *t, (const float*)work);
   return LTB_OK;
 }
 

@@ -1332,6 +1332,52 @@ int ora_tree_nodes_bwd(const ltb_tree_node* nodes_host, const ltb_tree_node*, in
   for (int i = first; i < first + count; ++i) { int rc = ora_tree_node_bwd(nodes_host + i); if (rc) return rc; }
   return LTB_OK;
 }
+// A whole tree: its nodes one after the other, children before parents and back.
+static bool tree_nodes_of(const ltb_tree* t, std::vector<ltb_tree_node>& v) {
+  if (!t || t->nodes < 1 || t->levels < 1 || t->hidden < 1 || t->in_len < 1 || !t->topo_host || !t->values || !t->table) return false;
+  const int n = t->nodes, p = LTB_TREE_PITCH(t->hidden);
+  const int32_t *left = t->topo_host, *right = left + n, *score = right + n, *word = score + n;
+  v.assign((size_t)n, ltb_tree_node{});
+  auto V = [&](int i) { return t->values + (size_t)i * LTB_TREE_VALUES(t->hidden); };
+  auto G = [&](int i) { return t->grads ? t->grads + (size_t)i * LTB_TREE_GRADS(t->hidden) : nullptr; };
+  const int cc = t->classify_cell;
+  for (int i = 0; i < n; ++i) {
+    ltb_tree_node& q = v[(size_t)i];
+    q.hidden = t->hidden; q.classes = t->classes; q.classify_cell = cc; q.inner = left[i] >= 0;
+    if (!q.inner) {
+      q.in_len = t->in_len; q.in[0] = t->table + (size_t)word[i] * t->in_len;
+      for (int g : {0, 3, 4}) { q.W[g][0] = t->leaf_W[g]; q.dW[g][0] = t->leaf_dW[g]; q.bias[g] = t->leaf_bias[g]; q.dbias[g] = t->leaf_dbias[g]; }
+    } else {
+      const int kid[2] = {left[i], right[i]};
+      q.in_len = t->hidden;
+      for (int k = 0; k < 2; ++k) { q.in[k] = V(kid[k]) + (cc ? 5 : 7) * p; if (t->grads) q.din[k] = G(kid[k]) + (cc ? 0 : p); }
+      q.cl = V(kid[0]) + (cc ? 7 : 5) * p; q.cr = V(kid[1]) + (cc ? 7 : 5) * p;
+      q.loss_l = V(kid[0]) + 8 * p + 32; q.loss_r = V(kid[1]) + 8 * p + 32;
+      if (t->grads) {
+        q.dcl = G(kid[0]) + (cc ? p : 0); q.dcr = G(kid[1]) + (cc ? p : 0);
+        q.dloss_l = G(kid[0]) + 2 * p; q.dloss_r = G(kid[1]) + 2 * p;
+      }
+      for (int g = 0; g < 5; ++g) { for (int k = 0; k < 2; ++k) { q.W[g][k] = t->W[g][k]; q.dW[g][k] = t->dW[g][k]; } q.bias[g] = t->bias[g]; q.dbias[g] = t->dbias[g]; }
+    }
+    q.Why = t->Why; q.by = t->by; q.dWhy = t->dWhy; q.dby = t->dby; q.score = score + i;
+    float* x = V(i); float* d = G(i);
+    q.gates = x; q.c = x + 5 * p; q.tc = x + 6 * p; q.h = x + 7 * p; q.logp = x + 8 * p; q.loss = x + 8 * p + 32;
+    if (d) { q.dc = d; q.dh = d + p; q.dloss = d + 2 * p; }
+  }
+  return true;
+}
+int ora_tree_fwd(const ltb_tree* t) {
+  std::vector<ltb_tree_node> v;
+  REQUIRE(tree_nodes_of(t, v), "tree_fwd: bad argument");
+  for (auto& q : v) { int rc = ora_tree_node_fwd(&q); if (rc) return rc; }
+  return LTB_OK;
+}
+int ora_tree_bwd(const ltb_tree* t) {
+  std::vector<ltb_tree_node> v;
+  REQUIRE(tree_nodes_of(t, v) && t->grads, "tree_bwd: bad argument");
+  for (size_t i = v.size(); i > 0; --i) { int rc = ora_tree_node_bwd(&v[i - 1]); if (rc) return rc; }
+  return LTB_OK;
+}
 }  // extern "C"
 
 // ------------------------------------------------------------------ staging / replay: plain host equivalents.

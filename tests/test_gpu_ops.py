@@ -1132,6 +1132,103 @@ def test_tree_levels_and_gradient(ora, gpu, classify_cell):
     check(f, ora, gpu)
 
 
+def _tree_topology(rng, leaves, chain, table_rows, classes):
+    """A random binary tree (chain: every right child is a leaf) in the order and layout ltb_tree wants: left, right, score, word, first node of each level."""
+    kids, depth, todo = {}, {}, [(leaves, None, 0)]
+    n = 0
+    while todo:
+        share, parent, which = todo.pop()
+        me, n = n, n + 1
+        if parent is not None:
+            kids.setdefault(parent, [None, None])[which] = me
+        if share > 1:
+            part = share - 1 if chain else int(rng.integers(1, share))
+            todo += [(part, me, 0), (share - part, me, 1)]
+
+    def height(i):
+        if i not in depth:
+            depth[i] = 0 if i not in kids else 1 + max(height(k) for k in kids[i])
+        return depth[i]
+    order = sorted(range(n), key=height)
+    pos = {node: i for i, node in enumerate(order)}
+    levels = max(depth.values()) + 1
+    left = [pos[kids[i][0]] if i in kids else -1 for i in order]
+    right = [pos[kids[i][1]] if i in kids else -1 for i in order]
+    first = [sum(height(i) < lv for i in order) for lv in range(levels + 1)]
+    return n, levels, np.array(left + right + list(rng.integers(0, classes, n)) + list(rng.integers(0, table_rows, n)) + first, np.int32)
+
+
+# leaves, hidden, embedding, classes, chain: one node, levels of more nodes than are worked on at once, a chain, the limits and odd sizes
+@pytest.mark.parametrize("classify_cell", [0, 1])
+@pytest.mark.parametrize("leaves,Hd,E,K,chain", [(1, 150, 300, 5, 0), (2, 150, 300, 5, 0), (25, 150, 300, 5, 0), (60, 150, 300, 5, 0), (14, 150, 300, 5, 1), (9, 160, 320, 32, 0),
+                                                 (7, 33, 17, 3, 0), (5, 1, 1, 1, 0), (40, 64, 96, 2, 0)])
+def test_a_whole_tree_per_call(ora, gpu, leaves, Hd, E, K, chain, classify_cell):
+    """ltb_tree_fwd / ltb_tree_bwd against the oracle's node by node, parameter gradients added to what is there, twice (the second tree's calls
+    meet the first one's barrier counters)."""
+    import ctypes
+    from lantern_b200._ffi import parse_struct
+    Tree = parse_struct("ltb_tree")
+    rng = R(leaves * 7 + Hd)
+    n, levels, topo0 = _tree_topology(rng, leaves, chain, 11, K)
+    v = lambda *shape, scale=1.0: (rng.standard_normal(shape) * scale).astype(np.float32)
+    W = {"leaf%d" % g: v(Hd, E, scale=1 / np.sqrt(E)) for g in (0, 3, 4)}
+    W.update({"in%d%d" % (g, k): v(Hd, Hd, scale=1 / np.sqrt(Hd)) for g in range(5) for k in (0, 1)})
+    W.update({"bl%d" % g: v(Hd, scale=0.1) for g in (0, 3, 4)}); W.update({"bi%d" % g: v(Hd, scale=0.1) for g in (0, 1, 3, 4)})
+    W["Why"], W["by"] = v(K, Hd, scale=0.3), v(K, scale=0.1)
+    table0 = v(11, E, scale=0.5)
+    pitch = (Hd + 63) // 64 * 64
+
+    def f(b):
+        lib = b.lib
+        w = {k: TensorR(b.fromNumpy(a), b.fromNumpy(a * 0.25)) for k, a in W.items()}
+        table, topo = b.fromNumpy(table0), b.fromNumpy(topo0)
+        out = {}
+        for turn in range(2):
+            vals, grads = b.fill((n, 8 * pitch + 64), 0.0), b.fill((n, 2 * pitch + 64), 0.0)
+            t = Tree(nodes=n, levels=levels, hidden=Hd, in_len=E, classes=K, classify_cell=classify_cell)
+            for g in (0, 3, 4):
+                t.leaf_W[g], t.leaf_dW[g], t.leaf_bias[g], t.leaf_dbias[g] = w["leaf%d" % g].x.ptr, w["leaf%d" % g].d.ptr, w["bl%d" % g].x.ptr, w["bl%d" % g].d.ptr
+            for g in range(5):
+                bk = "bi%d" % (1 if g == 2 else g)
+                for k in (0, 1):
+                    t.W[g][k], t.dW[g][k] = w["in%d%d" % (g, k)].x.ptr, w["in%d%d" % (g, k)].d.ptr
+                t.bias[g], t.dbias[g] = w[bk].x.ptr, w[bk].d.ptr
+            t.Why, t.by, t.dWhy, t.dby = w["Why"].x.ptr, w["by"].x.ptr, w["Why"].d.ptr, w["by"].d.ptr
+            t.table, t.topo_host, t.topo, t.values, t.grads = table.ptr, topo0.ctypes.data, topo.ptr, vals.ptr, grads.ptr
+            lib.tree_fwd(ctypes.addressof(t))
+            one = np.array([1.0], np.float32)
+            lib.h2d(grads.ptr + 4 * ((n - 1) * (2 * pitch + 64) + 2 * pitch), one.ctypes.data, 4)
+            lib.tree_bwd(ctypes.addressof(t))
+            out["vals%d" % turn] = vals.toCPU()[:, 5 * pitch:]
+            out["grads%d" % turn] = grads.toCPU()
+        out.update({"d" + k: x.d.toCPU() for k, x in w.items()})
+        return out
+    check(f, ora, gpu)
+
+
+def test_a_tree_that_is_none_is_refused(gpu):
+    """Sizes beyond the limits, and links that would send the kernels out of the arrays or round in circles."""
+    import ctypes
+    from lantern_b200._ffi import parse_struct
+    Tree = parse_struct("ltb_tree")
+    some = gpu.fill((4096,), 0.0).ptr
+
+    def attempt(topo, n=3, levels=2, hidden=8, in_len=8, classes=5):
+        topo = np.array(topo, np.int32)
+        t = Tree(nodes=n, levels=levels, hidden=hidden, in_len=in_len, classes=classes)
+        for g in range(5):
+            t.leaf_W[g] = t.leaf_bias[g] = t.W[g][0] = t.W[g][1] = t.bias[g] = some
+        t.Why = t.by = t.table = t.topo = t.values = some
+        t.topo_host = topo.ctypes.data
+        with pytest.raises(LanternError):
+            gpu.lib.tree_fwd(ctypes.addressof(t))
+    good = [-1, -1, 0, -1, -1, 1, 0, 0, 0, 0, 0, 0, 0, 2, 3]       # left, right, score, word of three nodes; first
+    attempt(good, hidden=161); attempt(good, in_len=321); attempt(good, classes=33); attempt(good, n=0); attempt(good, n=120)
+    for at, value in ((2, 2), (2, 1), (5, 7), (6, 5), (9, -1), (13, 3), (14, 4), (12, 1)):
+        bad = list(good); bad[at] = value
+        attempt(bad)
+
+
 @pytest.mark.parametrize("shape", [(128, 64, 16, 16), (128, 1024, 4, 4), (256, 64, 32, 32)])
 def test_fusion_level_two_changes_no_result(gpu, shape):
     """ltb_set_fusion(2): the batch-norm backward / add gradient that absorbs a held in-place ReLU gradient applies the mask on
