@@ -506,24 +506,34 @@ __global__ void skinny_k_kernel(const float* __restrict__ a, int64_t sam, int64_
 // are added in slice order through shared memory (a lane's loop over k is a chain of dependent steps: the classifier's weight
 // gradient, 10 x 2048 over a batch of 128, took 89 us as sixteen blocks walking all of K, 19 us as sixteen slabs and a second
 // launch).  With blockIdx.y > 1 a block's sum goes to its own slab and skinny_sum_kernel adds the slabs in order.
-constexpr int kSkinnyMSlices = 8;
+constexpr int kSkinnyMSlices = 8, kSkinnyMChunk = 32 * kSkinnyMSlices;
 template <bool ACC>
 __global__ void __launch_bounds__(32 * kSkinnyMSlices) skinny_m_kernel(const float* __restrict__ a, int64_t sam, int64_t sak, const float* __restrict__ b, int64_t sbk,
                                                                        int64_t sbn, float* c, int64_t scm, int64_t scn, int M, int N, int K, float alpha, float* part) {
   pdl_enter();
   __shared__ float sums[kSkinnyMSlices][16][33];
-  const int n = blockIdx.x * 32 + threadIdx.x, slice = threadIdx.y;
+  __shared__ float rows[16][kSkinnyMChunk + 1];                                     // a's share: every lane of a column's loop reads the same ones
+  const int n = blockIdx.x * 32 + threadIdx.x, slice = threadIdx.y, tid = slice * 32 + threadIdx.x;
   const int q0 = (int)((int64_t)K * blockIdx.y / gridDim.y), q1 = (int)((int64_t)K * (blockIdx.y + 1) / gridDim.y);
-  const int k0 = q0 + (int)((int64_t)(q1 - q0) * slice / kSkinnyMSlices), k1 = q0 + (int)((int64_t)(q1 - q0) * (slice + 1) / kSkinnyMSlices);
   float acc[16];
 #pragma unroll
   for (int m = 0; m < 16; ++m) acc[m] = 0.0f;
-  if (n < N) {
-#pragma unroll 4
-    for (int k = k0; k < k1; ++k) {
-      const float bv = b[(int64_t)k * sbk + (int64_t)n * sbn];
+  for (int c0 = q0; c0 < q1; c0 += kSkinnyMChunk) {
+    const int len = min(kSkinnyMChunk, q1 - c0), k0 = len * slice / kSkinnyMSlices, k1 = len * (slice + 1) / kSkinnyMSlices;
+    __syncthreads();
+    if (sak == 1) { for (int m = slice; m < M; m += kSkinnyMSlices) for (int k = threadIdx.x; k < len; k += 32) rows[m][k] = a[(int64_t)m * sam + c0 + k]; }
+    else for (int i = tid; i < M * len; i += 32 * kSkinnyMSlices) { const int k = i / M, m = i - k * M; rows[m][k] = a[(int64_t)m * sam + (int64_t)(c0 + k) * sak]; }
+    __syncthreads();
+    if (n >= N) continue;
+    const float* p = b + (int64_t)(c0 + k0) * sbk + (int64_t)n * sbn;
+    for (int k = k0; k < k1; k += 8, p += 8 * sbk) {                             // eight loads in flight
+      float v[8];
 #pragma unroll
-      for (int m = 0; m < 16; ++m) if (m < M) acc[m] += a[(int64_t)m * sam + (int64_t)k * sak] * bv;
+      for (int e = 0; e < 8; ++e) v[e] = k + e < k1 ? p[e * sbk] : 0.0f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int m = 0; m < 16; ++m) if (m < M && k + e < k1) acc[m] += rows[m][k + e] * v[e];
     }
   }
 #pragma unroll

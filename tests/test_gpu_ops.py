@@ -232,6 +232,42 @@ def test_softmax_family_and_nll(ora, gpu, rows, cols):
     check(f, ora, gpu, rtol=2e-4)
 
 
+# the lengths where a row stops fitting 1, 8 and 32 registers of a lane
+@pytest.mark.parametrize("rows,cols", [(1, 1), (9, 32), (5, 33), (3, 256), (4, 257), (3, 1000), (2, 1024), (7, 1025)])
+def test_softmax_rows_of_every_form(ora, gpu, rows, cols):
+    v = (R(cols).standard_normal((rows, cols)) * 3).astype(np.float32)
+    if cols > 1:
+        v[0, 0], v[rows - 1, cols - 1] = -np.inf, 80.0          # a class that is ruled out, and one that takes everything
+    dy = R(3).standard_normal(v.shape).astype(np.float32)
+
+    def f(b):
+        out = {}
+        for name, fwd, bwd in (("s", b.softmax, b.softmax_grad), ("l", b.logSoftmax, b.logSoftmax_grad)):
+            x = TensorR(b.fromNumpy(v), b.fromNumpy(dy * 0.5))
+            y = fwd(x.x)
+            bwd(x, TensorR(y, b.fromNumpy(dy)))
+            out.update({name: np.exp(y.toCPU()), name + "d": x.d.toCPU()})
+        return out
+    check(f, ora, gpu)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("math,M,N,K", [(0, 33, 20, 70), (0, 5, 300, 900), (0, 10, 2048, 128), (1, 256, 96, 320), (1, 1000, 1001, 257), (1, 128, 10, 2048)])
+def test_product_gradients_into_unset_buffers(gpu, ta, tb, math, M, N, K):
+    """Poisoned buffers declared unset against zeros: the gradients are written where they would have been added."""
+    b = gpu
+    a, c, dc = (b.fromNumpy(R(i).standard_normal(s).astype(np.float32)) for i, s in enumerate((((K, M) if ta else (M, K)), ((N, K) if tb else (K, N)), (M, N))))
+    b.lib.set_math(math); b.lib.set_deterministic(1)
+    try:
+        zero, fresh = [[f(b, a.shape), f(b, c.shape)] for f in (lambda b, s: b.fill(s, 0.0), _poisoned)]
+        for da, dc_ in (zero, fresh):
+            b.lib.gemm_grad(a.ptr, da.ptr, ta, c.ptr, dc_.ptr, tb, 0.5, dc.ptr, M, N, K)
+        for x, y in zip(zero, fresh):
+            assert np.array_equal(x.toCPU(), y.toCPU())
+    finally:
+        b.lib.set_math(1); b.lib.set_deterministic(0)
+
+
 def test_reductions_concat_trans_geam(ora, gpu):
     v = R(1).standard_normal((6, 5, 8)).astype(np.float32)
     big = R(2).standard_normal(300001).astype(np.float32)
