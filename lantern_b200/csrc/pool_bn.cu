@@ -489,16 +489,19 @@ __global__ void __launch_bounds__(512, 2) bn_bwd_cluster_kernel(const float* __r
 // cheaper than two cluster barriers, and with 1024 or 2048 channels of a few hundred values each the launch is bound by
 // the rate at which CTAs can be dispatched (measured: 9.5 us at 512 CTAs, 18 us at 2048 CTAs for the same 4 MB).  Here a
 // CTA is G rows of T threads (T a multiple of 32: warps never straddle rows), row g owns channel blockIdx.x * G + g.
-struct BnPackedPlan { int T, G; };
+// Threads rather than items per thread while all channels' threads fit the machine once (1024 per SM): one or two items per thread leave room to
+// fetch everything a channel needs before the sums, a single memory latency instead of two.
+struct BnPackedPlan { int T, G, vpt; };
 static bool bn_packed_plan(int N, int C, int HW, int vpt, BnPackedPlan& p) {
   const int64_t items = (int64_t)N * (HW >> 2);
   if (items > (int64_t)vpt * 512) return false;
-  int T = 32; while (T < 512 && (int64_t)T * 4 < items) T <<= 1;      // about four float4 per thread
-  while ((int64_t)T * vpt < items) T <<= 1;
-  if (T > 512) return false;
-  int G = 512 / T;
+  for (p.vpt = 1;; p.vpt <<= 1) {
+    p.T = 32; while ((int64_t)p.T * p.vpt < items) p.T <<= 1;
+    if (p.vpt == vpt || (p.T <= 512 && (int64_t)p.T * C <= (int64_t)1024 * g.sm_count)) break;
+  }
+  int G = 512 / p.T;
   while (G > 1 && (C + G - 1) / G < 128) G >>= 1;                       // keep at least 128 CTAs when there are channels for them
-  p.T = T; p.G = G;
+  p.G = G;
   return true;
 }
 // Sums of a and b over the T threads of this thread's row; every thread of the row returns the totals.  red: 2 x 16 floats.
@@ -529,11 +532,11 @@ __global__ void __launch_bounds__(512, 2) bn_fwd_packed_kernel(const float* x, f
   const float old_mean = run_mean && live ? run_mean[c] : 0.0f, old_var = run_var && live ? run_var[c] : 0.0f;
   const float k = live ? x[(int64_t)c * HW] : 0.0f;                     // shift: a sample of the channel (see bn_reduce_kernel)
   float a = 0.0f, b = 0.0f;
-  float4 keep[VPT];
+  float4 keep[VPT], plus[VPT <= 2 ? VPT : 1];
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const int t = j * T + (int)threadIdx.x;
-    if (live && t < total) { int i; const int n = geo.hw4.divmod(t, i); keep[j] = reinterpret_cast<const float4*>(x + ((int64_t)n * C + c) * HW)[i]; }
+    if (live && t < total) { int i; const int n = geo.hw4.divmod(t, i); keep[j] = reinterpret_cast<const float4*>(x + ((int64_t)n * C + c) * HW)[i]; if (VPT <= 2 && add) plus[j] = reinterpret_cast<const float4*>(add + ((int64_t)n * C + c) * HW)[i]; }
   }
   zero_fill(extra.zero);                                                // while the loads are on their way
 #pragma unroll
@@ -565,7 +568,7 @@ __global__ void __launch_bounds__(512, 2) bn_fwd_packed_kernel(const float* x, f
       int i; const int n = geo.hw4.divmod(t, i);
       float4 v = keep[j];
       v.x = (v.x - mu) * sc + sh; v.y = (v.y - mu) * sc + sh; v.z = (v.z - mu) * sc + sh; v.w = (v.w - mu) * sc + sh;
-      if (add) v = add4(v, reinterpret_cast<const float4*>(add + ((int64_t)n * C + c) * HW)[i]);
+      if (add) v = add4(v, VPT <= 2 ? plus[VPT <= 2 ? j : 0] : reinterpret_cast<const float4*>(add + ((int64_t)n * C + c) * HW)[i]);
       if (relu) { v.x = v.x < 0.0f ? 0.0f : v.x; v.y = v.y < 0.0f ? 0.0f : v.y; v.z = v.z < 0.0f ? 0.0f : v.z; v.w = v.w < 0.0f ? 0.0f : v.w; }
       reinterpret_cast<float4*>(y + ((int64_t)n * C + c) * HW)[i] = v;
       if (extra.cl) {
@@ -588,7 +591,8 @@ __global__ void __launch_bounds__(512, 2) bn_bwd_packed_kernel(const float* __re
   const int hw4 = HW >> 2, total = N * hw4;
   const float mu = live ? mean[c] : 0.0f, is = live ? istd[c] : 0.0f, ga = live ? gamma[c] : 0.0f;
   float a = 0.0f, b = 0.0f;
-  float4 kx[VPT], kd[VPT];
+  float4 kx[VPT], kd[VPT], o[VPT];
+  const float4 nothing = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const int t = j * T + (int)threadIdx.x;
@@ -596,11 +600,13 @@ __global__ void __launch_bounds__(512, 2) bn_bwd_packed_kernel(const float* __re
       int i; const int n = geo.hw4.divmod(t, i);
       const int64_t off = ((int64_t)n * C + c) * HW;
       kx[j] = reinterpret_cast<const float4*>(x + off)[i]; kd[j] = reinterpret_cast<const float4*>(dy + off)[i];
+      if (VPT <= 2) o[j] = dx && !(fresh & 1) ? reinterpret_cast<const float4*>(dx + off)[i] : nothing;
       if (mask_y) { kd[j] = relu_mask(kd[j], reinterpret_cast<const float4*>(mask_y + off)[i]); if (!(fresh & 2)) reinterpret_cast<float4*>(dy + off)[i] = kd[j]; }
       if (extra) {
         float4 e = (fresh & 4) ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(extra + off)[i];
         e.x += kd[j].x; e.y += kd[j].y; e.z += kd[j].z; e.w += kd[j].w;
         reinterpret_cast<float4*>(extra + off)[i] = e;
+        if (VPT <= 2 && extra == dx) o[j] = e;                          // a block whose shortcut is the batch norm's own input
       }
     }
   }
@@ -619,12 +625,12 @@ __global__ void __launch_bounds__(512, 2) bn_bwd_packed_kernel(const float* __re
   if (dx == nullptr) { if (first) { if (dbeta) dbeta[c] += a; if (dgamma) dgamma[c] += b; } return; }
   const float m = (float)N * (float)HW;
   const float ca = ga * is, cb = a / m, cc = b / m;
-  float4 o[VPT];
+  if (VPT > 2)
 #pragma unroll
-  for (int j = 0; j < VPT; ++j) {
-    const int t = j * T + (int)threadIdx.x;
-    if (t < total) { int i; const int n = geo.hw4.divmod(t, i); o[j] = (fresh & 1) ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(dx + ((int64_t)n * C + c) * HW)[i]; }
-  }
+    for (int j = 0; j < VPT; ++j) {
+      const int t = j * T + (int)threadIdx.x;
+      if (t < total) { int i; const int n = geo.hw4.divmod(t, i); o[j] = (fresh & 1) ? nothing : reinterpret_cast<const float4*>(dx + ((int64_t)n * C + c) * HW)[i]; }
+    }
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const int t = j * T + (int)threadIdx.x;
@@ -664,9 +670,15 @@ int bn_fwd_issue(const Pending& p, bool relu, const BnExtra& extra) {
   BnPackedPlan pk;
   if (bn_fwd_packed(p, pk)) {
     PdlUnlessLarge scope(ceil_div(p.C, pk.G));
-    LTB_LAUNCH(bn_fwd_packed_kernel<kBnVpt>, (unsigned)ceil_div(p.C, pk.G), dim3(pk.T, pk.G), 0, p.x, y, p.gamma, p.beta, p.run_mean, p.run_var,
-               p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, p.eps, p.momentum, r, add, extra);
-    return LTB_OK;
+    auto go = [&](auto kernel) -> int {
+      LTB_LAUNCH(kernel, (unsigned)ceil_div(p.C, pk.G), dim3(pk.T, pk.G), 0, p.x, y, p.gamma, p.beta, p.run_mean, p.run_var,
+                 p.save_mean, p.save_istd, bn_geo(p.N, p.HW), p.N, p.C, p.HW, p.eps, p.momentum, r, add, extra);
+      return LTB_OK;
+    };
+    g.label = "bn_fwd_packed_kernel";
+    const int rc = pk.vpt == 1 ? go(bn_fwd_packed_kernel<1>) : pk.vpt == 2 ? go(bn_fwd_packed_kernel<2>) : pk.vpt == 4 ? go(bn_fwd_packed_kernel<4>) : go(bn_fwd_packed_kernel<kBnVpt>);
+    g.label = nullptr;
+    return rc;
   }
   PdlUnlessLarge scope((int64_t)p.C * c.K);
   if (c.per_cta <= kBnVpt * c.threads)
@@ -788,9 +800,14 @@ int ltb_bn_bwd(const float* x, float* dx, const float* dy, const float* gamma, f
     BnPackedPlan pk;
     if ((p.K == 1 || C >= 96) && bn_packed_plan(N, C, HW, kBnVptBwd, pk)) {
       PdlUnlessLarge scope(ceil_div(C, pk.G));
-      LTB_LAUNCH(bn_bwd_packed_kernel<kBnVptBwd>, (unsigned)ceil_div(C, pk.G), dim3(pk.T, pk.G), 0, x, dyw, dx, gamma, dgamma, dbeta,
-                 save_mean, save_istd, bn_geo(N, HW), N, C, HW, mask_y, fresh, extra);
-      return LTB_OK;
+      auto go = [&](auto kernel) -> int {
+        LTB_LAUNCH(kernel, (unsigned)ceil_div(C, pk.G), dim3(pk.T, pk.G), 0, x, dyw, dx, gamma, dgamma, dbeta, save_mean, save_istd, bn_geo(N, HW), N, C, HW, mask_y, fresh, extra);
+        return LTB_OK;
+      };
+      g.label = "bn_bwd_packed_kernel";
+      const int rc = pk.vpt == 1 ? go(bn_bwd_packed_kernel<1>) : pk.vpt == 2 ? go(bn_bwd_packed_kernel<2>) : go(bn_bwd_packed_kernel<kBnVptBwd>);
+      g.label = nullptr;
+      return rc;
     }
     PdlUnlessLarge scope((int64_t)C * p.K);
     if (p.per_cta <= kBnVptBwd * p.threads)

@@ -1336,6 +1336,36 @@ def test_bn_backward_absorbs_the_add_gradient(gpu, shape, other_fresh):
     assert res[1][4] == res[0][4] - 1                                                        # one launch fewer: the add gradient went into the batch norm
 
 
+# one, two, four items per thread, and clusters
+@pytest.mark.parametrize("shape", [(8, 256, 4, 4), (128, 2048, 2, 2), (128, 1024, 4, 4), (32, 96, 8, 8), (128, 64, 16, 16)])
+@pytest.mark.parametrize("fresh", [False, True])
+def test_bn_backward_into_the_buffer_its_shortcut_shares(gpu, shape, fresh):
+    """relu(bn(x) + x): the batch norm's input gradient and the shortcut's are one buffer, which both add to."""
+    b, lib = gpu, gpu.lib
+    C = shape[1]
+    x0, out0, d0, pre = (R(i).standard_normal(shape).astype(np.float32) for i in (31, 32, 33, 34))
+    res = []
+    for level in (0, 2):
+        lib.set_fusion(level)
+        try:
+            x = TensorR(b.fromNumpy(x0), _poisoned(b, shape) if fresh else b.fromNumpy(pre))
+            gam, bet = TensorR(b.fill((C,), 1.5), b.fill((C,), 0.0)), TensorR(b.fill((C,), 0.1), b.fill((C,), 0.0))
+            z, sm, si, _ = b.batchNormTraining(x.x, gam.x, bet.x, b.fill((C,), 0.0), b.fill((C,), 1.0))
+            lib.sync()
+            zr = TensorR(z, _poisoned(b, shape))
+            out = TensorR(b.fromNumpy(out0), b.fromNumpy(d0))
+            b.relu_grad(out, out, inPlace=True)
+            sh = np.array(shape, np.int32)
+            lib.ew_binary_grad(0, zr.x.ptr, zr.d.ptr, sh.ctypes.data, x.x.ptr, x.d.ptr, sh.ctypes.data, out.d.ptr, 4)
+            b.batchNorm_grad(x, zr, gam, bet, sm, si)
+            lib.sync()
+            res.append([x.d.toCPU(), gam.d.toCPU(), bet.d.toCPU()])
+        finally:
+            lib.set_fusion(0)
+    for u, v in zip(*res):
+        assert np.isfinite(v).all() and np.array_equal(u, v)
+
+
 @pytest.mark.parametrize("shape", [(128, 256, 16, 16), (128, 64, 32, 32), (128, 512, 8, 8), (128, 1024, 4, 4), (64, 2048, 2, 2), (8, 20, 6, 6), (4, 6, 5, 5)])
 @pytest.mark.parametrize("order", ["bn_first", "shortcut_first"])
 def test_bn_forward_absorbs_the_add_and_relu(gpu, shape, order):
