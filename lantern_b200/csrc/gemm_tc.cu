@@ -39,7 +39,7 @@ namespace cg = cooperative_groups;
 
 namespace ltb {
 
-constexpr int kMaxStages = 4;
+constexpr int kMaxStages = 6;
 constexpr int kPartPitch = 129;                    // floats per column of a CTA's partial tile in shared memory (odd: reads along either axis are conflict-free)
 constexpr int kTapChunk = 40, kTapPitch = 161;     // TC_EPI_TAPS staging: floats from chunk to chunk of 32 columns (lanes = 8 channels x 4 chunks hit 32 banks) and from row to row
 constexpr int kTcThreads = 320;                    // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
@@ -116,6 +116,34 @@ __device__ __forceinline__ void tma_load(const CUtensorMap* map, uint64_t* bar, 
     asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
                  ::"r"(d), "l"(m), "r"(b), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]) : "memory");
 }
+// The same for a CTA of a pair: `bar` is a barrier of the pair's first CTA, as an address of the cluster's shared memory.
+__device__ __forceinline__ void tma_load_pair(const CUtensorMap* map, uint32_t b, void* dst, int rank, const int* c) {
+  const uint32_t d = smem_u32(dst);
+  const uint64_t m = reinterpret_cast<uint64_t>(map);
+  if (rank == 2)
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(d), "l"(m), "r"(b), "r"(c[0]), "r"(c[1]) : "memory");
+  else if (rank == 3)
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(d), "l"(m), "r"(b), "r"(c[0]), "r"(c[1]), "r"(c[2]) : "memory");
+  else if (rank == 4)
+    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 ::"r"(d), "l"(m), "r"(b), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]) : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+                 ::"r"(d), "l"(m), "r"(b), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]) : "memory");
+}
+__device__ __forceinline__ void tma_im2col_pair(const CUtensorMap* map, uint32_t b, void* dst, int c, int w, int h, int n, int s, int r) {
+  asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(b), "r"(c), "r"(w), "r"(h), "r"(n), "h"((uint16_t)s), "h"((uint16_t)r) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t first_of_pair(const void* p) {      // where p's namesake lies in the pair's first CTA
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(cluster_rank() & ~1u));
+  return a;
+}
+__device__ __forceinline__ void pair_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // One im2col-mode load: the map's walk starts at base pixel (w, h) of image n, tap (s, r) is added as an offset.
 __device__ __forceinline__ void tma_im2col(const CUtensorMap* map, uint64_t* bar, void* dst, int c, int w, int h, int n, int s, int r) {
   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
@@ -133,6 +161,13 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {        // arrives at this barrier of both CTAs
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)(3u << (cluster_rank() & ~1u))) : "memory");
+}
+__device__ __forceinline__ void tc_mma_tf32_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
@@ -214,20 +249,27 @@ struct BoxLane {
   // Issues a stage's loads and moves on to the next k-iteration.  GEN false: one box per operand, issued by the elected lane, which gets the
   // coordinates by shuffles.  GEN true: up to eight boxes per operand; every lane issues its own (the shuffles would cost more than the
   // compiler's loop over the lanes: 56 x 56, 3x3 layer 323 us instead of 282).
-  template <bool GEN>
-  __device__ __forceinline__ void issue(const TcParams& P, bool both, const CUtensorMap* map_a, const CUtensorMap* map_b, const TcOperandDev& o, int lane, uint64_t* bar, uint8_t* stage) {
+  // PAIR: `pair_bar` instead of bar.
+  template <bool GEN, bool PAIR>
+  __device__ __forceinline__ void issue(const TcParams& P, bool both, const CUtensorMap* map_a, const CUtensorMap* map_b, const TcOperandDev& o, int lane, uint64_t* bar, uint32_t pair_bar, uint8_t* stage) {
     if (!GEN) {
       int va[5], vb[5];
 #pragma unroll
       for (int j = 0; j < 5; ++j) { va[j] = __shfl_sync(0xffffffffu, c[j], 0); vb[j] = __shfl_sync(0xffffffffu, c[j], 8); }
       if (elect_one()) {
-        if (both) tma_load(map_a, bar, stage, P.a.rank, va);
-        tma_load(map_b, bar, stage + P.a.stage_bytes, P.b.rank, vb);
+        if (PAIR) { tma_load_pair(map_a, pair_bar, stage, P.a.rank, va); tma_load_pair(map_b, pair_bar, stage + P.a.stage_bytes, P.b.rank, vb); }
+        else {
+          if (both) tma_load(map_a, bar, stage, P.a.rank, va);
+          tma_load(map_b, bar, stage + P.a.stage_bytes, P.b.rank, vb);
+        }
       }
     } else {
       const CUtensorMap* const map = lane & 8 ? map_b : map_a;
-      if (load != TC_LOAD_IM2COL && load != TC_LOAD_IM2COL_MN) { if (active) tma_load(map, bar, stage + offset, rank, c); }
-      else if (active) tma_im2col(map, bar, stage + offset, c[0], o.im.low_w + pi * o.im.step_w, o.im.low_h + pj * o.im.step_h, pn, c[1], c[2]);
+      if (load != TC_LOAD_IM2COL && load != TC_LOAD_IM2COL_MN) { if (active) { if (PAIR) tma_load_pair(map, pair_bar, stage + offset, rank, c); else tma_load(map, bar, stage + offset, rank, c); } }
+      else if (active) {
+        const int w = o.im.low_w + pi * o.im.step_w, h = o.im.low_h + pj * o.im.step_h;
+        if (PAIR) tma_im2col_pair(map, pair_bar, stage + offset, c[0], w, h, pn, c[1], c[2]); else tma_im2col(map, bar, stage + offset, c[0], w, h, pn, c[1], c[2]);
+      }
     }
     if (GEN && load == TC_LOAD_IM2COL_MN) {
       pi += o.im.adv_i; pj += o.im.adv_j; pn += o.im.adv_n;
@@ -290,8 +332,12 @@ __device__ __forceinline__ long long out_column(const TcParams& P, int n) {
 // EPI (TcEpilogue) and MODE (0 store, 1 accumulate, 2 atomic accumulate) are compile-time: each launch then carries one
 // epilogue instead of six, a third of the instructions -- these CTAs live for a few microseconds and the instruction cache
 // starts cold (measured hit rate 66 % with all variants in one kernel).
-template <int EPI, int MODE, bool GEN>
-__global__ void __launch_bounds__(kTcThreads, 2)
+// PAIR: a cluster of two CTAs along x works on 256 rows.  Each loads its own 128 rows of A and half of B's columns, signalling the first one's barriers; the
+// first one issues the MMAs over both CTAs' shared memory (cta_group::2), whose commits arrive in both; each has its rows' accumulator and stores them.
+// The arrivals at the other CTA's barriers are relaxed (the copies are what the barrier orders): released at cluster scope, each waited about a
+// microsecond and a product took twice as long.
+template <int EPI, int MODE, bool GEN, bool PAIR>
+__global__ void __launch_bounds__(kTcThreads, PAIR ? 1 : 2)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ TcParams P) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];
@@ -302,6 +348,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // the shuffle tells the compiler that warp is uniform
   const int m_tile = blockIdx.x, n_tile = blockIdx.y;
+  const bool second_cta = PAIR && (blockIdx.x & 1);
   const int k_begin = blockIdx.z * P.k_per_split;
   const int k_end = min(P.k_iters, k_begin + P.k_per_split);
   const int n_iter = k_end - k_begin;
@@ -318,7 +365,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint32_t tx = 0;             // bytes a stage receives through TMA
   if (warp == 0) {
     if (lane < 2) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(lane ? &map_b : &map_a)) : "memory");
-    tx = box.init<GEN>(P, m_tile, n_tile, k_begin, lane, gather);
+    tx = box.init<GEN>(P, m_tile, PAIR ? 2 * n_tile + (second_cta ? 1 : 0) : n_tile, k_begin, lane, gather);
     asm volatile("bar.sync 5, 64;" ::: "memory");
     pdl_wait();
   }
@@ -326,7 +373,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (lane == 0) {
       // a stage is full when the TMA bytes have landed (one arrival with the byte count) and, in gather mode, the eight
       // gathering warps have stored their rows (one arrival each)
-      for (int s = 0; s < stages; ++s) { mbar_init(&full_bar[s], gather ? 9 : 1); mbar_init(&empty_bar[s], 1); }
+      for (int s = 0; s < stages; ++s) { mbar_init(&full_bar[s], PAIR ? 2 : gather ? 9 : 1); mbar_init(&empty_bar[s], 1); }      // (of a pair: an arrival with the byte count from each CTA)
       mbar_init(&accum_bar, 1);
       abort_flag = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -334,8 +381,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     __syncwarp();
     asm volatile("bar.sync 5, 64;" ::: "memory");
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)P.bn) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)P.bn) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)P.bn) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   // gather mode: the first two k-iterations' loads leave before the warps meet
   float4 cur[4], nxt[4], nx2[4];                                               // the loads of two k-iterations are in flight while one is stored
@@ -359,7 +411,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // The producer goes on issuing; the others meet here (the tensor memory's address, the barriers), so that the first MMA waits for
   // its own stage only.
   tc_fence_before();
-  if (warp != 0) asm volatile("bar.sync 6, 288;" ::: "memory");
+  if (PAIR) { __syncwarp(); pair_sync(); }                     // both CTAs' barriers and tensor memory are there
+  else if (warp != 0) asm volatile("bar.sync 6, 288;" ::: "memory");
   tc_fence_after();
   const uint32_t tmem_base = warp != 0 ? tmem_slot : 0u;
 
@@ -371,14 +424,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const bool ok = mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag, P.status, 1, P.wait_cycles);
         if (!__all_sync(0xffffffffu, ok)) break;
       }
-      if (elect_one()) mbar_expect_tx(&full_bar[s], tx);
+      uint32_t pair_bar = 0;
+      if (PAIR) {
+        pair_bar = first_of_pair(&full_bar[s]);
+        if (elect_one()) asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(pair_bar), "r"(tx) : "memory");
+      } else if (elect_one()) mbar_expect_tx(&full_bar[s], tx);
       __syncwarp();
-      box.issue<GEN>(P, !gather, &map_a, &map_b, o, lane, &full_bar[s], stage_base + (size_t)s * stage_bytes);
+      box.issue<GEN, PAIR>(P, !gather, &map_a, &map_b, o, lane, &full_bar[s], pair_bar, stage_base + (size_t)s * stage_bytes);
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
     __syncwarp();          // the block-wide barrier below needs converged warps
   } else if (warp == 1) {
-    if (n_iter > 0) {
+    if (n_iter > 0 && !second_cta) {
       int s = 0; uint32_t ph = 0;
       // descriptor pieces that do not change: kept in registers so that an MMA costs two additions and the instruction
       uint32_t koa[4], kob[4];
@@ -397,10 +454,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int k = 0; k < 4; ++k) {
           const uint64_t adesc = a_hi | (uint64_t)(a_lo | ((sa + koa[k]) & 0x3FFFu));
           const uint64_t bdesc = b_hi | (uint64_t)(b_lo | ((sb + kob[k]) & 0x3FFFu));
-          tc_mma_tf32(tmem_base, adesc, bdesc, idesc, (it > 0 || k > 0) ? 1u : 0u);
+          if (PAIR) tc_mma_tf32_pair(tmem_base, adesc, bdesc, idesc, (it > 0 || k > 0) ? 1u : 0u);
+          else tc_mma_tf32(tmem_base, adesc, bdesc, idesc, (it > 0 || k > 0) ? 1u : 0u);
         }
+        if (PAIR) { tc_commit_pair(&empty_bar[s]); if (it + 1 == n_iter) tc_commit_pair(&accum_bar); }
+        else {
         tc_commit(&empty_bar[s]);       // the stage may be refilled once these MMAs have read it
         if (it + 1 == n_iter) tc_commit(&accum_bar);    // accumulator complete
+        }
         }
         __syncwarp();
         if (++s == stages) { s = 0; ph ^= 1u; }
@@ -569,17 +630,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __syncthreads();
   if (P.cluster_z > 1) {
     // ---- the cluster sums its partial tiles in a fixed order.  The hardware cluster barrier is safe to wait at: the CTAs
-    // of a cluster are scheduled together.  CTA number zr of the cluster owns a slice of the tile -- columns for the
+    // of a cluster are scheduled together.  CTA (of a pair's halves each) number zr of the cluster owns a slice of the tile -- columns for the
     // pixel-major epilogue, rows for the row-major one, so that its global stores coalesce -- reads that slice from the
     // shared memory of every CTA of the cluster, rank 0 first, and writes the result the way the epilogue would.
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     if (warp >= 2 && !abort_flag) {
-      const int cz = P.cluster_z, zr = (int)cluster.block_rank();
+      const int cz = P.cluster_z, zr = (int)cluster.block_rank() >> (PAIR ? 1 : 0);
       float* part = reinterpret_cast<float*>(stage_base);
       const float* remote[8];
 #pragma unroll
-      for (int z = 0; z < 8; ++z) remote[z] = z < cz ? cluster.map_shared_rank(part, z) : part;
+      for (int z = 0; z < 8; ++z) remote[z] = z < cz ? cluster.map_shared_rank(part, PAIR ? 2 * z + (second_cta ? 1 : 0) : z) : part;
       const int t = threadIdx.x - 64;                                  // 0 .. 255
       const int n0 = n_tile * P.bn;
       float* const out_base = P.out + (long long)(blockIdx.z / cz) * P.split_stride;
@@ -638,9 +699,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     cluster.sync();                // no CTA leaves while its shared memory may still be read
   }
+  if (PAIR) { __syncwarp(); pair_sync(); }           // neither CTA's barriers, stages or tensor memory are used by the other any more
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.bn) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.bn) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)P.bn) : "memory");
   }
 }
 
@@ -966,12 +1029,13 @@ static void temp_free(float* p, size_t floats);
 static float* temp_alloc(size_t floats);
 
 typedef void (*EngineFn)(const CUtensorMap, const CUtensorMap, const TcParams);
-#define LTB_ENGINE(GEN)                                                                                                      \
-  {tc_gemm_kernel<TC_EPI_PIXEL, 0, GEN>, tc_gemm_kernel<TC_EPI_PIXEL, 1, GEN>, tc_gemm_kernel<TC_EPI_PIXEL, 2, GEN>,            \
-   tc_gemm_kernel<TC_EPI_ROWMAJOR, 0, GEN>, tc_gemm_kernel<TC_EPI_ROWMAJOR, 1, GEN>, tc_gemm_kernel<TC_EPI_ROWMAJOR, 2, GEN>,   \
-   tc_gemm_kernel<TC_EPI_TAPS, 0, GEN>, tc_gemm_kernel<TC_EPI_TAPS, 1, GEN>, tc_gemm_kernel<TC_EPI_TAPS, 2, GEN>}
-static const EngineFn kEngine[2][9] = {LTB_ENGINE(false), LTB_ENGINE(true)};    // by load modes, epilogue and store mode
-#undef LTB_ENGINE
+#define LTB_MODES(EPI, GEN, PAIR) tc_gemm_kernel<EPI, 0, GEN, PAIR>, tc_gemm_kernel<EPI, 1, GEN, PAIR>, tc_gemm_kernel<EPI, 2, GEN, PAIR>
+static const EngineFn kEngine[2][9] = {                                          // by load modes, epilogue and store mode
+    {LTB_MODES(TC_EPI_PIXEL, false, false), LTB_MODES(TC_EPI_ROWMAJOR, false, false), LTB_MODES(TC_EPI_TAPS, false, false)},
+    {LTB_MODES(TC_EPI_PIXEL, true, false), LTB_MODES(TC_EPI_ROWMAJOR, true, false), LTB_MODES(TC_EPI_TAPS, true, false)}};
+static const EngineFn kEnginePair[2][6] = {{LTB_MODES(TC_EPI_PIXEL, false, true), LTB_MODES(TC_EPI_ROWMAJOR, false, true)},
+                                           {LTB_MODES(TC_EPI_PIXEL, true, true), LTB_MODES(TC_EPI_ROWMAJOR, true, true)}};
+#undef LTB_MODES
 static size_t plan_out_floats(const TcPlan& p) {
   return p.epilogue == TC_EPI_PIXEL ? (size_t)ceil_div(p.M, p.pix_pad ? p.pix_pad : p.pix_per_img ? p.pix_per_img : 1) * (size_t)p.img_stride : (size_t)p.M * (size_t)p.ld;
 }
@@ -1020,7 +1084,7 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr,
   if (!to_dev(p.a, P.a) || !to_dev(p.b, P.b)) return fail(LTB_E_STATE, "tensor-core plan whose k-iteration order has no incremental walk");
   P.M = p.M; P.N = p.N; P.bn = p.bn; P.k_iters = p.k_iters;
   // Split-K: up to eight splits of a tile form a thread-block cluster and add their partial tiles up inside the kernel
-  // (through distributed shared memory, in a fixed order).  More than eight splits: every cluster of eight writes a slab of
+  // (through distributed shared memory, in a fixed order).  More than eight splits (four, of pairs): every cluster writes a slab of
   // partial results (a staging block with the layout of the output) and one more launch adds the slabs up, again in a fixed
   // order, and applies alpha, bias and accumulation.  No atomics, no zero fill, the same bits on every run.
   // That is the deterministic mode (ltb_set_deterministic): measured, it costs the contraction kernels about a third more
@@ -1029,7 +1093,7 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr,
   int splits = p.splits < 1 ? 1 : p.splits, cz = 1, nslabs = 1;
   const bool atomic = splits > 1 && !g.deterministic;
   if (splits > 1 && !atomic) {
-    cz = splits <= 2 ? 2 : splits <= 4 ? 4 : 8;
+    cz = splits <= 2 ? 2 : splits <= 4 || p.pair ? 4 : 8;                           // (four pairs)
     nslabs = (int)ceil_div(splits, cz);
   }
   const size_t out_floats = plan_out_floats(p);
@@ -1045,7 +1109,7 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr,
   P.epilogue = p.epilogue; P.accumulate = ws ? 0 : p.accumulate; P.atomic = atomic ? 1 : 0;
   if (atomic && !p.accumulate && !clear.done) LTB_CUDA(cudaMemsetAsync(p.out, 0, out_floats * 4, g.stream));     // overwrite semantics: start from zero, then add
   // tf32 x tf32 -> f32: D format 1 at [4,6), A/B format 2 at [7,10)/[10,13), major bits 15/16, N>>3 at [17,23), M>>4 at [24,29)
-  P.idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)p.a.mn_major << 15) | ((uint32_t)p.b.mn_major << 16) | ((uint32_t)(p.bn >> 3) << 17) | ((128u >> 4) << 24);
+  P.idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)p.a.mn_major << 15) | ((uint32_t)p.b.mn_major << 16) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(p.pair ? 256 : 128) >> 4 << 24);
   P.out = ws ? ws : p.out; P.bias = ws ? nullptr : p.bias; P.alpha = ws ? 1.0f : p.alpha; P.split_stride = ws ? (long long)out_floats : 0;
   P.pix_per_img = p.pix_per_img ? p.pix_per_img : 1; P.by_pix = FastDiv((int)(p.pix_pad ? p.pix_pad : P.pix_per_img));
   P.img_stride = p.img_stride; P.chan_stride = p.chan_stride; P.ld = p.ld; P.col_mod = p.col_mod; P.col_mul = p.col_mul;
@@ -1054,24 +1118,26 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr,
   if (P.relu) *relu = false;
   P.status = g.dev_status; P.wait_cycles = g.wait_limit_cycles;
   // 4 stages, except 3 for 128-wide tiles so that two CTAs (2 x 97 KB) share an SM and one's epilogue overlaps the other's main loop
-  // (256-wide tiles: four stages of 48 KB, one CTA per SM).
-  P.stages = p.bn == 128 ? 3 : kMaxStages;
+  // (256-wide tiles: four stages of 48 KB, one CTA per SM; six of 32 KB in a pair).
+  P.stages = p.pair ? kMaxStages : p.bn == 128 ? 3 : 4;
   const size_t smem = (size_t)P.stages * (p.a.stage_bytes + p.b.stage_bytes) + 1024;
   if (cz > 1 && (size_t)128 * (p.bn + 1) * 4 > smem - 1024) return fail(LTB_E_STATE, "tensor-core plan whose partial tile does not fit the pipeline stages");
   if (!smem_opted_in) {
-    const int max_smem = kMaxStages * (16384 + 32768) + 1024;
+    const int max_smem = 4 * (16384 + 32768) + 1024;                              // as much as six of 32 KB
     for (auto& set : kEngine) for (auto k : set) LTB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+    for (auto& set : kEnginePair) for (auto k : set) LTB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     smem_opted_in = true;
   }
   const int mode = atomic ? 2 : (P.accumulate ? 1 : 0);
-  const EngineFn kernel = kEngine[p.a.load != TC_LOAD_BOX || p.b.load != TC_LOAD_BOX][p.epilogue * 3 + mode];
+  const bool gen = p.a.load != TC_LOAD_BOX || p.b.load != TC_LOAD_BOX;
+  const EngineFn kernel = p.pair ? kEnginePair[gen][p.epilogue * 3 + mode] : kEngine[gen][p.epilogue * 3 + mode];
   {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.m_tiles, p.n_tiles, splits); cfg.blockDim = dim3(kTcThreads); cfg.dynamicSmemBytes = smem; cfg.stream = g.stream;
+    cfg.gridDim = dim3(p.pair ? (p.m_tiles + 1) / 2 * 2 : p.m_tiles, p.n_tiles, splits); cfg.blockDim = dim3(kTcThreads); cfg.dynamicSmemBytes = smem; cfg.stream = g.stream;
     cudaLaunchAttribute attr[2];
     pdl_attribute(attr[1]);
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)cz;
+    attr[0].val.clusterDim.x = p.pair ? 2 : 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)cz;
     cfg.attrs = attr; cfg.numAttrs = g.profiling ? 1 : 2;
     if (g.profiling) profile_before(label);
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mb, P);

@@ -337,6 +337,16 @@ int pick_bn(int n_extent, int m_tiles, int sm_count, int k_iters = 0) {
   return 128;
 }
 
+// A pair of CTAs per 256 x 256 outputs, where there are 256-wide tiles and an even number of row tiles (or an A operand whose loads beyond the last tile
+// only read zeros): a CTA then takes in 32 KB per k-iteration instead of 48, and that is what the loop waits for (at 48 KB a product of 4096 x 4096 x 2048
+// took 13 TB/s out of the L2).  Measured, one CTA against a pair, us: 4096 x 4096 x 2048 119 / 111, 8192 x 1000 x 2048 67 / 61 and 87 / 74 with B N-major,
+// 1920 x 4096 x 4096 108 / 100, 8192 x 2048 x 1000 (32 k-iterations) 73 / 72; with 16 k-iterations (16384 x 512 x 512) 24.2 / 25.4: the pair's meetings
+// before the first MMA and after the last are not earned back, hence the line at 32.  Returns the width of B's loads.
+int pick_pair(TcPlan& p, int m_tiles, int k_iters) {
+  p.pair = p.bn == 256 && k_iters >= 32 && m_tiles >= 2 && (m_tiles % 2 == 0 || p.a.load == TC_LOAD_BOX || p.a.load == TC_LOAD_BOXES) ? 1 : 0;
+  return p.pair ? p.bn / 2 : p.bn;
+}
+
 void finish(TcPlan& p, int M, int N, int k_iters, int sm_count, bool may_split) {
   p.M = M; p.N = N; p.k_iters = k_iters;
   p.m_tiles = cdiv(M, kTileM); p.n_tiles = cdiv(N, p.bn);
@@ -400,7 +410,7 @@ bool tc_plan_conv_fwd(TcPlan& p, const float* x, bool a_rows, const float* w, in
   const int M = n_img * pix;
   if (!(a_rows ? operand_k_rows(p.a, x, M, ck, kTileM, &ka) : operand_mn_pixels(p.a, x, n_img, ck, pix, &ka))) return false;
   p.bn = pick_bn(co, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_k_rows(p.b, w, co, ldw, p.bn, &kb) || ka != kb) return false;      // columns ck..ldw of w are zero padding
+  if (!operand_k_rows(p.b, w, co, ldw, a_rows ? p.bn : pick_pair(p, cdiv(M, kTileM), ka), &kb) || ka != kb) return false;      // columns ck..ldw of w are zero padding
   finish(p, M, co, ka, sm_count, true);             // split-K for small outputs: the launcher zeroes y first
   p.epilogue = TC_EPI_PIXEL; p.out = y; p.bias = bias; p.alpha = 1.0f; p.accumulate = 0;
   p.pix_per_img = pix; p.img_stride = (int64_t)co * pix; p.chan_stride = pix;
@@ -414,7 +424,7 @@ bool tc_plan_conv_dgrad(TcPlan& p, const float* dy, bool a_rows, const float* w,
   const int M = n_img * pix;
   if (!(a_rows ? operand_k_rows(p.a, dy, M, co, kTileM, &ka) : operand_mn_pixels(p.a, dy, n_img, co, pix, &ka))) return false;
   p.bn = pick_bn(ck, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_mn_cols(p.b, w, co, ldw, p.bn, &kb) || ka != kb) return false;      // columns ck .. ldw of w are zero padding
+  if (!operand_mn_cols(p.b, w, co, ldw, a_rows ? p.bn : pick_pair(p, cdiv(M, kTileM), ka), &kb) || ka != kb) return false;      // columns ck .. ldw of w are zero padding
   finish(p, M, ck, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = dx; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = accumulate ? 1 : 0;
   p.pix_per_img = pix; p.img_stride = (int64_t)ck * pix; p.chan_stride = pix;
@@ -446,7 +456,7 @@ bool tc_plan_conv_taps_fwd(TcPlan& p, const float* xr, const float* wt, const fl
   // output pixel (oh, ow) reads input (oh - ph + r, ow - pw + s)
   if (!operand_k_window(p.a, xr, g.n_img, g.H, g.W, g.C, g.oH, g.oW, g.R, g.S, -g.ph, -g.pw, +1, &ka)) return false;
   p.bn = pick_bn(g.K, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_k_taps(p.b, wt, g.R * g.S, g.K, g.C, p.bn, &kb) || ka != kb) return false;
+  if (!operand_k_taps(p.b, wt, g.R * g.S, g.K, g.C, pick_pair(p, cdiv(M, kTileM), ka), &kb) || ka != kb) return false;
   finish(p, M, g.K, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = y; p.bias = bias; p.alpha = 1.0f; p.accumulate = 0;
   p.pix_per_img = (int64_t)g.oH * g.oW; p.img_stride = (int64_t)g.K * g.oH * g.oW; p.chan_stride = (int64_t)g.oH * g.oW;
@@ -461,7 +471,7 @@ bool tc_plan_conv_taps_dgrad(TcPlan& p, const float* dyr, const float* wt, float
   // input pixel (h, w) receives dy(h + ph - r, w + pw - s) * w[k][c][r][s]
   if (!operand_k_window(p.a, dyr, g.n_img, g.oH, g.oW, g.K, g.H, g.W, g.R, g.S, g.ph, g.pw, -1, &ka)) return false;
   p.bn = pick_bn(g.C, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_mn_taps(p.b, wt, g.R * g.S, g.K, g.C, p.bn, &kb) || ka != kb) return false;
+  if (!operand_mn_taps(p.b, wt, g.R * g.S, g.K, g.C, pick_pair(p, cdiv(M, kTileM), ka), &kb) || ka != kb) return false;
   finish(p, M, g.C, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = dx; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = accumulate ? 1 : 0;
   p.pix_per_img = (int64_t)g.H * g.W; p.img_stride = (int64_t)g.C * g.H * g.W; p.chan_stride = (int64_t)g.H * g.W;
@@ -500,7 +510,7 @@ bool tc_plan_conv_any_fwd(TcPlan& p, const float* xr, const float* wt, const flo
   const int M = g.n_img * g.oH * g.oW;
   if (!operand_im2col(p.a, xr, g.n_img, g.H, g.W, g.C, g.ldc, g.oH, g.oW, g.sh, g.sw, -g.ph, -g.pw, g.R, g.S, &ka) || !corner_ok(p.a)) return false;
   p.bn = pick_bn(g.K, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_k_taps(p.b, wt, g.R * g.S, g.K, g.ldc, p.bn, &kb) || ka != kb) return false;
+  if (!operand_k_taps(p.b, wt, g.R * g.S, g.K, g.ldc, pick_pair(p, cdiv(M, kTileM), ka), &kb) || ka != kb) return false;
   finish(p, M, g.K, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = y; p.bias = bias; p.alpha = 1.0f; p.accumulate = 0;
   p.pix_per_img = (int64_t)g.oH * g.oW; p.img_stride = (int64_t)g.K * g.oH * g.oW; p.chan_stride = (int64_t)g.oH * g.oW;
@@ -515,12 +525,13 @@ bool tc_plan_conv_any_dgrad(TcPlan& p, const float* dyr, const float* wp, float*
   // dx is the convolution of dy with the filter turned round: tap (r', s') = (R - 1 - r, S - 1 - s), padding R - 1 - ph
   if (!operand_im2col(p.a, dyr, g.n_img, g.oH, g.oW, g.K, g.ldk, g.H, g.W, 1, 1, g.ph - g.R + 1, g.pw - g.S + 1, g.R, g.S, &ka) || !corner_ok(p.a)) return false;
   p.bn = pick_bn(g.C, cdiv(M, kTileM), sm_count, ka);
+  const int width = pick_pair(p, cdiv(M, kTileM), ka);
   // the taps in reverse
   if (g.C % 32 == 0) {
-    if (!operand_mn_taps(p.b, wp, g.R * g.S, g.K, g.C, p.bn, &kb) || ka != kb) return false;
+    if (!operand_mn_taps(p.b, wp, g.R * g.S, g.K, g.C, width, &kb) || ka != kb) return false;
     p.b.c_off[3] = g.R * g.S - 1; p.b.k_mul[3] = -1;
   } else {
-    if (!operand_k_taps(p.b, wp, g.R * g.S, g.C, g.ldk, p.bn, &kb) || ka != kb) return false;
+    if (!operand_k_taps(p.b, wp, g.R * g.S, g.C, g.ldk, width, &kb) || ka != kb) return false;
     p.b.c_off[2] = g.R * g.S - 1; p.b.k_mul[2] = -1;
   }
   finish(p, M, g.C, ka, sm_count, true);
@@ -549,7 +560,7 @@ bool tc_plan_conv_ragged_fwd(TcPlan& p, const float* x, const float* w, int ldw,
   if (co < 8 || ck < 8 || ldw < ck || (int64_t)n_img * pix > (1ll << 29) || !operand_mn_ragged(p.a, x, n_img, ck, pix, &ka, &tpi)) return false;
   const int M = n_img * tpi * kTileM;
   p.bn = pick_bn(co, n_img * tpi, sm_count, ka);
-  if (!operand_k_rows(p.b, w, co, ldw, p.bn, &kb) || ka != kb) return false;
+  if (!operand_k_rows(p.b, w, co, ldw, pick_pair(p, n_img * tpi, ka), &kb) || ka != kb) return false;
   finish(p, M, co, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = y; p.bias = bias; p.alpha = 1.0f; p.accumulate = 0;
   p.pix_per_img = pix; p.pix_pad = (int64_t)tpi * kTileM; p.img_stride = (int64_t)co * pix; p.chan_stride = pix;
@@ -562,7 +573,7 @@ bool tc_plan_conv_ragged_dgrad(TcPlan& p, const float* dy, const float* w, int l
   if (co < 8 || ck < 8 || ldw < ck || (int64_t)n_img * pix > (1ll << 29) || !operand_mn_ragged(p.a, dy, n_img, co, pix, &ka, &tpi)) return false;
   const int M = n_img * tpi * kTileM;
   p.bn = pick_bn(ck, n_img * tpi, sm_count, ka);
-  if (!operand_mn_cols(p.b, w, co, ldw, p.bn, &kb) || ka != kb) return false;
+  if (!operand_mn_cols(p.b, w, co, ldw, pick_pair(p, n_img * tpi, ka), &kb) || ka != kb) return false;
   finish(p, M, ck, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = dx; p.bias = nullptr; p.alpha = 1.0f; p.accumulate = accumulate ? 1 : 0;
   p.pix_per_img = pix; p.pix_pad = (int64_t)tpi * kTileM; p.img_stride = (int64_t)ck * pix; p.chan_stride = pix;
@@ -589,7 +600,8 @@ bool tc_plan_gemm_ld(TcPlan& p, const float* a, bool a_kmajor, int lda, const fl
   bool ok = a_kmajor ? operand_k_rows(p.a, a, M, lda, kTileM, &ka) : operand_mn_cols(p.a, a, K, lda, kTileM, &ka);
   if (!ok) return false;
   p.bn = pick_bn(N, cdiv(M, kTileM), sm_count, ka);
-  ok = b_kmajor ? operand_k_rows(p.b, b, N, ldb, p.bn, &kb) : operand_mn_cols(p.b, b, K, ldb, p.bn, &kb);
+  const int width = pick_pair(p, cdiv(M, kTileM), ka);
+  ok = b_kmajor ? operand_k_rows(p.b, b, N, ldb, width, &kb) : operand_mn_cols(p.b, b, K, ldb, width, &kb);
   if (!ok || ka != kb) return false;
   finish(p, M, N, ka, sm_count, true);
   p.epilogue = TC_EPI_ROWMAJOR; p.out = c; p.bias = nullptr; p.alpha = alpha; p.accumulate = accumulate ? 1 : 0; p.ld = N;

@@ -103,6 +103,7 @@ struct TcPlan {
   TcOperand a, b;             // a: the M-side operand (128 rows per tile), b: the N-side operand (bn columns per tile)
   int M, N;                   // logical extents of D
   int bn;                     // tile width: 64, 128 or 256
+  int pair;                   // two neighbouring row tiles share a CTA pair: one MMA over 256 rows, each CTA loads its own rows of A and half of B's columns (b is planned with tiles of bn / 2)
   int m_tiles, n_tiles, k_iters, splits;
   int epilogue;
   float* out;

@@ -168,19 +168,21 @@ static bool walk_matches(const TcOperand& o, int tile, int k_iters) {
 
 static bool run_plan(const TcPlan& p, size_t out_count) {
   if (p.a.nk != p.b.nk) { printf("nk mismatch\n"); return false; }
-  if (!walk_matches(p.a, p.m_tiles - 1, p.k_iters) || !walk_matches(p.b, p.n_tiles - 1, p.k_iters)) return false;
+  if (!walk_matches(p.a, p.m_tiles - 1, p.k_iters) || !walk_matches(p.b, (p.pair + 1) * p.n_tiles - 1, p.k_iters)) return false;
+  if (p.pair && (p.bn != 256 || p.gather_src || p.epilogue == TC_EPI_TAPS)) { printf("a pair where the kernel has none\n"); return false; }
   for (const TcOperand* o : {&p.a, &p.b}) if (o->load == TC_LOAD_IM2COL_MN && !pixel_walk_matches(*o, p.k_iters)) return false;
   // overwrite semantics under split-K: the partial results of the splits are summed and then stored; emulated by zeroing first
   if (p.splits > 1 && !p.accumulate) for (size_t i = 0; i < out_count; ++i) p.out[i] = 0.0f;
-  std::vector<float> sa, sb;
+  std::vector<float> sa, sb, sc;
   for (int mt = 0; mt < p.m_tiles; ++mt) for (int nt = 0; nt < p.n_tiles; ++nt) for (int z = 0; z < p.splits; ++z) {
     int per = (p.k_iters + p.splits - 1) / p.splits, k0 = z * per, k1 = k0 + per < p.k_iters ? k0 + per : p.k_iters;
     if (k0 >= k1) continue;
     std::vector<double> D((size_t)128 * p.bn, 0.0);
     for (int it = k0; it < k1; ++it) {
-      if (!(p.gather_src ? gather_load(p, mt, it, sa) : tma_load(p.a, mt, it, sa)) || !tma_load(p.b, nt, it, sb)) return false;
+      if (!(p.gather_src ? gather_load(p, mt, it, sa) : tma_load(p.a, mt, it, sa)) || !tma_load(p.b, p.pair ? 2 * nt : nt, it, sb)) return false;
+      if (p.pair && !tma_load(p.b, 2 * nt + 1, it, sc)) return false;             // the other CTA's half of the columns
       for (int ks = 0; ks < p.a.nk; ++ks) for (int r = 0; r < 128; ++r) for (int c = 0; c < p.bn; ++c) {
-        double s = 0; for (int kk = 0; kk < 8; ++kk) s += (double)umma_fetch(p.a, sa, ks, r, kk) * umma_fetch(p.b, sb, ks, c, kk);
+        double s = 0; for (int kk = 0; kk < 8; ++kk) s += (double)umma_fetch(p.a, sa, ks, r, kk) * (p.pair && c >= 128 ? umma_fetch(p.b, sc, ks, c - 128, kk) : umma_fetch(p.b, sb, ks, c, kk));
         D[(size_t)r * p.bn + c] += s;
       }
     }

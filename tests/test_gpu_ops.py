@@ -519,10 +519,11 @@ def test_gemm_of_ragged_rows_tf32(ora, gpu, ta, tb, M, N, K):
 
 
 @pytest.mark.parametrize("det", [0, 1])
-@pytest.mark.parametrize("M,N,K,ta,tb", [(4740, 1000, 516, 0, 1), (512, 508, 20000, 1, 0), (4096, 1196, 996, 0, 1)])
+@pytest.mark.parametrize("M,N,K,ta,tb", [(4740, 1000, 516, 0, 1), (512, 508, 20000, 1, 0), (4096, 1196, 996, 0, 1), (2564, 1476, 1028, 0, 1), (1284, 508, 7172, 1, 0)])
 def test_gemm_in_wide_tiles_tf32(ora, gpu, M, N, K, ta, tb, det):
     """256-wide tiles: enough of them, a product of 13 splits that is stored, and a gradient of 3 splits that is added; by atomics and, in
-    deterministic mode, by clusters (13 splits: two clusters of eight and a sum of their slabs)."""
+    deterministic mode, by clusters (13 splits: clusters of four and a sum of their slabs).  With 32 k-iterations and
+    more the tiles are worked on by pairs of CTAs: an odd number of row tiles, a ragged last half of the columns, one split and several."""
     gpu.lib.set_deterministic(det)
     try:
         test_gemm_of_ragged_rows_tf32(ora, gpu, ta=ta, tb=tb, M=M, N=N, K=K)
