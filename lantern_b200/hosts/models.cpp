@@ -74,9 +74,9 @@ struct Model {
   float* stage_x = nullptr;  // pinned staging for the batch
   int32_t* stage_y = nullptr;
   float* loss_host = nullptr;  // pinned, 1 float
-  void* graph = nullptr;
+  void* graph[3] = {nullptr, nullptr, nullptr};        // the recorded step: in its general form, and reading staging pair 0 or 1 (1 + slot)
   bool use_graph = false;
-  float graph_lr = 0.f;
+  float graph_lr[3] = {0.f, 0.f, 0.f};
   size_t zero_bytes = 0;       // bytes of zero-initialised gradient buffers the largest step so far asked for (0: not known yet)
   bool early_reduce = false;   // this step runs data-parallel with an update: finished gradient ranges are summed during backward
   bool branches = true;        // independent runs of calls (shortcut convolutions) are issued as branch regions
@@ -91,6 +91,7 @@ struct Model {
   float* dev_logits = nullptr; int64_t logit_count = 0; TR last_logits;
   // Two steps in flight (submit / collect): staging pair p = step & 1; marker p = its upload done, marker 2 + p = its step done.
   bool feeding = false;
+  int slot = -1;               // while feeding: the staging pair that the step being issued reads its batch from and leaves its loss in
   int64_t submitted = 0;
   float* feed_x[2] = {nullptr, nullptr}; int32_t* feed_y[2] = {nullptr, nullptr}; float* feed_loss = nullptr;
   float* dstage_x[2] = {nullptr, nullptr}; int32_t* dstage_y[2] = {nullptr, nullptr};   // device side of the two staging pairs (uploads run beside the step before)
@@ -141,7 +142,8 @@ struct Model {
     int64_t nin = (int64_t)batch * in_c * in_h * in_w;
     TR x; x.rank = 4; x.shape[0] = batch; x.shape[1] = in_c; x.shape[2] = in_h; x.shape[3] = in_w; x.is_input = true;
     int32_t* y;
-    if (resident) {           // batch already in device memory (measurement of the device-side step alone)
+    if (slot >= 0) { x.x = dstage_x[slot]; y = dstage_y[slot]; }
+    else if (resident) {      // batch already in device memory (measurement of the device-side step alone)
       x.x = dev_x; y = dev_y;
     } else {                  // the generated programs upload every batch: resnet50FromOnnx.scala:173-174
       x.x = alloc_value(nin);
@@ -153,10 +155,11 @@ struct Model {
     last_logits = TR();
     TR loss = forward(tape, x, y);
     if (dev_logits && last_logits.x && last_logits.count() == logit_count) BK(d2d)(dev_logits, last_logits.x, (size_t)logit_count * 4);
+    if (slot < 0) BK(d2d)(dev_loss, loss.x, 4);
     BK(fill)(loss.d, 1.0f, 1);                       // gradR_loss: y.d.setAsOne(), TD.scala:1763-1780
-    BK(d2d)(dev_loss, loss.x, 4);
     tape.backward();
-    BK(d2h_async)(loss_host, dev_loss, 4);
+    if (slot >= 0) BK(d2h_async)(feed_loss + slot, loss.x, 4);
+    else BK(d2h_async)(loss_host, dev_loss, 4);
     if (update) apply_update(lr);
     if (tracing()) dump_trace();
     { const size_t asked = zero_pool_end(); if (asked > zero_bytes) zero_bytes = asked; }   // the largest step so far: a smaller tree leaves part of the block unused
@@ -214,18 +217,20 @@ struct Model {
     copy_to_staging(stage_x, xh, (size_t)batch * in_c * in_h * in_w * 4);
     memcpy(stage_y, yh, (size_t)label_count * 4);
   }
+  void drop_graphs() { for (void*& rec : graph) if (rec) { BK(graph_destroy)(rec); rec = nullptr; } }
   int step_async(const float* xh, const int32_t* yh, float lr, bool update) {
     if (!resident && xh) load(xh, yh);
     if (!feeding && draw_host_data(0)) return LTB_E_CUDA;
     if (use_graph && update && zero_bytes > 0) {        // the first step runs eagerly: it measures the gradient pool
-      if (graph && graph_lr != lr) { BK(graph_destroy)(graph); graph = nullptr; }
-      if (!graph) {
+      void*& rec = graph[1 + slot];
+      if (rec && graph_lr[1 + slot] != lr) { BK(graph_destroy)(rec); rec = nullptr; }
+      if (!rec) {
         int rc = BK(graph_begin)(); if (rc) return rc;
         enqueue(lr, true);
-        graph = BK(graph_end)(); graph_lr = lr;
-        if (!graph) return LTB_E_CUDA;
+        rec = BK(graph_end)(); graph_lr[1 + slot] = lr;
+        if (!rec) return LTB_E_CUDA;
       }
-      return BK(graph_launch)(graph);
+      return BK(graph_launch)(rec);
     }
     enqueue(lr, update);
     return 0;
@@ -237,18 +242,21 @@ struct Model {
   }
   // Training with two steps in flight.  The generated programs upload a batch, run the step and block on the loss copy
   // (resnet50FromOnnx.scala:173-186), so the device idles while the host prepares the next batch.  submit() copies the
-  // batch into one of two pinned staging pairs, queues the upload, the step (reading the batch at its fixed device
-  // address, so the recorded step is the same every time) and a 4-byte loss copy, and returns; collect(k) waits for
-  // step k alone.  The staging pair of step k is refilled by step k + 2, after its upload marker has fired.
+  // batch into one of two pinned staging pairs, queues the upload and the step, and returns; collect(k) waits for
+  // step k alone.  The staging pair of step k is refilled by step k + 2, after its upload marker has fired.  A step is recorded
+  // once per pair: it reads the batch where the upload puts it and leaves its loss in the pair's pinned word.  (One recording
+  // for both, with the batch, its labels and the loss copied to and from fixed addresses around it: five more nodes a step,
+  // each 2 to 4 us on the device between two kernels: the RNN of one row 90 -> 74 us a step, the MNIST CNN 185 -> 163.)
   void feed_mode(bool on) {
     if (feeding == on) return;
-    if (graph) { BK(graph_destroy)(graph); graph = nullptr; }      // the recorded step reads the batch from another place
+    drop_graphs();
     if (on && !feed_loss) {
       const size_t xb = (size_t)batch * in_c * in_h * in_w * 4;
       for (int p = 0; p < 2; ++p) { feed_x[p] = (float*)BK(host_alloc)(xb); feed_y[p] = (int32_t*)BK(host_alloc)((size_t)label_count * 4); }
       feed_loss = (float*)BK(host_alloc)(8);
     }
-    if (on) BK(sync)();
+    BK(sync)();
+    if (!on && submitted) *loss_host = feed_loss[(submitted - 1) & 1];
     feeding = resident = on;
   }
   // Staging pair for the next submit, free to be written (a loader decodes a batch straight into it).
@@ -266,11 +274,11 @@ struct Model {
     const int p = (int)(submitted & 1);
     const size_t xb = (size_t)batch * in_c * in_h * in_w * 4;
     if (draw_host_data(p)) return -1;
-    // The upload runs on the copy stream beside the step before it (marker 4 + p: the device staging pair was read for the last
-    // time by step submitted - 2; marker p: the upload has left the host staging pair); the compute stream then waits for the
-    // upload on the device and moves the batch to where the recorded step reads it.
+    // The upload runs on the copy stream beside the step before it (marker 2 + p: step submitted - 2, the last one that read the
+    // device staging pair, is done; marker p: the upload has left the host staging pair); the compute stream then waits for the
+    // upload on the device.
     const size_t yb = (size_t)label_count * 4;
-    int after = submitted >= 2 ? 4 + p : -1;
+    int after = submitted >= 2 ? 2 + p : -1;
     if (xh) {
       memcpy(sy, yh, yb);
       for (size_t at = 0; at < xb; at += kUploadPiece, after = -1) {
@@ -280,9 +288,11 @@ struct Model {
       }
     } else if (BK(upload)(dstage_x[p], sx, xb, after)) return -1;
     if (BK(upload)(dstage_y[p], sy, yb, -1) || BK(upload_marker)(p)) return -1;
-    if (BK(stream_wait_marker)(p) || BK(d2d)(dev_x, dstage_x[p], xb) || BK(d2d)(dev_y, dstage_y[p], yb) || BK(marker_record)(4 + p)) return -1;
-    if (step_async(nullptr, nullptr, lr, true)) return -1;
-    if (BK(d2h_async)(feed_loss + p, dev_loss, 4) || BK(marker_record)(2 + p)) return -1;
+    if (BK(stream_wait_marker)(p)) return -1;
+    slot = p;
+    const int rc = step_async(nullptr, nullptr, lr, true);
+    slot = -1;
+    if (rc || BK(marker_record)(2 + p)) return -1;
     return submitted++;
   }
   int collect(int64_t k, float* loss) {
@@ -323,10 +333,8 @@ struct Mnist : Model {
     for (int64_t i = 0; i < n; ++i) mask_host[p][i] = ((float)rand() / RAND_MAX > kRate) ? scale : 0.0f;
     if (!feeding) return BK(h2d)(mask_dev, mask_host[p], (size_t)n * 4);
     // beside the step before, as the batch (Model::submit): staging block p was read for the last time by step submitted - 2
-    int rc = BK(upload)(mask_stage[p], mask_host[p], (size_t)n * 4, submitted >= 2 ? 4 + p : -1);
-    if (!rc) rc = BK(upload_marker)(p);                                 // marker p: the whole staging pair has left, mask included
-    if (!rc) rc = BK(stream_wait_marker)(p);
-    return rc ? rc : BK(d2d)(mask_dev, mask_stage[p], (size_t)n * 4);
+    int rc = BK(upload)(mask_stage[p], mask_host[p], (size_t)n * 4, submitted >= 2 ? 2 + p : -1);
+    return rc ? rc : BK(upload_marker)(p);                              // marker p: the whole staging pair has left, mask included
   }
   TR forward(Tape& t, const TR& x, const int32_t* y) override {   // MnistCNN.scala:43-59
     TR b1 = P(c1b), b2 = P(c2b);
@@ -335,7 +343,7 @@ struct Mnist : Model {
     TR s2 = t.conv(s1, P(c2w), &b2, 1, 0);
     TR s25 = t.max_pool(t.relu(s2, false), 2, 2);
     TR flat = view(s25, {batch, 320});
-    TR s3 = t.dropout_masked(t.plus_bias(t.dot(flat, P(l1w)), P(l1b)), mask_dev);
+    TR s3 = t.dropout_masked(t.plus_bias(t.dot(flat, P(l1w)), P(l1b)), slot >= 0 ? mask_stage[slot] : mask_dev);
     TR out = t.plus_bias(t.dot(s3, P(l2w)), P(l2b));
     last_logits = out;
     return t.sum(t.nll(t.log_softmax(out), y));
@@ -700,7 +708,7 @@ void* HOST_FN(model_create)(const char* name, int batch, int seed) {
 }
 void HOST_FN(model_destroy)(void* m) {
   Model* M = (Model*)m;
-  if (M->graph) BK(graph_destroy)(M->graph);
+  M->drop_graphs();
   BK(host_free)(M->stage_x); BK(host_free)(M->stage_y); BK(host_free)(M->loss_host);
   for (int p = 0; p < 2; ++p) { BK(host_free)(M->feed_x[p]); BK(host_free)(M->feed_y[p]); }
   BK(host_free)(M->feed_loss);
@@ -725,7 +733,7 @@ int64_t HOST_FN(model_label_count)(void* m) { return ((Model*)m)->label_count; }
 // on: 0 operator by operator, 1 one call per gate / cell, 2 (default) in addition the vanilla RNN's whole sequence in one call.
 int HOST_FN(model_use_fused_cells)(void* m, int on) {
   Model* M = (Model*)m;
-  if (M->graph) { BK(graph_destroy)(M->graph); M->graph = nullptr; }
+  M->drop_graphs();
   M->fused_cells = on != 0; M->whole_sequence = on >= 2; M->whole_tree = on >= 3; return 0;
 }
 // Issue independent runs of calls as branch regions (default) or everything in program order on one stream.
@@ -734,7 +742,7 @@ int HOST_FN(model_use_fused_cells)(void* m, int on) {
 int HOST_FN(model_use_deferred_zero)(void*, int on) { deferred_grads() = on != 0; return 0; }
 int HOST_FN(model_use_branches)(void* m, int on) {
   Model* M = (Model*)m;
-  if (M->graph) { BK(graph_destroy)(M->graph); M->graph = nullptr; }
+  M->drop_graphs();
   M->branches = on != 0; return 0;
 }
 // A recorded step can only be replayed when every step issues the same operations: not so for one tree per step.
@@ -743,7 +751,7 @@ int HOST_FN(model_use_graph)(void* m, int on) { Model* M = (Model*)m; M->use_gra
 int HOST_FN(model_set_resident)(void* m, const float* x_host, const int32_t* y_host) {
   Model* M = (Model*)m;
   M->feed_mode(false);
-  if (M->graph) { BK(graph_destroy)(M->graph); M->graph = nullptr; }
+  M->drop_graphs();
   if (!x_host) { M->resident = false; return 0; }
   M->load(x_host, y_host);
   BK(h2d)(M->dev_x, M->stage_x, (size_t)M->batch * M->in_c * M->in_h * M->in_w * 4);
@@ -768,7 +776,7 @@ int HOST_FN(model_step_async)(void* m, const float* x_host, const int32_t* y_hos
 // loss.  Only the last two submitted steps can be collected.
 int64_t HOST_FN(model_submit)(void* m, const float* x_host, const int32_t* y_host, float lr) { return ((Model*)m)->submit(x_host, y_host, lr); }
 int HOST_FN(model_collect)(void* m, int64_t step, float* loss) { return ((Model*)m)->collect(step, loss); }
-float HOST_FN(model_last_loss)(void* m) { return *((Model*)m)->loss_host; }
+float HOST_FN(model_last_loss)(void* m) { const Model* M = (Model*)m; return M->feeding && M->submitted ? M->feed_loss[(M->submitted - 1) & 1] : *M->loss_host; }
 // The classifier's output of the last step (batch x classes floats); returns the number of floats, 0 for programs without one.
 int64_t HOST_FN(model_logits)(void* m, float* host_out) {
   Model* M = (Model*)m;

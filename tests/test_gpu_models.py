@@ -82,6 +82,38 @@ def test_step_loss_and_every_gradient(oracle_lib, cuda_lib, name, batch, kind, m
     oracle_lib.reset(mo_mark); cuda_lib.reset(mg_mark)
 
 
+@pytest.mark.parametrize("name,batch,kind", [("mnist", 20, "uniform"), ("rnn_26_50", 3, "normal")])
+def test_two_steps_in_flight_give_the_losses_of_blocking_steps(cuda_lib, name, batch, kind):
+    """Seven submitted steps, each with a batch of its own (and, for MNIST, its own dropout mask), the step recorded once per staging pair:
+    losses and parameters are those of blocking steps, bit for bit in deterministic FP32; so is the loss read after leaving the mode."""
+    import ctypes
+    from lantern_b200.hosts import HostPrograms
+    libc, mark, res = ctypes.CDLL(None), cuda_lib.mark(), []
+    cuda_lib.set_math(0); cuda_lib.set_deterministic(1)
+    try:
+        for feed in (False, True):
+            m = HostPrograms(cuda_lib).model(name, batch, seed=5)
+            libc.srand(3)
+            rng = np.random.default_rng(11)
+            batches = [(rng.standard_normal(m.input_count).astype(np.float32), rng.integers(0, 10, m.label_count).astype(np.int32)) for _ in range(7)]
+            losses = []
+            if feed:
+                m.use_graph(True)
+                for k, (x, y) in enumerate(batches):
+                    m.submit(x, y, 0.01)
+                    if k:
+                        losses.append(m.collect(k - 1))
+                losses.append(m.collect(6))
+                assert m.last_loss() == losses[-1]
+            else:
+                losses = [m.step(x, y, 0.01) for x, y in batches]
+            res.append((losses, m.slab_params()))
+            m.close(); cuda_lib.reset(mark)
+    finally:
+        cuda_lib.set_math(1); cuda_lib.set_deterministic(0)
+    assert res[0][0] == res[1][0] and np.array_equal(res[0][1], res[1][1])
+
+
 def test_training_trajectory_and_graph_replay(oracle_lib, cuda_lib):
     """Ten SGD steps of the MNIST program: oracle vs CUDA; then the ResNet-50 step replayed from a recorded graph
     must reproduce the eagerly issued step bit for bit."""
