@@ -75,7 +75,8 @@ void*  LTB_FN(get_stream)(void);
 int    LTB_FN(sync)(void);
 int    LTB_FN(set_math)(int mode);                      /* LTB_MATH_TF32 (default) or LTB_MATH_FP32 */
 /* Look-ahead fusion, off by default. When on, batch normalisation (training or inference), a convolution with a bias and same-shape
- * add are issued one call late so that an in-place ReLU of their result joins the same kernel, and an in-place ReLU gradient is held
+ * add are issued one call late so that an in-place ReLU of their result joins the same kernel, a log-softmax, the negative log likelihood of its result and
+ * the sum or mean of that are one kernel, a fill of one element, the sum's gradient that reads it and the gradients of those two are another, and an in-place ReLU gradient is held
  * so that the batch-norm backward, convolution backward with a bias or add gradient that reads it applies it on the fly. Results are those of the separate calls; only the moment
  * of the launch moves: a held operation is issued by the next call of this library whatever it is, or joined by it; a batch norm and
  * the ReLU that joined it are held for one call more, so that a convolution of the result can have them prepare its output (sync, copies,

@@ -18,9 +18,11 @@ constexpr size_t kGranule = 256;      // arena granule (TMA wants 16 B bases/str
 // for one call.  BN forward or a same-shape add followed by an in-place ReLU of their result become one kernel; an in-place
 // ReLU gradient followed by BN backward or by the add's gradient reading that buffer become one kernel.  A convolution and the
 // in-place ReLU of its result share the contraction's epilogue, and a held ReLU gradient joins the bias-gradient pass of the
-// convolution backward that reads it.  Any other call
+// convolution backward that reads it.  A log-softmax, the negative log likelihood of its result and the sum (mean) of that are one kernel,
+// and so are the seed of the loss's gradient (a fill of one element) and the three gradients.  Any other call
 // first issues the held operation on its own, so results never change; only the moment of the launch does.
-enum { PEND_NONE = 0, PEND_BN_FWD = 1, PEND_ADD = 2, PEND_RELU_GRAD = 3, PEND_RELU_ADD_GRAD = 4, PEND_BN_ADD = 5, PEND_CONV = 6, PEND_BN_INF = 7, PEND_BN_RELU = 8 };
+enum { PEND_NONE = 0, PEND_BN_FWD = 1, PEND_ADD = 2, PEND_RELU_GRAD = 3, PEND_RELU_ADD_GRAD = 4, PEND_BN_ADD = 5, PEND_CONV = 6, PEND_BN_INF = 7, PEND_BN_RELU = 8,
+       PEND_LSM = 9, PEND_NLL = 10, PEND_SEED = 11, PEND_SUM_GRAD = 12, PEND_NLL_GRAD = 13 };
 struct ConvDims { int N, C, H, W, K, R, S, sh, sw, ph, pw, oH, oW; };
 struct Pending {
   int kind = PEND_NONE;
@@ -29,6 +31,9 @@ struct Pending {
   const float *x = nullptr, *gamma = nullptr, *beta = nullptr;
   float *y = nullptr, *run_mean = nullptr, *run_var = nullptr, *save_mean = nullptr, *save_istd = nullptr;
   int N = 0, C = 0, HW = 0; float eps = 0, momentum = 0;
+  // PEND_LSM: y = log softmax of x, N rows of C; PEND_NLL: and out = -y[target].  PEND_SEED: d[0] = value; PEND_SUM_GRAD: and da[0..n) += scale d[0]
+  // (seeded: whether the first part is there); PEND_NLL_GRAD: and db[row][target] -= da[row], N rows of C
+  const int32_t* target = nullptr; float value = 0, scale = 0; bool seeded = false;
   // PEND_ADD: out = a + b
   const float *a = nullptr, *b = nullptr; float* out = nullptr;
   // PEND_RELU_GRAD: d = relu_y > 0 ? d : 0
@@ -62,6 +67,7 @@ struct Context {
   int64_t launches = 0;
   bool capturing = false;
   int64_t capture_launch_base = 0;
+  unsigned* tickets = nullptr;        // two device words, zero between launches: how many CTAs of a launch are done (one for each of the streams a branch region has)
   int* dev_status = nullptr;          // device word set by kernels whose bounded waits run out
   int* host_status = nullptr;         // pinned mirror
   int64_t wait_limit_cycles = 2000000000ll;   // bound of every device-side spin wait (about a second; ltb_set_wait_limit)
@@ -119,6 +125,8 @@ ZeroFill take_clear(Clear* c);                             // what a kernel is g
 int issue_ahead(Clear* clear = nullptr, float* cl = nullptr);
 int add_issue(const float* a, const float* b, float* out, int64_t n, bool relu);
 int relu_issue(float* x, int64_t n);
+int fill_issue(float* x, float v, int64_t n);
+int head_issue(const Pending& p);                          // PEND_LSM, PEND_NLL, PEND_SUM_GRAD, PEND_NLL_GRAD on their own (reduce.cu)
 int relu_grad_issue(const float* y, float* d, int64_t n);
 // Host waits while a communicator exists: bounded, with NCCL's asynchronous error state polled (comm.cu).
 void filter_cache_clear();           // gemm_tc.cu

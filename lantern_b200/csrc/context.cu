@@ -95,6 +95,7 @@ static int init_steps(int device, size_t heap_bytes) {
   g.heap_bytes = heap_bytes; g.used = 0;
   LTB_CUDA(cudaMalloc((void**)&g.dev_status, 256));
   LTB_CUDA(cudaMemset(g.dev_status, 0, 256));
+  g.tickets = reinterpret_cast<unsigned*>(g.dev_status) + 32;
   LTB_CUDA(cudaMallocHost((void**)&g.host_status, 256));
   g.host_status[0] = 0;
   g.scratch_bytes = (size_t)8 << 20;

@@ -458,6 +458,10 @@ int relu_issue(float* x, int64_t n) { return launch_map<1>(x, nullptr, nullptr, 
 int relu_grad_issue(const float* y, float* d, int64_t n) {
   return launch_map<2>(y, d, nullptr, d, n, [] __device__(float yv, float g0, float) { return yv > 0.0f ? g0 : 0.0f; });
 }
+int fill_issue(float* x, float v, int64_t n) {
+  if (n) LTB_LAUNCH(fill_kernel, grid_for(n, 256), 256, 0, x, v, n);
+  return LTB_OK;
+}
 int flush_pending() {
   const Pending p = g.pending;
   g.pending.kind = PEND_NONE;
@@ -469,6 +473,8 @@ int flush_pending() {
     case PEND_ADD: return add_issue(p.a, p.b, p.out, p.n, false);
     case PEND_RELU_GRAD: return relu_grad_issue(p.relu_y, p.d, p.n);
     case PEND_RELU_ADD_GRAD: return relu_add_grad_issue(p);
+    case PEND_SEED: return fill_issue(p.d, p.value, 1);
+    case PEND_LSM: case PEND_NLL: case PEND_SUM_GRAD: case PEND_NLL_GRAD: return head_issue(p);
     case PEND_BN_ADD: {                                         // no ReLU came: the two operations on their own, y written
       Pending q = p; q.kind = PEND_BN_FWD;
       int rc = bn_fwd_issue(q, false);
@@ -542,8 +548,8 @@ static size_t shape_count(const int* shape, int rank) {
 // fill / fillInPlace: TensorDslCPU.scala:30-35, 65-67.
 int ltb_fill(float* x, float v, int64_t n) {
   LTB_INITED(); filter_cache_note_write(x, (size_t)(n > 0 ? n : 0) * 4); LTB_REQUIRE(x && n >= 0, "ltb_fill: bad argument");
-  if (n) LTB_LAUNCH(fill_kernel, grid_for(n, 256), 256, 0, x, v, n);
-  return LTB_OK;
+  if (n == 1 && g.fusion) { Pending h; h.kind = PEND_SEED; h.n = 1; h.d = x; h.value = v; g.pending = h; return LTB_OK; }   // the gradient of a sum that reads it may join it
+  return fill_issue(x, v, n);
 }
 // fillWithBias: TensorDslCPU.scala:41-61.
 int ltb_fill_with_bias(float* out, const float* bias, int outer, int c, int inner) {

@@ -36,8 +36,8 @@ __global__ void sum_kernel(const float* __restrict__ x, float* out, int64_t n, f
 }
 __global__ void add_scalar_from_kernel(float* dx, const float* __restrict__ dout, float scale, int64_t n) {
   pdl_enter();
-  float v = dout[0] * scale;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) dx[i] += v;
+  const float v = dout[0];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) dx[i] = fmaf(v, scale, dx[i]);
 }
 // out[o, l] = sum_s x[o, s, l]
 __global__ void sum_dim_kernel(const float* __restrict__ x, float* out, int outer, int d, int inner) {
@@ -72,12 +72,9 @@ __global__ void sum_dim_grad_kernel(float* dx, const float* __restrict__ dout, i
 
 // One warp per row. MODE 0 softmax, 1 logSoftmax (TensorDslCPU.scala:783-832).  VPT > 0: a row of at most 32 VPT columns stays in registers, all its
 // loads in flight at once (8192 x 1000: 17 us walking the row three times, 15 so); VPT 0: any length.
+// Returns log sum exp of the row (MODE 1).
 template <int MODE, int VPT>
-__global__ void softmax_kernel(const float* __restrict__ x, float* y, int rows, int cols) {
-  pdl_enter();
-  int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; int lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  const float* p = x + r * cols; float* q = y + r * cols;
+__device__ __forceinline__ float softmax_row(const float* p, float* q, int cols, int lane) {
   float mx = -FLT_MAX, s = 0.0f;
   if constexpr (VPT > 0) {
     float v[VPT];
@@ -92,14 +89,52 @@ __global__ void softmax_kernel(const float* __restrict__ x, float* y, int rows, 
     const float logsum = mx + logf(s);
 #pragma unroll
     for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols) q[i] = MODE == 0 ? expf(v[j] - mx) / s : v[j] - logsum; }
-    return;
+    return logsum;
   }
   for (int i = lane; i < cols; i += 32) mx = fmaxf(mx, p[i]);
   mx = warp_max(mx);
   for (int i = lane; i < cols; i += 32) s += expf(p[i] - mx);
   s = warp_sum(s);
-  if (MODE == 0) { for (int i = lane; i < cols; i += 32) q[i] = expf(p[i] - mx) / s; }
-  else { float logsum = mx + logf(s); for (int i = lane; i < cols; i += 32) q[i] = p[i] - logsum; }
+  const float logsum = mx + logf(s);
+  for (int i = lane; i < cols; i += 32) q[i] = MODE == 0 ? expf(p[i] - mx) / s : p[i] - logsum;
+  return logsum;
+}
+template <int MODE, int VPT>
+__global__ void softmax_kernel(const float* __restrict__ x, float* y, int rows, int cols) {
+  pdl_enter();
+  int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; int lane = threadIdx.x & 31;
+  if (r < rows) softmax_row<MODE, VPT>(x + r * cols, y + r * cols, cols, lane);
+}
+// Log-softmax of a row, the negative log likelihood of its target (nll_kernel) and, with `sum`, scale times the sum of those: three launches of some
+// 3 us each on a batch of a few hundred rows, of which there is next to nothing to compute.  The last CTA to finish adds the rows up, in the order in
+// which sum_kernel's one CTA of 1024 threads does, so the result is the same to the bit.
+template <int VPT>
+__global__ void __launch_bounds__(256) softmax_nll_kernel(const float* __restrict__ x, float* y, const int32_t* __restrict__ t, float* nll, float* sum, float scale,
+                                                          int rows, int cols, unsigned* ticket) {
+  pdl_enter();
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (r < rows) {
+    const int k = t[r];
+    const bool in = k >= 0 && k < cols;
+    const float xk = in ? x[r * cols + k] : 0.0f;
+    const float logsum = softmax_row<1, VPT>(x + r * cols, y + r * cols, cols, lane);
+    if (lane == 0) nll[r] = in ? -1.0f * (xk - logsum) : 0.0f;
+  }
+  if (!sum) return;
+  __shared__ bool last;
+  __shared__ float part[32];
+  __syncthreads();
+  if (threadIdx.x == 0) { __threadfence(); last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1; __threadfence(); }      // back at zero after the last
+  __syncthreads();
+  if (!last) return;
+  for (int q = 0; q < 4; ++q) {
+    float s = 0.0f;
+    for (int i = threadIdx.x + 256 * q; i < rows; i += 1024) s += __ldcg(nll + i);
+    s = warp_sum(s);
+    if (lane == 0) part[w + 8 * q] = s;
+  }
+  __syncthreads();
+  if (w == 0) { const float s = warp_sum(part[lane]); if (lane == 0) sum[0] = s * scale; }
 }
 // MODE 0: dx += y*(dy - sum dy*y) (cudnnSoftmaxBackward ACCURATE, TensorDslCudnn.scala:1465-1504);
 // MODE 1: dx += dy - exp(y)*sum dy (TensorDslCPU.scala:837-846).  VPT as above.
@@ -131,6 +166,41 @@ __global__ void softmax_grad_kernel(float* dx, const float* __restrict__ y, cons
     for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
 #pragma unroll
     for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; if (i < cols) o[i] = old[j] + (MODE == 0 ? w[j] * (v[j] - s) : v[j] - expf(w[j]) * s); }
+  }
+}
+// What leads from the gradient of a loss to that of the logits, a warp per row: dnll += scale dout (dout set to `value` first when it is seeded here),
+// dlogp[target] -= dnll, dx += dlogp - exp(y) sum dlogp; every buffer ends up as the separate launches leave it (four of 2.5 to 4 us each).
+template <int VPT>
+__global__ void __launch_bounds__(256) nll_softmax_grad_kernel(float* dx, const float* __restrict__ y, float* dlogp, float* dnll, float* dout, bool seeded, float value,
+                                                               float scale, const int32_t* __restrict__ t, int rows, int cols) {
+  pdl_enter();
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; const int lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const int k = t[r];
+  const float dn = fmaf(seeded ? value : dout[0], scale, dnll[r]);
+  if (lane == 0) { dnll[r] = dn; if (seeded && r == 0) dout[0] = value; }
+  const float* yy = y + r * cols; float* d = dlogp + r * cols; float* o = dx + r * cols;
+  float s = 0.0f;
+  if constexpr (VPT > 0) {
+    float v[VPT], w[VPT], old[VPT];
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols && i == k) { v[j] += -1.0f * dn; d[i] = v[j]; } if (i < cols) s += v[j]; }
+    s = warp_sum(s);
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols) o[i] = old[j] + (v[j] - expf(w[j]) * s); }
+    return;
+  }
+#pragma unroll 8
+  for (int i = lane; i < cols; i += 32) { float v = d[i]; if (i == k) { v += -1.0f * dn; d[i] = v; } s += v; }
+  s = warp_sum(s);
+  for (int i0 = lane; i0 < cols; i0 += 128) {            // each lane reads back what it wrote itself
+    float v[4], w[4], old[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; if (i < cols) o[i] = old[j] + (v[j] - expf(w[j]) * s); }
   }
 }
 __global__ void nll_kernel(const float* __restrict__ x, const int32_t* __restrict__ t, float* out, int rows, int cols) {
@@ -214,6 +284,60 @@ static int full_sum(const float* x, float* out, int64_t n, float scale) {
   return LTB_OK;
 }
 
+// ---- the calls around a classifier's loss that look-ahead fusion joins
+constexpr int kHeadSumRows = 1 << 16;                       // one CTA adds them up, as in full_sum
+static int softmax_nll_issue(const Pending& p, float* sum, float scale) {
+  const unsigned grid = (unsigned)ceil_div((int64_t)p.N * 32, 256);
+  unsigned* const ticket = g.tickets + (g.in_branch ? 1 : 0);
+  if (p.C <= 32) LTB_LAUNCH((softmax_nll_kernel<1>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
+  else if (p.C <= 256) LTB_LAUNCH((softmax_nll_kernel<8>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
+  else if (p.C <= 1024) LTB_LAUNCH((softmax_nll_kernel<32>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
+  else LTB_LAUNCH((softmax_nll_kernel<0>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
+  return LTB_OK;
+}
+static int nll_softmax_grad_issue(const Pending& p, float* dx, const float* y) {
+  const unsigned grid = (unsigned)ceil_div((int64_t)p.N * 32, 256);
+  if (p.C <= 32) LTB_LAUNCH((nll_softmax_grad_kernel<1>), grid, 256, 0, dx, y, p.db, p.da, p.d, p.seeded, p.value, p.scale, p.target, p.N, p.C);
+  else if (p.C <= 256) LTB_LAUNCH((nll_softmax_grad_kernel<8>), grid, 256, 0, dx, y, p.db, p.da, p.d, p.seeded, p.value, p.scale, p.target, p.N, p.C);
+  else LTB_LAUNCH((nll_softmax_grad_kernel<0>), grid, 256, 0, dx, y, p.db, p.da, p.d, p.seeded, p.value, p.scale, p.target, p.N, p.C);
+  return LTB_OK;
+}
+static int sum_grad_issue(float* dx, const float* dout, float scale, int64_t n) {
+  if (n) LTB_LAUNCH(add_scalar_from_kernel, grid_for(n, 256), 256, 0, dx, dout, scale, n);
+  return LTB_OK;
+}
+static int nll_grad_issue(float* dx, const float* dout, const int32_t* t, int rows, int cols) {
+  LTB_LAUNCH(nll_grad_kernel, (rows + 127) / 128, 128, 0, dx, dout, t, rows, cols);
+  return LTB_OK;
+}
+int head_issue(const Pending& p) {
+  if (p.kind == PEND_LSM) return softmax_issue<1>(p.x, p.y, p.N, p.C);
+  if (p.kind == PEND_NLL) return softmax_nll_issue(p, nullptr, 0.0f);
+  int rc = p.seeded ? fill_issue(p.d, p.value, 1) : LTB_OK;
+  if (!rc) rc = sum_grad_issue(p.da, p.d, p.scale, p.n);
+  return rc || p.kind == PEND_SUM_GRAD ? rc : nll_grad_issue(p.db, p.da, p.target, p.N, p.C);
+}
+// Whether [p, p + floats) keeps clear of [q, q + n).
+static bool apart(const void* p, int64_t floats, const void* q, int64_t n) { return (const float*)p + floats <= (const float*)q || (const float*)q + n <= (const float*)p; }
+static int full_sum_joining(const float* x, float* out, int64_t n, float scale) {
+  if (g.pending.kind == PEND_NLL && g.pending.out == x && g.pending.N == n && n <= kHeadSumRows) {
+    const Pending p = g.pending; g.pending.kind = PEND_NONE;
+    return softmax_nll_issue(p, out, scale);               // (the last CTA writes out: nothing is read any more)
+  }
+  if (g.pending.kind) { int rc = flush_pending(); if (rc) return rc; }
+  return full_sum(x, out, n, scale);
+}
+// dx += scale dout.  A held call that cannot be joined is issued before anything else of this one, its zero fills included.
+static int sum_grad_joining(float* dx, const float* dout, float scale, int64_t n) {
+  const bool clear = apart(dx, n, dout, 1), seeded = g.pending.kind == PEND_SEED && g.pending.d == dout && clear;
+  if (g.pending.kind && !seeded) { int rc = flush_pending(); if (rc) return rc; }
+  Pending h; h.kind = PEND_SUM_GRAD; h.n = n; h.da = dx; h.d = const_cast<float*>(dout); h.scale = scale; h.seeded = seeded; h.value = g.pending.value;
+  LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_WRITES(dx, n);
+  g.pending = h;
+  if (g.fusion && n > 0 && clear) return LTB_OK;           // the gradient of a negative log likelihood may join it
+  return flush_pending();
+}
+
 }  // namespace ltb
 
 using namespace ltb;
@@ -221,17 +345,15 @@ using namespace ltb;
 extern "C" {
 
 // sum / mean and their grads: TensorDslCPU.scala:1115-1124.
-int ltb_sum(const float* x, float* out, int64_t n) { LTB_INITED(); LTB_REQUIRE(x && out && n >= 0, "ltb_sum: bad argument"); LTB_WRITES(out, 1); return full_sum(x, out, n, 1.0f); }
-int ltb_mean(const float* x, float* out, int64_t n) { LTB_INITED(); LTB_REQUIRE(x && out && n > 0, "ltb_mean: bad argument"); LTB_WRITES(out, 1); return full_sum(x, out, n, 1.0f / (float)n); }
+int ltb_sum(const float* x, float* out, int64_t n) { LTB_INITED_NOFLUSH(); LTB_REQUIRE(x && out && n >= 0, "ltb_sum: bad argument"); LTB_WRITES(out, 1); return full_sum_joining(x, out, n, 1.0f); }
+int ltb_mean(const float* x, float* out, int64_t n) { LTB_INITED_NOFLUSH(); LTB_REQUIRE(x && out && n > 0, "ltb_mean: bad argument"); LTB_WRITES(out, 1); return full_sum_joining(x, out, n, 1.0f / (float)n); }
 int ltb_sum_grad(float* dx, const float* dout, int64_t n) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && n >= 0, "ltb_sum_grad: bad argument"); LTB_WRITES(dx, n);
-  if (n) LTB_LAUNCH(add_scalar_from_kernel, grid_for(n, 256), 256, 0, dx, dout, 1.0f, n);
-  return LTB_OK;
+  LTB_INITED_NOFLUSH(); LTB_REQUIRE(dx && dout && n >= 0, "ltb_sum_grad: bad argument");
+  return sum_grad_joining(dx, dout, 1.0f, n);
 }
 int ltb_mean_grad(float* dx, const float* dout, int64_t n) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && n > 0, "ltb_mean_grad: bad argument"); LTB_WRITES(dx, n);
-  LTB_LAUNCH(add_scalar_from_kernel, grid_for(n, 256), 256, 0, dx, dout, 1.0f / (float)n, n);
-  return LTB_OK;
+  LTB_INITED_NOFLUSH(); LTB_REQUIRE(dx && dout && n > 0, "ltb_mean_grad: bad argument");
+  return sum_grad_joining(dx, dout, 1.0f / (float)n, n);
 }
 // sum(dim) / sum_grad(dim): TensorDslCPU.scala:1125-1164.
 int ltb_sum_dim(const float* x, float* out, int outer, int d, int inner) {
@@ -301,24 +423,48 @@ int ltb_softmax(const float* x, float* y, int rows, int cols) {
 }
 int ltb_log_softmax(const float* x, float* y, int rows, int cols) {
   LTB_INITED(); LTB_REQUIRE(x && y && rows > 0 && cols > 0, "ltb_log_softmax: bad argument"); LTB_WRITES(y, (size_t)rows * cols);
-  return softmax_issue<1>(x, y, rows, cols);
+  if (!g.fusion) return softmax_issue<1>(x, y, rows, cols);
+  Pending h; h.kind = PEND_LSM; h.x = x; h.y = y; h.N = rows; h.C = cols;      // the negative log likelihood of y may join it
+  g.pending = h;
+  return LTB_OK;
 }
 int ltb_softmax_grad(float* dx, const float* y, const float* dy, int rows, int cols) {
   LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_softmax_grad: bad argument"); LTB_WRITES(dx, (size_t)rows * cols);
   return softmax_grad_issue<0>(dx, y, dy, rows, cols);
 }
 int ltb_log_softmax_grad(float* dx, const float* y, const float* dy, int rows, int cols) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_log_softmax_grad: bad argument"); LTB_WRITES(dx, (size_t)rows * cols);
-  return softmax_grad_issue<1>(dx, y, dy, rows, cols);
+  LTB_INITED_NOFLUSH(); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_log_softmax_grad: bad argument");
+  const Pending p = g.pending;
+  const int64_t n = (int64_t)rows * cols;
+  const bool joins = p.kind == PEND_NLL_GRAD && p.db == dy && p.N == rows && p.C == cols && apart(dx, n, dy, n) && apart(dx, n, p.da, rows) && apart(dx, n, p.d, 1) &&
+                     apart(dx, n, p.target, rows) && apart(y, n, dx, n) && apart(y, n, dy, n) && apart(y, n, p.da, rows) && apart(y, n, p.d, 1);
+  if (joins) g.pending.kind = PEND_NONE;
+  else if (p.kind) { int rc = flush_pending(); if (rc) return rc; }
+  LTB_SETTLE(dx); LTB_SETTLE(dy); LTB_WRITES(dx, (size_t)rows * cols);
+  return joins ? nll_softmax_grad_issue(p, dx, y) : softmax_grad_issue<1>(dx, y, dy, rows, cols);
 }
 // nllLoss / nllLoss_grad: TensorDslCPU.scala:1090-1110.
 int ltb_nll(const float* x, const int32_t* t, float* out, int rows, int cols) {
-  LTB_INITED(); LTB_REQUIRE(x && t && out && rows > 0 && cols > 0, "ltb_nll: bad argument"); LTB_WRITES(out, rows);
+  LTB_INITED_NOFLUSH(); LTB_REQUIRE(x && t && out && rows > 0 && cols > 0, "ltb_nll: bad argument"); LTB_WRITES(out, rows);
+  const int64_t n = (int64_t)rows * cols;
+  if (g.pending.kind == PEND_LSM && g.pending.y == x && g.pending.N == rows && g.pending.C == cols && apart(out, rows, x, n) && apart(out, rows, g.pending.x, n) &&
+      apart(out, rows, t, rows) && apart(t, rows, x, n)) {
+    g.pending.kind = PEND_NLL; g.pending.target = t; g.pending.out = out;                           // their sum or mean may join it
+    return LTB_OK;
+  }
+  if (g.pending.kind) { int rc = flush_pending(); if (rc) return rc; }
   LTB_LAUNCH(nll_kernel, (rows + 127) / 128, 128, 0, x, t, out, rows, cols); return LTB_OK;
 }
 int ltb_nll_grad(float* dx, const float* dout, const int32_t* t, int rows, int cols) {
-  LTB_INITED(); LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_REQUIRE(dx && dout && t && rows > 0 && cols > 0, "ltb_nll_grad: bad argument"); LTB_WRITES(dx, (size_t)rows * cols);
-  LTB_LAUNCH(nll_grad_kernel, (rows + 127) / 128, 128, 0, dx, dout, t, rows, cols); return LTB_OK;
+  LTB_INITED_NOFLUSH(); LTB_REQUIRE(dx && dout && t && rows > 0 && cols > 0, "ltb_nll_grad: bad argument");
+  const int64_t n = (int64_t)rows * cols;
+  const bool joins = g.pending.kind == PEND_SUM_GRAD && g.pending.da == dout && g.pending.n == rows && apart(dx, n, dout, rows) && apart(dx, n, g.pending.d, 1) &&
+                     apart(t, rows, dx, n) && apart(t, rows, dout, rows) && apart(t, rows, g.pending.d, 1);
+  if (!joins && g.pending.kind) { int rc = flush_pending(); if (rc) return rc; }
+  LTB_SETTLE(dx); LTB_SETTLE(dout); LTB_WRITES(dx, (size_t)rows * cols);
+  if (!joins) return nll_grad_issue(dx, dout, t, rows, cols);
+  g.pending.kind = PEND_NLL_GRAD; g.pending.db = dx; g.pending.target = t; g.pending.N = rows; g.pending.C = cols;      // the log-softmax's gradient may join it
+  return LTB_OK;
 }
 
 // vectorVectorDot / matrixVectorDot and the (1,1), (2,1) cases of dot_grad: TensorDslCPU.scala:135-206.

@@ -518,6 +518,43 @@ def test_gemm_of_ragged_rows_tf32(ora, gpu, ta, tb, M, N, K):
         assert_close(ref[k], got[k], FP32_RTOL, k)
 
 
+@pytest.mark.parametrize("rows,cols,mean", [(1, 2, 0), (7, 32, 1), (8, 33, 0), (9, 256, 1), (1030, 10, 1), (2500, 300, 0), (77, 1025, 1), (65536, 3, 1), (65537, 3, 0)])
+def test_loss_head_in_one_kernel_each_way(gpu, rows, cols, mean):
+    """log-softmax, negative log likelihood and their sum or mean, and the way back from a seeded gradient: with look-ahead fusion one kernel each, and
+    every buffer as the separate calls leave it, bit for bit (the same operations in the same order): with destinations that hold something already,
+    targets out of range, and a sequence broken off after each of its calls."""
+    import torch
+    lib = gpu.lib
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, device="cuda", generator=gen) * 3
+    t = torch.randint(-1, cols + 1, (rows,), device="cuda", generator=gen, dtype=torch.int32)
+    old = [torch.randn(n, device="cuda", generator=gen) for n in (rows, rows * cols, rows * cols)]
+    names = ("logp", "nll", "loss", "dloss", "dnll", "dlogp", "dx")
+
+    def run(fusion, stop):
+        lib.set_fusion(fusion)
+        b = [torch.zeros(n, device="cuda") for n in (rows * cols, rows, 1, 1)] + [o.clone() for o in old]
+        p = [v.data_ptr() for v in b]
+        torch.cuda.synchronize()
+        before = lib.kernel_launches()
+        calls = [lambda: lib.log_softmax(x.data_ptr(), p[0], rows, cols), lambda: lib.nll(p[0], t.data_ptr(), p[1], rows, cols),
+                 lambda: (lib.mean if mean else lib.sum)(p[1], p[2], rows), lambda: lib.fill(p[3], 0.75, 1),
+                 lambda: (lib.mean_grad if mean else lib.sum_grad)(p[4], p[3], rows), lambda: lib.nll_grad(p[5], p[4], t.data_ptr(), rows, cols),
+                 lambda: lib.log_softmax_grad(p[6], p[0], p[5], rows, cols)]
+        for c in calls[:stop]:
+            c()
+        lib.sync()
+        launches = lib.kernel_launches() - before
+        lib.set_fusion(0)
+        return b, launches
+    for stop in range(1, 8):
+        a, many = run(0, stop)
+        f, few = run(1, stop)
+        for name, u, v in zip(names, a, f):
+            assert torch.equal(u, v), (stop, name)
+        assert stop < 7 or few == (2 if rows <= 65536 else 4), (many, few)
+
+
 @pytest.mark.parametrize("det", [0, 1])
 @pytest.mark.parametrize("M,N,K,ta,tb", [(4740, 1000, 516, 0, 1), (512, 508, 20000, 1, 0), (4096, 1196, 996, 0, 1), (2564, 1476, 1028, 0, 1), (1284, 508, 7172, 1, 0)])
 def test_gemm_in_wide_tiles_tf32(ora, gpu, M, N, K, ta, tb, det):
