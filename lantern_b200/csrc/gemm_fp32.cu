@@ -596,10 +596,106 @@ static int skinny_gemm(const float* a, int64_t sam, int64_t sak, const float* b,
   return LTB_OK;
 }
 
+// ---- small products: so few outputs that one round of 32 x 32 tiles covers them ------------------------------------------------
+// The time of such a product is latency: the tiles above walk K in steps of 16, each a round trip to memory and a barrier.  Here a CTA of sixteen warps
+// fetches all of k of both operands at once (up to sixteen loads of a thread in flight; 4-byte cp.async leave an SM at one warp's worth per 18 cycles:
+// 100 x 50 x 320 8.4 us), each warp takes a sixteenth of k and the whole T x T tile, and their sums meet in shared memory in warp order: the same bits on
+// every run, and shorter chains than the tiles above have.  T is 16 while such tiles fit one round of the SMs: a quarter of the arithmetic per SM.
+constexpr int kSmallWarps = 16, kSmallPart = 33;
+template <int T> constexpr int kSmallK = 16384 / T;       // what shared memory holds of both operands: 1024 of k, or 512
+template <int T>
+__device__ __forceinline__ void small_fetch(float* dst, const float* p, int64_t row, int64_t kst, int rows, int len, int units, int warp, int lane) {
+  const bool along_k = kst == 1 && row != 1;                                          // a warp reads 8 of k by 4 rows (whole sectors), or T rows
+  auto at = [&](int u, int& k, int& m) {
+    if (along_k) { k = u / (T / 4) * 8 + (lane & 7); m = u % (T / 4) * 4 + (lane >> 3); }
+    else { k = u * (32 / T) + lane / T; m = lane % T; }
+  };
+  for (int u0 = warp; u0 < units; u0 += 16 * kSmallWarps) {
+    float v[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) { int k, m; at(u0 + e * kSmallWarps, k, m); v[e] = k < len && m < rows ? p[m * row + k * kst] : 0.0f; }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) { int k, m; at(u0 + e * kSmallWarps, k, m); if (u0 + e * kSmallWarps < units) dst[k * (T + 4) + m] = v[e]; }     // pitch T + 4: 8 of k by 4 rows hit 32 banks
+  }
+}
+template <bool ACC, int T>
+__global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_kernel(const float* __restrict__ a, int64_t sam, int64_t sak, const float* __restrict__ b, int64_t sbk, int64_t sbn,
+                                                                      float* c, int64_t scm, int64_t scn, int M, int N, int K, float alpha) {
+  extern __shared__ __align__(16) float small_smem[];
+  constexpr int TM = T / 8, TN = T / 4, P = T + 4;                                    // a lane's rows and columns
+  pdl_enter();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m0 = blockIdx.x * T, n0 = blockIdx.y * T;
+  const int lenp = (K + 15) / 16 * 16, per = lenp / kSmallWarps;
+  float* const as = small_smem; float* const bs = small_smem + lenp * P;
+  small_fetch<T>(as, a + m0 * sam, sam, sak, M - m0, K, lenp * T / 32, warp, lane);
+  small_fetch<T>(bs, b + n0 * sbn, sbn, sbk, N - n0, K, lenp * T / 32, warp, lane);
+  __syncthreads();
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+  const int lm = lane & 7, ln = lane >> 3;                                            // rows TM lm .., columns TN ln ..
+#pragma unroll 4
+  for (int k = warp * per; k < (warp + 1) * per; ++k) {
+    float u[TM], v[TN];
+#pragma unroll
+    for (int i = 0; i < TM; i += 2) { const float2 x = *reinterpret_cast<const float2*>(as + k * P + TM * lm + i); u[i] = x.x; u[i + 1] = x.y; }
+#pragma unroll
+    for (int j = 0; j < TN; j += 4) { const float4 y = *reinterpret_cast<const float4*>(bs + k * P + TN * ln + j); v[j] = y.x; v[j + 1] = y.y; v[j + 2] = y.z; v[j + 3] = y.w; }
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] += u[i] * v[j];
+  }
+  __syncthreads();
+  constexpr int kWarpSums = TM * TN * kSmallPart;
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) small_smem[warp * kWarpSums + (i * TN + j) * kSmallPart + lane] = acc[i][j];
+  __syncthreads();
+  const bool by_rows = scm == 1 && scn != 1;                                          // neighbouring lanes: neighbouring addresses of c
+#pragma unroll
+  for (int e = threadIdx.x; e < T * T; e += kSmallWarps * 32) {
+    const int m = by_rows ? e % T : e / T, n = by_rows ? e / T : e % T;
+    const float* q = small_smem + (m % TM * TN + n % TN) * kSmallPart + n / TN * 8 + m / TM;
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kSmallWarps; ++w) v += q[w * kWarpSums];
+    if (m0 + m < M && n0 + n < N) {
+      float* d = c + (m0 + m) * scm + (n0 + n) * scn;
+      *d = ACC ? *d + alpha * v : alpha * v;
+    }
+  }
+}
+// One round of CTAs and one fetch.  Measured with the probe's call overhead of 5 us included, tiles above against this, us: 100 x 50 x 320 11.3 / 5.8,
+// 128 x 128 x 128 8.1 / 5.5, 128 x 128 x 512 9.8 / 5.4, 64 x 64 x 1024 9.9 / 8.5, 240 x 240 x 300 12.3 / 7.5, 384 x 384 x 64 5.7 / 5.5, 384 x 384 x 512 14.6 / 9.3;
+// walking a longer K in several fetches (32 x 32 tiles) lost: 200 x 300 x 1500 20.9 / 24.8, 128 x 128 x 2048 16 / 33.
+template <int T> static bool small_takes(int M, int N, int K) { return K <= kSmallK<T> && ceil_div(M, T) * ceil_div(N, T) <= g.sm_count; }
+template <int T>
+static int small_gemm(const float* a, int64_t sam, int64_t sak, const float* b, int64_t sbk, int64_t sbn, float* c, int64_t scm, int64_t scn,
+                      int M, int N, int K, float alpha, bool accumulate) {
+  constexpr int kMost = 2 * kSmallK<T> * (T + 4) * 4, kSums = kSmallWarps * T * T / 32 * kSmallPart * 4;
+  static bool ready = false;
+  if (!ready) {
+    LTB_CUDA(cudaFuncSetAttribute((small_gemm_kernel<false, T>), cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+    LTB_CUDA(cudaFuncSetAttribute((small_gemm_kernel<true, T>), cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+    ready = true;
+  }
+  const int panels = 2 * ((K + 15) / 16 * 16) * (T + 4) * 4, smem = panels > kSums ? panels : kSums;
+  const dim3 grid((unsigned)ceil_div(M, T), (unsigned)ceil_div(N, T));
+  if (accumulate) LTB_LAUNCH((small_gemm_kernel<true, T>), grid, kSmallWarps * 32, smem, a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha);
+  else LTB_LAUNCH((small_gemm_kernel<false, T>), grid, kSmallWarps * 32, smem, a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha);
+  return LTB_OK;
+}
+
 // C[M,N] (op)= alpha * A B with arbitrary strides; accumulate selects += (gradients) over = (forward).
 static int strided_gemm(const float* a, int64_t sam, int64_t sak, const float* b, int64_t sbk, int64_t sbn, float* c, int64_t scm,
                         int64_t scn, int M, int N, int K, float alpha, bool accumulate) {
   { bool taken = false; int rc = skinny_gemm(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate, &taken); if (rc || taken) return rc; }
+  if (small_takes<16>(M, N, K)) return small_gemm<16>(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate);
+  if (small_takes<32>(M, N, K)) return small_gemm<32>(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate);
   // m of the kernel is the contiguous index of C
   const bool swap = scn == 1 && scm != 1;
   const int m = swap ? N : M, n = swap ? M : N;

@@ -518,6 +518,41 @@ def test_gemm_of_ragged_rows_tf32(ora, gpu, ta, tb, M, N, K):
         assert_close(ref[k], got[k], FP32_RTOL, k)
 
 
+@pytest.mark.parametrize("acc", [0, 1])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(17, 17, 17), (33, 31, 64), (1, 300, 45), (300, 1, 21), (193, 190, 33), (192, 190, 1024), (100, 50, 320), (385, 383, 17), (380, 381, 512), (190, 190, 513), (50, 100, 1025)])
+def test_small_products_fp32(gpu, M, N, K, ta, tb, acc):
+    """Products of one round of 16 x 16 or 32 x 32 tiles, at the edges of tiles, of the sixteenths of K and of the rules, against float64.  The sum of K
+    products in any order differs from the exact one by at most K roundings of the sum of their magnitudes."""
+    import torch
+    gpu.lib.set_math(0)
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn((K, M) if ta else (M, K), device="cuda", generator=gen)
+    b = torch.randn((N, K) if tb else (K, N), device="cuda", generator=gen)
+    torch.cuda.synchronize()
+    A, B = (a.double().T if ta else a.double()), (b.double().T if tb else b.double())
+    if not acc:
+        c = torch.full((M, N), float("nan"), device="cuda"); torch.cuda.synchronize()
+        gpu.lib.gemm(a.data_ptr(), ta, b.data_ptr(), tb, 0.5, c.data_ptr(), M, N, K)
+        gpu.lib.sync()
+        assert ((c.double() - 0.5 * (A @ B)).abs() <= K * 2.0 ** -24 * (A.abs() @ B.abs())).all()
+    else:                                                # both gradients of a product of M x K by K x N, added to what is there
+        dc = torch.randn(M, N, device="cuda", generator=gen)
+        da, db = torch.randn(a.shape, device="cuda", generator=gen), torch.randn(b.shape, device="cuda", generator=gen)
+        da0, db0 = da.double(), db.double()
+        torch.cuda.synchronize()
+        gpu.lib.gemm_grad(a.data_ptr(), da.data_ptr(), ta, b.data_ptr(), db.data_ptr(), tb, 0.5, dc.data_ptr(), M, N, K)
+        gpu.lib.sync()
+        D = dc.double()
+        ra, rb = D @ B.T, A.T @ D
+        ma, mb = D.abs() @ B.abs().T, A.abs().T @ D.abs()
+        for got, old, r, m, n, t in ((da, da0, ra, ma, N, ta), (db, db0, rb, mb, M, tb)):
+            r, m = (r.T, m.T) if t else (r, m)
+            want = old + 0.5 * r
+            assert ((got.double() - want).abs() <= (n + 2) * 2.0 ** -24 * (m + old.abs())).all()
+    gpu.lib.set_math(1)
+
+
 @pytest.mark.parametrize("rows,cols,mean", [(1, 2, 0), (7, 32, 1), (8, 33, 0), (9, 256, 1), (1030, 10, 1), (2500, 300, 0), (77, 1025, 1), (65536, 3, 1), (65537, 3, 0)])
 def test_loss_head_in_one_kernel_each_way(gpu, rows, cols, mean):
     """log-softmax, negative log likelihood and their sum or mean, and the way back from a seeded gradient: with look-ahead fusion one kernel each, and
