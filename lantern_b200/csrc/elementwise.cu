@@ -45,17 +45,29 @@ __device__ __forceinline__ float un_grad(int op, float x, float y, float dy) {
 
 // ---- generic vectorised map over up to three inputs -------------------------------------------------------------
 // F: float f(float a, float b, float c); a/b/c may be null (then 0 is passed). out may alias any input.
-template <int NIN, class F>
-__global__ void map_vec4(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c,
-                         float* out, int64_t n4, F f) {
+// U items of a thread in flight: 4 where the tensor gives every thread of the GPU one and more (a 3x3 layer with batch norm and ReLU on 32 x 64 x 56 x 56, forward and
+// backward, 212 -> 210 us; SqueezeNet at batch 64 776 -> 763), else 1 on as many
+// CTAs as there are.
+template <int NIN, int U, class F>
+__global__ void __launch_bounds__(256) map_vec4(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c,
+                                                float* out, int64_t n4, F f) {
   pdl_enter();
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n4; i += stride) {
-    float4 va = reinterpret_cast<const float4*>(a)[i];
-    float4 vb = NIN > 1 ? reinterpret_cast<const float4*>(b)[i] : make_float4(0, 0, 0, 0);
-    float4 vc = NIN > 2 ? reinterpret_cast<const float4*>(c)[i] : make_float4(0, 0, 0, 0);
+  const int64_t i0 = (int64_t)blockIdx.x * 256 * U + threadIdx.x;
+  float4 va[U], vb[U], vc[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t i = i0 + 256 * u;
+    if (i >= n4) break;
+    va[u] = reinterpret_cast<const float4*>(a)[i];
+    vb[u] = NIN > 1 ? reinterpret_cast<const float4*>(b)[i] : make_float4(0, 0, 0, 0);
+    vc[u] = NIN > 2 ? reinterpret_cast<const float4*>(c)[i] : make_float4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t i = i0 + 256 * u;
+    if (i >= n4) break;
     float4 r;
-    r.x = f(va.x, vb.x, vc.x); r.y = f(va.y, vb.y, vc.y); r.z = f(va.z, vb.z, vc.z); r.w = f(va.w, vb.w, vc.w);
+    r.x = f(va[u].x, vb[u].x, vc[u].x); r.y = f(va[u].y, vb[u].y, vc[u].y); r.z = f(va[u].z, vb[u].z, vc[u].z); r.w = f(va[u].w, vb[u].w, vc[u].w);
     reinterpret_cast<float4*>(out)[i] = r;
   }
 }
@@ -70,7 +82,9 @@ int launch_map(const float* a, const float* b, const float* c, float* out, int64
   if (n <= 0) return LTB_OK;
   bool vec = aligned16(a) && aligned16(out) && (NIN < 2 || aligned16(b)) && (NIN < 3 || aligned16(c));
   int64_t n4 = vec ? n / 4 : 0;
-  if (n4 > 0) LTB_LAUNCH((map_vec4<NIN, F>), grid_for(n4, 256), 256, 0, a, b, c, out, n4, f);
+  LTB_REQUIRE(n4 <= (int64_t)256 * 0x7fffffff, "elementwise operation on too many elements");
+  if (n4 > (int64_t)g.sm_count * 2048) LTB_LAUNCH((map_vec4<NIN, 4, F>), (unsigned)ceil_div(n4, 1024), 256, 0, a, b, c, out, n4, f);
+  else if (n4 > 0) LTB_LAUNCH((map_vec4<NIN, 1, F>), (unsigned)ceil_div(n4, 256), 256, 0, a, b, c, out, n4, f);
   if (n4 * 4 < n) LTB_LAUNCH((map_scalar<NIN, F>), grid_for(n - n4 * 4, 256), 256, 0, a, b, c, out, n4 * 4, n, f);
   return LTB_OK;
 }
