@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_kernel(const floa
     }
   }
 }
-// One round of CTAs and one fetch.  Measured with the probe's call overhead of 5 us included, tiles above against this, us: 100 x 50 x 320 11.3 / 5.8,
+// One round of CTAs and one fetch.  Measured from Python, 5 us of call overhead included, tiles above against this, us: 100 x 50 x 320 11.3 / 5.8,
 // 128 x 128 x 128 8.1 / 5.5, 128 x 128 x 512 9.8 / 5.4, 64 x 64 x 1024 9.9 / 8.5, 240 x 240 x 300 12.3 / 7.5, 384 x 384 x 64 5.7 / 5.5, 384 x 384 x 512 14.6 / 9.3;
 // walking a longer K in several fetches (32 x 32 tiles) lost: 200 x 300 x 1500 20.9 / 24.8, 128 x 128 x 2048 16 / 33.
 template <int T> static bool small_takes(int M, int N, int K) { return K <= kSmallK<T> && ceil_div(M, T) * ceil_div(N, T) <= g.sm_count; }
