@@ -28,6 +28,7 @@ _SIGS = {
     "model_set_resident": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
     "model_step": (ctypes.c_float, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float, ctypes.c_int]),
     "model_step_async": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float]),
+    "model_status": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_int]),
     "model_last_loss": (ctypes.c_float, [ctypes.c_void_p]),
     "model_logits": (ctypes.c_int64, [ctypes.c_void_p, ctypes.c_void_p]),
     "model_submit": (ctypes.c_int64, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float]),
@@ -112,22 +113,29 @@ class Model:
         assert x.size == self.input_count and y.size == self.label_count
         return x, y
 
+    def _failure(self):
+        buf = ctypes.create_string_buffer(512)
+        rc = self.hp.fn["model_status"](self.h, buf, 512)
+        return "%d %s" % (rc, buf.value.decode(errors="replace")) if rc else ""
+
     def step(self, x, y, lr, update=True):
         x, y = self._arrs(x, y)
-        return float(self.hp.fn["model_step"](self.h, x.ctypes.data, y.ctypes.data, lr, int(update)))
+        loss = float(self.hp.fn["model_step"](self.h, x.ctypes.data, y.ctypes.data, lr, int(update)))
+        if loss != loss and self._failure():             # a failed step's loss is a NaN, and so is a diverged network's
+            raise RuntimeError("model_step failed: " + self._failure())
+        return loss
 
     def step_async(self, x, y, lr):
         x, y = self._arrs(x, y)
-        rc = self.hp.fn["model_step_async"](self.h, x.ctypes.data, y.ctypes.data, lr)
-        if rc:
-            raise RuntimeError("model_step_async failed: %d %s" % (rc, self.lib.error_message()))
+        if self.hp.fn["model_step_async"](self.h, x.ctypes.data, y.ctypes.data, lr):
+            raise RuntimeError("model_step_async failed: " + self._failure())
 
     def submit(self, x, y, lr):
         """Queue one training step on host arrays and return its number without waiting (two steps stay in flight)."""
         x, y = self._arrs(x, y)
         k = self.hp.fn["model_submit"](self.h, x.__array_interface__["data"][0], y.__array_interface__["data"][0], lr)
         if k < 0:
-            raise RuntimeError("model_submit failed: %s" % self.lib.error_message())
+            raise RuntimeError("model_submit failed: " + (self._failure() or self.lib.error_message()))
         return k
 
     def collect(self, step):
@@ -174,7 +182,8 @@ class Model:
             self.hp.fn["model_set_resident"](self.h, None, None)
             return
         x, y = self._arrs(x, y)
-        self.hp.fn["model_set_resident"](self.h, x.ctypes.data, y.ctypes.data)
+        if self.hp.fn["model_set_resident"](self.h, x.ctypes.data, y.ctypes.data):
+            raise RuntimeError("model_set_resident failed: " + self._failure())
 
     def trace(self, x, y):
         """Debug: one row per operator output of one step without update, in forward order: (index, count, shape, sum|x|,

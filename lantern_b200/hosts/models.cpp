@@ -132,11 +132,19 @@ struct Model {
     mark = BK(mark)();
   }
   virtual TR forward(Tape& t, const TR& x, const int32_t* y) = 0;
+  // What became of the last step: 0, or the code of what kept it from being run, with the reason if it was this program's own (else the
+  // library has it).  A step that fails leaves the parameters as they were.
+  int status = 0;
+  std::string reason;
+  void note(int rc) { if (rc && !status) status = rc; }
+  int refuse(int rc, const char* why) { status = rc; reason = why; return rc; }
+  // Labels that no call may see (null: the labels are fine): they would send a kernel, or the program itself, outside an array.
+  virtual const char* bad_labels(const int32_t*) { return nullptr; }
   // Data that a step draws on the host (a dropout mask): into staging block p, and from there to where the step reads it.
   virtual int draw_host_data(int) { return 0; }
 
   // One training step's device work, in the order of the generated programs.
-  void enqueue(float lr, bool update) {
+  int enqueue(float lr, bool update) {
     Tape tape;
     zero_pool_begin(zero_bytes);
     int64_t nin = (int64_t)batch * in_c * in_h * in_w;
@@ -154,16 +162,18 @@ struct Model {
     early_reduce = update && BK(comm_world)() > 1;
     last_logits = TR();
     TR loss = forward(tape, x, y);
+    if (status) { zero_pool_end(); BK(reset)(mark); return status; }
     if (dev_logits && last_logits.x && last_logits.count() == logit_count) BK(d2d)(dev_logits, last_logits.x, (size_t)logit_count * 4);
     if (slot < 0) BK(d2d)(dev_loss, loss.x, 4);
     BK(fill)(loss.d, 1.0f, 1);                       // gradR_loss: y.d.setAsOne(), TD.scala:1763-1780
     tape.backward();
     if (slot >= 0) BK(d2h_async)(feed_loss + slot, loss.x, 4);
     else BK(d2h_async)(loss_host, dev_loss, 4);
-    if (update) apply_update(lr);
+    if (update && !status) apply_update(lr);
     if (tracing()) dump_trace();
     { const size_t asked = zero_pool_end(); if (asked > zero_bytes) zero_bytes = asked; }   // the largest step so far: a smaller tree leaves part of the block unused
     BK(reset)(mark);
+    return status;
   }
   // Data parallelism: pushed on the tape at a point of the forward pass, this fires in the backward pass once every layer
   // after that point is done, i.e. when the gradients of the parameters declared from `first_decl` up to offset `hi` of the
@@ -219,26 +229,34 @@ struct Model {
   }
   void drop_graphs() { for (void*& rec : graph) if (rec) { BK(graph_destroy)(rec); rec = nullptr; } }
   int step_async(const float* xh, const int32_t* yh, float lr, bool update) {
-    if (!resident && xh) load(xh, yh);
+    status = 0; reason.clear();
+    return status = issue_step(xh, yh, lr, update);
+  }
+  int issue_step(const float* xh, const int32_t* yh, float lr, bool update) {
+    if (!resident && xh) {
+      if (const char* why = bad_labels(yh)) return refuse(LTB_E_ARG, why);
+      load(xh, yh);
+    }
     if (!feeding && draw_host_data(0)) return LTB_E_CUDA;
     if (use_graph && update && zero_bytes > 0) {        // the first step runs eagerly: it measures the gradient pool
       void*& rec = graph[1 + slot];
       if (rec && graph_lr[1 + slot] != lr) { BK(graph_destroy)(rec); rec = nullptr; }
       if (!rec) {
         int rc = BK(graph_begin)(); if (rc) return rc;
-        enqueue(lr, true);
+        rc = enqueue(lr, true);
         rec = BK(graph_end)(); graph_lr[1 + slot] = lr;
         if (!rec) return LTB_E_CUDA;
+        if (rc) { BK(graph_destroy)(rec); rec = nullptr; return rc; }
       }
       return BK(graph_launch)(rec);
     }
-    enqueue(lr, update);
-    return 0;
+    return enqueue(lr, update);
   }
+  // The loss of this batch, a NaN if the step failed (`status` tells one from the loss of a diverged network).
   float step(const float* xh, const int32_t* yh, float lr, bool update) {
     step_async(xh, yh, lr, update);
-    BK(sync)();
-    return *loss_host;
+    note(BK(sync)());
+    return status ? NAN : *loss_host;
   }
   // Training with two steps in flight.  The generated programs upload a batch, run the step and block on the loss copy
   // (resnet50FromOnnx.scala:173-186), so the device idles while the host prepares the next batch.  submit() copies the
@@ -270,7 +288,9 @@ struct Model {
   // xh == nullptr: the caller has filled the pair returned by feed_slot.
   int64_t submit(const float* xh, const int32_t* yh, float lr) {
     float* sx; int32_t* sy;
+    status = 0; reason.clear();
     if (feed_slot(&sx, &sy)) return -1;
+    if (const char* why = bad_labels(xh ? yh : sy)) { refuse(LTB_E_ARG, why); return -1; }
     const int p = (int)(submitted & 1);
     const size_t xb = (size_t)batch * in_c * in_h * in_w * 4;
     if (draw_host_data(p)) return -1;
@@ -555,11 +575,31 @@ struct TreeLstm : Model {
     int32_t* dev = (int32_t*)BK(malloc_uninit)(topo.size() * 4);
     BK(h2d)(dev, topo.data(), topo.size() * 4);
     tree.topo_host = topo.data(); tree.topo = dev;
-    BK(tree_fwd)(&tree);
-    t.push([this] { BK(tree_bwd)(&tree); });
+    note(BK(tree_fwd)(&tree));
+    t.push([this] { note(BK(tree_bwd)(&tree)); });
     TR loss; loss.rank = 1; loss.shape[0] = 1;
     loss.x = tree.values + (n - 1) * vstride + 8 * LTB_TREE_PITCH(Hd) + 32; loss.d = tree.grads + (n - 1) * gstride + 2 * LTB_TREE_PITCH(Hd);
     return loss;
+  }
+  // Every node, whether node 0 reaches it or not: links inside the arrays and round no circle, scores of the classifier, words of the table.
+  const char* bad_labels(const int32_t* host) override {
+    const int n = host[0];
+    if (n < 1 || n > MAXN) return nullptr;             // an empty step
+    const int32_t *scores = host + 1, *words = host + 1 + MAXN, *lch = host + 1 + 2 * MAXN, *rch = host + 1 + 3 * MAXN;
+    int parents[MAXN] = {}, top[MAXN], left = 0;
+    for (int i = 0; i < n; ++i) {
+      if (scores[i] < 0 || scores[i] >= O) return "a score outside the classes";
+      if (lch[i] < 0) { if (words[i] < 0 || words[i] >= VOCAB) return "a leaf's word outside the embedding table"; continue; }
+      if (lch[i] >= n || rch[i] < 0 || rch[i] >= n) return "a child outside the tree";
+      ++parents[lch[i]]; ++parents[rch[i]];
+    }
+    for (int i = 0; i < n; ++i) if (!parents[i]) top[left++] = i;
+    int done = 0;
+    while (left > 0) {                                 // parents before children: what never comes up goes round in a circle
+      const int i = top[--left]; ++done;
+      if (lch[i] >= 0) for (int k : {lch[i], rch[i]}) if (!--parents[k]) top[left++] = k;
+    }
+    return done == n ? nullptr : "a node that is its own descendant";
   }
   TR forward(Tape& t, const TR&, const int32_t* y) override {
     const int n = stage_y[0];
@@ -753,6 +793,8 @@ int HOST_FN(model_set_resident)(void* m, const float* x_host, const int32_t* y_h
   M->feed_mode(false);
   M->drop_graphs();
   if (!x_host) { M->resident = false; return 0; }
+  M->status = 0; M->reason.clear();
+  if (const char* why = M->bad_labels(y_host)) return M->refuse(LTB_E_ARG, why);
   M->load(x_host, y_host);
   BK(h2d)(M->dev_x, M->stage_x, (size_t)M->batch * M->in_c * M->in_h * M->in_w * 4);
   BK(h2d)(M->dev_y, M->stage_y, (size_t)M->label_count * 4);
@@ -760,7 +802,7 @@ int HOST_FN(model_set_resident)(void* m, const float* x_host, const int32_t* y_h
   M->resident = true;
   return 0;
 }
-// Blocking step: returns the loss of this batch. update=0 leaves the parameter gradients in place for inspection.
+// Blocking step: returns the loss of this batch (a NaN if the step failed: model_status). update=0 leaves the parameter gradients in place for inspection.
 float HOST_FN(model_step)(void* m, const float* x_host, const int32_t* y_host, float lr, int update) {
   Model* M = (Model*)m;
   if (M->feeding) M->feed_mode(false);
@@ -775,6 +817,12 @@ int HOST_FN(model_step_async)(void* m, const float* x_host, const int32_t* y_hos
 // Two steps in flight: submit returns the step's number (or -1) without waiting; collect(k) waits for step k and gives its
 // loss.  Only the last two submitted steps can be collected.
 int64_t HOST_FN(model_submit)(void* m, const float* x_host, const int32_t* y_host, float lr) { return ((Model*)m)->submit(x_host, y_host, lr); }
+// What became of the last step: 0, or a negative code with the reason in buf.  model_step, model_step_async and model_submit set it.
+int HOST_FN(model_status)(void* m, char* buf, int len) {
+  const Model* M = (Model*)m;
+  if (buf && len > 0) { strncpy(buf, M->reason.c_str(), len - 1); buf[len - 1] = 0; if (M->status && M->reason.empty()) BK(last_error)(buf, len); }
+  return M->status;
+}
 int HOST_FN(model_collect)(void* m, int64_t step, float* loss) { return ((Model*)m)->collect(step, loss); }
 float HOST_FN(model_last_loss)(void* m) { const Model* M = (Model*)m; return M->feeding && M->submitted ? M->feed_loss[(M->submitted - 1) & 1] : *M->loss_host; }
 // The classifier's output of the last step (batch x classes floats); returns the number of floats, 0 for programs without one.

@@ -319,3 +319,21 @@ def test_treelstm_gradients_and_adagrad_step(oracle_lib, cuda_lib, variant):
     mo.close(); mg.close()
     cuda_lib.set_math(1)
     oracle_lib.reset(mo_mark); cuda_lib.reset(mg_mark)
+
+
+def test_treelstm_labels_that_are_no_tree_raise(cuda_lib):
+    """What the kernels would refuse, or walk out of an array on, is an error of the step and no loss; the steps after it are as ever."""
+    from lantern_b200.hosts import HostPrograms
+    from tests.test_oracle_hosts import GOOD_TREE, _labels
+    mark = cuda_lib.mark()
+    m, x = HostPrograms(cuda_lib).model("treelstm", 1, seed=42), np.zeros(1, np.float32)
+    before = m.slab_params()
+    for node, field, value in ((0, 0, 5), (3, 1, 1000), (2, 2, 5), (2, 2, 0)):
+        bad = [list(v) for v in GOOD_TREE]
+        bad[node][field] = value
+        with pytest.raises(RuntimeError, match="outside|descendant"):
+            m.step(x, _labels(bad), 0.05)
+    assert np.array_equal(m.slab_params(), before)
+    loss = m.step(x, _labels(GOOD_TREE), 0.05)
+    assert abs(loss - 5 * np.log(5.0)) < 0.05 * 5 and not np.array_equal(m.slab_params(), before)
+    m.close(); cuda_lib.reset(mark)

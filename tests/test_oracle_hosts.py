@@ -89,6 +89,36 @@ def test_treelstm_node_call_equals_operator_by_operator(oracle_lib, variant):
                 assert np.abs(a - b).max() <= 1e-5 * max(np.abs(b).max(), 1e-12), (leaves, i)
 
 
+def _labels(nodes, maxn=99):
+    """Tree labels of the host program from (score, word, left, right) per node."""
+    y = np.zeros(1 + 4 * maxn, dtype=np.int32)
+    y[0] = len(nodes)
+    for f in range(4):
+        y[1 + f * maxn:1 + f * maxn + len(nodes)] = [node[f] for node in nodes]
+    return y
+
+
+GOOD_TREE = [(1, 0, 1, 2), (0, 7, -1, -1), (4, 0, 3, 4), (2, 999, -1, -1), (3, 5, -1, -1)]
+
+
+@pytest.mark.parametrize("node,field,value", [(0, 0, 5), (3, 0, -1), (3, 1, 1000), (1, 1, -1), (2, 2, 5), (2, 3, 5), (2, 3, -1), (2, 2, 0), (2, 3, 2)])
+def test_labels_that_are_no_tree_raise(oracle_lib, node, field, value):
+    """A score outside the classes, a word outside the table, a child outside the tree and a circle: every way to issue a step raises, no
+    parameter changes, and the program goes on working."""
+    mark = oracle_lib.mark()
+    m = _model(oracle_lib, "treelstm", 1)
+    x, bad = np.zeros(1, np.float32), [list(v) for v in GOOD_TREE]
+    bad[node][field] = value
+    before = m.slab_params()
+    for issue in (lambda: m.step(x, _labels(bad), 0.05), lambda: m.step_async(x, _labels(bad), 0.05), lambda: m.submit(x, _labels(bad), 0.05),
+                  lambda: m.set_resident(x, _labels(bad))):
+        with pytest.raises(RuntimeError, match="outside|descendant"):
+            issue()
+    assert np.array_equal(m.slab_params(), before)
+    assert np.isfinite(m.step(x, _labels(GOOD_TREE), 0.05)) and not np.array_equal(m.slab_params(), before)
+    m.close(); oracle_lib.reset(mark)
+
+
 def test_rnn_fused_cell_equals_operator_by_operator(oracle_lib):
     """The recurrent cell and the output layer as one fused call each (affine_act_rows) against the operator-by-operator form."""
     mark = oracle_lib.mark()
