@@ -287,8 +287,10 @@ int LTB_FN(tree_nodes_bwd)(const ltb_tree_node* nodes_host, const ltb_tree_node*
  * [levels + 1].  values: LTB_TREE_VALUES(hidden) floats per node, 16-byte aligned -- with p = LTB_TREE_PITCH(hidden): gates at 0, c at 5 p, tanh(c) at 6 p, h at 7 p, log
  * probabilities at 8 p, accumulated loss at 8 p + 32.  grads: LTB_TREE_GRADS(hidden) floats per node -- dc at 0, dh at p, dloss at 2 p; the caller
  * sets the root's dloss, the rest is zero before tree_bwd.  Results are those of tree_node_fwd / tree_node_bwd node by node with the
- * children's second state (classify_cell ? h : c) feeding the cell and their first (classify_cell ? c : h) the gates.  Limits (LTB_E_LIMIT beyond: the calls per level and
- * per node remain): hidden 160, in_len 320, 119 nodes. */
+ * children's second state (classify_cell ? h : c) feeding the cell and their first (classify_cell ? c : h) the gates.  Refused with LTB_E_ARG, before anything
+ * is launched: levels that do not cover the nodes, a child that is not in a level below, a node with two parents, a score outside the classes (a
+ * node with two parents can go through the calls per node).  The loss is the last node's: a node that is no one's child has no part in it.  Limits (LTB_E_LIMIT
+ * beyond: the calls per level and per node remain): hidden 160, in_len 320, 119 nodes. */
 #define LTB_TREE_PITCH(hidden) (((hidden) + 63) / 64 * 64)
 #define LTB_TREE_VALUES(hidden) (8 * LTB_TREE_PITCH(hidden) + 64)
 #define LTB_TREE_GRADS(hidden) (2 * LTB_TREE_PITCH(hidden) + 64)

@@ -480,7 +480,13 @@ struct TreeLstm : Model {
     TR pred = fused_cells ? t.affine_act(-1, P(Why), in, nullptr, nullptr, P(by)) : t.plus_bias(t.dot(P(Why), in), P(by));
     return t.nll(t.log_softmax(view(pred, {1, O})), score);
   }
-  State visit(Tape& t, const int32_t* host, const int32_t* dev, int i) {
+  std::vector<State> known;                  // of the nodes visited so far, for one that is the child of two
+  std::vector<char> visited;
+  const State& visit(Tape& t, const int32_t* host, const int32_t* dev, int i) {
+    if (!visited[i]) { State s = node(t, host, dev, i); known[i] = s; visited[i] = 1; }
+    return known[i];
+  }
+  State node(Tape& t, const int32_t* host, const int32_t* dev, int i) {
     const int32_t *scores = dev + 1, *words = host + 1 + MAXN, *lch = host + 1 + 2 * MAXN, *rch = host + 1 + 3 * MAXN;
     State s;
     if (fused_cells && whole_sequence) {               // the whole node in one call forward and one backward (ltb_tree_node_fwd / _bwd)
@@ -537,7 +543,16 @@ struct TreeLstm : Model {
     s.first = cell; s.second = hidden;
     return s;
   }
-  // The whole tree in one call each way (ltb_tree_fwd / _bwd): the nodes sorted by height, their links uploaded once.
+  // Whether node 0 is the root of a tree of all n nodes, as the whole-tree call takes them.  The labels may also say less (nodes that node 0 does not
+  // reach, which have no part in the loss) or more (a node under two parents, whose loss counts twice): such a step goes node by node from node 0.
+  static bool is_one_tree(const int32_t* host, int n) {
+    const int32_t *lch = host + 1 + 2 * MAXN, *rch = host + 1 + 3 * MAXN;
+    int parents[MAXN] = {};
+    for (int i = 0; i < n; ++i) if (lch[i] >= 0) { ++parents[lch[i]]; ++parents[rch[i]]; }
+    for (int i = 1; i < n; ++i) if (parents[i] != 1) return false;
+    return parents[0] == 0;
+  }
+  // The whole tree in one call each way (ltb_tree_fwd / _bwd): the nodes sorted by height (node 0 is the last), their links uploaded once.
   ltb_tree tree = {};
   std::vector<int32_t> topo;                       // kept until the backward call has been issued
   TR forward_tree(Tape& t, const int32_t* host, int n) {
@@ -604,7 +619,8 @@ struct TreeLstm : Model {
   TR forward(Tape& t, const TR&, const int32_t* y) override {
     const int n = stage_y[0];
     if (n < 1 || n > MAXN) { TR z = make({1}); BK(fill)(z.x, 0.0f, 1); return z; }
-    if (fused_cells && whole_sequence && whole_tree) return forward_tree(t, stage_y, n);
+    if (fused_cells && whole_sequence && whole_tree && is_one_tree(stage_y, n)) return forward_tree(t, stage_y, n);
+    known.assign((size_t)n, State()); visited.assign((size_t)n, 0);
     return visit(t, stage_y, y, 0).loss;
   }
   void apply_update(float lr) override { BK(adagrad_update)(slab_x, slab_d, slab_h, lr, pldi19 ? 1.0f : 3.0e38f, 1, slab_count); }

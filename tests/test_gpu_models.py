@@ -337,3 +337,23 @@ def test_treelstm_labels_that_are_no_tree_raise(cuda_lib):
     loss = m.step(x, _labels(GOOD_TREE), 0.05)
     assert abs(loss - 5 * np.log(5.0)) < 0.05 * 5 and not np.array_equal(m.slab_params(), before)
     m.close(); cuda_lib.reset(mark)
+
+
+@pytest.mark.parametrize("variant", ["treelstm", "treelstm_nips18"])
+def test_treelstm_labels_that_are_more_or_less_than_a_tree(oracle_lib, cuda_lib, variant):
+    """Parts that node 0 does not reach and nodes under two parents, against the oracle's walk from node 0."""
+    from tests.test_oracle_hosts import ODD_TREES, _labels
+    mo_mark, mg_mark = oracle_lib.mark(), cuda_lib.mark()
+    cuda_lib.set_math(0); oracle_lib.set_math(0)
+    mo, mg = _pair(oracle_lib, cuda_lib, variant, 1)
+    mo.use_fused_cells(0)
+    x = np.zeros(1, np.float32)
+    for nodes in ODD_TREES:
+        lo, lg = mo.step(x, _labels(nodes), 0.0, update=False), mg.step(x, _labels(nodes), 0.0, update=False)
+        assert abs(lo - lg) <= FP32_RTOL * max(1.0, abs(lo)), (nodes, lo, lg)
+        for i in range(mo.num_params):
+            assert_close(mo.grad(i), mg.grad(i), FP32_RTOL, "treelstm grad %d" % i)
+        mo.step(x, _labels(nodes), 0.0); mg.step(x, _labels(nodes), 0.0)              # lr 0: only clears the gradients
+    mo.close(); mg.close()
+    cuda_lib.set_math(1)
+    oracle_lib.reset(mo_mark); cuda_lib.reset(mg_mark)

@@ -119,6 +119,38 @@ def test_labels_that_are_no_tree_raise(oracle_lib, node, field, value):
     m.close(); oracle_lib.reset(mark)
 
 
+# A part that node 0 does not reach and that is higher than its tree, a node 0 that is the child of another, a leaf and an inner node under
+# two parents, one under the same parent twice.
+ODD_TREES = [[(1, 0, 1, 2), (0, 7, -1, -1), (4, 3, -1, -1), (2, 0, 4, 5), (3, 5, -1, -1), (1, 0, 6, 7), (0, 9, -1, -1), (2, 11, -1, -1)],
+             [(1, 8, -1, -1), (0, 0, 0, 2), (4, 3, -1, -1)],
+             [(1, 0, 1, 2), (0, 0, 3, 4), (4, 0, 3, 5), (2, 6, -1, -1), (3, 5, -1, -1), (1, 2, -1, -1)],
+             [(1, 0, 1, 2), (0, 0, 2, 3), (4, 0, 4, 5), (2, 6, -1, -1), (3, 5, -1, -1), (1, 2, -1, -1)],
+             [(1, 0, 1, 1), (0, 0, 2, 3), (4, 1, -1, -1), (2, 6, -1, -1)]]
+
+
+@pytest.mark.parametrize("variant", ["treelstm", "treelstm_nips18"])
+@pytest.mark.parametrize("nodes", ODD_TREES, ids=["unreached", "child", "leaf shared", "node shared", "twins"])
+def test_labels_that_are_more_or_less_than_a_tree(oracle_lib, variant, nodes):
+    """The reference walks the arrays from node 0: a part it does not reach counts nothing, a node under two parents counts under both.
+    The loss is that walk's (recomputed here from per-node losses of an untrained classifier) and every form of the program gives it."""
+    mark = oracle_lib.mark()
+
+    def count(i):
+        return 1 + (0 if nodes[i][2] < 0 else count(nodes[i][2]) + count(nodes[i][3]))
+    res = []
+    for level in (3, 2, 1, 0):
+        m = _model(oracle_lib, variant, 1)
+        m.use_fused_cells(level)
+        loss = m.step(np.zeros(1, np.float32), _labels(nodes), 0.0, update=False)
+        res.append((loss, [m.grad(i) for i in range(m.num_params)]))
+        m.close(); oracle_lib.reset(mark)
+    assert abs(res[3][0] - count(0) * np.log(5.0)) < 0.01 * count(0)
+    for r in res[:3]:
+        assert abs(r[0] - res[3][0]) <= 1e-6 * abs(res[3][0])
+        for i, (a, b) in enumerate(zip(r[1], res[3][1])):
+            assert np.abs(a - b).max() <= 1e-5 * max(np.abs(b).max(), 1e-12), i
+
+
 def test_rnn_fused_cell_equals_operator_by_operator(oracle_lib):
     """The recurrent cell and the output layer as one fused call each (affine_act_rows) against the operator-by-operator form."""
     mark = oracle_lib.mark()
