@@ -617,11 +617,12 @@ struct TreeLstm : Model {
     return done == n ? nullptr : "a node that is its own descendant";
   }
   TR forward(Tape& t, const TR&, const int32_t* y) override {
-    const int n = stage_y[0];
+    const int32_t* const host = slot >= 0 ? feed_y[slot] : stage_y;      // y as the host has it
+    const int n = host[0];
     if (n < 1 || n > MAXN) { TR z = make({1}); BK(fill)(z.x, 0.0f, 1); return z; }
-    if (fused_cells && whole_sequence && whole_tree && is_one_tree(stage_y, n)) return forward_tree(t, stage_y, n);
+    if (fused_cells && whole_sequence && whole_tree && is_one_tree(host, n)) return forward_tree(t, host, n);
     known.assign((size_t)n, State()); visited.assign((size_t)n, 0);
-    return visit(t, stage_y, y, 0).loss;
+    return visit(t, host, y, 0).loss;
   }
   void apply_update(float lr) override { BK(adagrad_update)(slab_x, slab_d, slab_h, lr, pldi19 ? 1.0f : 3.0e38f, 1, slab_count); }
   // Replaces the embedding table (rows x 300 floats, rows <= VOCAB) by the caller's.

@@ -119,6 +119,21 @@ def test_labels_that_are_no_tree_raise(oracle_lib, node, field, value):
     m.close(); oracle_lib.reset(mark)
 
 
+def test_submitted_trees_are_the_trees_of_their_steps(oracle_lib):
+    """submit() puts the labels into a staging pair; the program builds the step from that pair, not from what a blocking step left behind."""
+    from tests.test_gpu_models import _random_tree
+    mark = oracle_lib.mark()
+    rng, x = np.random.default_rng(8), np.zeros(1, np.float32)
+    trees = [_random_tree(rng, leaves) for leaves in (3, 9, 2, 6)]
+    runs = []
+    for submit in (False, True):
+        m = _model(oracle_lib, "treelstm", 1)
+        m.step(x, trees[0], 0.05)
+        runs.append([m.collect(m.submit(x, y, 0.05)) if submit else m.step(x, y, 0.05) for y in trees])
+        m.close(); oracle_lib.reset(mark)
+    assert runs[0] == runs[1]
+
+
 # A part that node 0 does not reach and that is higher than its tree, a node 0 that is the child of another, a leaf and an inner node under
 # two parents, one under the same parent twice.
 ODD_TREES = [[(1, 0, 1, 2), (0, 7, -1, -1), (4, 3, -1, -1), (2, 0, 4, 5), (3, 5, -1, -1), (1, 0, 6, 7), (0, 9, -1, -1), (2, 11, -1, -1)],
