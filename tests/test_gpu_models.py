@@ -357,3 +357,24 @@ def test_treelstm_labels_that_are_more_or_less_than_a_tree(oracle_lib, cuda_lib,
     mo.close(); mg.close()
     cuda_lib.set_math(1)
     oracle_lib.reset(mo_mark); cuda_lib.reset(mg_mark)
+
+
+def test_treelstm_submitted_trees_are_the_trees_of_their_steps(cuda_lib):
+    """Two trees in flight give the losses of blocking steps (shared bias gradients are added up in the order of arrival: FP32 rounding)."""
+    from lantern_b200.hosts import HostPrograms
+    rng, x, mark = np.random.default_rng(8), np.zeros(1, np.float32), cuda_lib.mark()
+    trees = [_random_tree(rng, leaves) for leaves in (3, 50, 2, 25, 6)]
+    runs = []
+    for submit in (False, True):
+        m = HostPrograms(cuda_lib).model("treelstm", 1, seed=42)
+        losses = []
+        for k, y in enumerate(trees):
+            if not submit:
+                losses.append(m.step(x, y, 0.01))
+                continue
+            m.submit(x, y, 0.01)
+            if k:
+                losses.append(m.collect(k - 1))
+        runs.append(losses + ([m.collect(len(trees) - 1)] if submit else []))
+        m.close(); cuda_lib.reset(mark)
+    np.testing.assert_allclose(runs[1], runs[0], rtol=1e-4)
