@@ -448,7 +448,7 @@ int ltb_nll(const float* x, const int32_t* t, float* out, int rows, int cols) {
   LTB_INITED_NOFLUSH(); LTB_REQUIRE(x && t && out && rows > 0 && cols > 0, "ltb_nll: bad argument"); LTB_WRITES(out, rows);
   const int64_t n = (int64_t)rows * cols;
   if (g.pending.kind == PEND_LSM && g.pending.y == x && g.pending.N == rows && g.pending.C == cols && apart(out, rows, x, n) && apart(out, rows, g.pending.x, n) &&
-      apart(out, rows, t, rows) && apart(t, rows, x, n)) {
+      apart(out, rows, t, rows) && apart(t, rows, x, n) && apart(g.pending.x, n, x, n)) {
     g.pending.kind = PEND_NLL; g.pending.target = t; g.pending.out = out;                           // their sum or mean may join it
     return LTB_OK;
   }

@@ -590,6 +590,28 @@ def test_loss_head_in_one_kernel_each_way(gpu, rows, cols, mean):
         assert stop < 7 or few == (2 if rows <= 65536 else 4), (many, few)
 
 
+@pytest.mark.parametrize("rows,cols", [(9, 10), (300, 200), (77, 1000), (40, 1500)])
+def test_loss_head_over_its_own_logits(gpu, rows, cols):
+    """A log-softmax in place: the likelihood is that of the values before, with look-ahead fusion as without, and the calls are not joined (the
+    joined kernel reads a row's target after it may have written the row)."""
+    import torch
+    lib = gpu.lib
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, cols, device="cuda", generator=gen) * 3
+    t = torch.randint(-1, cols + 1, (rows,), device="cuda", generator=gen, dtype=torch.int32)
+    got = []
+    for fusion in (0, 1):
+        y, nll, loss = x.clone(), torch.zeros(rows, device="cuda"), torch.zeros(1, device="cuda")
+        torch.cuda.synchronize()
+        lib.set_fusion(fusion)
+        before = lib.kernel_launches()
+        lib.log_softmax(y.data_ptr(), y.data_ptr(), rows, cols); lib.nll(y.data_ptr(), t.data_ptr(), nll.data_ptr(), rows, cols); lib.mean(nll.data_ptr(), loss.data_ptr(), rows)
+        lib.sync()
+        got.append((y, nll, loss, lib.kernel_launches() - before))
+        lib.set_fusion(0)
+    assert all(torch.equal(u, v) for u, v in zip(got[0][:3], got[1][:3])) and got[1][3] == 3
+
+
 @pytest.mark.parametrize("det", [0, 1])
 @pytest.mark.parametrize("M,N,K,ta,tb", [(4740, 1000, 516, 0, 1), (512, 508, 20000, 1, 0), (4096, 1196, 996, 0, 1), (2564, 1476, 1028, 0, 1), (1284, 508, 7172, 1, 0)])
 def test_gemm_in_wide_tiles_tf32(ora, gpu, M, N, K, ta, tb, det):
