@@ -13,6 +13,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <string>
 #include <vector>
 
 #include "../lantern_b200/csrc/tc_plan.h"
@@ -173,7 +175,12 @@ static bool run_plan(const TcPlan& p, size_t out_count) {
   for (const TcOperand* o : {&p.a, &p.b}) if (o->load == TC_LOAD_IM2COL_MN && !pixel_walk_matches(*o, p.k_iters)) return false;
   // overwrite semantics under split-K: the partial results of the splits are summed and then stored; emulated by zeroing first
   if (p.splits > 1 && !p.accumulate) for (size_t i = 0; i < out_count; ++i) p.out[i] = 0.0f;
-  std::vector<float> sa, sb, sc;
+  std::vector<float> sa, sb, sc, fa(128 * 8), fb((size_t)p.bn * 8);
+  // a pair's second CTA loads what stands where a row tile beyond the last one would be; nothing of it is stored
+  if (p.pair && p.m_tiles % 2) {
+    if (p.a.load != TC_LOAD_BOX && p.a.load != TC_LOAD_BOXES) { printf("a pair whose second row tile has no place to be read from\n"); return false; }
+    for (int it = 0; it < p.k_iters; it += 7) if (!tma_load(p.a, p.m_tiles, it, sa)) return false;
+  }
   for (int mt = 0; mt < p.m_tiles; ++mt) for (int nt = 0; nt < p.n_tiles; ++nt) for (int z = 0; z < p.splits; ++z) {
     int per = (p.k_iters + p.splits - 1) / p.splits, k0 = z * per, k1 = k0 + per < p.k_iters ? k0 + per : p.k_iters;
     if (k0 >= k1) continue;
@@ -181,9 +188,13 @@ static bool run_plan(const TcPlan& p, size_t out_count) {
     for (int it = k0; it < k1; ++it) {
       if (!(p.gather_src ? gather_load(p, mt, it, sa) : tma_load(p.a, mt, it, sa)) || !tma_load(p.b, p.pair ? 2 * nt : nt, it, sb)) return false;
       if (p.pair && !tma_load(p.b, 2 * nt + 1, it, sc)) return false;             // the other CTA's half of the columns
-      for (int ks = 0; ks < p.a.nk; ++ks) for (int r = 0; r < 128; ++r) for (int c = 0; c < p.bn; ++c) {
-        double s = 0; for (int kk = 0; kk < 8; ++kk) s += (double)umma_fetch(p.a, sa, ks, r, kk) * (p.pair && c >= 128 ? umma_fetch(p.b, sc, ks, c - 128, kk) : umma_fetch(p.b, sb, ks, c, kk));
-        D[(size_t)r * p.bn + c] += s;
+      for (int ks = 0; ks < p.a.nk; ++ks) {
+        for (int r = 0; r < 128; ++r) for (int kk = 0; kk < 8; ++kk) fa[r * 8 + kk] = umma_fetch(p.a, sa, ks, r, kk);
+        for (int c = 0; c < p.bn; ++c) for (int kk = 0; kk < 8; ++kk) fb[c * 8 + kk] = p.pair && c >= 128 ? umma_fetch(p.b, sc, ks, c - 128, kk) : umma_fetch(p.b, sb, ks, c, kk);
+        for (int r = 0; r < 128; ++r) for (int c = 0; c < p.bn; ++c) {
+          double s = 0; for (int kk = 0; kk < 8; ++kk) s += (double)fa[r * 8 + kk] * fb[c * 8 + kk];
+          D[(size_t)r * p.bn + c] += s;
+        }
       }
     }
     bool atomic = p.splits > 1;
@@ -237,7 +248,13 @@ static bool close(const std::vector<float>& a, const std::vector<float>& b, cons
   return true;
 }
 
-static int conv_case(int n_img, int ck, int co, int pix) {
+static std::map<std::string, int> pairs, split_pairs, odd_pairs;      // by planner: plans for pairs of CTAs emulated, those with splits, those of an odd number of row tiles
+static bool holds(const TcPlan& p, const std::vector<float>& want, const std::vector<float>& got, const char* what) {
+  if (p.pair) { ++pairs[what]; split_pairs[what] += p.splits > 1; odd_pairs[what] += p.m_tiles % 2; }
+  return run_plan(p, got.size()) && close(want, got, what);
+}
+
+static int conv_case(int n_img, int ck, int co, int pix, int sms = 148) {
   auto x = rnd((size_t)n_img * ck * pix, 1), w = rnd((size_t)co * ck, 2), dy = rnd((size_t)n_img * co * pix, 3), bias = rnd(co, 4);
   // TMA bases must be 16-byte aligned: std::vector<float> storage from operator new is.
   std::vector<float> y((size_t)n_img * co * pix, 7.0f), yr(y.size()), dx((size_t)n_img * ck * pix, 0.5f), dxr(dx), dw((size_t)co * ck, -1.0f), dwr(dw);
@@ -267,23 +284,23 @@ static int conv_case(int n_img, int ck, int co, int pix) {
   auto padded = [&](int ld) { std::vector<float> o((size_t)co * ld, 0.0f); for (int c = 0; c < co; ++c) for (int k = 0; k < ck; ++k) o[(size_t)c * ld + k] = w[(size_t)c * ck + k]; return o; };
   const int ld4 = (ck + 3) / 4 * 4;
   const std::vector<float> w4 = padded(ld4);
-  if (tc_plan_conv_fwd(p, rows ? xt.data() : x.data(), rows, w4.data(), ld4, bias.data(), y.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "fwd")) return -1; }
-  if (tc_plan_conv_dgrad(p, rows ? dyt.data() : dy.data(), rows, w4.data(), ld4, dx.data(), n_img, ck, co, pix, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "dgrad")) return -1; }
+  if (tc_plan_conv_fwd(p, rows ? xt.data() : x.data(), rows, w4.data(), ld4, bias.data(), y.data(), n_img, ck, co, pix, sms)) { ++taken; if (!holds(p, yr, y, "fwd")) return -1; }
+  if (tc_plan_conv_dgrad(p, rows ? dyt.data() : dy.data(), rows, w4.data(), ld4, dx.data(), n_img, ck, co, pix, true, sms)) { ++taken; if (!holds(p, dxr, dx, "dgrad")) return -1; }
   // the same two contractions with the kernel gathering the activation itself (small images: 4 or 16 pixels)
   if (rows && tc_gather_possible(x.data(), ck, pix) && tc_gather_possible(dy.data(), co, pix)) {
     std::fill(y.begin(), y.end(), 7.0f); std::fill(dx.begin(), dx.end(), 0.5f);
-    if (tc_plan_conv_fwd(p, x.data(), true, w4.data(), ld4, bias.data(), y.data(), n_img, ck, co, pix, 148)) {
-      tc_plan_gather(p, x.data(), n_img, ck, pix); ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "fwd (gather)")) return -1; }
-    if (tc_plan_conv_dgrad(p, dy.data(), true, w4.data(), ld4, dx.data(), n_img, ck, co, pix, true, 148)) {
-      tc_plan_gather(p, dy.data(), n_img, co, pix); ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "dgrad (gather)")) return -1; }
+    if (tc_plan_conv_fwd(p, x.data(), true, w4.data(), ld4, bias.data(), y.data(), n_img, ck, co, pix, sms)) {
+      tc_plan_gather(p, x.data(), n_img, ck, pix); ++taken; if (!holds(p, yr, y, "fwd (gather)")) return -1; }
+    if (tc_plan_conv_dgrad(p, dy.data(), true, w4.data(), ld4, dx.data(), n_img, ck, co, pix, true, sms)) {
+      tc_plan_gather(p, dy.data(), n_img, co, pix); ++taken; if (!holds(p, dxr, dx, "dgrad (gather)")) return -1; }
   }
-  if (tc_plan_conv_wgrad(p, x.data(), dy.data(), dw.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "wgrad")) return -1; }
+  if (tc_plan_conv_wgrad(p, x.data(), dy.data(), dw.data(), n_img, ck, co, pix, sms)) { ++taken; if (!holds(p, dwr, dw, "wgrad")) return -1; }
   printf("conv n=%d ck=%d co=%d pix=%d: %d of 3 plans (5 with the gathered ones) taken, all match\n", n_img, ck, co, pix, taken);
   return taken;
 }
 
 // Images of a size that fills no tiles, straight from x[n][k][p].
-static int ragged_case(int n_img, int ck, int co, int pix) {
+static int ragged_case(int n_img, int ck, int co, int pix, int sms = 148) {
   auto x = rnd((size_t)n_img * ck * pix, 1), w = rnd((size_t)co * ck, 2), dy = rnd((size_t)n_img * co * pix, 3), bias = rnd(co, 4);
   std::vector<float> y(dy.size(), 7.0f), yr(y.size()), dx(x.size(), 0.5f), dxr(dx), dw(w.size(), -1.0f), dwr(dw);
   for (int n = 0; n < n_img; ++n) for (int q = 0; q < pix; ++q) {
@@ -303,16 +320,16 @@ static int ragged_case(int n_img, int ck, int co, int pix) {
   const int ld = (ck + 3) / 4 * 4; std::vector<float> wp((size_t)co * ld, 0.0f);
   for (int c = 0; c < co; ++c) for (int k = 0; k < ck; ++k) wp[(size_t)c * ld + k] = w[(size_t)c * ck + k];
   int taken = 0; TcPlan p;
-  if (tc_plan_conv_ragged_fwd(p, x.data(), wp.data(), ld, bias.data(), y.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "ragged fwd")) return -1; }
-  if (tc_plan_conv_ragged_dgrad(p, dy.data(), wp.data(), ld, dx.data(), n_img, ck, co, pix, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "ragged dgrad")) return -1; }
-  if (tc_plan_conv_ragged_wgrad(p, x.data(), dy.data(), dw.data(), n_img, ck, co, pix, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "ragged wgrad")) return -1; }
+  if (tc_plan_conv_ragged_fwd(p, x.data(), wp.data(), ld, bias.data(), y.data(), n_img, ck, co, pix, sms)) { ++taken; if (!holds(p, yr, y, "ragged fwd")) return -1; }
+  if (tc_plan_conv_ragged_dgrad(p, dy.data(), wp.data(), ld, dx.data(), n_img, ck, co, pix, true, sms)) { ++taken; if (!holds(p, dxr, dx, "ragged dgrad")) return -1; }
+  if (tc_plan_conv_ragged_wgrad(p, x.data(), dy.data(), dw.data(), n_img, ck, co, pix, sms)) { ++taken; if (!holds(p, dwr, dw, "ragged wgrad")) return -1; }
   printf("ragged conv n=%d ck=%d co=%d pix=%d: %d of 3 plans taken, all match\n", n_img, ck, co, pix, taken);
   return taken;
 }
 
 // R x S convolution against a direct evaluation: through the tap-loop plans (stride 1), and through the im2col-mode plans from
 // channels-last copies whose channels are padded to a multiple of 4.
-static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph, int pw, int sh = 1, int sw = 1) {
+static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph, int pw, int sh = 1, int sw = 1, int sms = 148) {
   const int oH = (H + 2 * ph - R) / sh + 1, oW = (W + 2 * pw - S) / sw + 1, taps = R * S;
   TcConvGeom g{n_img, C, H, W, K, R, S, ph, pw, oH, oW};
   auto x = rnd((size_t)n_img * C * H * W, 11), w = rnd((size_t)K * C * taps, 12), dy = rnd((size_t)n_img * K * oH * oW, 13), bias = rnd(K, 14);
@@ -340,9 +357,9 @@ static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph
   }
   int taken = 0; TcPlan p;
   if (sh == 1 && sw == 1) {
-    if (tc_plan_conv_taps_fwd(p, xr.data(), wt.data(), bias.data(), y.data(), g, 148)) { ++taken; if (!run_plan(p, y.size()) || !close(yr, y, "taps fwd")) return -1; }
-    if (tc_plan_conv_taps_dgrad(p, dyr.data(), wt.data(), dx.data(), g, true, 148)) { ++taken; if (!run_plan(p, dx.size()) || !close(dxr, dx, "taps dgrad")) return -1; }
-    if (tc_plan_conv_taps_wgrad(p, dyr.data(), xr.data(), dw.data(), g, 148)) { ++taken; if (!run_plan(p, dw.size()) || !close(dwr, dw, "taps wgrad")) return -1; }
+    if (tc_plan_conv_taps_fwd(p, xr.data(), wt.data(), bias.data(), y.data(), g, sms)) { ++taken; if (!holds(p, yr, y, "taps fwd")) return -1; }
+    if (tc_plan_conv_taps_dgrad(p, dyr.data(), wt.data(), dx.data(), g, true, sms)) { ++taken; if (!holds(p, dxr, dx, "taps dgrad")) return -1; }
+    if (tc_plan_conv_taps_wgrad(p, dyr.data(), xr.data(), dw.data(), g, sms)) { ++taken; if (!holds(p, dwr, dw, "taps wgrad")) return -1; }
   }
   // im2col mode; the data gradient of a strided convolution is a stride-1 one of dy with zeros between its pixels
   const int ldc = (C + 3) / 4 * 4, ldk = (K + 3) / 4 * 4, uH = H + 2 * ph - R + 1, uW = W + 2 * pw - S + 1;
@@ -358,9 +375,9 @@ static int taps_case(int n_img, int C, int K, int H, int W, int R, int S, int ph
   std::fill(y.begin(), y.end(), 7.0f); std::fill(dx.begin(), dx.end(), 0.5f); std::fill(dw.begin(), dw.end(), -1.0f);
   TcConvAny a{n_img, C, H, W, K, R, S, sh, sw, ph, pw, oH, oW, ldc, ldk}, u{n_img, C, H, W, K, R, S, 1, 1, ph, pw, uH, uW, ldc, ldk};
   int any = 0;
-  if (tc_plan_conv_any_fwd(p, xp.data(), wtp.data(), bias.data(), y.data(), a, 148)) { ++any; if (!run_plan(p, y.size()) || !close(yr, y, "im2col fwd")) return -1; }
-  if (tc_plan_conv_any_dgrad(p, up.data(), C % 32 == 0 ? wtp.data() : wdp.data(), dx.data(), u, true, 148)) { ++any; if (!run_plan(p, dx.size()) || !close(dxr, dx, "im2col dgrad")) return -1; }
-  if (tc_plan_conv_any_wgrad(p, dyp.data(), xp.data(), dw.data(), a, 148)) { ++any; if (!run_plan(p, dw.size()) || !close(dwr, dw, "im2col wgrad")) return -1; }
+  if (tc_plan_conv_any_fwd(p, xp.data(), wtp.data(), bias.data(), y.data(), a, sms)) { ++any; if (!holds(p, yr, y, "im2col fwd")) return -1; }
+  if (tc_plan_conv_any_dgrad(p, up.data(), C % 32 == 0 ? wtp.data() : wdp.data(), dx.data(), u, true, sms)) { ++any; if (!holds(p, dxr, dx, "im2col dgrad")) return -1; }
+  if (tc_plan_conv_any_wgrad(p, dyp.data(), xp.data(), dw.data(), a, sms)) { ++any; if (!holds(p, dwr, dw, "im2col wgrad")) return -1; }
   if (any != 3) { printf("only %d of 3 im2col plans taken\n", any); return -1; }
   printf("taps conv n=%d C=%d K=%d %dx%d k%dx%d pad %d,%d stride %d,%d: %d of 3 window plans and 3 im2col plans taken, all match\n", n_img, C, K, H, W, R, S, ph, pw, sh, sw, taken);
   return taken;
@@ -377,20 +394,42 @@ static int gemm_case(int M, int N, int K, bool ak, bool bk, bool acc, int sms = 
   const int wa = ak ? K : M, ha = ak ? M : K, wb = bk ? K : N, hb = bk ? N : K;
   if (wa % 4 == 0 && wb % 4 == 0) {
     if (!tc_plan_gemm(p, a.data(), ak, b.data(), bk, c.data(), M, N, K, 0.5f, acc, sms)) { printf("gemm %dx%dx%d ak=%d bk=%d: not eligible\n", M, N, K, ak, bk); return 0; }
-    if (!run_plan(p, c.size()) || !close(cr, c, "gemm")) return -1;
+    if (!holds(p, cr, c, "gemm")) return -1;
   } else {                     // rows of no whole 16-byte unit: copies padded with zeros, as the library makes them
     const int lda = (wa + 3) / 4 * 4, ldb = (wb + 3) / 4 * 4;
     std::vector<float> ap((size_t)ha * lda, 0.0f), bp((size_t)hb * ldb, 0.0f);
     for (int i = 0; i < ha; ++i) for (int j = 0; j < wa; ++j) ap[(size_t)i * lda + j] = a[(size_t)i * wa + j];
     for (int i = 0; i < hb; ++i) for (int j = 0; j < wb; ++j) bp[(size_t)i * ldb + j] = b[(size_t)i * wb + j];
     if (!tc_plan_gemm_ld(p, ap.data(), ak, lda, bp.data(), bk, ldb, c.data(), M, N, K, 0.5f, acc, sms)) { printf("gemm %dx%dx%d ak=%d bk=%d: padded copies not eligible\n", M, N, K, ak, bk); return -1; }
-    if (!run_plan(p, c.size()) || !close(cr, c, "padded gemm")) return -1;
+    if (!holds(p, cr, c, "padded gemm")) return -1;
   }
   printf("gemm %dx%dx%d ak=%d bk=%d acc=%d: bn=%d splits=%d match\n", M, N, K, ak, bk, acc, p.bn, p.splits);
   return 1;
 }
 
-int main() {
+// "forward splits, data-gradient splits" of a layer on 148 SMs, 0 where its plan is not for pairs of CTAs, in the order in which the library asks the planners.
+static int print_pairs(char** v) {
+  int n[8]; for (int i = 0; i < 8; ++i) n[i] = atoi(v[i]);
+  const int N = n[0], C = n[1], H = n[2], W = n[3], K = n[4], R = n[5], st = n[6], pad = n[7], oH = (H + 2 * pad - R) / st + 1, oW = (W + 2 * pad - R) / st + 1;
+  alignas(16) static float some[4];
+  TcPlan f{}, d{};
+  bool ok = true;
+  if (R == 1 && st == 1 && tc_conv_needs_rows(H * W)) {
+    ok = tc_plan_conv_ragged_fwd(f, some, some, (C + 3) / 4 * 4, nullptr, some, N, C, K, H * W, 148) && tc_plan_conv_ragged_dgrad(d, some, some, (C + 3) / 4 * 4, some, N, C, K, H * W, true, 148);
+  } else if (R == 1 && st == 1) {
+    ok = tc_plan_conv_fwd(f, some, false, some, (C + 3) / 4 * 4, nullptr, some, N, C, K, H * W, 148) && tc_plan_conv_dgrad(d, some, false, some, (C + 3) / 4 * 4, some, N, C, K, H * W, true, 148);
+  } else {
+    const TcConvGeom g{N, C, H, W, K, R, R, pad, pad, oH, oW};
+    const TcConvAny a{N, C, H, W, K, R, R, st, st, pad, pad, oH, oW, (C + 3) / 4 * 4, (K + 3) / 4 * 4};
+    ok = ((st == 1 && tc_plan_conv_taps_fwd(f, some, some, nullptr, some, g, 148)) || tc_plan_conv_any_fwd(f, some, some, nullptr, some, a, 148)) &&
+         ((st == 1 && tc_plan_conv_taps_dgrad(d, some, some, some, g, true, 148)) || tc_plan_conv_any_dgrad(d, some, some, some, a, true, 148));
+  }
+  printf("%d %d\n", f.pair ? f.splits : 0, d.pair ? d.splits : 0);
+  return ok ? 0 : 1;
+}
+
+int main(int argc, char** argv) {
+  if (argc == 9) return print_pairs(argv + 1);
   int bad = slices_cover() ? 0 : 1, taken = 0;
   const int convs[][4] = {{2, 64, 64, 256}, {3, 64, 256, 256}, {4, 128, 96, 64}, {5, 256, 128, 64}, {11, 256, 128, 16}, {35, 512, 64, 4}, {1, 32, 48, 1024},
                           {8, 576, 64, 256}, {2, 40, 64, 32}, {3, 64, 64, 36}, {2, 2048, 512, 4}, {9, 1024, 256, 16}, {70, 512, 32, 1},
@@ -421,6 +460,24 @@ int main() {
   for (auto& c : any) {
     int r = taps_case(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9], c[10]); if (r < 0) ++bad; else taken += r;
   }
+  // Pairs of CTAs, as larger layers have them on the real machine: every planner that can choose one, without splits and with, with an odd number of
+  // row tiles where the planner allows that (images that a tiled load can leave out; not the im2col mode's), a last half of the columns that is not full.
+  const int pair_convs[][5] = {{2, 1024, 256, 128, 2}, {2, 256, 1024, 128, 2}, {3, 2052, 252, 128, 6}, {3, 252, 2052, 128, 6}};
+  for (auto& c : pair_convs) { int r = conv_case(c[0], c[1], c[2], c[3], c[4]); if (r < 0) ++bad; else taken += r; }
+  const int pair_ragged[][5] = {{1, 1056, 200, 132, 2}, {1, 200, 1056, 132, 2}, {1, 2056, 200, 260, 6}, {1, 200, 2056, 260, 6}};
+  for (auto& c : pair_ragged) { int r = ragged_case(c[0], c[1], c[2], c[3], c[4]); if (r < 0) ++bad; else taken += r; }
+  // images, channels in and out, size, filter size, padding, stride, SMs
+  const int pair_taps[][8] = {{4, 256, 256, 8, 3, 1, 1, 4}, {5, 256, 224, 8, 3, 1, 1, 6}, {5, 224, 256, 8, 3, 1, 1, 6}, {4, 256, 512, 8, 3, 1, 1, 8}, {4, 512, 256, 8, 3, 1, 1, 8}, {3, 196, 160, 9, 3, 1, 1, 2},
+                              {3, 160, 196, 17, 3, 1, 2, 2}, {6, 132, 512, 7, 3, 1, 1, 8}};
+  for (auto& c : pair_taps) { int r = taps_case(c[0], c[1], c[2], c[3], c[3], c[4], c[4], c[5], c[5], c[6], c[6], c[7]); if (r < 0) ++bad; else taken += r; }
+  { int r = gemm_case(380, 508, 1040, true, true, true, 4); if (r < 0) ++bad; else taken += r; }
+  { int r = gemm_case(256, 244, 3100, false, false, false, 6); if (r < 0) ++bad; else taken += r; }
+  for (const char* what : {"fwd", "dgrad", "ragged fwd", "ragged dgrad", "taps fwd", "taps dgrad", "im2col fwd", "im2col dgrad"}) {
+    const bool im2col = !strncmp(what, "im2col", 6);
+    printf("pairs of CTAs, %s: %d plans, %d split, %d with an odd number of row tiles\n", what, pairs[what], split_pairs[what], odd_pairs[what]);
+    if (pairs[what] < 2 || !split_pairs[what] || pairs[what] == split_pairs[what] || (im2col ? odd_pairs[what] != 0 : !odd_pairs[what])) ++bad;
+  }
+  if (pairs["gemm"] < 1 || pairs["padded gemm"] + pairs["gemm"] < 2) { printf("pairs of CTAs: too few products\n"); ++bad; }
   printf("%d plans emulated, %d failures\n", taken, bad);
   return bad ? 1 : (taken >= 140 ? 0 : 2);
 }

@@ -464,6 +464,10 @@ ANY_CONVS = [  # N, C, H, W, K, R, stride, pad: image sizes, strides and channel
 @pytest.mark.parametrize("cfg", ANY_CONVS, ids=[str(c) for c in ANY_CONVS])
 def test_conv_of_any_size_tf32(ora, gpu, cfg, cache, det):
     """Factors of ten mantissa bits: their TF32 products are exact, so the FP32 oracle's result must come out to FP32 rounding."""
+    _conv_exact_factors(ora, gpu, cfg, [(cache, det)])
+
+
+def _conv_exact_factors(ora, gpu, cfg, modes):
     N, C, H, W, K, Rk, s, p = cfg
 
     def exact(a):
@@ -479,13 +483,28 @@ def test_conv_of_any_size_tf32(ora, gpu, cfg, cache, det):
         b.conv2D_batch_grad(x, None, w, TensorR(y, b.fromNumpy(dy0)), bias, (p, p), (s, s))
         return {"y": y.toCPU(), "dx": x.d.toCPU(), "dw": w.d.toCPU(), "db": bias.d.toCPU()}
     ref = f(ora)
-    gpu.lib.set_filter_cache(cache); gpu.lib.set_deterministic(det)
-    try:
-        got = f(gpu)
-    finally:
-        gpu.lib.set_filter_cache(0); gpu.lib.set_deterministic(0)
-    for k in ref:
-        assert_close(ref[k], got[k], FP32_RTOL, k)
+    for cache, det in modes:
+        gpu.lib.set_filter_cache(cache); gpu.lib.set_deterministic(det)
+        try:
+            got = f(gpu)
+        finally:
+            gpu.lib.set_filter_cache(0); gpu.lib.set_deterministic(0)
+        for k in ref:
+            assert_close(ref[k], got[k], FP32_RTOL, k)
+
+
+# Layers whose forward or data-gradient runs in pairs of CTAs on 148 SMs, and in how many splits (test_tc_plan.py asks the planner): the tap loop, the
+# im2col mode, images straight from memory that fill tiles and that do not; an odd number of row tiles, a last half of the columns that is not full.
+# N, C, H, W, K, R, stride, pad; splits of the forward and of the data-gradient (0: no pair)
+PAIR_CONVS = [((37, 256, 16, 16, 256, 3, 1, 1), 2, 2), ((150, 512, 4, 4, 512, 3, 1, 1), 3, 3), ((238, 256, 8, 8, 256, 3, 1, 1), 1, 1), ((160, 1024, 4, 4, 256, 3, 1, 1), 6, 2),
+              ((16, 256, 28, 28, 256, 3, 1, 1), 2, 2), ((78, 196, 14, 14, 252, 3, 1, 1), 1, 1), ((37, 2048, 16, 16, 256, 1, 1, 0), 2, 0), ((37, 256, 16, 16, 2048, 1, 1, 0), 0, 2),
+              ((60, 1024, 14, 14, 256, 1, 1, 0), 1, 0), ((60, 256, 14, 14, 1024, 1, 1, 0), 0, 1), ((41, 1024, 18, 18, 256, 1, 1, 0), 1, 0), ((41, 200, 18, 18, 1028, 1, 1, 0), 0, 1)]
+
+
+@pytest.mark.parametrize("cfg", [c[0] for c in PAIR_CONVS], ids=[str(c[0]) for c in PAIR_CONVS])
+def test_conv_in_pairs_of_ctas_tf32(ora, gpu, cfg):
+    """By atomics and, in deterministic mode, by clusters of up to four pairs and a sum of their slabs.  The tolerance is that of any FP32 sum here."""
+    _conv_exact_factors(ora, gpu, cfg, [(0, 0), (1, 1)])
 
 
 # Stride-1 filters on maps that tiles fill: rows and chunks (a tap of 32 channels) that end inside a tile, taps that wrap inside one, with and
