@@ -339,11 +339,14 @@ int pick_bn(int n_extent, int m_tiles, int sm_count, int k_iters = 0) {
 
 // A pair of CTAs per 256 x 256 outputs, where there are 256-wide tiles and an even number of row tiles (or an A operand whose loads beyond the last tile
 // only read zeros): a CTA then takes in 32 KB per k-iteration instead of 48, and that is what the loop waits for (at 48 KB a product of 4096 x 4096 x 2048
-// took 13 TB/s out of the L2).  Measured, one CTA against a pair, us: 4096 x 4096 x 2048 119 / 111, 8192 x 1000 x 2048 67 / 61 and 87 / 74 with B N-major,
-// 1920 x 4096 x 4096 108 / 100, 8192 x 2048 x 1000 (32 k-iterations) 73 / 72; with 16 k-iterations (16384 x 512 x 512) 24.2 / 25.4: the pair's meetings
-// before the first MMA and after the last are not earned back, hence the line at 32.  Returns the width of B's loads.
-int pick_pair(TcPlan& p, int m_tiles, int k_iters) {
-  p.pair = p.bn == 256 && k_iters >= 32 && m_tiles >= 2 && (m_tiles % 2 == 0 || p.a.load == TC_LOAD_BOX || p.a.load == TC_LOAD_BOXES) ? 1 : 0;
+// took 13 TB/s out of the L2).  Measured, one CTA against a pair, us.  Products: 4096 x 4096 x 2048 127 / 114, 8192 x 1000 x 2048 73 / 62 and 97 / 88 with A
+// M-major, 1920 x 4096 x 4096 124 / 112, 8192 x 4096 x 1024 (32 k-iterations) 142.5 / 142.2; of 84 of 32 k-iterations and more 77 are faster, by 7 % in the
+// middle, and one much slower (1000 x 2048 x 8192 with neither operand along k, 84 / 94).  With 16 k-iterations (16384 x 512 x 512) 24.2 / 25.4: the pair's
+// meetings before the first MMA and after the last are not earned back, hence the line at 32.  Tap loop: 256 channels, 256 images of 16 x 16, 126 / 123
+// forward and 151 / 144 back; 1x1 on images that fill tiles: 2048 -> 512, 128 of 16 x 16, 149 / 134.  `pays` is what a planner says of its own loads
+// (the reasons beside those that say no).  Returns the width of B's loads.
+int pick_pair(TcPlan& p, int m_tiles, int k_iters, bool pays = true) {
+  p.pair = pays && p.bn == 256 && k_iters >= 32 && m_tiles >= 2 && (m_tiles % 2 == 0 || p.a.load == TC_LOAD_BOX || p.a.load == TC_LOAD_BOXES) ? 1 : 0;
   return p.pair ? p.bn / 2 : p.bn;
 }
 
@@ -503,6 +506,10 @@ static bool corner_ok(const TcOperand& o) {
   return m.low_w >= -128 && m.low_h >= -128 && m.upper_w >= -128 && m.upper_h >= -128 && m.upper_w <= 127 && m.upper_h <= 127 && m.low_w <= 127 && m.low_h <= 127;
 }
 
+// In im2col mode a pair pays where the pixels' channels are not whole 32-byte sectors (a load then reads one more for each of its 128 rows): 28 x 28, 3x3 on 64
+// images, 196 -> 252 channels 131 / 104 us with a pair, 200 -> 256 99 / 103, 256 -> 256 109 / 112; 27 x 27, 5x5, 196 -> 252 113 / 84, 256 -> 200 90 / 93.
+// Of 230 launches over whole sectors one gained 2 % and 124 lost 2 to 7 %; of 22 others 18 gained 14 to 28 % and none lost.
+static bool im2col_pair_pays(int ld) { return ld % 8 != 0; }
 bool tc_plan_conv_any_fwd(TcPlan& p, const float* xr, const float* wt, const float* bias, float* y, const TcConvAny& g, int sm_count) {
   std::memset(&p, 0, sizeof p);
   if (!any_geometry_ok(g)) return false;
@@ -510,7 +517,7 @@ bool tc_plan_conv_any_fwd(TcPlan& p, const float* xr, const float* wt, const flo
   const int M = g.n_img * g.oH * g.oW;
   if (!operand_im2col(p.a, xr, g.n_img, g.H, g.W, g.C, g.ldc, g.oH, g.oW, g.sh, g.sw, -g.ph, -g.pw, g.R, g.S, &ka) || !corner_ok(p.a)) return false;
   p.bn = pick_bn(g.K, cdiv(M, kTileM), sm_count, ka);
-  if (!operand_k_taps(p.b, wt, g.R * g.S, g.K, g.ldc, pick_pair(p, cdiv(M, kTileM), ka), &kb) || ka != kb) return false;
+  if (!operand_k_taps(p.b, wt, g.R * g.S, g.K, g.ldc, pick_pair(p, cdiv(M, kTileM), ka, im2col_pair_pays(g.ldc)), &kb) || ka != kb) return false;
   finish(p, M, g.K, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = y; p.bias = bias; p.alpha = 1.0f; p.accumulate = 0;
   p.pix_per_img = (int64_t)g.oH * g.oW; p.img_stride = (int64_t)g.K * g.oH * g.oW; p.chan_stride = (int64_t)g.oH * g.oW;
@@ -525,7 +532,7 @@ bool tc_plan_conv_any_dgrad(TcPlan& p, const float* dyr, const float* wp, float*
   // dx is the convolution of dy with the filter turned round: tap (r', s') = (R - 1 - r, S - 1 - s), padding R - 1 - ph
   if (!operand_im2col(p.a, dyr, g.n_img, g.oH, g.oW, g.K, g.ldk, g.H, g.W, 1, 1, g.ph - g.R + 1, g.pw - g.S + 1, g.R, g.S, &ka) || !corner_ok(p.a)) return false;
   p.bn = pick_bn(g.C, cdiv(M, kTileM), sm_count, ka);
-  const int width = pick_pair(p, cdiv(M, kTileM), ka);
+  const int width = pick_pair(p, cdiv(M, kTileM), ka, im2col_pair_pays(g.ldk));
   // the taps in reverse
   if (g.C % 32 == 0) {
     if (!operand_mn_taps(p.b, wp, g.R * g.S, g.K, g.C, width, &kb) || ka != kb) return false;
@@ -560,7 +567,9 @@ bool tc_plan_conv_ragged_fwd(TcPlan& p, const float* x, const float* w, int ldw,
   if (co < 8 || ck < 8 || ldw < ck || (int64_t)n_img * pix > (1ll << 29) || !operand_mn_ragged(p.a, x, n_img, ck, pix, &ka, &tpi)) return false;
   const int M = n_img * tpi * kTileM;
   p.bn = pick_bn(co, n_img * tpi, sm_count, ka);
-  if (!operand_k_rows(p.b, w, co, ldw, pick_pair(p, n_img * tpi, ka), &kb) || ka != kb) return false;
+  // a pair pays for one column of tiles only: 14 x 14, 2048 -> 256 channels, 37 images 32.2 / 31.1 us with a pair, 74 images 48.1 / 45.2 (256 images 150 / 156);
+  // 1024 -> 512, 37 images 27.1 / 29.0, 128 images 88.5 / 94.5.  (The data-gradient takes it always: 512 -> 2048 channels 47.1 / 46.1, 500 -> 1024 137 / 127.)
+  if (!operand_k_rows(p.b, w, co, ldw, pick_pair(p, n_img * tpi, ka, co <= 256), &kb) || ka != kb) return false;
   finish(p, M, co, ka, sm_count, true);
   p.epilogue = TC_EPI_PIXEL; p.out = y; p.bias = bias; p.alpha = 1.0f; p.accumulate = 0;
   p.pix_per_img = pix; p.pix_pad = (int64_t)tpi * kTileM; p.img_stride = (int64_t)co * pix; p.chan_stride = pix;

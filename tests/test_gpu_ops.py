@@ -497,8 +497,9 @@ def _conv_exact_factors(ora, gpu, cfg, modes):
 # im2col mode, images straight from memory that fill tiles and that do not; an odd number of row tiles, a last half of the columns that is not full.
 # N, C, H, W, K, R, stride, pad; splits of the forward and of the data-gradient (0: no pair)
 PAIR_CONVS = [((37, 256, 16, 16, 256, 3, 1, 1), 2, 2), ((150, 512, 4, 4, 512, 3, 1, 1), 3, 3), ((238, 256, 8, 8, 256, 3, 1, 1), 1, 1), ((160, 1024, 4, 4, 256, 3, 1, 1), 6, 2),
-              ((16, 256, 28, 28, 256, 3, 1, 1), 2, 2), ((78, 196, 14, 14, 252, 3, 1, 1), 1, 1), ((37, 2048, 16, 16, 256, 1, 1, 0), 2, 0), ((37, 256, 16, 16, 2048, 1, 1, 0), 0, 2),
-              ((60, 1024, 14, 14, 256, 1, 1, 0), 1, 0), ((60, 256, 14, 14, 1024, 1, 1, 0), 0, 1), ((41, 1024, 18, 18, 256, 1, 1, 0), 1, 0), ((41, 200, 18, 18, 1028, 1, 1, 0), 0, 1)]
+              ((16, 252, 28, 28, 252, 3, 1, 1), 2, 2), ((78, 196, 14, 14, 252, 3, 1, 1), 1, 1), ((25, 1020, 10, 10, 252, 3, 1, 1), 6, 2), ((16, 256, 28, 28, 256, 3, 1, 1), 0, 0), ((37, 2048, 16, 16, 256, 1, 1, 0), 2, 0), ((37, 256, 16, 16, 2048, 1, 1, 0), 0, 2),
+              ((60, 1024, 14, 14, 256, 1, 1, 0), 1, 0), ((60, 256, 14, 14, 1024, 1, 1, 0), 0, 1), ((41, 1024, 18, 18, 256, 1, 1, 0), 1, 0), ((41, 200, 18, 18, 1028, 1, 1, 0), 0, 1),
+              ((60, 1024, 14, 14, 512, 1, 1, 0), 0, 0), ((37, 252, 16, 16, 2048, 1, 1, 0), 0, 2)]
 
 
 @pytest.mark.parametrize("cfg", [c[0] for c in PAIR_CONVS], ids=[str(c[0]) for c in PAIR_CONVS])
