@@ -45,9 +45,12 @@ __device__ __forceinline__ float un_grad(int op, float x, float y, float dy) {
 
 // ---- generic vectorised map over up to three inputs -------------------------------------------------------------
 // F: float f(float a, float b, float c); a/b/c may be null (then 0 is passed). out may alias any input.
-// U items of a thread in flight: 4 where the tensor gives every thread of the GPU one and more (a 3x3 layer with batch norm and ReLU on 32 x 64 x 56 x 56, forward and
-// backward, 212 -> 210 us; SqueezeNet at batch 64 776 -> 763), else 1 on as many
-// CTAs as there are.
+// U items of a thread in flight, bound by memory or, in the L2, by the number of loads under way.  Four of them (1 / 4, us): what lies in the L2 gains from 3.6 million
+// elements on (ReLU 3.7 million 4.2 / 3.8, 5.6 million 6.1 / 4.6, 10.3 million 11.3 / 7.6, sum 5.6 million 6.2 / 5.2, ReLU gradient 5.5 / 5.1), fewer leave threads
+// without work (sum 2.5 million 3.0 / 3.4, 1.3 million 2.2 / 3.1; with three inputs 2.5 million 3.6 / 3.4, 1.3 million 2.4 / 2.9).  From memory a map of one input gains (25.7 million, ReLU 32.0 / 31.6, tanh 33.3 / 31.7; 100 million
+// 121 / 118 and 128 / 117), one of several loses (sum 44.5 / 45.7, 100 million 170 / 173): those go four at a time while their tensors fit the L2 (in place, 10.3
+// million, 11.5 / 9.5), which costs them 1 to 2 % if they happen not to be there.
+constexpr int64_t kMapL2Bytes = (int64_t)126 << 20;
 template <int NIN, int U, class F>
 __global__ void __launch_bounds__(256) map_vec4(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c,
                                                 float* out, int64_t n4, F f) {
@@ -83,7 +86,9 @@ int launch_map(const float* a, const float* b, const float* c, float* out, int64
   bool vec = aligned16(a) && aligned16(out) && (NIN < 2 || aligned16(b)) && (NIN < 3 || aligned16(c));
   int64_t n4 = vec ? n / 4 : 0;
   LTB_REQUIRE(n4 <= (int64_t)256 * 0x7fffffff, "elementwise operation on too many elements");
-  if (n4 > (int64_t)g.sm_count * 2048) LTB_LAUNCH((map_vec4<NIN, 4, F>), (unsigned)ceil_div(n4, 1024), 256, 0, a, b, c, out, n4, f);
+  const bool in_place = out == a || (NIN > 1 && out == b) || (NIN > 2 && out == c);
+  const bool four = n4 > (int64_t)g.sm_count * (NIN > 2 ? 4096 : 6144) && (NIN == 1 || n4 * 16 * (NIN + (in_place ? 0 : 1)) <= kMapL2Bytes);
+  if (four) LTB_LAUNCH((map_vec4<NIN, 4, F>), (unsigned)ceil_div(n4, 1024), 256, 0, a, b, c, out, n4, f);
   else if (n4 > 0) LTB_LAUNCH((map_vec4<NIN, 1, F>), (unsigned)ceil_div(n4, 256), 256, 0, a, b, c, out, n4, f);
   if (n4 * 4 < n) LTB_LAUNCH((map_scalar<NIN, F>), grid_for(n - n4 * 4, 256), 256, 0, a, b, c, out, n4 * 4, n, f);
   return LTB_OK;

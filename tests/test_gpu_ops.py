@@ -610,6 +610,27 @@ def test_loss_head_in_one_kernel_each_way(gpu, rows, cols, mean):
         assert stop < 7 or few == (2 if rows <= 65536 else 4), (many, few)
 
 
+# Maps of four items a thread and of one: both sides of the lines (148 x 6144 x 4 elements, 148 x 4096 x 4 with three inputs; 126 MB of tensors), remainders of a CTA's 4096 and of 4.
+@pytest.mark.parametrize("n", [2424832, 2424841, 3637248, 3637252, 3637248 + 4093, 3637248 + 8191, 11010045, 11010052, 16515072, 16515080])
+def test_large_elementwise_maps(gpu, n):
+    import ctypes
+    import torch
+    lib, shape = gpu.lib, (ctypes.c_int * 1)(n)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x, y, d = (torch.randint(-8, 9, (n,), device="cuda", generator=gen).float() for _ in range(3))      # sums and products of these are exact
+    out, dx, s = torch.empty_like(x), d.clone(), x.clone()
+    torch.cuda.synchronize()
+    p = lambda t: t.data_ptr()
+    lib.unary(0, p(x), p(out), n); lib.sync()                                        # ReLU
+    assert torch.equal(out, x.clamp(min=0))
+    lib.ew_binary(0, p(x), shape, p(y), shape, p(out), 1); lib.sync()                # a sum into a third tensor
+    assert torch.equal(out, x + y)
+    lib.ew_binary(0, p(s), shape, p(y), shape, p(s), 1); lib.sync()                  # and over its own operand
+    assert torch.equal(s, x + y)
+    lib.unary_grad(6, p(x), p(dx), 0, p(y), n, 0); lib.sync()                        # the gradient of a square: three operands, one of them the result
+    assert torch.equal(dx, d + y * x * 2)
+
+
 @pytest.mark.parametrize("rows,cols", [(9, 10), (300, 200), (77, 1000), (40, 1500)])
 def test_loss_head_over_its_own_logits(gpu, rows, cols):
     """A log-softmax in place: the likelihood is that of the values before, with look-ahead fusion as without, and the calls are not joined (the
