@@ -655,8 +655,11 @@ static int bn_splits(int N, int C) {
 
 // Issues a BN forward described by `p` (the cluster path), optionally with the ReLU of its result; a PEND_BN_ADD also adds
 // p.a and writes p.out instead of p.y.
-// The channels-last copy leaves a packed kernel as single floats, 4 C bytes apart: 16 us of stores per million of them (512 thousand, 256 x 4 x 4 at
-// batch 128: 12.2 us, 4.4 without the copy), where the copy as a launch of its own takes 3.5 us on the smallest maps and 5 on these.
+// The channels-last copy leaves a packed kernel as single floats, 4 C bytes apart: stores that cost more and more beside a launch of its own, which on small
+// maps is mostly launch.  Batch norm, ReLU and the 3x3 convolution behind them alone in a recording, us with the copy apart / written here, by the number of
+// elements: 16 to 131 thousand 0.4 to 1.2 us saved in each of nine shapes (8 x 256 x 4 x 4 13.6 / 12.4), 164 to 400 thousand 0.1 to 2.8 in each of sixteen
+// (32 x 128 x 8 x 8 16.9 / 14.4), 524 thousand 18.8 / 16.9, 22.9 / 22.0, 22.0 / 22.1, 33.4 / 33.4, a million 23.7 / 24.7, 29.4 / 31.4.  In a training step the line is
+// lower, 131 thousand: with 262 or 524 thousand ResNet-50 takes 1693 us instead of 1688 at batch 32, 3093 instead of 3088 at 128, 2113 instead of 2115 at 64.
 static bool bn_fwd_packed(const Pending& p, BnPackedPlan& pk) { return (bn_cluster_plan(p.N, p.C, p.HW).K == 1 || p.C >= 96) && bn_packed_plan(p.N, p.C, p.HW, kBnVpt, pk); }
 bool bn_fwd_writes_copy(const Pending& p) {
   BnPackedPlan pk;

@@ -971,7 +971,9 @@ def test_lookahead_fusion_flushes_on_any_other_call(ora, gpu):
 # N, C, H, K, R, stride, pad: convolutions whose results are cleared by a kernel before them, each kind of batch-norm kernel and of staging
 @pytest.mark.parametrize("reuse", [False, True])
 @pytest.mark.parametrize("cfg", [(8, 256, 4, 1024, 1, 1, 0), (8, 256, 4, 256, 3, 1, 1), (8, 64, 16, 64, 3, 1, 1), (128, 64, 16, 64, 1, 1, 0), (8, 128, 8, 256, 3, 2, 1),
-                                 (8, 256, 8, 512, 1, 2, 0), (3, 36, 6, 40, 3, 1, 1), (16, 512, 2, 512, 3, 1, 1), (2, 64, 32, 24, 5, 1, 2), (5, 10, 3, 12, 3, 1, 1)])
+                                 (8, 256, 8, 512, 1, 2, 0), (3, 36, 6, 40, 3, 1, 1), (16, 512, 2, 512, 3, 1, 1), (2, 64, 32, 24, 5, 1, 2), (5, 10, 3, 12, 3, 1, 1),
+                                 # the copy for the convolution in the batch norm's kernel up to 2^17 elements, and beyond
+                                 (8, 256, 8, 64, 3, 1, 1), (9, 256, 8, 64, 3, 1, 1), (6, 96, 14, 40, 3, 1, 1), (64, 512, 2, 64, 3, 1, 1)])
 def test_a_convolution_takes_over_the_batch_norm_before_it(gpu, cfg, reuse):
     """Batch norm, in-place ReLU, convolution and its backward call: as three kernels that prepare for one another and one by one.  The convolution writes
     into a buffer full of NaN, or (reuse) into the batch norm's own input."""
