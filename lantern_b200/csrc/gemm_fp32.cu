@@ -67,7 +67,11 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
 constexpr int kTables = 4;
 // How an operand's elements are fetched.  FEED_ROW: single elements, neighbouring threads on neighbouring rows (a thread keeps its row);
 // FEED_K: neighbouring threads on neighbouring k (a thread keeps its k).  _4: four neighbours at a time with one 16-byte load, where
-// groups of four along the contiguous index are aligned and lie inside together.
+// groups of four along the contiguous index are aligned and lie inside together.  That doubles the kernels (and their build), for, us one by one / four at a time:
+// products, 32 of eight sizes and both orders of each operand, 0 to 14 % (2048^3 408 / 370 with both along k, 390 / 353 with neither, 397 / 397 and 399 / 393 mixed;
+// 512 x 512 x 4096 100 / 92 to 84; 300 x 2000 x 320 23.5 / 21.6); 1x1 layers, fourteen, forward 0 to 7 % (128 -> 256 at 28 x 28 on 8 images 18.4 / 17.3), data-gradient
+// 0 to 11 % (48 -> 192 at 8 x 8 on 64 images 12.7 / 11.3), weight gradient 1 to 6 %; larger filters, whose taps leave one operand as it was, 0 to 1 % forward
+// (64 -> 64 3x3 at 28 x 28 on 32 images 72.2 / 71.5) and 1 to 3 % of the weight gradient (16 -> 64 at 16 x 16 on 64 images 24.0 / 23.2).  None was slower.
 enum { FEED_ROW = 0, FEED_K = 1, FEED_ROW4 = 2, FEED_K4 = 3 };
 // One operand's share of a step: T rows x BKK, fetched to registers, then stored k by k.
 template <int T, int FEED, class OP>

@@ -4,6 +4,7 @@
 // kernels (DslAPI.scala:506-516) and cublasSdot/Sgemv (TensorDslCublas.scala:173-201, 257-264).  Semantics follow
 // TensorDslCPU.scala (cited per entry point).  Rows are reduced by one warp each with shuffles; full reductions
 // use a block tree in shared memory and, for large inputs, a second pass over per-block partials.
+#include <algorithm>
 #include <cfloat>
 
 #include "common.cuh"
@@ -107,19 +108,23 @@ __global__ void softmax_kernel(const float* __restrict__ x, float* y, int rows, 
 }
 // Log-softmax of a row, the negative log likelihood of its target (nll_kernel) and, with `sum`, scale times the sum of those: three launches of some
 // 3 us each on a batch of a few hundred rows, of which there is next to nothing to compute.  The last CTA to finish adds the rows up, in the order in
-// which sum_kernel's one CTA of 1024 threads does, so the result is the same to the bit.
+// which sum_kernel's one CTA of 1024 threads does, so the result is the same to the bit: thirty-two loads of a thread in flight (one after the other the sum of
+// 8192 rows took 9 us), rows of at most 32 columns (VPT 1) on as many CTAs as the GPU holds, so that there are fewer tickets to wait for (65536 x 10 24.5 -> 18.2 us).
 template <int VPT>
 __global__ void __launch_bounds__(256) softmax_nll_kernel(const float* __restrict__ x, float* y, const int32_t* __restrict__ t, float* nll, float* sum, float scale,
                                                           int rows, int cols, unsigned* ticket) {
   pdl_enter();
-  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (r < rows) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t first = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  auto row = [&](int64_t r) {
     const int k = t[r];
     const bool in = k >= 0 && k < cols;
     const float xk = in ? x[r * cols + k] : 0.0f;
     const float logsum = softmax_row<1, VPT>(x + r * cols, y + r * cols, cols, lane);
     if (lane == 0) nll[r] = in ? -1.0f * (xk - logsum) : 0.0f;
-  }
+  };
+  if constexpr (VPT == 1) { for (int64_t r = first; r < rows; r += (int64_t)gridDim.x * 8) row(r); }
+  else if (first < rows) row(first);
   if (!sum) return;
   __shared__ bool last;
   __shared__ float part[32];
@@ -127,14 +132,22 @@ __global__ void __launch_bounds__(256) softmax_nll_kernel(const float* __restric
   if (threadIdx.x == 0) { __threadfence(); last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1; __threadfence(); }      // back at zero after the last
   __syncthreads();
   if (!last) return;
-  for (int q = 0; q < 4; ++q) {
-    float s = 0.0f;
-    for (int i = threadIdx.x + 256 * q; i < rows; i += 1024) s += __ldcg(nll + i);
-    s = warp_sum(s);
-    if (lane == 0) part[w + 8 * q] = s;
+  float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  for (int i0 = threadIdx.x; i0 < rows; i0 += 8192) {
+    float v[8][4];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { const int i = i0 + 1024 * e + 256 * q; v[e][q] = i < rows ? __ldcg(nll + i) : 0.0f; }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] += v[e][q];
   }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { const float a = warp_sum(s[q]); if (lane == 0) part[w + 8 * q] = a; }
   __syncthreads();
-  if (w == 0) { const float s = warp_sum(part[lane]); if (lane == 0) sum[0] = s * scale; }
+  if (w == 0) { const float a = warp_sum(part[lane]); if (lane == 0) sum[0] = a * scale; }
 }
 // MODE 0: dx += y*(dy - sum dy*y) (cudnnSoftmaxBackward ACCURATE, TensorDslCudnn.scala:1465-1504);
 // MODE 1: dx += dy - exp(y)*sum dy (TensorDslCPU.scala:837-846).  VPT as above.
@@ -169,9 +182,10 @@ __global__ void softmax_grad_kernel(float* dx, const float* __restrict__ y, cons
   }
 }
 // What leads from the gradient of a loss to that of the logits, a warp per row: dnll += scale dout (dout set to `value` first when it is seeded here),
-// dlogp[target] -= dnll, dx += dlogp - exp(y) sum dlogp; every buffer ends up as the separate launches leave it (four of 2.5 to 4 us each).
+// dlogp[target] -= dnll, dx += dlogp - exp(y) sum dlogp; every buffer ends up as the separate launches leave it (four of 2.5 to 4 us each).  Nothing is stored before
+// a row's sum, so that its loads go out together (us, 8192 x 1000 apart 25.9, joined 29.4 with the store first, 22.0 so; 1024 x 4096 24.7, 40.1, 22.7; 8192 x 100 6.9, 4.2).
 template <int VPT>
-__global__ void __launch_bounds__(256) nll_softmax_grad_kernel(float* dx, const float* __restrict__ y, float* dlogp, float* dnll, float* dout, bool seeded, float value,
+__global__ void __launch_bounds__(256) nll_softmax_grad_kernel(float* __restrict__ dx, const float* __restrict__ y, float* __restrict__ dlogp, float* dnll, float* dout, bool seeded, float value,
                                                                float scale, const int32_t* __restrict__ t, int rows, int cols) {
   pdl_enter();
   const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; const int lane = threadIdx.x & 31;
@@ -179,7 +193,7 @@ __global__ void __launch_bounds__(256) nll_softmax_grad_kernel(float* dx, const 
   const int k = t[r];
   const float dn = fmaf(seeded ? value : dout[0], scale, dnll[r]);
   if (lane == 0) { dnll[r] = dn; if (seeded && r == 0) dout[0] = value; }
-  const float* yy = y + r * cols; float* d = dlogp + r * cols; float* o = dx + r * cols;
+  const float* __restrict__ yy = y + r * cols; float* __restrict__ d = dlogp + r * cols; float* __restrict__ o = dx + r * cols;
   float s = 0.0f;
   if constexpr (VPT > 0) {
     float v[VPT], w[VPT], old[VPT];
@@ -193,14 +207,17 @@ __global__ void __launch_bounds__(256) nll_softmax_grad_kernel(float* dx, const 
     return;
   }
 #pragma unroll 8
-  for (int i = lane; i < cols; i += 32) { float v = d[i]; if (i == k) { v += -1.0f * dn; d[i] = v; } s += v; }
+  for (int i = lane; i < cols; i += 32) { float v = d[i]; if (i == k) v += -1.0f * dn; s += v; }
   s = warp_sum(s);
-  for (int i0 = lane; i0 < cols; i0 += 128) {            // each lane reads back what it wrote itself
+  for (int i0 = lane; i0 < cols; i0 += 128) {
     float v[4], w[4], old[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; if (i < cols) o[i] = old[j] + (v[j] - expf(w[j]) * s); }
+    for (int j = 0; j < 4; ++j) {
+      const int i = i0 + 32 * j;
+      if (i < cols) { if (i == k) { v[j] += -1.0f * dn; d[i] = v[j]; } o[i] = old[j] + (v[j] - expf(w[j]) * s); }
+    }
   }
 }
 __global__ void nll_kernel(const float* __restrict__ x, const int32_t* __restrict__ t, float* out, int rows, int cols) {
@@ -285,11 +302,15 @@ static int full_sum(const float* x, float* out, int64_t n, float scale) {
 }
 
 // ---- the calls around a classifier's loss that look-ahead fusion joins
-constexpr int kHeadSumRows = 1 << 16;                       // one CTA adds them up, as in full_sum
+// The rows up to which the sum joins: as many as the GPU holds at once (the kernel's registers allow eight CTAs of eight rows an SM, three at 257 to 1024
+// columns; at most 32 columns a CTA takes several rows).  A CTA waits for its ticket before it makes room for another, which costs more than the two launches
+// saved: apart / joined, us, 3000 x 1000 8.9 / 7.8, 4096 x 1000 10.9 / 11.7, 8192 x 1000 15.1 / 17.1; 8192 x 100 6.3 / 5.8, 16384 x 100 9.0 / 10.0; 8192 x 10 5.3 / 5.0,
+// 20000 x 10 8.1 / 7.6, 65536 x 10 17.3 / 18.2.  (One CTA adds them up, as in full_sum: 65536 in all.)
+static int head_sum_rows(int cols) { return cols <= 32 ? 1 << 16 : std::min(1 << 16, g.sm_count * 8 * (cols <= 256 || cols > 1024 ? 8 : 3)); }
 static int softmax_nll_issue(const Pending& p, float* sum, float scale) {
-  const unsigned grid = (unsigned)ceil_div((int64_t)p.N * 32, 256);
+  const unsigned grid = (unsigned)ceil_div((int64_t)p.N * 32, 256), most = (unsigned)g.sm_count * 8;      // a warp per row
   unsigned* const ticket = g.tickets + (g.in_branch ? 1 : 0);
-  if (p.C <= 32) LTB_LAUNCH((softmax_nll_kernel<1>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
+  if (p.C <= 32) LTB_LAUNCH((softmax_nll_kernel<1>), std::min(grid, most), 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
   else if (p.C <= 256) LTB_LAUNCH((softmax_nll_kernel<8>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
   else if (p.C <= 1024) LTB_LAUNCH((softmax_nll_kernel<32>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
   else LTB_LAUNCH((softmax_nll_kernel<0>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
@@ -320,7 +341,7 @@ int head_issue(const Pending& p) {
 // Whether [p, p + floats) keeps clear of [q, q + n).
 static bool apart(const void* p, int64_t floats, const void* q, int64_t n) { return (const float*)p + floats <= (const float*)q || (const float*)q + n <= (const float*)p; }
 static int full_sum_joining(const float* x, float* out, int64_t n, float scale) {
-  if (g.pending.kind == PEND_NLL && g.pending.out == x && g.pending.N == n && n <= kHeadSumRows) {
+  if (g.pending.kind == PEND_NLL && g.pending.out == x && g.pending.N == n && n <= head_sum_rows(g.pending.C)) {
     const Pending p = g.pending; g.pending.kind = PEND_NONE;
     return softmax_nll_issue(p, out, scale);               // (the last CTA writes out: nothing is read any more)
   }

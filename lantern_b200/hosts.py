@@ -219,8 +219,8 @@ class Model:
 
     def use_fused_cells(self, on=3):
         """Recursive models: 0 one call per operator, as the reference stages them; 1 one fused call per gate or cell; 2 in
-        addition the vanilla RNN's whole unrolled sequence and a whole tree-LSTM node in one call; 3 (the default) a whole
-        LEVEL of the tree in one call."""
+        addition the vanilla RNN's whole unrolled sequence and a whole tree-LSTM node in one call; 3 (the default) the whole
+        tree in one call."""
         self.hp.fn["model_use_fused_cells"](self.h, int(on))
 
     def use_branches(self, on=True):

@@ -264,7 +264,9 @@ struct Model {
   // step k alone.  The staging pair of step k is refilled by step k + 2, after its upload marker has fired.  A step is recorded
   // once per pair: it reads the batch where the upload puts it and leaves its loss in the pair's pinned word.  (One recording
   // for both, with the batch, its labels and the loss copied to and from fixed addresses around it: five more nodes a step,
-  // each 2 to 4 us on the device between two kernels: the RNN of one row 90 -> 74 us a step, the MNIST CNN 185 -> 163.)
+  // each 2 to 4 us on the device between two kernels: the RNN of one row 90 -> 74 us a step, the MNIST CNN 185 -> 163.  The second recording costs
+  // the host as much again as the first, once a program and once a change of the learning rate: 2.4 ms for ResNet-50, 0.9 for SqueezeNet, 0.34 for the
+  // MNIST CNN, 0.1 to 0.2 for the RNN, part of it beside the step on the device; five to a hundred steps earn it back.)
   void feed_mode(bool on) {
     if (feeding == on) return;
     drop_graphs();
@@ -787,7 +789,8 @@ int HOST_FN(model_set_table)(void* m, const float* host, int rows) {
 }
 int64_t HOST_FN(model_label_count)(void* m) { return ((Model*)m)->label_count; }
 // Recursive models: gates as single fused calls (default) or operator by operator, as the reference stages them.
-// on: 0 operator by operator, 1 one call per gate / cell, 2 (default) in addition the vanilla RNN's whole sequence in one call.
+// on: 0 operator by operator, 1 one call per gate / cell, 2 in addition the vanilla RNN's whole sequence and a whole tree node in one call, 3 (default) the
+// whole tree.
 int HOST_FN(model_use_fused_cells)(void* m, int on) {
   Model* M = (Model*)m;
   M->drop_graphs();

@@ -578,6 +578,16 @@ def test_loss_head_in_one_kernel_each_way(gpu, rows, cols, mean):
     """log-softmax, negative log likelihood and their sum or mean, and the way back from a seeded gradient: with look-ahead fusion one kernel each, and
     every buffer as the separate calls leave it, bit for bit (the same operations in the same order): with destinations that hold something already,
     targets out of range, and a sequence broken off after each of its calls."""
+    _loss_head(gpu, rows, cols, mean, 2 if rows <= 65536 else 4)
+
+
+@pytest.mark.parametrize("rows,cols,mean,launches", [(9472, 100, 1, 2), (9473, 100, 1, 3), (3552, 257, 0, 2), (3553, 257, 0, 3), (9473, 33, 1, 3), (9475, 1025, 0, 3), (30000, 32, 1, 2)])
+def test_loss_head_of_more_rows_than_the_gpu_holds(gpu, rows, cols, mean, launches):
+    """Both sides of the line up to which the sum joins; several rows of at most 32 columns per warp."""
+    _loss_head(gpu, rows, cols, mean, launches)
+
+
+def _loss_head(gpu, rows, cols, mean, launches_joined):
     import torch
     lib = gpu.lib
     gen = torch.Generator(device="cuda").manual_seed(rows + cols)
@@ -607,7 +617,7 @@ def test_loss_head_in_one_kernel_each_way(gpu, rows, cols, mean):
         f, few = run(1, stop)
         for name, u, v in zip(names, a, f):
             assert torch.equal(u, v), (stop, name)
-        assert stop < 7 or few == (2 if rows <= 65536 else 4), (many, few)
+        assert stop < 7 or few == launches_joined, (many, few)
 
 
 # Maps of four items a thread and of one: both sides of the lines (148 x 6144 x 4 elements, 148 x 4096 x 4 with three inputs; 126 MB of tensors), remainders of a CTA's 4096 and of 4.

@@ -77,7 +77,7 @@ def test_treelstm_node_call_equals_operator_by_operator(oracle_lib, variant):
     for leaves in (1, 2, 9, 30):
         y = _random_tree(np.random.default_rng(12 + leaves), leaves)
         res = []
-        for level in (3, 2, 0):                      # a whole level of the tree per call, a whole node per call, operator by operator
+        for level in (3, 2, 0):                      # the whole tree per call, a whole node per call, operator by operator
             m = _model(oracle_lib, variant, 1)
             m.use_fused_cells(level)
             loss = m.step(x, y, 0.0, update=False)
