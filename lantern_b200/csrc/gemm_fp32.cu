@@ -604,7 +604,7 @@ static int skinny_gemm(const float* a, int64_t sam, int64_t sak, const float* b,
 // The time of such a product is latency: the tiles above walk K in steps of 16, each a round trip to memory and a barrier.  Here a CTA of sixteen warps
 // fetches all of k of both operands at once (up to sixteen loads of a thread in flight; 4-byte cp.async leave an SM at one warp's worth per 18 cycles:
 // 100 x 50 x 320 8.4 us), each warp takes a sixteenth of k and the whole T x T tile, and their sums meet in shared memory in warp order: the same bits on
-// every run, and shorter chains than the tiles above have.  T is 16 while such tiles fit one round of the SMs: a quarter of the arithmetic per SM.
+// every run, and shorter chains than the tiles above have.  T is 16 where that is the faster tile: a quarter of the arithmetic per SM.
 constexpr int kSmallWarps = 16, kSmallPart = 33;
 template <int T> constexpr int kSmallK = 16384 / T;       // what shared memory holds of both operands: 1024 of k, or 512
 template <int T>
@@ -673,10 +673,27 @@ __global__ void __launch_bounds__(kSmallWarps * 32) small_gemm_kernel(const floa
     }
   }
 }
-// One round of CTAs and one fetch.  Measured from Python, 5 us of call overhead included, tiles above against this, us: 100 x 50 x 320 11.3 / 5.8,
-// 128 x 128 x 128 8.1 / 5.5, 128 x 128 x 512 9.8 / 5.4, 64 x 64 x 1024 9.9 / 8.5, 240 x 240 x 300 12.3 / 7.5, 384 x 384 x 64 5.7 / 5.5, 384 x 384 x 512 14.6 / 9.3;
-// walking a longer K in several fetches (32 x 32 tiles) lost: 200 x 300 x 1500 20.9 / 24.8, 128 x 128 x 2048 16 / 33.
-template <int T> static bool small_takes(int M, int N, int K) { return K <= kSmallK<T> && ceil_div(M, T) * ceil_div(N, T) <= g.sm_count; }
+// The tile of a small product, or 0: the tiles above.  One round of CTAs, one fetch of all of k (walking a longer K in several fetches lost: 200 x 300 x 1500 20.9 / 24.8 us,
+// 128 x 128 x 2048 16 / 33), and where that was the faster one of the three; sums that may be added atomically are split over CTAs by the tiles above, from K = 128 on.
+// Measured in recordings of twenty, us, tiles above / 16 / 32:
+//                    stored                                                               added
+//   64 x 64          K 48 3.2/3.2/3.7, 64 3.9/3.2/3.8, 512 7.8/4.8/8.4, 1024 8.0/8.0        K 32 3.1/3.1/3.7, 64 4.3/3.2/3.8, 400 5.9/4.4, 512 5.3/4.9, 640 4.5/6.5
+//   8 x 8            K 48 2.6/3.0/3.3, 64 3.2/3.1/3.4, 512 6.2/4.4/7.7, 640 6.3/6.4         K 48 2.9/2.9/3.3, 320 4.2/3.7/6.1, 512 4.2/4.5, 640 3.6/6.1
+//   192 x 192        K 64 4.1/5.0/3.9, 128 6.6/5.4/4.4, 400 8.7/6.6/7.6, 640 8.2/10.9, 768 8.1/7.1   K 64 4.9/4.7/4.1, 192 5.8/5.2/5.4, 256 5.5/5.5/5.8
+//   384 x 384 (32)   K 48 3.4/3.9, 64 4.0/4.0, 512 12.0/8.7                                 K 48 4.6/4.2, 400 9.0/7.9
+// (More than one CTA of 16 x 16 for two SMs is slow where two of them fit one SM, up to K = 640: they are not spread evenly.)
+static int small_tile(int M, int N, int K, bool adds) {
+  const int64_t t16 = ceil_div(M, 16) * ceil_div(N, 16), t32 = ceil_div(M, 32) * ceil_div(N, 32), sms = g.sm_count;
+  const bool few = 2 * t16 <= sms;
+  if (K < (adds ? 48 : 64)) return 0;
+  if (adds) {
+    if (few) return K <= (t16 >= 8 && t16 <= 32 ? 512 : 400) ? 16 : 0;
+    return t32 <= sms && K <= (5 * t32 >= 2 * sms ? 400 : 192) ? 32 : 0;
+  }
+  if (K > 512) return t16 >= 16 && t16 <= sms && K <= kSmallK<16> && (K >= 704 || t16 <= 32) ? 16 : 0;
+  if (t16 <= sms && (few || K > 256)) return 16;
+  return t32 <= sms ? 32 : 0;
+}
 template <int T>
 static int small_gemm(const float* a, int64_t sam, int64_t sak, const float* b, int64_t sbk, int64_t sbn, float* c, int64_t scm, int64_t scn,
                       int M, int N, int K, float alpha, bool accumulate) {
@@ -698,15 +715,16 @@ static int small_gemm(const float* a, int64_t sam, int64_t sak, const float* b, 
 static int strided_gemm(const float* a, int64_t sam, int64_t sak, const float* b, int64_t sbk, int64_t sbn, float* c, int64_t scm,
                         int64_t scn, int M, int N, int K, float alpha, bool accumulate) {
   { bool taken = false; int rc = skinny_gemm(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate, &taken); if (rc || taken) return rc; }
-  if (small_takes<16>(M, N, K)) return small_gemm<16>(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate);
-  if (small_takes<32>(M, N, K)) return small_gemm<32>(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate);
+  const bool adds = accumulate && !g.deterministic;
+  if (const int tile = small_tile(M, N, K, adds))
+    return tile == 16 ? small_gemm<16>(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate) : small_gemm<32>(a, sam, sak, b, sbk, sbn, c, scm, scn, M, N, K, alpha, accumulate);
   // m of the kernel is the contiguous index of C
   const bool swap = scn == 1 && scm != 1;
   const int m = swap ? N : M, n = swap ? M : N;
   const long long sm = swap ? scn : scm, sn = swap ? scm : scn;
   const float* pa = swap ? b : a; const float* pb = swap ? a : b;
   const int64_t ar = swap ? sbn : sam, ak = swap ? sbk : sak, br = swap ? sam : sbn, bk = swap ? sak : sbk;
-  const Tiling t = choose_tiling(m, n, K, !g.deterministic && accumulate);
+  const Tiling t = choose_tiling(m, n, K, adds);
   const MatPut st{c, sm, sn, alpha, t.groups > 1 ? 2 : accumulate ? 1 : 0, sm == 1 && sn % 4 == 0 && aligned16(c)};
   const int64_t most = ((int64_t)1 << 31) - 1;
   if (m * ar + K * ak > most || n * br + K * bk > most) {

@@ -540,7 +540,9 @@ def test_gemm_of_ragged_rows_tf32(ora, gpu, ta, tb, M, N, K):
 
 @pytest.mark.parametrize("acc", [0, 1])
 @pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
-@pytest.mark.parametrize("M,N,K", [(17, 17, 17), (33, 31, 64), (1, 300, 45), (300, 1, 21), (193, 190, 33), (192, 190, 1024), (100, 50, 320), (385, 383, 17), (380, 381, 512), (190, 190, 513), (50, 100, 1025)])
+@pytest.mark.parametrize("M,N,K", [(17, 17, 17), (33, 31, 64), (1, 300, 45), (300, 1, 21), (193, 190, 33), (192, 190, 1024), (100, 50, 320), (385, 383, 17), (380, 381, 512), (190, 190, 513), (50, 100, 1025),
+                                   # the lines of the rule in k: 63 | 64, 512 | 513, 703 | 704; of gradients 47 | 48, 192 | 193, 400 | 401, 512 | 513
+                                   (17, 17, 63), (65, 70, 513), (130, 130, 703), (130, 131, 704), (10, 10, 600), (200, 190, 257), (47, 48, 60), (193, 192, 200), (400, 401, 34), (513, 512, 70)])
 def test_small_products_fp32(gpu, M, N, K, ta, tb, acc):
     """Products of one round of 16 x 16 or 32 x 32 tiles, at the edges of tiles, of the sixteenths of K and of the rules, against float64.  The sum of K
     products in any order differs from the exact one by at most K roundings of the sum of their magnitudes."""
