@@ -997,11 +997,20 @@ static int conv_direct(const float* in, const float* w, float* out, DirectGeo& G
   return launch_direct<4, 2, FLIP>(in, w, out, G, G.Ci <= G.Co ? 6 : 16, label);
 }
 // 3x3, stride 1, padding 1 on maps of 4 to 32 rows and columns (powers of two: whole groups of 32 runs), 16-byte aligned tensors, at least a step of
-// channels on both sides.
-static bool direct_takes(const ConvDims& d, const float* a, const float* b) {
+// channels on both sides; and where it is the faster one.  Measured against the matrix form on 1328 sizes each way (4 to 32 rows, 1 to 128 images, 8 to 512 channels): from 24
+// channels summed over it takes 0.4 to 1.0 of the time but where less than half of a group's pixels exist and there are splits all the same (128 -> 512, one
+// image of 8 x 8, 10.1 us in matrix form, 18.2 here; 96 -> 256, two images, 9.5 / 12.5); with fewer a chain is too short for what it costs, so that only large outputs
+// gain (16 channels: 24 outputs on 16 images of 8 x 8 6.9 / 9.0, 96 outputs on 32 of 32 x 32 32.2 / 26.1; 12, a step and a half, at 32 x 32 on 16 images, 256 outputs
+// 26.7 / 33.7), and maps of 4 rows, whose tiles are half as wide (16 -> 64, 8.2 / 5.6; back from 8 channels to fewer than 32, 4.9 / 5.8).
+static bool direct_takes(const ConvDims& d, const float* a, const float* b, bool back) {
   if (d.R != 3 || d.S != 3 || d.sh != 1 || d.sw != 1 || d.ph != 1 || d.pw != 1 || !aligned16(a) || !aligned16(b)) return false;
   if (d.W != 4 && d.W != 8 && d.W != 16 && d.W != 32) return false;
   if (d.C < 8 || d.K < 8) return false;
+  const int from = back ? d.K : d.C, to = back ? d.C : d.K;
+  const int64_t pixels = (int64_t)d.N * d.H * d.W;
+  const bool wide = d.W >= 8 && d.H >= 8;
+  if (from < 24 && (from % 8 || (wide ? pixels * ceil_div(to, 32) * 32 < 1200000 : back && from == 8 && to < 32))) return false;
+  if (wide && from > 64 && from <= to && pixels <= 128) return false;
   return d.H <= 32 && (d.H & (d.H - 1)) == 0 && d.H >= 4 && (int64_t)d.C * d.H * d.W * 32 < (1ll << 31) && (int64_t)d.K * d.H * d.W * 32 < (1ll << 31);
 }
 
@@ -1014,7 +1023,7 @@ static bool narrow(const ConvDims& d) {
 static bool plain_pixels(const ConvDims& d) { return d.R == 1 && d.S == 1 && d.sh == 1 && d.sw == 1 && d.ph == 0 && d.pw == 0 && d.H * d.W % 4 == 0; }
 int conv_fwd_fp32(const float* x, const float* w, const float* bias, float* y, const ConvDims& d, bool relu) {
   const int hw = d.oH * d.oW, M = d.N * hw, Kd = d.C * d.R * d.S;
-  if (direct_takes(d, x, y)) {
+  if (direct_takes(d, x, y, false)) {
     DirectGeo G{d.N, d.C, d.K, d.H, d.W, 0, 0, 0, 0, bias, relu ? 1 : 0};
     return conv_direct<false>(x, w, y, G, "direct[conv_fwd]");
   }
@@ -1029,7 +1038,7 @@ int conv_fwd_fp32(const float* x, const float* w, const float* bias, float* y, c
 }
 int conv_dgrad_fp32(const float* dy, const float* w, float* dx, const ConvDims& d) {
   const int hw = d.H * d.W, M = d.N * hw, rs = d.R * d.S, Kd = d.K * rs;
-  if (direct_takes(d, dy, dx)) {
+  if (direct_takes(d, dy, dx, true)) {
     DirectGeo G{d.N, d.K, d.C, d.H, d.W, 0, 0, 0, 0, nullptr, 0};
     return conv_direct<true>(dy, w, dx, G, "direct[conv_dgrad]");
   }

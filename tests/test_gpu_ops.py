@@ -144,6 +144,9 @@ def test_conv_fwd_bwd_fp32(ora, gpu, cfg):
 # time and one by one; strides; filters whose rows and columns do not fit a table entry's bits.
 FP32_FORMS = [(1, 8, 4, 4, 8, 3, 3, 1, 1), (9, 13, 4, 4, 70, 3, 3, 1, 1), (3, 40, 8, 8, 33, 3, 3, 1, 1), (5, 17, 16, 16, 9, 3, 3, 1, 1), (2, 9, 32, 32, 34, 3, 3, 1, 1),
               (2, 64, 8, 16, 16, 3, 3, 1, 1), (3, 16, 32, 4, 48, 3, 3, 1, 1), (2, 24, 4, 32, 40, 3, 3, 1, 1), (2, 70, 16, 8, 100, 3, 3, 1, 1),
+              # the same edges with 24 channels and more on both sides, and both sides of the lines between the direct form and the matrix form
+              (9, 29, 4, 4, 70, 3, 3, 1, 1), (5, 27, 16, 16, 25, 3, 3, 1, 1), (2, 25, 32, 32, 34, 3, 3, 1, 1), (74, 16, 16, 16, 64, 3, 3, 1, 1), (73, 16, 16, 16, 64, 3, 3, 1, 1),
+              (2, 96, 8, 8, 130, 3, 3, 1, 1), (3, 96, 8, 8, 130, 3, 3, 1, 1), (7, 8, 4, 4, 31, 3, 3, 1, 1), (7, 31, 4, 4, 8, 3, 3, 1, 1), (7, 32, 4, 4, 8, 3, 3, 1, 1),
               (3, 20, 6, 6, 36, 1, 1, 1, 0), (3, 18, 5, 5, 34, 1, 1, 1, 0), (4, 10, 12, 9, 12, 3, 5, 3, 2), (2, 6, 11, 13, 8, 4, 3, 2, 3), (1, 2, 16, 17, 5, 15, 15, 1, 2), (2, 3, 20, 18, 5, 17, 16, 2, 4)]
 
 
