@@ -78,18 +78,31 @@ template <int MODE, int VPT>
 __device__ __forceinline__ float softmax_row(const float* p, float* q, int cols, int lane) {
   float mx = -FLT_MAX, s = 0.0f;
   if constexpr (VPT > 0) {
+    constexpr int G = VPT < 4 ? VPT : 4;                      // pieces of 128 columns, those beyond the row left out
     float v[VPT];
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; v[j] = i < cols ? p[i] : -FLT_MAX; }
+    for (int g = 0; g < VPT; g += G) if (g == 0 || 32 * g < cols) {
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) mx = fmaxf(mx, v[j]);
+      for (int j = g; j < g + G; ++j) { const int i = lane + 32 * j; v[j] = i < cols ? p[i] : -FLT_MAX; }
+    }
+#pragma unroll
+    for (int g = 0; g < VPT; g += G) if (g == 0 || 32 * g < cols) {
+#pragma unroll
+      for (int j = g; j < g + G; ++j) mx = fmaxf(mx, v[j]);
+    }
     mx = warp_max(mx);
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) if (lane + 32 * j < cols) s += expf(v[j] - mx);
+    for (int g = 0; g < VPT; g += G) if (g == 0 || 32 * g < cols) {
+#pragma unroll
+      for (int j = g; j < g + G; ++j) if (lane + 32 * j < cols) s += expf(v[j] - mx);
+    }
     s = warp_sum(s);
     const float logsum = mx + logf(s);
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols) q[i] = MODE == 0 ? expf(v[j] - mx) / s : v[j] - logsum; }
+    for (int g = 0; g < VPT; g += G) if (g == 0 || 32 * g < cols) {
+#pragma unroll
+      for (int j = g; j < g + G; ++j) { const int i = lane + 32 * j; if (i < cols) q[i] = MODE == 0 ? expf(v[j] - mx) / s : v[j] - logsum; }
+    }
     return logsum;
   }
   for (int i = lane; i < cols; i += 32) mx = fmaxf(mx, p[i]);
@@ -149,8 +162,13 @@ __global__ void __launch_bounds__(256) softmax_nll_kernel(const float* __restric
   __syncthreads();
   if (w == 0) { const float a = warp_sum(part[lane]); if (lane == 0) sum[0] = a * scale; }
 }
+// The gradient's forms.  VPT 1, 8: a row of at most 32 VPT columns in registers, as above.  Longer rows are read twice, VPT 0 in loops that the compiler unrolls by four,
+// VPT -1 with four pieces of 32 columns at a time, those of the row's end together too, where the loops' last turns would go one by one.
+static int softmax_grad_form(int cols) { return cols <= 32 ? 1 : cols <= 256 ? 8 : cols < 1280 && cols % 128 >= 64 ? -1 : 0; }
 // MODE 0: dx += y*(dy - sum dy*y) (cudnnSoftmaxBackward ACCURATE, TensorDslCudnn.scala:1465-1504);
-// MODE 1: dx += dy - exp(y)*sum dy (TensorDslCPU.scala:837-846).  VPT as above.
+// MODE 1: dx += dy - exp(y)*sum dy (TensorDslCPU.scala:837-846).
+// us, VPT 0 / -1 (MODE 1): 1024 columns, 1 row 3.8 / 4.6, 1000 rows 5.6 / 6.8; 4096 columns, 300 rows 15.3 / 20.2; 1000 columns, 1 row 5.4 / 4.6, 1000 rows 7.4 / 6.8,
+// 9623 rows 31.4 / 28.7; 600 columns 3.6 / 3.4, 5.0 / 4.8, 11.9 / 10.8.  A row of 1000 in 96 registers: 72 us on 8192 of them, 25 in this form.
 template <int MODE, int VPT>
 __global__ void softmax_grad_kernel(float* dx, const float* __restrict__ y, const float* __restrict__ dy, int rows, int cols) {
   pdl_enter();
@@ -167,58 +185,72 @@ __global__ void softmax_grad_kernel(float* dx, const float* __restrict__ y, cons
     s = warp_sum(s);
 #pragma unroll
     for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols) o[i] = old[j] + (MODE == 0 ? w[j] * (v[j] - s) : v[j] - expf(w[j]) * s); }
-    return;
-  }
-#pragma unroll 8
-  for (int i = lane; i < cols; i += 32) s += MODE == 0 ? d[i] * yy[i] : d[i];
-  s = warp_sum(s);
-  // four of the row's 128-byte pieces in flight (a row of 1000 in 96 registers: 72 us on 8192 x 1000, where this takes 24)
-  for (int i0 = lane; i0 < cols; i0 += 128) {
-    float v[4], w[4], old[4];
+  } else if constexpr (VPT == 0) {
+    for (int i = lane; i < cols; i += 32) s += MODE == 0 ? d[i] * yy[i] : d[i];
+    s = warp_sum(s);
+    for (int i = lane; i < cols; i += 32) o[i] += MODE == 0 ? yy[i] * (d[i] - s) : d[i] - expf(yy[i]) * s;
+  } else {
+    for (int i0 = lane; i0 < cols; i0 += 256) {
+      float v[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
+      for (int j = 0; j < 8; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? (MODE == 0 ? d[i] * yy[i] : d[i]) : 0.0f; }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; if (i < cols) o[i] = old[j] + (MODE == 0 ? w[j] * (v[j] - s) : v[j] - expf(w[j]) * s); }
+      for (int j = 0; j < 8; ++j) s += v[j];
+    }
+    s = warp_sum(s);
+    for (int i0 = lane; i0 < cols; i0 += 128) {
+      float v[4], w[4], old[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; if (i < cols) o[i] = old[j] + (MODE == 0 ? w[j] * (v[j] - s) : v[j] - expf(w[j]) * s); }
+    }
   }
 }
 // What leads from the gradient of a loss to that of the logits, a warp per row: dnll += scale dout (dout set to `value` first when it is seeded here),
 // dlogp[target] -= dnll, dx += dlogp - exp(y) sum dlogp; every buffer ends up as the separate launches leave it (four of 2.5 to 4 us each).  Nothing is stored before
-// a row's sum, so that its loads go out together (us, 8192 x 1000 apart 25.9, joined 29.4 with the store first, 22.0 so; 1024 x 4096 24.7, 40.1, 22.7; 8192 x 100 6.9, 4.2).
+// a row's sum, so that its loads go out together (us, 8192 x 1000 apart 25.4, joined 29.4 with the store first, 21.4 so; 8192 x 100 6.8, 4.4).  Rows of 1280 columns and
+// more are not joined: the target in the way, the compiler's loops are slow (8192 x 2000 225), and the other form gains nothing (2048 x 2000 apart 15.0, joined 15.0;
+// 1024 x 4096 19.1, 23.3).
 template <int VPT>
 __global__ void __launch_bounds__(256) nll_softmax_grad_kernel(float* __restrict__ dx, const float* __restrict__ y, float* __restrict__ dlogp, float* dnll, float* dout, bool seeded, float value,
                                                                float scale, const int32_t* __restrict__ t, int rows, int cols) {
   pdl_enter();
   const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; const int lane = threadIdx.x & 31;
   if (r >= rows) return;
-  const int k = t[r];
+  const int target = t[r], k = target < cols ? target : -1;         // (a target may lie beyond the row)
   const float dn = fmaf(seeded ? value : dout[0], scale, dnll[r]);
   if (lane == 0) { dnll[r] = dn; if (seeded && r == 0) dout[0] = value; }
   const float* __restrict__ yy = y + r * cols; float* __restrict__ d = dlogp + r * cols; float* __restrict__ o = dx + r * cols;
+  auto with = [&](int i, float v) { return i == k ? v + -1.0f * dn : v; };
   float s = 0.0f;
   if constexpr (VPT > 0) {
     float v[VPT], w[VPT], old[VPT];
 #pragma unroll
     for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols && i == k) { v[j] += -1.0f * dn; d[i] = v[j]; } if (i < cols) s += v[j]; }
+    for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols) { if (i == k) { v[j] += -1.0f * dn; d[i] = v[j]; } s += v[j]; } }
     s = warp_sum(s);
 #pragma unroll
     for (int j = 0; j < VPT; ++j) { const int i = lane + 32 * j; if (i < cols) o[i] = old[j] + (v[j] - expf(w[j]) * s); }
     return;
   }
-#pragma unroll 8
-  for (int i = lane; i < cols; i += 32) { float v = d[i]; if (i == k) v += -1.0f * dn; s += v; }
+  for (int i0 = lane; i0 < cols; i0 += 256) {                       // VPT 0: as softmax_grad_kernel's -1
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? d[i] : 0.0f; }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += with(i0 + 32 * j, v[j]);
+  }
   s = warp_sum(s);
   for (int i0 = lane; i0 < cols; i0 += 128) {
     float v[4], w[4], old[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; v[j] = i < cols ? d[i] : 0.0f; w[j] = i < cols ? yy[i] : 0.0f; old[j] = i < cols ? o[i] : 0.0f; }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int i = i0 + 32 * j;
-      if (i < cols) { if (i == k) { v[j] += -1.0f * dn; d[i] = v[j]; } o[i] = old[j] + (v[j] - expf(w[j]) * s); }
-    }
+    for (int j = 0; j < 4; ++j) { const int i = i0 + 32 * j; if (i < cols) o[i] = old[j] + (with(i, v[j]) - expf(w[j]) * s); }
   }
+  if (k >= 0 && lane == (k & 31)) d[k] = with(k, d[k]);             // by the lane that read it
 }
 __global__ void nll_kernel(const float* __restrict__ x, const int32_t* __restrict__ t, float* out, int rows, int cols) {
   pdl_enter();
@@ -280,6 +312,7 @@ static int softmax_issue(const float* x, float* y, int rows, int cols) {
   const unsigned grid = (unsigned)ceil_div((int64_t)rows * 32, 256);
   if (cols <= 32) LTB_LAUNCH((softmax_kernel<MODE, 1>), grid, 256, 0, x, y, rows, cols);
   else if (cols <= 256) LTB_LAUNCH((softmax_kernel<MODE, 8>), grid, 256, 0, x, y, rows, cols);
+  else if (cols <= 512) LTB_LAUNCH((softmax_kernel<MODE, 16>), grid, 256, 0, x, y, rows, cols);
   else if (cols <= 1024) LTB_LAUNCH((softmax_kernel<MODE, 32>), grid, 256, 0, x, y, rows, cols);
   else LTB_LAUNCH((softmax_kernel<MODE, 0>), grid, 256, 0, x, y, rows, cols);
   return LTB_OK;
@@ -287,9 +320,11 @@ static int softmax_issue(const float* x, float* y, int rows, int cols) {
 template <int MODE>
 static int softmax_grad_issue(float* dx, const float* y, const float* dy, int rows, int cols) {
   const unsigned grid = (unsigned)ceil_div((int64_t)rows * 32, 256);
-  if (cols <= 32) LTB_LAUNCH((softmax_grad_kernel<MODE, 1>), grid, 256, 0, dx, y, dy, rows, cols);
-  else if (cols <= 256) LTB_LAUNCH((softmax_grad_kernel<MODE, 8>), grid, 256, 0, dx, y, dy, rows, cols);
-  else LTB_LAUNCH((softmax_grad_kernel<MODE, 0>), grid, 256, 0, dx, y, dy, rows, cols);
+  const int form = softmax_grad_form(cols);
+  if (form == 1) LTB_LAUNCH((softmax_grad_kernel<MODE, 1>), grid, 256, 0, dx, y, dy, rows, cols);
+  else if (form == 8) LTB_LAUNCH((softmax_grad_kernel<MODE, 8>), grid, 256, 0, dx, y, dy, rows, cols);
+  else if (form == 0) LTB_LAUNCH((softmax_grad_kernel<MODE, 0>), grid, 256, 0, dx, y, dy, rows, cols);
+  else LTB_LAUNCH((softmax_grad_kernel<MODE, -1>), grid, 256, 0, dx, y, dy, rows, cols);
   return LTB_OK;
 }
 
@@ -302,16 +337,17 @@ static int full_sum(const float* x, float* out, int64_t n, float scale) {
 }
 
 // ---- the calls around a classifier's loss that look-ahead fusion joins
-// The rows up to which the sum joins: as many as the GPU holds at once (the kernel's registers allow eight CTAs of eight rows an SM, three at 257 to 1024
-// columns; at most 32 columns a CTA takes several rows).  A CTA waits for its ticket before it makes room for another, which costs more than the two launches
-// saved: apart / joined, us, 3000 x 1000 8.9 / 7.8, 4096 x 1000 10.9 / 11.7, 8192 x 1000 15.1 / 17.1; 8192 x 100 6.3 / 5.8, 16384 x 100 9.0 / 10.0; 8192 x 10 5.3 / 5.0,
-// 20000 x 10 8.1 / 7.6, 65536 x 10 17.3 / 18.2.  (One CTA adds them up, as in full_sum: 65536 in all.)
+// The rows up to which the sum joins: not many more than the GPU works on at once, eight CTAs of eight rows an SM, three at 257 to 1024 columns (at most 32
+// columns: a CTA takes several rows).  A CTA waits for its ticket before it makes room for another, which costs more than the launch saved: us, the sum apart /
+// joined, 4096 x 300 5.8 / 6.6, 5000 x 300 6.3 / 6.9, 4096 x 1000 8.4 / 8.9, 16384 x 100 8.5 / 10.0; 3000 x 1000 8.9 / 7.8, 8192 x 100 6.3 / 5.8, 20000 x 10 8.1 / 7.6,
+// but 65536 x 10 17.3 / 18.0.  (One CTA adds them up, as in full_sum: 65536 in all.)
 static int head_sum_rows(int cols) { return cols <= 32 ? 1 << 16 : std::min(1 << 16, g.sm_count * 8 * (cols <= 256 || cols > 1024 ? 8 : 3)); }
 static int softmax_nll_issue(const Pending& p, float* sum, float scale) {
   const unsigned grid = (unsigned)ceil_div((int64_t)p.N * 32, 256), most = (unsigned)g.sm_count * 8;      // a warp per row
   unsigned* const ticket = g.tickets + (g.in_branch ? 1 : 0);
   if (p.C <= 32) LTB_LAUNCH((softmax_nll_kernel<1>), std::min(grid, most), 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
   else if (p.C <= 256) LTB_LAUNCH((softmax_nll_kernel<8>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
+  else if (p.C <= 512) LTB_LAUNCH((softmax_nll_kernel<16>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
   else if (p.C <= 1024) LTB_LAUNCH((softmax_nll_kernel<32>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
   else LTB_LAUNCH((softmax_nll_kernel<0>), grid, 256, 0, p.x, p.y, p.target, p.out, sum, scale, p.N, p.C, ticket);
   return LTB_OK;
@@ -457,7 +493,7 @@ int ltb_log_softmax_grad(float* dx, const float* y, const float* dy, int rows, i
   LTB_INITED_NOFLUSH(); LTB_REQUIRE(dx && y && dy && rows > 0 && cols > 0, "ltb_log_softmax_grad: bad argument");
   const Pending p = g.pending;
   const int64_t n = (int64_t)rows * cols;
-  const bool joins = p.kind == PEND_NLL_GRAD && p.db == dy && p.N == rows && p.C == cols && apart(dx, n, dy, n) && apart(dx, n, p.da, rows) && apart(dx, n, p.d, 1) &&
+  const bool joins = p.kind == PEND_NLL_GRAD && p.C < 1280 && p.db == dy && p.N == rows && p.C == cols && apart(dx, n, dy, n) && apart(dx, n, p.da, rows) && apart(dx, n, p.d, 1) &&
                      apart(dx, n, p.target, rows) && apart(y, n, dx, n) && apart(y, n, dy, n) && apart(y, n, p.da, rows) && apart(y, n, p.d, 1);
   if (joins) g.pending.kind = PEND_NONE;
   else if (p.kind) { int rc = flush_pending(); if (rc) return rc; }
