@@ -490,7 +490,9 @@ __global__ void __launch_bounds__(512, 2) bn_bwd_cluster_kernel(const float* __r
 // the rate at which CTAs can be dispatched (measured: 9.5 us at 512 CTAs, 18 us at 2048 CTAs for the same 4 MB).  Here a
 // CTA is G rows of T threads (T a multiple of 32: warps never straddle rows), row g owns channel blockIdx.x * G + g.
 // Threads rather than items per thread while all channels' threads fit the machine once (1024 per SM): one or two items per thread leave room to
-// fetch everything a channel needs before the sums, a single memory latency instead of two.
+// fetch everything a channel needs before the sums, a single memory latency instead of two.  (Back to back on data in the L2 256 channels of 2048 values take
+// 4.8 us backward so and 3.8 with four items in 128 threads; in a training step it is the other way, ResNet-50 at batch 32 1692 us, 1689 with at most 256
+// threads a channel, 1709 with 128; at batch 64 2119, 2132, 2136; at batch 8 1301, 1301, 1319.)
 struct BnPackedPlan { int T, G, vpt; };
 static bool bn_packed_plan(int N, int C, int HW, int vpt, BnPackedPlan& p) {
   const int64_t items = (int64_t)N * (HW >> 2);

@@ -72,7 +72,8 @@ __global__ void sum_dim_grad_kernel(float* dx, const float* __restrict__ dout, i
 }
 
 // One warp per row. MODE 0 softmax, 1 logSoftmax (TensorDslCPU.scala:783-832).  VPT > 0: a row of at most 32 VPT columns stays in registers, all its
-// loads in flight at once (8192 x 1000: 17 us walking the row three times, 15 so); VPT 0: any length.
+// loads in flight at once, and the pieces beyond the row are left out (log-softmax, us, walking the row three times / so: 300 rows of 100 2.8 / 1.6, 9623 of 300 6.2 / 5.0,
+// of 1000 16.5 / 11.2, 3000 of 768 4.7 / 5.4, 20000 of 768 23.9 / 19.8); VPT 0: any length.
 // Returns log sum exp of the row (MODE 1).
 template <int MODE, int VPT>
 __device__ __forceinline__ float softmax_row(const float* p, float* q, int cols, int lane) {

@@ -235,8 +235,9 @@ def test_softmax_family_and_nll(ora, gpu, rows, cols):
     check(f, ora, gpu, rtol=2e-4)
 
 
-# the lengths where a row stops fitting 1, 8 and 32 registers of a lane
-@pytest.mark.parametrize("rows,cols", [(1, 1), (9, 32), (5, 33), (3, 256), (4, 257), (3, 1000), (2, 1024), (7, 1025)])
+# the lengths where a row stops fitting 1, 8, 16 and 32 registers of a lane, where it ends in a group of pieces, and where the gradient's form changes
+@pytest.mark.parametrize("rows,cols", [(1, 1), (9, 32), (5, 33), (3, 256), (4, 257), (3, 1000), (2, 1024), (7, 1025), (3, 319), (4, 320), (3, 384), (2, 511), (3, 512), (5, 513), (3, 640),
+                                       (2, 641), (3, 769), (2, 1215), (3, 1216), (2, 1279), (3, 1280)])
 def test_softmax_rows_of_every_form(ora, gpu, rows, cols):
     v = (R(cols).standard_normal((rows, cols)) * 3).astype(np.float32)
     if cols > 1:
