@@ -967,7 +967,7 @@ __global__ void __launch_bounds__(32 * kTreeUnits / CTAS, 1) tree_chain_fwd_kern
   cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster.block_rank();
   const int Hd = tree.hidden, Hs = (Hd + 31) / 32 * 32, n = T.n, u = rank * kWarps + warp;
-  const int inner = n / 2;                                   // of n nodes, in a tree of which every inner node has two children
+  const int inner = n / 2;                                   // room for: of n nodes no more have two children of their own (a tree has as many, nodes that are no one's children make it fewer)
   const int K = tree.classes;
   float* state = sm; float* kept = state + (size_t)n * 2 * Hs; float* why = kept + (size_t)kWarps * inner * 8; float* loss = why + K * Hd;
   int* left = reinterpret_cast<int*>(loss + n); int* right = left + n; int* first = right + n;
@@ -1044,7 +1044,7 @@ __global__ void __launch_bounds__(32 * kTreeUnits / CTAS, 1) tree_chain_fwd_kern
     tree_spread<CTAS>(cluster, state + (size_t)begin * 2 * Hs, 2 * (end - begin), Hs, rank);
     cluster.sync();                                          // the level's states are in every CTA
   }
-  for (int i = tid; i < inner * 8 * kWarps; i += kThreads) {          // neighbouring threads on neighbouring units
+  for (int i = tid; i < (n - leaves) * 8 * kWarps; i += kThreads) {   // neighbouring threads on neighbouring units
     const int ne = i / kWarps, a = i - ne * kWarps, q = ne >> 3, e = ne & 7, unit = rank * kWarps + a;
     if (unit < Hd) T.V(leaves + q)[(e < 5 ? e * Hd : e * T.p) + unit] = kept[((size_t)a * inner + q) * 8 + e];
   }

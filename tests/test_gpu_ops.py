@@ -1348,18 +1348,34 @@ def _tree_topology(rng, leaves, chain, table_rows, classes):
     return n, levels, np.array(left + right + list(rng.integers(0, classes, n)) + list(rng.integers(0, table_rows, n)) + first, np.int32)
 
 
-# leaves, hidden, embedding, classes, chain: one node, levels of more nodes than are worked on at once, a chain, the limits and odd sizes
+def _forest_topology(rng, trees, table_rows, classes):
+    """Two or three trees of one, two or three leaves side by side, as _tree_topology lays them out; the last node is a root, the others' are no one's children."""
+    levels = max(trees)
+    nodes = [(lv, t) for lv in range(levels) for t, size in enumerate(trees) for _ in range(size if lv == 0 else 1) if lv < size]
+    at = lambda lv, t: [i for i, v in enumerate(nodes) if v == (lv, t)]
+    left, right = [-1] * len(nodes), [-1] * len(nodes)
+    for i, (lv, t) in enumerate(nodes):
+        if lv:
+            left[i], right[i] = (at(0, t)[0] if lv == 1 else at(lv - 1, t)[0]), at(0, t)[lv]
+    first = [sum(v[0] < lv for v in nodes) for lv in range(levels + 1)]
+    n = len(nodes)
+    return n, levels, np.array(left + right + list(rng.integers(0, classes, n)) + list(rng.integers(0, table_rows, n)) + first, np.int32)
+
+
+# leaves (a tuple: of several trees), hidden, embedding, classes, chain: one node, levels of more nodes than are worked on at once, a chain, the limits and odd sizes
 @pytest.mark.parametrize("classify_cell", [0, 1])
 @pytest.mark.parametrize("leaves,Hd,E,K,chain", [(1, 150, 300, 5, 0), (2, 150, 300, 5, 0), (25, 150, 300, 5, 0), (60, 150, 300, 5, 0), (14, 150, 300, 5, 1), (9, 160, 320, 32, 0),
-                                                 (7, 33, 17, 3, 0), (5, 1, 1, 1, 0), (40, 64, 96, 2, 0)])
+                                                 (7, 33, 17, 3, 0), (5, 1, 1, 1, 0), (40, 64, 96, 2, 0),
+                                                 ((1, 1), 150, 300, 5, 0), ((1, 2), 150, 300, 5, 0), ((2, 1, 1, 3), 33, 17, 3, 0), ((2, 2), 64, 96, 2, 0)])
 def test_a_whole_tree_per_call(ora, gpu, leaves, Hd, E, K, chain, classify_cell):
     """ltb_tree_fwd / ltb_tree_bwd against the oracle's node by node, parameter gradients added to what is there, twice (the second tree's calls
-    meet the first one's barrier counters)."""
+    meet what the first one's left in shared memory); with nodes that are no one's children too.  What follows the nodes' values in memory keeps its 7."""
     import ctypes
     from lantern_b200._ffi import parse_struct
     Tree = parse_struct("ltb_tree")
-    rng = R(leaves * 7 + Hd)
-    n, levels, topo0 = _tree_topology(rng, leaves, chain, 11, K)
+    forest = isinstance(leaves, tuple)
+    rng = R((sum(leaves) if forest else leaves) * 7 + Hd)
+    n, levels, topo0 = _forest_topology(rng, leaves, 11, K) if forest else _tree_topology(rng, leaves, chain, 11, K)
     v = lambda *shape, scale=1.0: (rng.standard_normal(shape) * scale).astype(np.float32)
     W = {"leaf%d" % g: v(Hd, E, scale=1 / np.sqrt(E)) for g in (0, 3, 4)}
     W.update({"in%d%d" % (g, k): v(Hd, Hd, scale=1 / np.sqrt(Hd)) for g in range(5) for k in (0, 1)})
@@ -1374,7 +1390,8 @@ def test_a_whole_tree_per_call(ora, gpu, leaves, Hd, E, K, chain, classify_cell)
         table, topo = b.fromNumpy(table0), b.fromNumpy(topo0)
         out = {}
         for turn in range(2):
-            vals, grads = b.fill((n, 8 * pitch + 64), 0.0), b.fill((n, 2 * pitch + 64), 0.0)
+            vals, grads = b.fill((n + 3, 8 * pitch + 64), 0.0), b.fill((n, 2 * pitch + 64), 0.0)
+            lib.fill(vals.ptr + 4 * n * (8 * pitch + 64), 7.0, 3 * (8 * pitch + 64))
             t = Tree(nodes=n, levels=levels, hidden=Hd, in_len=E, classes=K, classify_cell=classify_cell)
             for g in (0, 3, 4):
                 t.leaf_W[g], t.leaf_dW[g], t.leaf_bias[g], t.leaf_dbias[g] = w["leaf%d" % g].x.ptr, w["leaf%d" % g].d.ptr, w["bl%d" % g].x.ptr, w["bl%d" % g].d.ptr
@@ -1389,7 +1406,9 @@ def test_a_whole_tree_per_call(ora, gpu, leaves, Hd, E, K, chain, classify_cell)
             one = np.array([1.0], np.float32)
             lib.h2d(grads.ptr + 4 * ((n - 1) * (2 * pitch + 64) + 2 * pitch), one.ctypes.data, 4)
             lib.tree_bwd(ctypes.addressof(t))
-            out["vals%d" % turn] = vals.toCPU()[:, 5 * pitch:]
+            got = vals.toCPU()
+            assert np.all(got[n:] == 7.0)
+            out["vals%d" % turn] = got[:n, 5 * pitch:]
             out["grads%d" % turn] = grads.toCPU()
         out.update({"d" + k: x.d.toCPU() for k, x in w.items()})
         return out
