@@ -438,14 +438,14 @@ static Tiling choose_tiling(int M, int N, int K, bool may_add_atomically) {
 template <int AF, int BF, class OA, class OB, class ST>
 static int launch_igemm(const char* label, const Tiling& t, int M, int N, int K, const OA& oa, const OB& ob, const ST& st) {
   const dim3 grid((unsigned)ceil_div(M, t.bm), (unsigned)ceil_div(N, t.bn), (unsigned)(t.cz * t.groups));
-  auto go = [&](auto igemm, int smem, bool& ready) -> int {
-    if (!ready) { LTB_CUDA(cudaFuncSetAttribute(igemm, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); ready = true; }
+  auto go = [&](auto igemm, int smem, int& ready) -> int {
+    if (ready != g.device) { LTB_CUDA(cudaFuncSetAttribute(igemm, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); ready = g.device; }
     g.label = label;
     LTB_LAUNCH_CLUSTER_Z(igemm, grid, 256, t.cz, smem, M, N, K, t.kps, oa, ob, st);
     g.label = nullptr;
     return LTB_OK;
   };
-  static bool ready[5];
+  static int ready[5] = {-1, -1, -1, -1, -1};              // the device whose kernels have been given the larger shared memory
 #define LTB_TILE(BM, BN, I) go(igemm_kernel<BM, BN, AF, BF, OA, OB, ST>, igemm_smem<BM, BN>(), ready[I])
   if (t.bm == 128) return t.bn == 128 ? LTB_TILE(128, 128, 0) : t.bn == 64 ? LTB_TILE(128, 64, 1) : LTB_TILE(128, 32, 2);
   return t.bn == 64 ? LTB_TILE(64, 64, 3) : LTB_TILE(64, 32, 4);
@@ -698,11 +698,11 @@ template <int T>
 static int small_gemm(const float* a, int64_t sam, int64_t sak, const float* b, int64_t sbk, int64_t sbn, float* c, int64_t scm, int64_t scn,
                       int M, int N, int K, float alpha, bool accumulate) {
   constexpr int kMost = 2 * kSmallK<T> * (T + 4) * 4, kSums = kSmallWarps * T * T / 32 * kSmallPart * 4;
-  static bool ready = false;
-  if (!ready) {
+  static int ready = -1;
+  if (ready != g.device) {
     LTB_CUDA(cudaFuncSetAttribute((small_gemm_kernel<false, T>), cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
     LTB_CUDA(cudaFuncSetAttribute((small_gemm_kernel<true, T>), cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
-    ready = true;
+    ready = g.device;
   }
   const int panels = 2 * ((K + 15) / 16 * 16) * (T + 4) * 4, smem = panels > kSums ? panels : kSums;
   const dim3 grid((unsigned)ceil_div(M, T), (unsigned)ceil_div(N, T));
@@ -980,8 +980,8 @@ static int launch_direct(const float* in, const float* w, float* out, DirectGeo&
   G.ci_per = (int)ceil_div(ceil_div(G.Ci, cz), kDirectCh) * kDirectCh;
   cz = (int)ceil_div(G.Ci, G.ci_per);
   const int smem = direct_smem<PX, NW>(G.imgs * (G.rows + 2) * G.rs + 4);
-  static int most = 0;
-  if (smem > most) { LTB_CUDA(cudaFuncSetAttribute((conv3x3_direct_kernel<PX, NW, FLIP>), cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); most = smem; }
+  static int most = 0, device = -1;
+  if (device != g.device || smem > most) { LTB_CUDA(cudaFuncSetAttribute((conv3x3_direct_kernel<PX, NW, FLIP>), cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); most = smem; device = g.device; }
   g.label = label;
   LTB_LAUNCH_CLUSTER_Z((conv3x3_direct_kernel<PX, NW, FLIP>), dim3((unsigned)groups, (unsigned)ceil_div(G.Co, NW * 8), (unsigned)cz), NW * 32, cz, smem, in, w, out, G);
   g.label = nullptr;

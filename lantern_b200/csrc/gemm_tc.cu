@@ -974,7 +974,7 @@ static EncodeTiledFn encode_tiled = nullptr;
 typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const int*, const int*,
                                    cuuint32_t, cuuint32_t, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeIm2colFn encode_im2col = nullptr;
-static bool smem_opted_in = false;
+static int smem_opted_device = -1;                 // the device whose kernels have been given the larger shared memory
 
 static void* driver_entry(const char* name) {
   void* fn = nullptr; cudaDriverEntryPointQueryResult qres;
@@ -1122,11 +1122,11 @@ static int launch_plan(const TcPlan& p, const char* label, bool* relu = nullptr,
   P.stages = p.pair ? kMaxStages : p.bn == 128 ? 3 : 4;
   const size_t smem = (size_t)P.stages * (p.a.stage_bytes + p.b.stage_bytes) + 1024;
   if (cz > 1 && (size_t)128 * (p.bn + 1) * 4 > smem - 1024) return fail(LTB_E_STATE, "tensor-core plan whose partial tile does not fit the pipeline stages");
-  if (!smem_opted_in) {
+  if (smem_opted_device != g.device) {
     const int max_smem = 4 * (16384 + 32768) + 1024;                              // as much as six of 32 KB
     for (auto& set : kEngine) for (auto k : set) LTB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     for (auto& set : kEnginePair) for (auto k : set) LTB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    smem_opted_in = true;
+    smem_opted_device = g.device;
   }
   const int mode = atomic ? 2 : (P.accumulate ? 1 : 0);
   const bool gen = p.a.load != TC_LOAD_BOX || p.b.load != TC_LOAD_BOX;

@@ -71,3 +71,23 @@ def test_ctypes_mirror_of_the_tree_node_struct_has_the_c_layout(tmp_path):
     got = [int(v) for v in subprocess.check_output([str(exe)]).split()]
     assert got[0] == ctypes.sizeof(node)
     assert got[1:] == [getattr(node, n).offset for n in names]
+
+
+def test_kernel_attributes_are_set_for_each_device():
+    """An attribute of a kernel holds for one device: after ltb_shutdown and ltb_init on another every opt-in to more shared memory has to come again, so what says that
+    it has been done is the device and not a flag."""
+    csrc = os.path.join(ROOT, "lantern_b200", "csrc")
+    seen = 0
+    for name in sorted(f for f in os.listdir(csrc) if f.endswith((".cu", ".cuh"))):
+        lines = open(os.path.join(csrc, name)).read().split("\n")
+        for i, line in enumerate(lines):
+            if "cudaFuncSetAttribute(" not in line:
+                continue
+            seen += 1
+            start = next(j for j in range(i, -1, -1) if lines[j] == "}")               # the end of the definition before
+            within = "\n".join(lines[start:i + 1])
+            if "static bool tree_set_up()" in within:                                   # called where the device changes
+                caller = "\n".join(lines).split("static int tree_ctas()")[1]
+                within = caller[:caller.index("tree_set_up<16>()")]
+            assert "!= g.device" in within, "%s:%d: %s" % (name, i + 1, line.strip())
+    assert seen
