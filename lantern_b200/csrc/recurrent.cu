@@ -775,6 +775,12 @@ __global__ void __launch_bounds__(kNodeThreads) tree_nodes_bwd_kernel(const ltb_
 
 extern "C" {
 
+// Gradients that were declared unset get their zeros: every one of these is added to.
+static int tree_node_settle(const ltb_tree_node& q) {
+  for (const float* d : std::initializer_list<const float*>{q.dc, q.dh, q.dloss, q.din[0], q.din[1], q.dcl, q.dcr, q.dloss_l, q.dloss_r, q.dWhy, q.dby}) LTB_SETTLE(d);
+  for (int s = 0; s < 5; ++s) for (float* d : {q.dW[s][0], q.dW[s][1], q.dbias[s]}) LTB_SETTLE(d);
+  return LTB_OK;
+}
 static int tree_node_check(const ltb_tree_node* n, const char* who) {
   LTB_REQUIRE(n, "tree_node: null node");
   const int G = n->inner ? 5 : 3;
@@ -801,6 +807,7 @@ int ltb_tree_node_fwd(const ltb_tree_node* n) {
 int ltb_tree_node_bwd(const ltb_tree_node* n) {
   LTB_INITED();
   if (int rc = tree_node_check(n, "ltb_tree_node_bwd")) return rc;
+  if (int rc = tree_node_settle(*n)) return rc;
   filter_cache_note_write(nullptr, 0);
   const int G = n->inner ? 5 : 3;
   LTB_REQUIRE(n->dc && n->dh && n->dloss && n->dWhy && n->dby, "ltb_tree_node_bwd: missing gradient operand");
@@ -842,6 +849,7 @@ int ltb_tree_nodes_bwd(const ltb_tree_node* nodes_host, const ltb_tree_node* nod
     for (int i = at; i < at + n; ++i) {
       const ltb_tree_node* q = nodes_host + i;
       if (int rc = tree_node_check(q, "ltb_tree_nodes_bwd")) return rc;
+      if (int rc = tree_node_settle(*q)) return rc;
       const int G = q->inner ? 5 : 3;
       LTB_REQUIRE(q->dc && q->dh && q->dloss && q->dWhy && q->dby, "ltb_tree_nodes_bwd: missing gradient operand");
       for (int g = 0; g < G; ++g) {
@@ -1357,6 +1365,8 @@ int ltb_tree_fwd(const ltb_tree* t) {
 int ltb_tree_bwd(const ltb_tree* t) {
   LTB_INITED();
   if (int rc = tree_check(t, true, "ltb_tree_bwd")) return rc;
+  for (float* d : {t->grads, t->dWhy, t->dby}) LTB_SETTLE(d);
+  for (int s = 0; s < 5; ++s) for (float* d : {t->leaf_dW[s], t->leaf_dbias[s], t->dW[s][0], t->dW[s][1], t->dbias[s]}) LTB_SETTLE(d);
   const int ctas = tree_ctas();
   if (!ctas) return fail(LTB_E_CUDA, "the tree kernels could not be set up");
   filter_cache_note_write(nullptr, 0);                  // what it writes is a score of vectors: everything is taken as stale

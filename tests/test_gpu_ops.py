@@ -1193,8 +1193,10 @@ def test_rnn_whole_sequence_kernels_at_their_edges(ora, gpu, T, B, V, H):
     test_rnn_whole_sequence_kernels(ora, gpu, T, B, V, H)
 
 
+# unset: the gradients added to are declared unset (ltb_grad_unset) and full of NaN
+@pytest.mark.parametrize("unset", [0, 1])
 @pytest.mark.parametrize("inner,classify_cell,Hd,L", [(1, 1, 150, 150), (1, 0, 150, 150), (0, 1, 150, 300), (0, 0, 150, 300), (1, 0, 40, 40)])
-def test_tree_node_and_gradient(ora, gpu, inner, classify_cell, Hd, L):
+def test_tree_node_and_gradient(ora, gpu, inner, classify_cell, Hd, L, unset):
     """ltb_tree_node_fwd / ltb_tree_node_bwd (a whole tree-LSTM node per launch) against the oracle issuing the gate-by-gate
     operator sequence: gates, cell, hidden, log-probabilities and loss; then every gradient accumulated onto non-zero
     destinations -- an inner node (five gates over two inputs, the two forget gates sharing one bias) and a leaf (three
@@ -1217,7 +1219,7 @@ def test_tree_node_and_gradient(ora, gpu, inner, classify_cell, Hd, L):
 
     def f(b):
         t = {k: b.fromNumpy(a) for k, a in data.items()}
-        d = {k: b.fromNumpy(data[k] * 0.25) for k in grads}                           # accumulate onto non-zero values
+        d = {k: _poisoned(b, data[k].shape) if unset else b.fromNumpy(data[k] * 0.25) for k in grads}                           # accumulate onto non-zero values
         score = b.fromNumpy(np.array([3], np.int32))
         out = {}
         for rep in range(2):
@@ -1249,8 +1251,9 @@ def test_tree_node_and_gradient(ora, gpu, inner, classify_cell, Hd, L):
     check(f, ora, gpu)
 
 
+@pytest.mark.parametrize("unset", [0, 1])
 @pytest.mark.parametrize("classify_cell", [0, 1])
-def test_tree_levels_and_gradient(ora, gpu, classify_cell):
+def test_tree_levels_and_gradient(ora, gpu, classify_cell, unset):
     """ltb_tree_nodes_fwd / ltb_tree_nodes_bwd: a small tree (four leaves, two inner nodes over them, the root) level by level --
     three calls forward, three backward, node descriptions read from an array in device memory -- against the oracle running
     the nodes one after the other: every node's cell, hidden vector and loss, the root's accumulated loss, and every weight
@@ -1271,7 +1274,7 @@ def test_tree_levels_and_gradient(ora, gpu, classify_cell):
 
     def f(b):
         lib = b.lib
-        w = {k: TensorR(b.fromNumpy(a), b.fromNumpy(a * 0.25)) for k, a in W.items()}
+        w = {k: TensorR(b.fromNumpy(a), _poisoned(b, a.shape) if unset else b.fromNumpy(a * 0.25)) for k, a in W.items()}
         e, scores = b.fromNumpy(emb), b.fromNumpy(scores0)
         pitch = 192
         vals, grads = b.fill((n, 8 * pitch + 64), 0.0), b.fill((n, 2 * pitch + 64), 0.0)
@@ -1363,11 +1366,12 @@ def _forest_topology(rng, trees, table_rows, classes):
 
 
 # leaves (a tuple: of several trees), hidden, embedding, classes, chain: one node, levels of more nodes than are worked on at once, a chain, the limits and odd sizes
+@pytest.mark.parametrize("unset", [0, 1])
 @pytest.mark.parametrize("classify_cell", [0, 1])
 @pytest.mark.parametrize("leaves,Hd,E,K,chain", [(1, 150, 300, 5, 0), (2, 150, 300, 5, 0), (25, 150, 300, 5, 0), (60, 150, 300, 5, 0), (14, 150, 300, 5, 1), (9, 160, 320, 32, 0),
                                                  (7, 33, 17, 3, 0), (5, 1, 1, 1, 0), (40, 64, 96, 2, 0),
                                                  ((1, 1), 150, 300, 5, 0), ((1, 2), 150, 300, 5, 0), ((2, 1, 1, 3), 33, 17, 3, 0), ((2, 2), 64, 96, 2, 0)])
-def test_a_whole_tree_per_call(ora, gpu, leaves, Hd, E, K, chain, classify_cell):
+def test_a_whole_tree_per_call(ora, gpu, leaves, Hd, E, K, chain, classify_cell, unset):
     """ltb_tree_fwd / ltb_tree_bwd against the oracle's node by node, parameter gradients added to what is there, twice (the second tree's calls
     meet what the first one's left in shared memory); with nodes that are no one's children too.  What follows the nodes' values in memory keeps its 7."""
     import ctypes
@@ -1386,7 +1390,7 @@ def test_a_whole_tree_per_call(ora, gpu, leaves, Hd, E, K, chain, classify_cell)
 
     def f(b):
         lib = b.lib
-        w = {k: TensorR(b.fromNumpy(a), b.fromNumpy(a * 0.25)) for k, a in W.items()}
+        w = {k: TensorR(b.fromNumpy(a), _poisoned(b, a.shape) if unset else b.fromNumpy(a * 0.25)) for k, a in W.items()}
         table, topo = b.fromNumpy(table0), b.fromNumpy(topo0)
         out = {}
         for turn in range(2):
