@@ -119,7 +119,7 @@ int    LTB_FN(params_changed)(void);
  * first -- usually the only -- operator that adds into it.  grad_unset(d, n) declares the n floats at d, a fresh block that
  * nothing has written, to be a gradient buffer whose zero fill is deferred: it COUNTS as zero.  The first entry point that
  * meets exactly that block as an accumulation destination and is able to -- conv2d_bwd (dx, tensor-core path), bn_bwd (dx),
- * the gradient of a same-shape add (da, db) -- writes its result instead of adding; every other entry point that is handed
+ * the gradient of a same-shape add (da, db), gemm_grad (da, db) -- writes its result instead of adding; every other entry point that is handed
  * the block (any gradient operator, the transfers) fills it with zeros first, so results never depend on the declaration.
  * grad_materialize(d, n) does that filling on request (before the caller reads the block by other means).  Declarations
  * end with the arena span that holds the block (ltb_reset, ltb_free). */

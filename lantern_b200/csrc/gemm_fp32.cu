@@ -18,8 +18,9 @@
 //   output     : m is the index that is contiguous in memory (the caller swaps the operands for row-major results), so a thread's
 //                four consecutive m leave as one 16-byte store or vector reduction.
 // Bound: the FP32 pipes (128 FMA per SM and cycle, 74 TFLOP/s at 1.97 GHz) and, for an 8 x 8 tile of a thread as much, the 32 floats per cycle that
-// shared memory delivers (four FMAs per float loaded); 55 TFLOP/s on 4096 x 4096 x 2048 with k contiguous, 51 without.  The 3x3 layers
-// that conv3x3_direct_kernel below takes make six FMAs per float.
+// shared memory delivers (four FMAs per float loaded); 55 TFLOP/s on 4096 x 4096 x 2048 with k contiguous, 51 without.  In the 3x3 layers
+// that conv3x3_direct_kernel below takes a lane makes 24 PX FMAs of the PX + 2 pixels and 24 weights it loads, 5.6 per float in runs of eight pixels and 3.2 in runs
+// of four; but a weight is one for the whole warp, so that six deliveries of 128 bytes hold them all and a warp makes 12 or 8 FMAs per delivery, where the tiles make four.
 #include <cooperative_groups.h>
 
 #include <type_traits>

@@ -84,8 +84,9 @@ def test_step_loss_and_every_gradient(oracle_lib, cuda_lib, name, batch, kind, m
 
 @pytest.mark.parametrize("name,batch,kind", [("mnist", 20, "uniform"), ("rnn_26_50", 3, "normal")])
 def test_two_steps_in_flight_give_the_losses_of_blocking_steps(cuda_lib, name, batch, kind):
-    """Seven submitted steps, each with a batch of its own (and, for MNIST, its own dropout mask), the step recorded once per staging pair:
-    losses and parameters are those of blocking steps, bit for bit in deterministic FP32; so is the loss read after leaving the mode."""
+    """Seven submitted steps, each with a batch of its own (and, for MNIST, its own dropout mask), the step recorded once per staging pair; then the mode
+    is left (its last loss can still be read), a blocking step, recorded anew, and two more submitted: losses and parameters are those of ten
+    blocking steps, bit for bit in deterministic FP32."""
     import ctypes
     from lantern_b200.hosts import HostPrograms
     libc, mark, res = ctypes.CDLL(None), cuda_lib.mark(), []
@@ -95,15 +96,20 @@ def test_two_steps_in_flight_give_the_losses_of_blocking_steps(cuda_lib, name, b
             m = HostPrograms(cuda_lib).model(name, batch, seed=5)
             libc.srand(3)
             rng = np.random.default_rng(11)
-            batches = [(rng.standard_normal(m.input_count).astype(np.float32), rng.integers(0, 10, m.label_count).astype(np.int32)) for _ in range(7)]
+            batches = [(rng.standard_normal(m.input_count).astype(np.float32), rng.integers(0, 10, m.label_count).astype(np.int32)) for _ in range(10)]
             losses = []
             if feed:
                 m.use_graph(True)
-                for k, (x, y) in enumerate(batches):
+                for k, (x, y) in enumerate(batches[:7]):
                     m.submit(x, y, 0.01)
                     if k:
                         losses.append(m.collect(k - 1))
                 losses.append(m.collect(6))
+                m.set_resident(None)
+                assert m.last_loss() == losses[-1]
+                losses.append(m.step(*batches[7], 0.01))
+                steps = [m.submit(x, y, 0.01) for x, y in batches[8:]]
+                losses += [m.collect(k) for k in steps]
                 assert m.last_loss() == losses[-1]
             else:
                 losses = [m.step(x, y, 0.01) for x, y in batches]

@@ -984,16 +984,17 @@ def test_lookahead_fusion_flushes_on_any_other_call(ora, gpu):
         assert_close(ref[k], got[k], 2e-4, k)
 
 
-# N, C, H, K, R, stride, pad: convolutions whose results are cleared by a kernel before them, each kind of batch-norm kernel and of staging
+# N, C, H, K, R, stride, pad, launches fewer than one by one (1: batch norm with the ReLU; 2: and the convolution's channels-last copy; 0: nine pixels, another batch
+# norm that is not held): convolutions whose results are cleared by a kernel before them, each kind of batch-norm kernel and of staging
 @pytest.mark.parametrize("reuse", [False, True])
-@pytest.mark.parametrize("cfg", [(8, 256, 4, 1024, 1, 1, 0), (8, 256, 4, 256, 3, 1, 1), (8, 64, 16, 64, 3, 1, 1), (128, 64, 16, 64, 1, 1, 0), (8, 128, 8, 256, 3, 2, 1),
-                                 (8, 256, 8, 512, 1, 2, 0), (3, 36, 6, 40, 3, 1, 1), (16, 512, 2, 512, 3, 1, 1), (2, 64, 32, 24, 5, 1, 2), (5, 10, 3, 12, 3, 1, 1),
+@pytest.mark.parametrize("cfg", [(8, 256, 4, 1024, 1, 1, 0, 1), (8, 256, 4, 256, 3, 1, 1, 2), (8, 64, 16, 64, 3, 1, 1, 2), (128, 64, 16, 64, 1, 1, 0, 1), (8, 128, 8, 256, 3, 2, 1, 1),
+                                 (8, 256, 8, 512, 1, 2, 0, 1), (3, 36, 6, 40, 3, 1, 1, 2), (16, 512, 2, 512, 3, 1, 1, 2), (2, 64, 32, 24, 5, 1, 2, 2), (5, 10, 3, 12, 3, 1, 1, 0),
                                  # the copy for the convolution in the batch norm's kernel up to 2^17 elements, and beyond
-                                 (8, 256, 8, 64, 3, 1, 1), (9, 256, 8, 64, 3, 1, 1), (6, 96, 14, 40, 3, 1, 1), (64, 512, 2, 64, 3, 1, 1)])
+                                 (8, 256, 8, 64, 3, 1, 1, 2), (9, 256, 8, 64, 3, 1, 1, 1), (6, 96, 14, 40, 3, 1, 1, 2), (64, 512, 2, 64, 3, 1, 1, 2)])
 def test_a_convolution_takes_over_the_batch_norm_before_it(gpu, cfg, reuse):
     """Batch norm, in-place ReLU, convolution and its backward call: as three kernels that prepare for one another and one by one.  The convolution writes
-    into a buffer full of NaN, or (reuse) into the batch norm's own input."""
-    N, C, H, K, Rk, s, p = cfg
+    into a buffer full of NaN, or (reuse) into the batch norm's own input (which then only the clearing is refused for)."""
+    N, C, H, K, Rk, s, p, saved = cfg
     oh = (H + 2 * p - Rk) // s + 1
     v, w0 = R(1).standard_normal((N, C, H, H)).astype(np.float32), (R(2).standard_normal((K, C, Rk, Rk)) / np.sqrt(C * Rk * Rk)).astype(np.float32)
     dy0 = R(4).standard_normal((N, K, oh, oh)).astype(np.float32)
@@ -1006,9 +1007,12 @@ def test_a_convolution_takes_over_the_batch_norm_before_it(gpu, cfg, reuse):
             x, w = b.fromNumpy(v), TensorR(b.fromNumpy(w0))
             y = x if reuse else b.fromNumpy(np.full((N, K, oh, oh), np.nan, np.float32))
             rm, rv = b.fill((C,), 0.0), b.fill((C,), 1.0)
-            z, sm, si, _ = b.batchNormTraining(x, b.fromNumpy(np.ones(C, np.float32)), b.fromNumpy(np.zeros(C, np.float32)), rm, rv)
+            ones, zeros = b.fromNumpy(np.ones(C, np.float32)), b.fromNumpy(np.zeros(C, np.float32))
+            b.lib.sync(); before = b.lib.kernel_launches()
+            z, sm, si, _ = b.batchNormTraining(x, ones, zeros, rm, rv)
             b.relu(z, True)
             b.lib.conv2d_fwd(z.ptr, w.x.ptr, 0, y.ptr, N, C, H, H, K, Rk, Rk, s, s, p, p)
+            b.lib.sync(); launches.append(b.lib.kernel_launches() - before)
             out = {"y": y.toCPU().reshape(-1)[:N * K * oh * oh].copy(), "z": z.toCPU(), "rm": rm.toCPU(), "rv": rv.toCPU()}
             zr = TensorR(z)
             b.conv2D_batch_grad(zr, None, w, TensorR(y, b.fromNumpy(dy0)), None, (p, p), (s, s))
@@ -1016,7 +1020,9 @@ def test_a_convolution_takes_over_the_batch_norm_before_it(gpu, cfg, reuse):
         finally:
             b.lib.set_fusion(0); b.lib.set_filter_cache(0)
         return out
+    launches = []
     plain, joined = f(gpu, 0), f(gpu, 2)
+    assert launches[0] - launches[1] == saved
     for k in plain:
         if k in ("z", "rm", "rv"):
             assert np.array_equal(plain[k], joined[k]), k
