@@ -567,6 +567,7 @@ static size_t shape_count(const int* shape, int rank) {
 // fill / fillInPlace: TensorDslCPU.scala:30-35, 65-67.
 int ltb_fill(float* x, float v, int64_t n) {
   LTB_INITED(); filter_cache_note_write(x, (size_t)(n > 0 ? n : 0) * 4); LTB_REQUIRE(x && n >= 0, "ltb_fill: bad argument");
+  LTB_SETTLE(x);                                            // no longer unset: a later call must not put zeros over the value
   if (n == 1 && g.fusion) { Pending h; h.kind = PEND_SEED; h.n = 1; h.d = x; h.value = v; g.pending = h; return LTB_OK; }   // the gradient of a sum that reads it may join it
   return fill_issue(x, v, n);
 }

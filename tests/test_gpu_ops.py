@@ -1629,6 +1629,21 @@ def test_conv_backward_into_an_unset_gradient_buffer(gpu, cfg, math):
         lib.set_deterministic(0); lib.set_math(1)
 
 
+@pytest.mark.parametrize("fusion", [0, 1])
+@pytest.mark.parametrize("n", [1, 5])
+def test_a_filled_buffer_is_no_longer_unset(gpu, n, fusion):
+    """The gradient of a loss in a buffer declared unset, then filled: the calls that read it see the value and not the zeros they would have put there."""
+    b, lib = gpu, gpu.lib
+    lib.set_fusion(fusion)
+    try:
+        d, dx = _poisoned(b, (n,)), b.fill((7,), 0.5)
+        lib.fill(d.ptr, 2.0, n)
+        lib.sum_grad(dx.ptr, d.ptr, 7)
+        assert np.array_equal(dx.toCPU(), np.full(7, 2.5, np.float32)) and np.array_equal(d.toCPU(), np.full(n, 2.0, np.float32))
+    finally:
+        lib.set_fusion(0)
+
+
 @pytest.mark.parametrize("shape", [(128, 64, 16, 16), (128, 256, 8, 8), (128, 1024, 4, 4), (32, 2048, 2, 2), (8, 5, 3, 3)])
 @pytest.mark.parametrize("with_relu", [False, True])
 def test_batch_norm_backward_into_an_unset_gradient_buffer(gpu, shape, with_relu):
